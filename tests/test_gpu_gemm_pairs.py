@@ -1,0 +1,86 @@
+"""The tensor-core GEMM at the sizes where its tiling can go wrong: weight rows around the 256-row
+pair tile, activation rows around the 16-row granularity and the 64 / 256-row tile limits, K loops of
+one to a few 256-wide units with a short last one, and decode batches whose K loops are cut evenly
+over all pairs (more than half as many row tiles as pairs) or uniformly."""
+import numpy as np
+import pytest
+
+import oracle
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+SEED = 299792458
+# Both operands are rounded to f16 (relative error <= 2^-11 per element, about 2^-11 / sqrt(3) rms each),
+# the sub-block scale and min of the weight once more: about 2^-11 in the result, 4 x that allowed.
+TOL = 4 * 2.0 ** -11
+
+
+@pytest.fixture(scope="module")
+def tq():
+    import tur_b200
+    return tur_b200
+
+
+def make_weight(dt, n, k, seed):
+    rng = np.random.default_rng(seed)
+    w = (rng.standard_normal((n, k)) * 0.02).astype(np.float32)
+    return oracle.quantize(dt, w)
+
+
+K_QUANT = [(oracle.Q4_K, 256), (oracle.Q5_K, 512), (oracle.Q6_K, 768)]
+
+
+@pytest.mark.parametrize("n", [1, 16, 255, 257, 400])
+@pytest.mark.parametrize("m", [17, 48, 64, 65, 129, 257])
+@pytest.mark.parametrize("dt,k", K_QUANT + [(oracle.Q8_0, 64), (oracle.Q8_0, 320), (oracle.Q8_0, 704)])
+def test_edges_of_the_pair_tile(tq, dt, k, n, m):
+    w = make_weight(dt, n, k, SEED + 7000 + n + k)
+    rng = np.random.default_rng(SEED + 7001 + m)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    bias = rng.standard_normal(n).astype(np.float32)
+    mm = tq.QMatMul.from_arc(tq.QTensor.new(w, tq.GgmlDType(dt), (n, k)))
+    y = mm.forward(torch.from_numpy(x).cuda(), bias=torch.from_numpy(bias).cuda(), mode=tq.Mode.TENSOR_CORE)
+    assert oracle.rel_fro(y.cpu().numpy(), oracle.matmul_f64(dt, w, n, k, x) + bias) < TOL
+    tq.context().poll_status()
+
+
+@pytest.mark.parametrize("dt,n,k", [(oracle.Q4_K, 10000, 768), (oracle.Q6_K, 19000, 256), (oracle.Q8_0, 9700, 320),
+                                    (oracle.Q8_0, 40000, 64), (oracle.Q5_K, 300, 8192), (oracle.Q8_0, 512, 4160)])
+def test_decode_batches_share_the_k_loop(tq, dt, n, k):
+    """Cuts inside a tile, pairs that hold several tiles and pairs that hold a part of one; the flags
+    between the pairs are left as they were found (the second call), and a row's bits do not depend
+    on the batch."""
+    w = make_weight(dt, n, k, SEED + 7100 + n + k)
+    x = np.random.default_rng(SEED + 7101).standard_normal((64, k)).astype(np.float32)
+    mm = tq.QMatMul.from_arc(tq.QTensor.new(w, tq.GgmlDType(dt), (n, k)))
+    xd = torch.from_numpy(x).cuda()
+    y = mm.forward(xd, mode=tq.Mode.TENSOR_CORE)
+    assert oracle.rel_fro(y.cpu().numpy(), oracle.matmul_f64(dt, w, n, k, x)) < TOL
+    assert torch.equal(mm.forward(xd, mode=tq.Mode.TENSOR_CORE), y)
+    assert torch.equal(mm.forward(xd[:21], mode=tq.Mode.TENSOR_CORE), y[:21])
+    tq.context().poll_status()
+
+
+@pytest.mark.parametrize("m", [33, 300])
+def test_weights_of_one_call_run_side_by_side(tq, m):
+    """Four weights of different types and sizes that share x: the later ones start beside the first
+    one and whatever follows the call has to wait for all of them."""
+    k = 1024
+    shapes = [(oracle.Q4_K, 4096), (oracle.Q6_K, 272), (oracle.Q5_K, 16), (oracle.Q4_K, 1000)]
+    ws = [make_weight(t, n, k, SEED + 7200 + n) for t, n in shapes]
+    mms = [tq.QMatMul.from_arc(tq.QTensor.new(w, tq.GgmlDType(t), (n, k))) for w, (t, n) in zip(ws, shapes)]
+    x = np.random.default_rng(SEED + 7201).standard_normal((m, k)).astype(np.float32)
+    xd = torch.from_numpy(x).cuda()
+    want = [mm.forward(xd, mode=tq.Mode.TENSOR_CORE) for mm in mms]
+    outs = [torch.empty(m, n, device="cuda") for _, n in shapes]
+    for _ in range(20):
+        for o in outs:
+            o.fill_(float("nan"))
+        tq.QMatMul.forward_multi(mms, xd, outs=outs, mode=tq.Mode.TENSOR_CORE)
+        got = torch.cat([o.flatten() for o in outs])       # a launch of another kind right behind the call
+        xd.mul_(1.0)
+        assert torch.equal(got, torch.cat([w_.flatten() for w_ in want]))
+    for o, w, (t, n) in zip(want, ws, shapes):
+        assert oracle.rel_fro(o.cpu().numpy(), oracle.matmul_f64(t, w, n, k, x)) < TOL
+    tq.context().poll_status()

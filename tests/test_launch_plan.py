@@ -22,6 +22,10 @@ long long split_start(int grid, int q, int r, long long total, int b) {
   return turq::gemv_split_start(p, total, b);
 }
 int gemm_bn(long long n, long long m, int sms, int force) { return turq::plan_gemm_bn(n, m, sms, force); }
+void gemm_work(long long n, long long m, long long k, int mt, int sms, int* out) {
+  turq::GemmWork w = turq::plan_gemm_work(n, m, k, mt, sms);
+  out[0] = w.pairs; out[1] = w.split_k;
+}
 int gemm_splits(long long n, long long m, long long k, int sms, int force) { return turq::plan_gemm_splits(n, m, k, sms, force); }
 }
 """
@@ -39,6 +43,7 @@ def plan():
         lib.split_start.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_int]
         lib.gemm_bn.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int, ctypes.c_int]
         lib.gemm_splits.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int, ctypes.c_int]
+        lib.gemm_work.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
         yield lib
 
 
@@ -107,3 +112,28 @@ def test_gemm_activation_tile_choice(plan):
     assert plan.gemm_bn(2560, 1024, sms, 0) == 256     # 20 x 4 tiles: doubling would spill into a second wave
     assert plan.gemm_bn(1024, 2048, sms, 0) == 128
     assert plan.gemm_bn(12288, 2048, sms, 128) == 128
+
+
+@pytest.mark.parametrize("n,k", [(8192, 5120), (1024, 5120), (5120, 25600), (2560, 2560), (640, 2560), (12288, 4096), (4096, 12288),
+                                 (151936, 4096), (272, 256), (1, 64), (9700, 320), (40000, 64), (10000, 768), (300, 8192)])
+def test_gemm_pairs_cover_the_work(plan, n, k):
+    """Decode batches: every pair has work, no more pairs than an SM each for two CTAs, a tile is shared
+    by at most 17 pairs, the same for every batch size. Prefill: never split, no more pairs than tiles."""
+    out = (ctypes.c_int * 2)()
+    tiles, ku = -(-n // 256), -(-k // 256)
+    total = tiles * ku
+    seen = set()
+    for m in (17, 40, 64):
+        plan.gemm_work(n, m, k, 1, 148, out)
+        seen.add((out[0], out[1]))
+    assert len(seen) == 1
+    pairs, split = seen.pop()
+    assert split == 1 and 1 <= pairs <= 74
+    starts = [total * p // pairs for p in range(pairs + 1)]
+    assert starts[0] == 0 and starts[-1] == total and all(b > a for a, b in zip(starts, starts[1:]))
+    splits = plan.gemm_splits(n, 64, k, 148, -1)
+    if splits > 1:
+        assert pairs == tiles * splits and all(t * ku in starts for t in range(tiles)), "no pair holds parts of two tiles"
+    assert max(sum(1 for a, b in zip(starts, starts[1:]) if a < (t + 1) * ku and b > t * ku) for t in range(tiles)) <= 17
+    plan.gemm_work(n, 1000, k, 4, 148, out)
+    assert out[1] == 0 and out[0] == min(74, 4 * tiles)

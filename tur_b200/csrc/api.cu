@@ -183,8 +183,11 @@ int32_t turq_ctx_create(int32_t device, turq_ctx** out) {
   *ctx->host_done = 0;
   ctx->sm_count = prop.multiProcessorCount;
   const size_t ws_bytes = turq::gemv_workspace_bytes(ctx->sm_count);
+  const size_t gemm_ws_bytes = turq::gemm_tc_workspace_bytes(ctx->sm_count);
   if (cudaMalloc(reinterpret_cast<void**>(&ctx->gemv_ws), ws_bytes) != cudaSuccess ||
-      cudaMemset(ctx->gemv_ws, 0, ws_bytes) != cudaSuccess) {
+      cudaMemset(ctx->gemv_ws, 0, ws_bytes) != cudaSuccess ||
+      cudaMalloc(reinterpret_cast<void**>(&ctx->gemm_ws), gemm_ws_bytes) != cudaSuccess ||
+      cudaMemset(ctx->gemm_ws, 0, gemm_ws_bytes) != cudaSuccess) {
     cudaGetLastError();
     turq_ctx_destroy(ctx);
     return TURQ_E_CUDA;
@@ -208,6 +211,7 @@ int32_t turq_ctx_destroy(turq_ctx* ctx) {
   if (ctx->host_status) cudaFreeHost(ctx->host_status);
   if (ctx->done_count) cudaFree(ctx->done_count);
   if (ctx->gemv_ws) cudaFree(ctx->gemv_ws);
+  if (ctx->gemm_ws) cudaFree(ctx->gemm_ws);
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   delete ctx;
   return TURQ_OK;
@@ -223,14 +227,8 @@ int32_t turq_ctx_reserve(turq_ctx* ctx, int64_t max_m, int64_t max_k, int64_t ma
   size_t need = turq::plan_act_pack(TQ_Q8_K, max_m, k256).total;
   const size_t q80 = turq::plan_act_pack(TQ_Q8_0, max_m, k256).total;
   if (q80 > need) need = q80;
-  // the tensor-core path's f16 operand and split-K partial sums (decode batches split the K loop)
-  for (int64_t mm : {max_m < 64 ? max_m : (int64_t)64, max_m}) {
-    const size_t tc = turq::gemm_tc_scratch_bytes(mm, k256, max_n, ctx->sm_count);
-    if (tc > need) need = tc;
-    // the widest split happens for weights of at most 128 rows
-    const size_t tc_small = turq::gemm_tc_scratch_bytes(mm, k256, max_n < 128 ? max_n : 128, ctx->sm_count);
-    if (tc_small > need) need = tc_small;
-  }
+  const size_t tc = turq::gemm_tc_scratch_bytes(max_m, k256);  // the tensor-core path's f16 operand
+  if (tc > need) need = tc;
   int32_t st = ensure(ctx, &ctx->scratch, &ctx->scratch_bytes, need);
   if (st != TURQ_OK) return st;
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
@@ -260,6 +258,7 @@ int32_t turq_ctx_poll_status(turq_ctx* ctx, void* stream) {
     *static_cast<volatile int*>(ctx->host_status) = 0;
     // a kernel that gave up may have left hand-over flags or claim counters set
     cudaMemsetAsync(ctx->gemv_ws, 0, turq::gemv_workspace_bytes(ctx->sm_count), s);
+    cudaMemsetAsync(ctx->gemm_ws, 0, turq::gemm_tc_workspace_bytes(ctx->sm_count), s);
     cudaStreamSynchronize(s);
     if (st == TURQ_E_INVALID_ARG) return fail(ctx, st, "an embedding lookup was given an id outside the table");
     return fail(ctx, st, "a kernel gave up a bounded device-side wait (status %d)", st);
@@ -484,10 +483,10 @@ int32_t turq_qmatmul(turq_ctx* ctx, const turq_qtensor* qt, const void* dev_x, i
   } else if (mode == TURQ_MODE_EXACT_F32) {
     e = turq::launch_gemv_f32(qt->dtype, qt->tiles, qt->n_rows, k, dev_x, x_dtype, m, dev_y, dev_bias, ctx->sm_count, s, &launches);
   } else if (mode == TURQ_MODE_TENSOR_CORE) {
-    int32_t st = ensure(ctx, &ctx->scratch, &ctx->scratch_bytes, turq::gemm_tc_scratch_bytes(m, k, qt->n_rows, ctx->sm_count));
+    int32_t st = ensure(ctx, &ctx->scratch, &ctx->scratch_bytes, turq::gemm_tc_scratch_bytes(m, k));
     if (st != TURQ_OK) return st;
     e = turq::launch_gemm_tc(qt->dtype, qt->tiles, qt->n_rows, k, dev_x, x_dtype, m, dev_y, dev_bias, ctx->scratch,
-                             ctx->sm_count, s, &launches, ctx->dev_status);
+                             ctx->gemm_ws, ctx->sm_count, s, &launches, ctx->dev_status);
   } else {
     return fail(ctx, TURQ_E_INVALID_ARG, "unknown mode %d", mode);
   }
@@ -520,20 +519,16 @@ static int32_t qmatmul_multi_impl(turq_ctx* ctx, int32_t count, const turq_qtens
       (x_dtype == TURQ_F32 || x_dtype == TURQ_BF16) && (uintptr_t)dev_x % 16 == 0) {
     // tensor-core scheme: x is converted to the f16 operand once for all the weights
     const int64_t k = qts[0]->n_cols;
-    size_t need = 0;
-    for (int i = 0; i < count; i++) {
+    for (int i = 0; i < count; i++)
       if (qts[i]->device != ctx->device) return fail(ctx, TURQ_E_INVALID_ARG, "tensor lives on device %d, context on %d", qts[i]->device, ctx->device);
-      const size_t b = turq::gemm_tc_scratch_bytes(m, k, qts[i]->n_rows, ctx->sm_count);
-      if (b > need) need = b;
-    }
     TQ_CUDA(ctx, cudaSetDevice(ctx->device));
-    int32_t st = ensure(ctx, &ctx->scratch, &ctx->scratch_bytes, need);
+    int32_t st = ensure(ctx, &ctx->scratch, &ctx->scratch_bytes, turq::gemm_tc_scratch_bytes(m, k));
     if (st != TURQ_OK) return st;
     for (int i = 0; i < count; i++) {
       int launches = 0;
       cudaError_t e = turq::launch_gemm_tc(qts[i]->dtype, qts[i]->tiles, qts[i]->n_rows, k, dev_x, x_dtype, m, dev_ys[i],
-                                           dev_biases ? dev_biases[i] : nullptr, ctx->scratch, ctx->sm_count,
-                                           static_cast<cudaStream_t>(stream), &launches, ctx->dev_status, i > 0);
+                                           dev_biases ? dev_biases[i] : nullptr, ctx->scratch, ctx->gemm_ws, ctx->sm_count,
+                                           static_cast<cudaStream_t>(stream), &launches, ctx->dev_status, i);
       ctx->launches += launches;
       if (e != cudaSuccess) return cuda_fail(ctx, e, "qmatmul_multi launch");
     }
@@ -832,12 +827,12 @@ int32_t qmatmul_for_exchange(turq_ctx* ctx, const turq_qtensor* qt, const void* 
     return TURQ_OK;
   }
   if (mode == TURQ_MODE_TENSOR_CORE && qt->n_cols % 64 == 0 && m <= INT32_MAX / 2) {
-    // the GEMM's epilogue (or its split-K reduction) picks the slot itself: no staging copy
-    int32_t st = ensure(ctx, &ctx->scratch, &ctx->scratch_bytes, gemm_tc_scratch_bytes(m, qt->n_cols, qt->n_rows, ctx->sm_count));
+    // the GEMM's epilogue picks the slot itself: no staging copy
+    int32_t st = ensure(ctx, &ctx->scratch, &ctx->scratch_bytes, gemm_tc_scratch_bytes(m, qt->n_cols));
     if (st != TURQ_OK) return st;
     int launches = 0;
     cudaError_t e = launch_gemm_tc(qt->dtype, qt->tiles, qt->n_rows, qt->n_cols, dev_x, x_dtype, m, s0, local_bias, ctx->scratch,
-                                   ctx->sm_count, s, &launches, ctx->dev_status, false, toggle, s1);
+                                   ctx->gemm_ws, ctx->sm_count, s, &launches, ctx->dev_status, 0, toggle, s1);
     ctx->launches += launches;
     if (e != cudaSuccess) return cuda_fail(ctx, e, "row-parallel GEMM launch");
     return TURQ_OK;

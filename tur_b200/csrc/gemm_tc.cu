@@ -1,27 +1,51 @@
-// Prefill-sized QMatMul::forward on the 5th-generation tensor cores (tcgen05 / TMEM).
+// QMatMul::forward on the 5th-generation tensor cores (tcgen05 / TMEM): prefill and decode batches
+// of more than 16 rows.
 //
 //   y[m, n] = sum_k x[m, k] * W[n, k]      W quantized (device fragment tiles), x f32 or bf16
 //
 // Step 1 (prep kernel): x -> f16 [M, K], each row scaled by a power of two that puts its largest
 // magnitude just below the top of the f16 range (the scale is undone exactly in the epilogue).
-// Step 2 (this kernel, one CTA per 128 weight rows x BN = 256 or 64 activation rows):
-//   * warp 0        TMA producer: activation tiles (256 rows x 64 k, f16) into 128B-swizzled
-//                   shared memory (cp.async.bulk.tensor, no multicast);
-//   * warps 2..17   dequantize (two groups of eight on alternate stages) the weight tile (128 rows x 64 k) from the fragment tiles to
-//                   f16 with packed half arithmetic and store it in the same K-major
-//                   128B-swizzled layout, then fence to the async proxy;
-//   * warp 1        one elected thread issues tcgen05.mma (M=128, N=256, K=16, f16 x f16 ->
-//                   f32 in TMEM), four per stage, and commits the stage back to the producers;
-//   * warps 2..17   epilogue: tcgen05.ld the accumulator, undo the row scale, add bias, store.
+// Step 2 (this kernel): pairs of CTAs (a cluster of two, cta_group::2) produce output tiles of 256
+// weight rows x `bn` <= 256 activation rows. Each CTA holds its 128 weight rows as the A operand and
+// half of the activation rows as its part of the B operand, so an activation byte crosses from L2
+// into shared memory once per 256 weight rows.
+//   * warp 0        streams the raw quantized tiles of the CTA's 128 weight rows (units of 256 k,
+//                   contiguous bytes per row-tile) into a ring with cp.async.bulk: how far the
+//                   weights run ahead is set by shared memory, not by registers;
+//   * warp 1        TMA of the activation tile (bn/2 rows x 64 k, f16, 128B swizzle, no multicast),
+//                   completing on the leader CTA's barrier;
+//   * warp 2        (leader CTA) one thread issues tcgen05.mma M=256, N=bn, K=16, f16 x f16 -> f32,
+//                   four per stage, and commits the stage back to the producers of both CTAs;
+//   * warps 3..6    epilogue: tcgen05.ld the accumulator, undo the row scale, add bias, store. The
+//                   accumulator is double buffered (2 x 256 TMEM columns), so the next tile's MMAs
+//                   run meanwhile;
+//   * warps 7..22   dequantize (two groups of eight on alternate 64-k blocks) from the raw ring to
+//                   f16 with packed half arithmetic, store in the K-major 128B-swizzled layout,
+//                   fence to the async proxy and arrive on the leader's barrier.
 // MMA roles: A = weights (rows = TMEM lanes), B = activations (columns).
-// Every mbarrier wait is bounded; on expiry the CTA records TURQ_E_TIMEOUT, releases its TMEM
-// and returns.
+// Work: more than 64 rows: whole tiles, dealt out to persistent pairs. Decode batches (<= 64 rows,
+// one activation tile): the K loop of a tile is shared between pairs; the pair that holds a tile's
+// first unit adds the others' partial sums in pair order (fixed order, no float atomics).
+//
+// What bounds it. Prefill: the tensor pipe (81 % of active cycles at 12288 x 4096 Q4_K, 2048 rows), the
+// power limit and the last wave of tiles. Decode batches: issue slots - the dequantization costs about
+// 75 warp instructions per 1024 weights - and some 8 us of hand-overs (conversion, first activation
+// tile, partial sums). Why it is split this way, measured with graph replay, conversion included, against
+// one CTA per 128 rows with weights prefetched into registers and one ring for both operands:
+//   Q4_K 12288 x 4096, 2048 rows  231 -> 163 us (1267 TFLOP/s)   Q6_K 4096 x 12288, 512 rows  105 -> 75 us
+//   Q4_K 12288 x 4096, 64 rows   31.5 -> 24 us                   Q6_K 5120 x 25600, 64 rows   85 -> 57 us
+// Steps on the way: an MMA loop whose control flow is warp-uniform (210 -> 173 us at 2048 rows: with
+// one divergent thread the descriptors of every MMA went through moves to uniform registers), remote
+// arrivals without a cluster-scope release (270 -> 210 us; the proxy fence already orders the operand
+// tile), two 64-k blocks per weight stage (fewer fences and barrier rounds per dequantize warp).
+// Every wait is bounded; on expiry the CTA records TURQ_E_TIMEOUT, releases its TMEM and returns.
 #include <cstdlib>
 #include <cuda.h>
 #include <cuda_fp16.h>
 
 #include <cstdio>
 
+#include "actquant.cuh"
 #include "device_utils.cuh"
 #include "gemv_tile.cuh"
 #include "launch_plan.h"
@@ -31,16 +55,21 @@ namespace turq {
 
 namespace {
 
-constexpr int BM = 128;      // weight rows per CTA (MMA M)
-constexpr int BK = 64;       // k per stage (one 128-byte swizzle row of f16)
-// Pipeline depth by activation-tile height: the ring must cover the L2 -> shared-memory latency of
-// the TMA loads (a slot is only refilled after the MMAs that read it have completed), so the
-// smaller tiles get more stages out of the same shared memory.
-constexpr int stages_for_bn(int bn) { return bn == 64 ? 8 : bn == 128 ? 6 : 4; }
-constexpr int A_BYTES = BM * BK * 2;  // 16 KB
+constexpr int BM = 128;      // weight rows per CTA; a pair's MMA covers 2 * BM
+constexpr int BK = 64;       // k per operand block (one 128-byte swizzle row of f16)
+constexpr int UNIT_K = 256;  // k per unit of raw weight bytes (four blocks)
+constexpr int MAX_ST = 8;    // operand stages
+constexpr int MAX_RAW = 8;   // raw ring slots
+constexpr int KA = 2;                 // blocks per weight stage: what one dequantize warp makes of a unit
+constexpr int A_BYTES = BM * BK * 2;  // 16 KB per block
+constexpr int DQ_WARP0 = 7;        // first dequantize warp; warps 3..6 are the epilogue, one per TMEM lane quarter (warp & 3)
 constexpr int DQ_WARPS = 8;        // warps that together produce one stage of the weight operand
 constexpr int DQ_GROUPS = 2;       // groups of DQ_WARPS warps working on alternate stages
-constexpr int TC_THREADS = (2 + DQ_WARPS * DQ_GROUPS) * 32;
+constexpr int HELPERS = 1 + DQ_WARPS * DQ_GROUPS / 4;  // warps per TMEM lane quarter that share a pair's last epilogue
+constexpr int TC_THREADS = (DQ_WARP0 + DQ_WARPS * DQ_GROUPS) * 32;
+// Register bound (72) of the kernel: leaves a CTA of the conversion kernel room beside it on an SM.
+constexpr int TC_REG_THREADS = 896;
+constexpr int TMEM_COLS = 512;     // two accumulators of 256 columns
 constexpr long long TC_WAIT_CYCLES = 4000000000ll;
 
 __device__ __forceinline__ uint32_t s_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -75,32 +104,28 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatil
   *abort_flag = 1;
   return false;
 }
-
-#ifdef TURQ_TRACE
-// Debug timeline of CTA (0,0,0): global-timer stamps of one dequantize warp and of the MMA
-// thread over a few consecutive stages (built only with -DTURQ_TRACE).
-__device__ unsigned long long g_gemm_trace[64 * 8];
-__device__ __forceinline__ unsigned long long gtime_tc() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
+// The barriers of a pair's leader collect arrivals of both CTAs.
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
 }
-#define TC_TRACE(row, col) do { if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (row) >= 0 && (row) < 64) g_gemm_trace[(row) * 8 + (col)] = gtime_tc(); } while (0)
-int read_gemm_trace(unsigned long long* host, int n) {
-  return (int)cudaMemcpyFromSymbol(host, g_gemm_trace, sizeof(unsigned long long) * n);
+__device__ __forceinline__ void bar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-#else
-#define TC_TRACE(row, col) do { } while (0)
-#endif
-
-// K-major, 128-byte swizzle shared-memory matrix descriptor (8-row groups 1024 B apart).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
-
-// byte offset of 16-byte chunk `ch` (8 f16 along k) of tile row r in the swizzled layout
-__device__ __forceinline__ uint32_t swz(int r, int ch) {
-  return (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((ch ^ (r & 7)) << 4));
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void commit_to_pair(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(s_u32(bar)),
+               "h"((unsigned short)3)
+               : "memory");
 }
 
 // ---- dequantization to f16 with packed half arithmetic (two elements per instruction).
@@ -110,134 +135,151 @@ __device__ __forceinline__ uint32_t swz(int r, int ch) {
 // of the tensor-core mode (the bit-exact f32 decode lives in decode.cuh).
 __device__ __forceinline__ __half2 u2h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 __device__ __forceinline__ uint32_t h22u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
-// bytes (b0, b1) / (b2, b3) of a word of small integers -> half2 (1024 + b0, 1024 + b1) / ...
+// The f16 operands keep the elements of every aligned group of four in the order 0, 2, 1, 3 (weights
+// here, activations in the conversion kernel): those are the pairs a word gives without a shuffle.
+// bytes (b0, b2) / (b1, b3) of a word of small integers -> half2 (1024 + b0, 1024 + b2) / ...
+__device__ __forceinline__ __half2 pair02(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5240)); }
+__device__ __forceinline__ __half2 pair13(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5341)); }
 __device__ __forceinline__ __half2 pair01(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5140)); }
 __device__ __forceinline__ __half2 pair23(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5342)); }
 
-// Raw fragment bytes of one lane for one stage (16 rows x 64 k), fetched from global memory a
-// few stages ahead of their use so that the HBM/L2 latency is off the critical path.
-template <int DT> struct StageRegs;
-template <> struct StageRegs<TQ_Q8_0> { uint4 q[2]; uint32_t d[2]; };       // d: f16 row g | row g+8 << 16, per tile
-template <> struct StageRegs<TQ_Q4_K> { uint4 q; uint4 hdr[2]; };
-template <> struct StageRegs<TQ_Q5_K> { uint4 q; uint4 qh; uint4 hdr[2]; };
-template <> struct StageRegs<TQ_Q6_K> { uint4 ql; uint4 qh; uint32_t sc[2]; uint32_t d; };
+// Raw bytes of one unit (16 weight rows x 256 k) as they lie in a ring slot.
+template <int DT> struct UnitGeom {
+  static constexpr int TILES = UNIT_K / TileGeom<DT>::ELEMS;  // device tiles per unit: 8 (Q8_0) or 1
+  static constexpr int BYTES = TILES * TileGeom<DT>::BYTES;   // per row-tile
+};
 
+// Scales of the two 64-k blocks of a unit that a warp dequantizes (Q4_K / Q5_K): lane 2r + e holds,
+// for row r of the row-tile and block e of the warp's two, the f16 scale and negated min of the
+// block's two sub-blocks. Worked out once per unit and row instead of by every lane that needs them.
+struct UnitScales { uint32_t dl, ml; };
 template <int DT>
-__device__ __forceinline__ void stage_load(StageRegs<DT>& r, const uint8_t* __restrict__ tiles_rt, int kb, int lane) {
-  const int g = lane >> 2;
-  if constexpr (DT == TQ_Q8_0) {
-#pragma unroll
-    for (int tt = 0; tt < 2; tt++) {
-      const uint8_t* t = tiles_rt + (size_t)(2 * kb + tt) * 544;
-      r.q[tt] = ld_stream_v4(t + TQ_Q8_0_QS + 16 * lane);
-      r.d[tt] = (uint32_t)ld_u16(t + 2 * g) | ((uint32_t)ld_u16(t + 2 * (g + 8)) << 16);
-    }
-  } else if constexpr (DT == TQ_Q4_K || DT == TQ_Q5_K) {
-    constexpr int TB = DT == TQ_Q4_K ? 2304 : 2816;
-    constexpr int QS = DT == TQ_Q4_K ? TQ_Q4K_QS : TQ_Q5K_QS;
-    const uint8_t* t = tiles_rt + (size_t)(kb >> 2) * TB;
-    r.q = ld_stream_v4(t + QS + 512 * (kb & 3) + 16 * lane);
-    if constexpr (DT == TQ_Q5_K) r.qh = ld_v4(t + TQ_Q5K_QH + 16 * lane);
-    r.hdr[0] = ld_v4(t + 16 * g);
-    r.hdr[1] = ld_v4(t + 16 * (g + 8));
-  } else {
-    const uint8_t* t = tiles_rt + (size_t)(kb >> 2) * 3360;
-    const int i = kb & 3;
-    r.ql = ld_stream_v4(t + TQ_Q6K_QL + 512 * i + 16 * lane);
-    r.qh = ld_v4(t + TQ_Q6K_QH + 512 * (i >> 1) + 16 * lane);
-    r.sc[0] = ld_u32(t + 16 * g + 4 * i);
-    r.sc[1] = ld_u32(t + 16 * (g + 8) + 4 * i);
-    r.d = (uint32_t)ld_u16(t + TQ_Q6K_D + 2 * g) | ((uint32_t)ld_u16(t + TQ_Q6K_D + 2 * (g + 8)) << 16);
+__device__ __forceinline__ UnitScales unit_scales(const uint8_t* t, int i, int lane) {
+  UnitScales u{0u, 0u};
+  if constexpr (DT == TQ_Q4_K || DT == TQ_Q5_K) {
+    const __half2 off = __float2half2_rn(1024.f);
+    const uint4 hd = lds_v4(t + 16 * (lane >> 1));
+    // Half arithmetic only (no int->float / float->half conversions, which share one narrow pipe):
+    // d * sc is exact in f32, so one f16 multiply rounds it the same way.
+    const __half2 dd = u2h2(__byte_perm(hd.x, 0u, 0x1010)), mm = u2h2(__byte_perm(hd.x, 0u, 0x3232));
+    // 6-bit scales / mins of sub-blocks 0..3 or 4..7, one per byte; block i needs bytes 2(i&1), 2(i&1)+1
+    const uint32_t scw = i >= 2 ? ((hd.w & 0x0F0F0F0Fu) | ((hd.y >> 2) & 0x30303030u)) : (hd.y & 0x3F3F3F3Fu);
+    const uint32_t mnw = i >= 2 ? (((hd.w >> 4) & 0x0F0F0F0Fu) | ((hd.z >> 2) & 0x30303030u)) : (hd.z & 0x3F3F3F3Fu);
+    const int sh = 16 * (i & 1);
+    u.dl = h22u(__hmul2(dd, __hsub2(pair01(scw >> sh), off)));
+    u.ml = h22u(__hneg2(__hmul2(mm, __hsub2(pair01(mnw >> sh), off))));
   }
+  return u;
 }
 
-// Dequantize one stage from registers and store it as f16: a_tile = swizzled 128 x 64 tile,
-// row0 = first of this warp's 16 rows inside it.
+// Dequantizes 64-k block i of a unit (t: the row-tile's raw bytes in shared memory), block e of the
+// warp's two, to f16 and stores it in the swizzled operand tile; `a_rows` points at the row-tile's 16
+// rows there. Odd rows store their two 64-byte halves in the other order than even ones: with the
+// same order rows g and g + 1 of a quarter-warp meet in the same banks and every store takes two passes.
 template <int DT>
-__device__ __forceinline__ void stage_dequant_store(const StageRegs<DT>& r, int kb, int lane, uint8_t* a_tile, int row0) {
-  const int g = lane >> 2, c = lane & 3;
+__device__ __forceinline__ void dequant_block(const uint8_t* t, const UnitScales& us, int i, int e, int lane, uint8_t* a_rows) {
+  const int g = lane >> 2, c = lane & 3, odd = g & 1;
+  uint8_t* const row = a_rows + g * 128;
   if constexpr (DT == TQ_Q8_0) {
     const __half2 off = __float2half2_rn(1152.f);  // 1024 + 128: bytes are biased by xor 0x80
+    const uint32_t o0 = (uint32_t)(((4 * odd + c) ^ g) << 4);
 #pragma unroll
-    for (int tt = 0; tt < 2; tt++) {
-      const uint4 q = r.q[tt];
+    for (int h = 0; h < 2; h++) {
+      const uint8_t* tt = t + (2 * i + (h ^ odd)) * 544;
+      const uint4 q = lds_v4(tt + TQ_Q8_0_QS + 16 * lane);
+      const uint32_t dd = lds_u16(tt + 2 * g) | (lds_u16(tt + 2 * (g + 8)) << 16);
       const uint32_t w[2][2] = {{q.x ^ 0x80808080u, q.y ^ 0x80808080u}, {q.z ^ 0x80808080u, q.w ^ 0x80808080u}};
 #pragma unroll
       for (int hr = 0; hr < 2; hr++) {
-        const __half2 d2 = __half2half2(__ushort_as_half((unsigned short)((r.d[tt] >> (16 * hr)) & 0xFFFFu)));
+        const __half2 d2 = u2h2(__byte_perm(dd, 0u, hr ? 0x3232 : 0x1010));
         uint4 o;
-        o.x = h22u(__hmul2(__hsub2(pair01(w[hr][0]), off), d2));
-        o.y = h22u(__hmul2(__hsub2(pair23(w[hr][0]), off), d2));
-        o.z = h22u(__hmul2(__hsub2(pair01(w[hr][1]), off), d2));
-        o.w = h22u(__hmul2(__hsub2(pair23(w[hr][1]), off), d2));
-        *reinterpret_cast<uint4*>(a_tile + swz(row0 + g + 8 * hr, 4 * tt + c)) = o;
+        o.x = h22u(__hmul2(__hsub2(pair02(w[hr][0]), off), d2));
+        o.y = h22u(__hmul2(__hsub2(pair13(w[hr][0]), off), d2));
+        o.z = h22u(__hmul2(__hsub2(pair02(w[hr][1]), off), d2));
+        o.w = h22u(__hmul2(__hsub2(pair13(w[hr][1]), off), d2));
+        *reinterpret_cast<uint4*>(row + hr * 1024 + (o0 ^ (h << 6))) = o;
       }
     }
   } else if constexpr (DT == TQ_Q4_K || DT == TQ_Q5_K) {
-    const int i = kb & 3;  // 64-element group inside the super-block: sub-blocks 2i, 2i+1
-    const uint32_t w[2][2] = {{r.q.x, r.q.y}, {r.q.z, r.q.w}};
-    uint32_t qh[2][2] = {{0, 0}, {0, 0}};
-    if constexpr (DT == TQ_Q5_K) {
-      qh[0][0] = r.qh.x; qh[0][1] = r.qh.y; qh[1][0] = r.qh.z; qh[1][1] = r.qh.w;
-    }
-    const __half2 off = __float2half2_rn(1024.f);
+    constexpr int QS = DT == TQ_Q4_K ? TQ_Q4K_QS : TQ_Q5K_QS;
+    const uint4 q = lds_v4(t + QS + 512 * i + 16 * lane);
+    const uint32_t w[2][2] = {{q.x, q.y}, {q.z, q.w}};
+    const uint32_t o0 = (uint32_t)(((4 * odd + c) ^ g) << 4);
+    uint32_t dl2[2], ml2[2];
 #pragma unroll
     for (int hr = 0; hr < 2; hr++) {
-      const uint4 hdr = r.hdr[hr];
-      // Sub-block scales in half arithmetic only (no int->float / float->half conversions, which
-      // share one narrow pipe): d * sc is exact in f32, so one f16 multiply rounds it the same way.
-      const __half2 dd = u2h2(__byte_perm(hdr.x, 0u, 0x1010)), mm = u2h2(__byte_perm(hdr.x, 0u, 0x3232));
-      // 6-bit scales / mins of sub-blocks 0..3 or 4..7, one per byte; this stage needs bytes
-      // 2*(i&1) and 2*(i&1)+1
-      const uint32_t scw = i < 2 ? (hdr.y & 0x3F3F3F3Fu) : ((hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u));
-      const uint32_t mnw = i < 2 ? (hdr.z & 0x3F3F3F3Fu) : (((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u));
-      const __half2 sc2 = __hsub2((i & 1) ? pair23(scw) : pair01(scw), off);
-      const __half2 mn2 = __hsub2((i & 1) ? pair23(mnw) : pair01(mnw), off);
-      const __half2 dl2 = __hmul2(dd, sc2), ml2 = __hneg2(__hmul2(mm, mn2));
+      const int src = 2 * (g + 8 * hr) + e;
+      dl2[hr] = __shfl_sync(0xFFFFFFFFu, us.dl, src);
+      ml2[hr] = __shfl_sync(0xFFFFFFFFu, us.ml, src);
+    }
 #pragma unroll
-      for (int nib = 0; nib < 2; nib++) {
-        const int j = 2 * i + nib;
-        const __half2 dl = nib ? __high2half2(dl2) : __low2half2(dl2);
-        const __half2 ml = nib ? __high2half2(ml2) : __low2half2(ml2);
-        uint32_t m0 = (nib ? (w[hr][0] >> 4) : w[hr][0]) & 0x0F0F0F0Fu;
-        uint32_t m1 = (nib ? (w[hr][1] >> 4) : w[hr][1]) & 0x0F0F0F0Fu;
-        if constexpr (DT == TQ_Q5_K) {
-          m0 |= ((qh[hr][0] >> j) << 4) & 0x10101010u;
-          m1 |= ((qh[hr][1] >> j) << 4) & 0x10101010u;
+    for (int h = 0; h < 2; h++) {
+      const int nib = h ^ odd;  // 0: sub-block 2i (low nibbles), 1: sub-block 2i + 1
+      const uint32_t sel = nib ? 0x3232u : 0x1010u;
+      if constexpr (DT == TQ_Q4_K) {
+        // A nibble becomes a half without being moved: under the exponent of 1024 the low nibble counts
+        // ones, under that of 64 the high nibble (16 units of 1/16) does; the offset subtracts exactly.
+        const uint32_t mask = nib ? 0x00F000F0u : 0x000F000Fu, magic = nib ? 0x54005400u : 0x64006400u;
+        const __half2 off = u2h2(magic);
+#pragma unroll
+        for (int hr = 0; hr < 2; hr++) {
+          const __half2 dl = u2h2(__byte_perm(dl2[hr], 0u, sel)), ml = u2h2(__byte_perm(ml2[hr], 0u, sel));
+          uint4 o;
+          o.x = h22u(__hfma2(__hsub2(u2h2((w[hr][0] & mask) | magic), off), dl, ml));
+          o.y = h22u(__hfma2(__hsub2(u2h2(((w[hr][0] >> 8) & mask) | magic), off), dl, ml));
+          o.z = h22u(__hfma2(__hsub2(u2h2((w[hr][1] & mask) | magic), off), dl, ml));
+          o.w = h22u(__hfma2(__hsub2(u2h2(((w[hr][1] >> 8) & mask) | magic), off), dl, ml));
+          *reinterpret_cast<uint4*>(row + hr * 1024 + (o0 ^ (h << 6))) = o;
         }
-        uint4 o;
-        o.x = h22u(__hfma2(__hsub2(pair01(m0), off), dl, ml));
-        o.y = h22u(__hfma2(__hsub2(pair23(m0), off), dl, ml));
-        o.z = h22u(__hfma2(__hsub2(pair01(m1), off), dl, ml));
-        o.w = h22u(__hfma2(__hsub2(pair23(m1), off), dl, ml));
-        *reinterpret_cast<uint4*>(a_tile + swz(row0 + g + 8 * hr, 4 * nib + c)) = o;
+      } else {
+        const __half2 off = __float2half2_rn(1024.f);
+        const uint4 h4 = lds_v4(t + TQ_Q5K_QH + 16 * lane);
+        const uint32_t qh[2][2] = {{h4.x, h4.y}, {h4.z, h4.w}};
+        const int rot = 4 - (2 * i + nib);  // brings the sub-block's bit to bit 4 of every byte
+#pragma unroll
+        for (int hr = 0; hr < 2; hr++) {
+          const __half2 dl = u2h2(__byte_perm(dl2[hr], 0u, sel)), ml = u2h2(__byte_perm(ml2[hr], 0u, sel));
+          const uint32_t m0 = ((w[hr][0] >> (4 * nib)) & 0x0F0F0F0Fu) | (__funnelshift_l(qh[hr][0], qh[hr][0], rot) & 0x10101010u);
+          const uint32_t m1 = ((w[hr][1] >> (4 * nib)) & 0x0F0F0F0Fu) | (__funnelshift_l(qh[hr][1], qh[hr][1], rot) & 0x10101010u);
+          uint4 o;
+          o.x = h22u(__hfma2(__hsub2(pair02(m0), off), dl, ml));
+          o.y = h22u(__hfma2(__hsub2(pair13(m0), off), dl, ml));
+          o.z = h22u(__hfma2(__hsub2(pair02(m1), off), dl, ml));
+          o.w = h22u(__hfma2(__hsub2(pair13(m1), off), dl, ml));
+          *reinterpret_cast<uint4*>(row + hr * 1024 + (o0 ^ (h << 6))) = o;
+        }
       }
     }
-  } else {  // Q6_K: the stage is sub-blocks 4i .. 4i+3 (16 elements each)
-    const int i = kb & 3;
-    const uint32_t qlw[2][2] = {{r.ql.x, r.ql.y}, {r.ql.z, r.ql.w}};
-    const uint32_t qhw[2] = {(i & 1) ? r.qh.y : r.qh.x, (i & 1) ? r.qh.w : r.qh.z};
+  } else {  // Q6_K: the block is sub-blocks 4i .. 4i+3 (16 elements each)
+    const uint4 ql = lds_v4(t + TQ_Q6K_QL + 512 * i + 16 * lane);
+    const uint4 q2 = lds_v4(t + TQ_Q6K_QH + 512 * (i >> 1) + 16 * lane);
+    const uint32_t db = lds_u16(t + TQ_Q6K_D + 2 * g) | (lds_u16(t + TQ_Q6K_D + 2 * (g + 8)) << 16);
     const __half2 off = __float2half2_rn(1056.f);  // 1024 + 32
     const __half2 off_sc = __float2half2_rn(1152.f);  // 1024 + 128: the int8 scales are biased by xor 0x80
+    const uint32_t o0 = (uint32_t)((((4 * odd) ^ (c >> 1) ^ g) << 4) + 8 * (c & 1));
 #pragma unroll
     for (int hr = 0; hr < 2; hr++) {
-      const int rr = g + 8 * hr;
+      const uint32_t wa = hr ? ql.z : ql.x, wb = hr ? ql.w : ql.y;
+      const uint32_t qhw = (i & 1) ? (hr ? q2.w : q2.y) : (hr ? q2.z : q2.x);
       // d * scale in half arithmetic (exact product, one rounding - as the f32 route gives)
-      const __half2 dd = u2h2(__byte_perm(r.d, 0u, hr ? 0x3232 : 0x1010));
-      const uint32_t scb = r.sc[hr] ^ 0x80808080u;
+      const __half2 dd = u2h2(__byte_perm(db, 0u, hr ? 0x3232 : 0x1010));
+      const uint32_t scb = ld_u32(t + 16 * (g + 8 * hr) + 4 * i) ^ 0x80808080u;
       const __half2 dl01 = __hmul2(dd, __hsub2(pair01(scb), off_sc)), dl23 = __hmul2(dd, __hsub2(pair23(scb), off_sc));
+      // odd rows take sub-blocks 2, 3, 0, 1
+      const uint32_t w2[2] = {odd ? wb : wa, odd ? wa : wb};
+      const uint32_t dl2[2] = {h22u(odd ? dl23 : dl01), h22u(odd ? dl01 : dl23)};
+      const uint32_t qv = odd ? __funnelshift_l(qhw, qhw, 28) : qhw;  // fields 2, 3 down to 0, 1 (and 0, 1 up, bytes rotated)
+      const uint32_t qu = odd ? __funnelshift_l(qhw, qhw, 4) : qhw;   // fields 0, 1 up to 2, 3
 #pragma unroll
       for (int jj = 0; jj < 4; jj++) {
-        const int tw = jj >> 1, nib = jj & 1, sh = 2 * jj;
-        const __half2 dlp = jj < 2 ? dl01 : dl23;
-        const __half2 dl = (jj & 1) ? __high2half2(dlp) : __low2half2(dlp);
-        uint32_t m = (nib ? (qlw[hr][tw] >> 4) : qlw[hr][tw]) & 0x0F0F0F0Fu;
-        m |= (sh <= 4 ? (qhw[hr] << (4 - sh)) : (qhw[hr] >> (sh - 4))) & 0x30303030u;
-        // elements 16*jj + 4c .. +3 of the stage: chunk 2*jj + (c >> 1), half (c & 1)
+        const int nib = jj & 1, sh = 2 * jj;
+        const __half2 dl = u2h2(__byte_perm(dl2[jj >> 1], 0u, nib ? 0x3232 : 0x1010));
+        uint32_t m = (nib ? (w2[jj >> 1] >> 4) : w2[jj >> 1]) & 0x0F0F0F0Fu;
+        m |= (sh <= 4 ? ((jj < 2 ? qv : qu) << (4 - sh)) : (qu >> (sh - 4))) & 0x30303030u;
         uint2 o;
-        o.x = h22u(__hmul2(__hsub2(pair01(m), off), dl));
-        o.y = h22u(__hmul2(__hsub2(pair23(m), off), dl));
-        *reinterpret_cast<uint2*>(a_tile + swz(row0 + rr, 2 * jj + (c >> 1)) + 8 * (c & 1)) = o;
+        o.x = h22u(__hmul2(__hsub2(pair02(m), off), dl));
+        o.y = h22u(__hmul2(__hsub2(pair13(m), off), dl));
+        *reinterpret_cast<uint2*>(row + hr * 1024 + (o0 ^ (jj << 5))) = o;
       }
     }
   }
@@ -246,246 +288,498 @@ __device__ __forceinline__ void stage_dequant_store(const StageRegs<DT>& r, int 
 struct GemmArgs {
   const uint8_t* tiles;
   int64_t n_rows;   // weight rows (output features)
-  int ktiles;       // fragment tiles per row-tile
-  int k;
+  int row_tiles;    // 16-row tiles of the weight
+  int ktiles;       // device tiles per row-tile
+  int kblocks;      // k / 64
+  int KU;           // units of 256 k per row (the last one of a Q8_0 weight may hold fewer blocks)
   int m;            // activation rows
+  int bn;           // activation rows per pair tile: a multiple of 16, at most 256
+  int mt;           // activation tiles
+  int total;        // split_k: units of all tiles, shared out evenly; else: tiles
+  int split_k;
+  int sibling;      // the preceding launch belongs to the same call and reads the same x (see the kernel)
+  int a_stages, b_stages, raw_slots;
   const float* rscale;  // [m] factor undoing the f16 row scaling
-  float* y;         // [m, n_rows]; with split-K: partial sums [splits][m][n_rows]
+  float* y;             // [m, n_rows]
   const float* bias;
+  float* partial;       // [CTA][bn / 4][128][4]: partial sums of a CTA that does not own its first tile
+  int* flags;           // [CTA][4 lane quarters][8, HELPERS used], all zero between launches
   int* status;
-  int splits;       // CTAs along K per output tile (gridDim.z); > 1: a reduction launch follows
   // exchange slots (tp.cu): with y_toggle set, the result goes to y_alt instead of y when the
   // word it points to, plus one, is odd - read after the preceding kernels have completed
   const unsigned* y_toggle;
   float* y_alt;
 };
 
-// BN = activation rows per CTA (MMA N): 256 for prefill (128 when that is needed to give every
-// SM a CTA), 64 for decode batches of a few dozen rows.
-template <int DT, int BN>
-__global__ void __launch_bounds__(TC_THREADS, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
+// The tiles (or shares of tiles) a pair works on, in order; every role of both CTAs walks the same list.
+struct Segments {
+  int u, u1, step, KU;
+  bool split;
+  __device__ __forceinline__ static int start(const GemmArgs& a, int pair, int pairs) {
+    return (int)((int64_t)a.total * pair / pairs);
+  }
+  __device__ __forceinline__ void init(const GemmArgs& a, int pair, int pairs) {
+    split = a.split_k != 0;
+    KU = a.KU;
+    u = split ? start(a, pair, pairs) : pair;
+    u1 = split ? start(a, pair + 1, pairs) : a.total;
+    step = pairs;
+  }
+  __device__ __forceinline__ bool last() const { return u >= u1; }  // after next(): nothing follows
+  // units [ka, kb) of tile `t`
+  __device__ __forceinline__ bool next(int& t, int& ka, int& kb) {
+    if (u >= u1) return false;
+    if (!split) {
+      t = u; ka = 0; kb = KU;
+      u += step;
+      return true;
+    }
+    t = u / KU;
+    ka = u - t * KU;
+    kb = ka + (u1 - u);
+    if (kb > KU) kb = KU;
+    u += kb - ka;
+    return true;
+  }
+};
+
+__device__ __forceinline__ int ld_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release(int* p, int v) { asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
+
+// Epilogue of one segment for one TMEM lane quarter (32 weight rows): columns in chunks of CH, the
+// chunks h0, h0 + hstep, ... A pair that does not hold the tile's first unit parks its sums in
+// the workspace; the one that does adds the others' in pair order. Ready flags are per lane quarter
+// and chunk residue modulo HELPERS, so whoever takes a chunk finds it complete whether the other
+// side's last epilogue was shared between warps or not.
+template <int CH, bool SPLIT>
+__device__ __forceinline__ void epilogue(const GemmArgs& a, float* ybase, int t, int ka, int kb, int pair, int pairs, int rank,
+                                         int quarter, int lane, uint32_t tmem, int h0, int hstep, volatile int* abort_flag) {
+  const int m0 = (t % a.mt) * a.bn;
+  const int cols = a.m - m0 < a.bn ? a.m - m0 : a.bn;
+  const int nchunks = (cols + CH - 1) / CH;
+  const int64_t n = (int64_t)(t / a.mt) * (2 * BM) + rank * BM + 32 * quarter + lane;
+  const bool owner = !SPLIT || ka == 0;
+  const int cta = 2 * pair + rank;
+  const int nflags = nchunks < HELPERS ? nchunks : HELPERS;
+  int nother = 0;  // pairs that hold the rest of this tile
+  if (SPLIT && owner && kb < a.KU) {
+    while (pair + 1 + nother < pairs && Segments::start(a, pair + 1 + nother, pairs) < (t + 1) * a.KU) nother++;
+    const long long t0 = clock64();
+    for (int f0 = h0; f0 < nflags; f0 += hstep)
+      for (int o = lane; o < nother; o += 32) {
+        const int* f = a.flags + ((cta + 2 * (o + 1)) * 4 + quarter) * 8 + f0;
+        while (ld_acquire(f) == 0) {
+          if (*abort_flag || clock64() - t0 > TC_WAIT_CYCLES) { *abort_flag = 1; break; }
+        }
+      }
+    __syncwarp();
+  }
+  const float bv = (owner && a.bias && n < a.n_rows) ? a.bias[n] : 0.f;
+  float* const yp = ybase + (int64_t)m0 * a.n_rows + n;
+  float* const part = a.partial + ((size_t)cta * (a.bn >> 2) * BM + (32 * quarter + lane)) * 4;
+  const size_t part_pair = (size_t)2 * (a.bn >> 2) * BM * 4;  // the same CTA of the next pair
+  for (int ch = h0; ch < nchunks; ch += hstep) {
+    const int col0 = ch * CH;
+    uint32_t v[CH];
+    const uint32_t taddr = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)col0;
+    if constexpr (CH == 16) {
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+          "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+            "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+          : "r"(taddr)
+          : "memory");
+    } else {
+      asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                   : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                   : "r"(taddr)
+                   : "memory");
+    }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    if (!owner) {
+#pragma unroll
+      for (int j = 0; j < CH; j += 4)
+        __stcg(reinterpret_cast<uint4*>(part + (size_t)((col0 + j) >> 2) * BM * 4), make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]));
+    } else {
+      if constexpr (SPLIT) {
+        constexpr int B = 2;  // other pairs whose sums are in flight at once
+        for (int o = 1; o <= nother; o += B) {
+          float4 p[B][CH / 4];
+#pragma unroll
+          for (int b = 0; b < B; b++)
+#pragma unroll
+            for (int j = 0; j < CH / 4; j++)
+              if (o + b <= nother) p[b][j] = __ldcg(reinterpret_cast<const float4*>(part + (o + b) * part_pair + (size_t)((col0 >> 2) + j) * BM * 4));
+#pragma unroll
+          for (int b = 0; b < B; b++)
+            if (o + b <= nother) {
+#pragma unroll
+              for (int j = 0; j < CH / 4; j++) {
+                v[4 * j] = __float_as_uint(__uint_as_float(v[4 * j]) + p[b][j].x);
+                v[4 * j + 1] = __float_as_uint(__uint_as_float(v[4 * j + 1]) + p[b][j].y);
+                v[4 * j + 2] = __float_as_uint(__uint_as_float(v[4 * j + 2]) + p[b][j].z);
+                v[4 * j + 3] = __float_as_uint(__uint_as_float(v[4 * j + 3]) + p[b][j].w);
+              }
+            }
+        }
+      }
+      if (n < a.n_rows) {
+#pragma unroll
+        for (int j = 0; j < CH; j++)
+          if (col0 + j < cols) yp[(int64_t)(col0 + j) * a.n_rows] = __uint_as_float(v[j]) * a.rscale[m0 + col0 + j] + bv;
+      }
+    }
+  }
+  if constexpr (SPLIT) {
+    if (!owner) {
+      __syncwarp();
+      if (lane == 0)
+        for (int f0 = h0; f0 < nflags; f0 += hstep) st_release(a.flags + (cta * 4 + quarter) * 8 + f0, 1);
+    } else {
+      __syncwarp();
+      for (int f0 = h0; f0 < nflags; f0 += hstep)  // consumed: zero again for the next launch
+        for (int o = lane; o < nother; o += 32) a.flags[((cta + 2 * (o + 1)) * 4 + quarter) * 8 + f0] = 0;
+    }
+  }
+}
+
+// SPLIT: decode batches of at most 64 rows (K loops shared between pairs).
+template <int DT, bool SPLIT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_REG_THREADS, 1)
+gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ GemmArgs a) {
   constexpr int TB = TileGeom<DT>::BYTES;
-  constexpr int B_BYTES = BN * BK * 2;
-  constexpr int TMEM_COLS = BN;
-  constexpr int ST = stages_for_bn(BN);
+  constexpr int UB = UnitGeom<DT>::BYTES;
+  constexpr int SLOT_BYTES = 8 * UB;
+  constexpr int KB = SPLIT ? 2 : 1;  // 64-k blocks per activation stage
+  constexpr int CH = SPLIT ? 8 : 16;  // columns per epilogue step
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  // 1024-byte alignment for the swizzled tiles
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  // 1024-byte alignment for the swizzled tiles; the same offsets in both CTAs of the pair
+  uint8_t* smem = smem_raw + ((1024u - (s_u32(smem_raw) & 1023u)) & 1023u);
+  const int SA = a.a_stages, SB = a.b_stages, RS = a.raw_slots;
+  const int b_bytes = a.bn * (BK * 2 / 2);  // this CTA's half of the activation tile, per block
   uint8_t* sA = smem;
-  uint8_t* sB = smem + ST * A_BYTES;
-  // full[s]: stage s holds its weight tile (one arrival per dequantize warp) and its
-  // activation tile (the TMA thread's arrival + transaction bytes)
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + ST * (A_BYTES + B_BYTES));
-  uint64_t* empty = full + ST;
-  uint64_t* accum = empty + ST;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
+  uint8_t* sB = sA + SA * KA * A_BYTES;
+  uint8_t* sRaw = sB + SB * KB * b_bytes;
+  // The two operands have rings of their own: an activation tile is a trip to L2 away and needs many
+  // stages in flight, a weight tile comes from this SM's raw ring and needs few.
+  // a_full[s] (leader only): both CTAs' weight tiles, one arrival per dequantize warp
+  // b_full[s] (leader only): both halves of the activation tile (transaction bytes of both CTAs)
+  uint64_t* a_full = reinterpret_cast<uint64_t*>(sRaw + RS * SLOT_BYTES);
+  uint64_t* a_empty = a_full + MAX_ST;
+  uint64_t* b_full = a_empty + MAX_ST;
+  uint64_t* b_empty = b_full + MAX_ST;
+  uint64_t* raw_full = b_empty + MAX_ST;
+  uint64_t* raw_empty = raw_full + MAX_RAW;
+  uint64_t* acc_full = raw_empty + MAX_RAW;
+  uint64_t* acc_empty = acc_full + 2;  // leader only
+  uint64_t* last_full = acc_empty + 2;  // the pair's last accumulator is complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(last_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * BM;  // first weight row
-  const int m0 = blockIdx.y * BN;  // first activation row
-  // this CTA's share of the K loop (split-K: an even share of the 64-element blocks)
-  const int kb_all = a.k / BK;
-  const int kb_begin = (int)((int64_t)kb_all * blockIdx.z / a.splits);
-  const int kblocks = (int)((int64_t)kb_all * (blockIdx.z + 1) / a.splits) - kb_begin;
+  const uint32_t rank = blockIdx.x & 1u;  // rank in the cluster of two
+  const int pair = (int)(blockIdx.x >> 1), pairs = (int)(gridDim.x >> 1);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < ST; s++) {
-      bar_init(&full[s], DQ_WARPS + 1);
-      bar_init(&empty[s], 1);
+    for (int s = 0; s < SA; s++) {
+      bar_init(&a_full[s], 2 * DQ_WARPS);
+      bar_init(&a_empty[s], 1);
     }
-    bar_init(accum, 1);
+    for (int s = 0; s < SB; s++) {
+      bar_init(&b_full[s], 1);
+      bar_init(&b_empty[s], 1);
+    }
+    for (int s = 0; s < RS; s++) {
+      bar_init(&raw_full[s], 1);
+      bar_init(&raw_empty[s], DQ_WARPS * DQ_GROUPS);
+    }
+    for (int s = 0; s < 2; s++) {
+      bar_init(&acc_full[s], 1);
+      bar_init(&acc_empty[s], 8);
+    }
+    bar_init(last_full, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_u32(tmem_slot)), "n"(TMEM_COLS)
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_u32(tmem_slot)), "n"(TMEM_COLS)
                  : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  cluster_sync_all();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
 
+  Segments seg;
+  seg.init(a, pair, pairs);
+  int t, ka, kb;
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer (activations)
+    // ------------------------------------------------------------ raw weight bytes -> ring
     if (lane == 0) {
-      // launched with programmatic stream serialization: the f16 operand comes from the
-      // conversion launch before this one (the weight side below starts without waiting)
-      asm volatile("griddepcontrol.wait;" ::: "memory");
-      for (int kb = 0; kb < kblocks; kb++) {
-        const int s = kb % ST;
-        const uint32_t ph = (uint32_t)(kb / ST) & 1u;
-        if (!bar_wait(&empty[s], ph ^ 1u, abort_flag)) break;
-        bar_expect_tx(&full[s], B_BYTES);
-        asm volatile(
-            "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                s_u32(sB + s * B_BYTES)),
-            "l"(&xmap), "r"((kb_begin + kb) * BK), "r"(m0), "r"(s_u32(&full[s]))
-            : "memory");
+      int slot = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      while (ok && seg.next(t, ka, kb)) {
+        const int rt0 = (t / a.mt) * 16 + (int)rank * 8;
+        int nlive = a.row_tiles - rt0;
+        nlive = nlive < 0 ? 0 : nlive > 8 ? 8 : nlive;
+        for (int ku = ka; ku < kb; ku++) {
+          ok = bar_wait(&raw_empty[slot], ph ^ 1u, abort_flag);
+          if (!ok) break;
+          int nt = a.ktiles - ku * UnitGeom<DT>::TILES;
+          if (nt > UnitGeom<DT>::TILES) nt = UnitGeom<DT>::TILES;
+          const uint32_t bytes = (uint32_t)(nt * TB);
+          bar_expect_tx(&raw_full[slot], bytes * (uint32_t)nlive);
+          const uint8_t* src = a.tiles + ((int64_t)rt0 * a.ktiles + (int64_t)ku * UnitGeom<DT>::TILES) * TB;
+          uint8_t* dst = sRaw + slot * SLOT_BYTES;
+          for (int r = 0; r < nlive; r++) {
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(s_u32(dst)),
+                         "l"(src), "r"(bytes), "r"(s_u32(&raw_full[slot]))
+                         : "memory");
+            src += (int64_t)a.ktiles * TB;
+            dst += UB;
+          }
+          if (++slot == RS) { slot = 0; ph ^= 1u; }
+        }
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
+    // ------------------------------------------------------------ TMA producer (activations)
     if (lane == 0) {
-      // instruction descriptor: f32 accumulate, f16 x f16, both K-major, N = BN, M = 128
-      constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-      // This one thread feeds the tensor core, so its own instruction count per stage is what
-      // separates consecutive stages' MMAs: descriptors are a constant high half plus a low
-      // half that advances by 2 (32 bytes >> 4) per 16-element K step, the stage index and
-      // phase are carried along, and one barrier covers both operands.
+      // Programmatic stream serialization: the f16 operand comes from the conversion launch before
+      // this one (the weight side starts without waiting). A sibling launch (the next weight of a
+      // call, same x) starts once every CTA of the GEMM before it has come past this point, so the
+      // operand is complete and everything older than the call has finished: it does not wait here
+      // and runs beside its predecessor; it waits before it ends (below), so that whoever waits for
+      // it has waited for all of the call.
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
+      if (!a.sibling) asm volatile("griddepcontrol.wait;" ::: "memory");
+      asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      while (ok && seg.next(t, ka, kb)) {
+        const int row = (t % a.mt) * a.bn + (int)rank * (a.bn >> 1);
+        const int k1 = kb * 4 < a.kblocks ? kb * 4 : a.kblocks;
+        for (int k = ka * 4; k < k1; k += KB) {
+          ok = bar_wait(&b_empty[s], ph ^ 1u, abort_flag);
+          if (!ok) break;
+          const int nk = k1 - k < KB ? k1 - k : KB;
+          if (rank == 0) bar_expect_tx(&b_full[s], 2u * (uint32_t)(nk * b_bytes));
+          for (int b = 0; b < nk; b++)
+            asm volatile(
+                "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                    s_u32(sB + (s * KB + b) * b_bytes)),
+                "l"(&xmap), "r"((k + b) * BK), "r"(row), "r"(map_to_rank(s_u32(&b_full[s]), 0))
+                : "memory");
+          if (++s == SB) { s = 0; ph ^= 1u; }
+        }
+      }
+    }
+  } else if (warp == 2) {
+    // ------------------------------------------------------------ MMA issuer
+    // The whole warp walks the loop and one elected lane issues: control flow and descriptors stay
+    // warp-uniform.
+    if (rank == 0) {
+      // instruction descriptor: f32 accumulate, f16 x f16, both K-major, N = bn, M = 256
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(a.bn >> 3) << 17) | ((uint32_t)(2 * BM >> 4) << 24);
+      // K-major, 128-byte swizzle matrix descriptors (8-row groups 1024 B apart): a constant high
+      // half plus a low half that advances by 2 (32 bytes >> 4) per 16-element K step
       constexpr uint64_t desc_hi = (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
       const uint32_t a_lo0 = (s_u32(sA) & 0x3FFFFu) >> 4, b_lo0 = (s_u32(sB) & 0x3FFFFu) >> 4;
+      const uint32_t b_step = (uint32_t)b_bytes >> 4;
       bool ok = true;
-      int s = 0;
-      uint32_t ph = 0, accumulate = 0;  // the first MMA of the tile overwrites the accumulator
-      for (int kb = 0; kb < kblocks; kb++) {
-        TC_TRACE(kb, 5);
-        ok = bar_wait(&full[s], ph, abort_flag);
+      int s = 0, sb = 0, nseg = 0;
+      uint32_t ph = 0, bph = 0;
+      while (ok && seg.next(t, ka, kb)) {
+        const int acc = nseg & 1;
+        const uint32_t aph = (uint32_t)(nseg >> 1) & 1u;
+        nseg++;
+        ok = bar_wait(&acc_empty[acc], aph ^ 1u, abort_flag);
+        ok = __all_sync(0xFFFFFFFFu, ok);
         if (!ok) break;
-        TC_TRACE(kb, 6);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint64_t da0 = desc_hi | (uint64_t)(a_lo0 + (uint32_t)s * (A_BYTES >> 4));
-        const uint64_t db0 = desc_hi | (uint64_t)(b_lo0 + (uint32_t)s * (B_BYTES >> 4));
+        const uint32_t d = tmem_base + (uint32_t)(acc * 256);
+        uint32_t accumulate = 0;  // the first MMA of the tile overwrites the accumulator
+        const int k1 = kb * 4 < a.kblocks ? kb * 4 : a.kblocks;
+        for (int k = ka * 4; k < k1 && ok; k += KA) {
+          const int nk = k1 - k < KA ? k1 - k : KA;
+          const uint64_t da0 = desc_hi | (uint64_t)(a_lo0 + (uint32_t)(s * KA) * (A_BYTES >> 4));
 #pragma unroll
-        for (int kk = 0; kk < BK / 16; kk++) {
-          asm volatile(
-              "{\n\t.reg .pred p;\n\t"
-              "setp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_base),
-              "l"(da0 + 2 * kk), "l"(db0 + 2 * kk), "r"(idesc), "r"(kk > 0 ? 1u : accumulate)
-              : "memory");
+          for (int b = 0; b < KA; b++) {
+            if (b < nk) {
+              if (b % KB == 0) {
+                ok = (b > 0 || bar_wait(&a_full[s], ph, abort_flag)) && bar_wait(&b_full[sb], bph, abort_flag);
+                ok = __all_sync(0xFFFFFFFFu, ok);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              }
+              const uint64_t db0 = desc_hi | (uint64_t)(b_lo0 + (uint32_t)(sb * KB + b % KB) * b_step);
+              if (elect_one()) {
+#pragma unroll
+                for (int kk = 0; kk < BK / 16; kk++) {
+                  asm volatile(
+                      "{\n\t.reg .pred p;\n\t"
+                      "setp.ne.b32 p, %4, 0;\n\t"
+                      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+                      "l"(da0 + (uint64_t)(b * (A_BYTES >> 4) + 2 * kk)), "l"(db0 + (uint64_t)(2 * kk)), "r"(idesc),
+                      "r"(b + kk > 0 ? 1u : accumulate)
+                      : "memory");
+                }
+                // release the stages to both CTAs' producers once these MMAs have read them
+                if (b % KB == KB - 1 || b == nk - 1) commit_to_pair(&b_empty[sb]);
+                if (b == nk - 1) commit_to_pair(&a_empty[s]);
+              }
+              __syncwarp();
+              if (b % KB == KB - 1 || b == nk - 1) {
+                if (++sb == SB) { sb = 0; bph ^= 1u; }
+              }
+            }
+          }
+          accumulate = 1u;
+          if (++s == SA) { s = 0; ph ^= 1u; }
         }
-        accumulate = 1u;
-        // release the stage to the producers once these MMAs have read it
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s_u32(&empty[s]))
-                     : "memory");
-        TC_TRACE(kb, 7);
-        if (++s == ST) { s = 0; ph ^= 1u; }
+        if (ok && elect_one()) commit_to_pair(seg.last() ? last_full : &acc_full[acc]);
+        __syncwarp();
       }
-      if (ok)
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s_u32(accum))
-                     : "memory");
+    }
+  } else if (warp < DQ_WARP0) {
+    // ------------------------------------------------------------ epilogue
+    if (!a.sibling) asm volatile("griddepcontrol.wait;" ::: "memory");  // y may still be read, the row scales still written
+    float* ybase = a.y;
+    if (a.y_toggle && ((*reinterpret_cast<const volatile unsigned*>(a.y_toggle) + 1u) & 1u)) ybase = a.y_alt;
+    const int quarter = warp & 3;
+    const uint32_t empty0 = map_to_rank(s_u32(&acc_empty[0]), 0);
+    int nseg = 0;
+    while (seg.next(t, ka, kb)) {
+      const int acc = nseg & 1;
+      const uint32_t aph = (uint32_t)(nseg >> 1) & 1u;
+      nseg++;
+      if (!(seg.last() ? bar_wait(last_full, 0, abort_flag) : bar_wait(&acc_full[acc], aph, abort_flag))) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // the last epilogue is shared with the dequantize warps, which have nothing left to do
+      epilogue<CH, SPLIT>(a, ybase, t, ka, kb, pair, pairs, (int)rank, quarter, lane, tmem_base + (uint32_t)(acc * 256), 0,
+                          seg.last() ? HELPERS : 1, abort_flag);
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) bar_arrive_cluster(empty0 + 8u * (uint32_t)acc);
     }
   } else {
-    // ------------------------------------------------------------ dequantize producers, then epilogue
-    const int dqw = warp - 2;           // 0..15
-    const int grp = dqw / DQ_WARPS;     // this warp's group takes stages kb = grp, grp + DQ_GROUPS, ...
-    const int dq = dqw % DQ_WARPS;      // row-tile of 16 rows inside the 128-row tile
-    const int64_t rt = (int64_t)(n0 >> 4) + dq;
-    const bool live = rt * TQ_TILE_ROWS < ((a.n_rows + 15) & ~(int64_t)15);
-    const uint8_t* tiles_rt = a.tiles + rt * a.ktiles * TB;
+    // ------------------------------------------------------------ dequantize
+    const int dqw = warp - DQ_WARP0;    // 0..15
+    const int grp = dqw / DQ_WARPS;     // this warp's group takes the blocks i = grp, grp + 2 of a unit
+    const int dq = dqw % DQ_WARPS;      // row-tile of 16 rows inside the CTA's 128 rows
+    const uint32_t a_full0 = map_to_rank(s_u32(&a_full[0]), 0);
+    int slot = 0, s = 0, nseg = 0;
+    uint32_t rph = 0, ph = 0;
     bool ok = true;
-    constexpr int PF = 4;  // stages of raw weight bytes kept in registers ahead of their use
-    StageRegs<DT> pre[PF];
-    // this warp's stages are kb = grp + DQ_GROUPS * t, t = 0, 1, ...
-    const int nmine = (kblocks - grp + DQ_GROUPS - 1) / DQ_GROUPS;
-    if (live) {
-#pragma unroll
-      for (int u = 0; u < PF - 1; u++)
-        if (u < nmine) stage_load<DT>(pre[u], tiles_rt, kb_begin + grp + DQ_GROUPS * u, lane);
-    }
-    for (int t0 = 0; t0 < nmine && ok; t0 += PF) {
-#pragma unroll
-      for (int u = 0; u < PF; u++) {
-        const int t = t0 + u;
-        if (t >= nmine) break;
-        const int kb = grp + DQ_GROUPS * t;
-        if (live && t + PF - 1 < nmine)
-          stage_load<DT>(pre[(u + PF - 1) % PF], tiles_rt, kb_begin + grp + DQ_GROUPS * (t + PF - 1), lane);
-        const int s = kb % ST;
-        const uint32_t ph = (uint32_t)(kb / ST) & 1u;
-        if (dq == 0 && lane == 0) TC_TRACE(kb, 0);
-        ok = bar_wait(&empty[s], ph ^ 1u, abort_flag);
+    int lt = 0, lka = 0, lkb = 0;  // the last segment
+    while (ok && seg.next(t, ka, kb)) {
+      lt = t; lka = ka; lkb = kb;
+      nseg++;
+      const bool live = (t / a.mt) * 16 + (int)rank * 8 + dq < a.row_tiles;  // rows beyond the weight are never stored
+      for (int ku = ka; ku < kb && ok; ku++) {
+        ok = bar_wait(&raw_full[slot], rph, abort_flag);
         if (!ok) break;
-        if (dq == 0 && lane == 0) TC_TRACE(kb, 1);
-        uint8_t* a_tile = sA + s * A_BYTES;
-        if (live) {
-          stage_dequant_store<DT>(pre[u], kb_begin + kb, lane, a_tile, 16 * dq);
-        } else {
-          // rows beyond the tensor: zeros
-          const int g = lane >> 2, c = lane & 3;
+        const uint8_t* raw = sRaw + slot * SLOT_BYTES + dq * UB;
+        int nb = a.kblocks - 4 * ku;
+        if (nb > 4) nb = 4;
+        nb -= KA * grp;  // this group makes the unit's blocks KA * grp, KA * grp + 1: one stage
+        if (nb > 0) {
+          const UnitScales us = unit_scales<DT>(raw, KA * grp + (lane & 1), lane);
+          int si = s + grp;
+          uint32_t phi = ph;
+          if (si >= SA) { si -= SA; phi ^= 1u; }
+          ok = bar_wait(&a_empty[si], phi ^ 1u, abort_flag);
+          if (!ok) break;
 #pragma unroll
-          for (int hr = 0; hr < 2; hr++)
-#pragma unroll
-            for (int h = 0; h < 2; h++)
-              *reinterpret_cast<uint4*>(a_tile + swz(16 * dq + g + 8 * hr, 4 * h + c)) = make_uint4(0, 0, 0, 0);
+          for (int b = 0; b < KA; b++)
+            if (live && b < nb) dequant_block<DT>(raw, us, KA * grp + b, b, lane, sA + (si * KA + b) * A_BYTES + dq * 16 * 128);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> visible to the MMA
+          __syncwarp();
+          if (lane == 0) bar_arrive_cluster(a_full0 + 8u * (uint32_t)si);
         }
-        if (dq == 0 && lane == 0) TC_TRACE(kb, 2);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> visible to the MMA
+        s += a.kblocks - 4 * ku > KA ? 2 : 1;
+        if (s >= SA) { s -= SA; ph ^= 1u; }
         __syncwarp();
-        if (dq == 0 && lane == 0) TC_TRACE(kb, 3);
-        if (lane == 0) bar_arrive(&full[s]);
-        if (dq == 0 && lane == 0) TC_TRACE(kb, 4);
+        if (lane == 0) bar_arrive(&raw_empty[slot]);
+        if (++slot == RS) { slot = 0; rph ^= 1u; }
       }
     }
-    // ---- epilogue: TMEM lanes 32*(warp%4).., columns split over the warps of each lane quarter
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the next launch may set up behind this one
-    asm volatile("griddepcontrol.wait;" ::: "memory");               // y / the partial sums may still be read by the predecessor
-    if (ok) ok = bar_wait(accum, 0, abort_flag);
-    if (ok) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int quarter = warp & 3;
-      constexpr int PARTS = BN >= 128 ? 4 : 2;       // column parts shared out over the warps of a lane quarter
-      const int col_part = dqw >> 2;                  // 0..3
-      const int64_t n = (int64_t)n0 + 32 * quarter + lane;
-      const float bv = (a.bias && a.splits == 1 && n < a.n_rows) ? a.bias[n] : 0.f;
+    // nothing left to dequantize: help with the epilogue of the last segment
+    if (ok && nseg > 0) {
+      if (!a.sibling) asm volatile("griddepcontrol.wait;" ::: "memory");
       float* ybase = a.y;
       if (a.y_toggle && ((*reinterpret_cast<const volatile unsigned*>(a.y_toggle) + 1u) & 1u)) ybase = a.y_alt;
-      float* const yout = ybase + (size_t)blockIdx.z * (size_t)a.m * (size_t)a.n_rows;
-#pragma unroll 1
-      for (int cb = 0; cb < BN / (32 * PARTS) && col_part < PARTS; cb++) {
-        const int col0 = (BN / PARTS) * col_part + 32 * cb;
-        uint32_t v[32];
-        const uint32_t taddr = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)col0;
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-            "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-              "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-              "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-              "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-            : "r"(taddr)
-            : "memory");
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (n < a.n_rows) {
-#pragma unroll
-          for (int j = 0; j < 32; j++) {
-            const int mrow = m0 + col0 + j;
-            if (mrow < a.m) yout[(int64_t)mrow * a.n_rows + n] = __uint_as_float(v[j]) * a.rscale[mrow] + bv;
-          }
-        }
+      const int acc = (nseg - 1) & 1;
+      if (bar_wait(last_full, 0, abort_flag)) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        epilogue<CH, SPLIT>(a, ybase, lt, lka, lkb, pair, pairs, (int)rank, warp & 3, lane, tmem_base + (uint32_t)(acc * 256),
+                            (warp - DQ_WARP0) / 4 + 1, HELPERS, abort_flag);
       }
     }
   }
+  __syncthreads();
+  if (*abort_flag) {
+    // a wait ran out: give copies still in flight time to land in this CTA's shared memory
+    for (int i = 0; i < 64; i++) __nanosleep(2000);
+    if (threadIdx.x == 0) {
+      *reinterpret_cast<volatile int*>(a.status) = 7;  // TURQ_E_TIMEOUT; the word may be mapped host memory
+      __threadfence_system();
+    }
+  }
+  // neither CTA leaves while the other may still arrive on its barriers or have its operands read
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 1) {
+  // (execution only: nothing but barriers and operand tiles is shared between the two)
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  if (warp == 2) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(TMEM_COLS) : "memory");
   }
-  if (threadIdx.x == 0 && *abort_flag) {
-    *reinterpret_cast<volatile int*>(a.status) = 7;  // TURQ_E_TIMEOUT; the word may be mapped host memory
-    __threadfence_system();
-  }
+  if (a.sibling && threadIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // x [m, k] (f32 / bf16) -> f16 [m, k] with a per-row power-of-two scale that brings the row's
 // largest magnitude into [8192, 16384): rows of large values do not overflow f16 and rows of
 // tiny values do not sink into its subnormals. rscale[m] undoes the scale exactly in the
 // epilogue. Rows that are all zero, or hold an infinity or NaN, are converted as they are.
-// One CTA per row.
-__global__ void __launch_bounds__(256) prep_act_kernel(const void* __restrict__ x, int is_bf16, int64_t k,
+// Every aligned group of four k keeps the order 0, 2, 1, 3 (pair02 / pair13 above). One CTA per row;
+// up to 4096 values stay in registers between the two passes. At 48 registers a thread a CTA fits
+// beside a CTA of the GEMM, so the conversion of the next call is resident before this call ends.
+__global__ void __launch_bounds__(256, 5) prep_act_kernel(const void* __restrict__ x, int is_bf16, int64_t k,
                                                         __half* __restrict__ xh, float* __restrict__ rscale) {
   __shared__ float wmax[8];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMM behind may start on its weights
   asm volatile("griddepcontrol.wait;" ::: "memory");               // x may still be written, the operand buffer still read
-  const int64_t row = blockIdx.x;
+  constexpr int KEEP = 2;
+  const int64_t row0 = (int64_t)blockIdx.x * k;
+  float v[KEEP][8];
   float amax = 0.f;
-  for (int64_t i = threadIdx.x; i < k; i += blockDim.x) amax = fmaxf(amax, fabsf(load_act_f32(x, is_bf16, row * k + i)));
+#pragma unroll
+  for (int j = 0; j < KEEP; j++) {
+    const int64_t i = ((int64_t)j * 256 + threadIdx.x) * 8;
+    if (i < k) {
+      load8(x, is_bf16, row0 + i, v[j]);
+#pragma unroll
+      for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(v[j][e]));
+    }
+  }
+#pragma unroll 2
+  for (int64_t i = ((int64_t)KEEP * 256 + threadIdx.x) * 8; i < k; i += 2048) {
+    float u[8];
+    load8(x, is_bf16, row0 + i, u);
+#pragma unroll
+    for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(u[e]));
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
   if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = amax;
@@ -501,38 +795,25 @@ __global__ void __launch_bounds__(256) prep_act_kernel(const void* __restrict__ 
     if (se > 126) se = 126;     // keep the scale and its reciprocal normal numbers
     s = ldexpf(1.f, se);
   }
-  if (threadIdx.x == 0) rscale[row] = 1.f / s;
-  for (int64_t i = threadIdx.x; i < k; i += blockDim.x)
-    xh[row * k + i] = __float2half_rn(load_act_f32(x, is_bf16, row * k + i) * s);
-}
-
-// y[i] = sum of the split-K partial sums (in split order) + bias
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ part, int splits, int64_t total,
-                                                             int64_t n_rows, const float* __restrict__ bias,
-                                                             float* __restrict__ y, const unsigned* y_toggle, float* y_alt) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (y_toggle && ((*reinterpret_cast<const volatile unsigned*>(y_toggle) + 1u) & 1u)) y = y_alt;
-  const int64_t i4 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-  if (i4 >= total) return;
-  if (i4 + 4 <= total && (n_rows & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
-    float4 acc = *reinterpret_cast<const float4*>(part + i4);
-    for (int z = 1; z < splits; z++) {
-      const float4 p = *reinterpret_cast<const float4*>(part + (size_t)z * total + i4);
-      acc.x += p.x; acc.y += p.y; acc.z += p.z; acc.w += p.w;
-    }
-    if (bias) {
-      const int64_t n = i4 % n_rows;
-      acc.x += bias[n]; acc.y += bias[n + 1]; acc.z += bias[n + 2]; acc.w += bias[n + 3];
-    }
-    *reinterpret_cast<float4*>(y + i4) = acc;
-  } else {
-    for (int64_t i = i4; i < total && i < i4 + 4; i++) {
-      float acc = part[i];
-      for (int z = 1; z < splits; z++) acc += part[(size_t)z * total + i];
-      if (bias) acc += bias[i % n_rows];
-      y[i] = acc;
-    }
+  if (threadIdx.x == 0) rscale[blockIdx.x] = 1.f / s;
+  auto store8 = [&](int64_t i, const float (&u)[8]) {
+    uint32_t o[4];
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) o[2 * h + e] = h22u(__floats2half2_rn(u[4 * h + e] * s, u[4 * h + e + 2] * s));
+    *reinterpret_cast<uint4*>(xh + row0 + i) = make_uint4(o[0], o[1], o[2], o[3]);
+  };
+#pragma unroll
+  for (int j = 0; j < KEEP; j++) {
+    const int64_t i = ((int64_t)j * 256 + threadIdx.x) * 8;
+    if (i < k) store8(i, v[j]);
+  }
+#pragma unroll 2
+  for (int64_t i = ((int64_t)KEEP * 256 + threadIdx.x) * 8; i < k; i += 2048) {
+    float u[8];
+    load8(x, is_bf16, row0 + i, u);
+    store8(i, u);
   }
 }
 
@@ -569,68 +850,83 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-template <int DT, int BN>
-cudaError_t launch_tc_bn(const CUtensorMap& map, const GemmArgs& a, cudaStream_t s) {
-  constexpr int ST = stages_for_bn(BN);
-  constexpr int SMEM = ST * (A_BYTES + BN * BK * 2) + (3 * ST + 1) * 8 + 16 + 1024;
+template <int DT, bool SPLIT>
+cudaError_t launch_tc_split(const CUtensorMap& map, GemmArgs a, int pairs, cudaStream_t s) {
+  constexpr int SLOT_BYTES = 8 * UnitGeom<DT>::BYTES;
+  constexpr int BAR_BYTES = (4 * MAX_ST + 2 * MAX_RAW + 5) * 8 + 8;
+  // Shared memory: three raw slots and weight stages (two where that leaves no room for four
+  // activation blocks in flight), the rest for activation stages and raw slots.
+  // (A dequantize warp only waits on the stages it fills itself. Behind a unit of one stage - an
+  // in-feature count that is no multiple of 256 - it is three stages on from its last wait; with two
+  // stages it could then wait two phases ahead of the barrier, which the parity does not tell apart.)
+  // 4 KB stay free for a CTA of the next call's conversion kernel.
+  const int budget = device_smem_optin() - 1024 - BAR_BYTES - 4096;
+  const int a_stage = KA * A_BYTES, b_stage = (SPLIT ? 2 : 1) * a.bn * BK;
+  int sa = 3, sb = SPLIT ? 3 : 4, rs = 3;
+  auto left = [&]() { return budget - sa * a_stage - sb * b_stage - rs * SLOT_BYTES; };
+  if (left() < 0 && a.kblocks % 4 == 0) sa = 2;
+  if (left() < 0) rs = 2;
+  if (left() < 0) sb = 3;
+  if (left() < 0) return cudaErrorInvalidConfiguration;
+  while (sb < MAX_ST && left() >= b_stage) sb++;
+  while (rs < MAX_RAW && left() >= SLOT_BYTES) rs++;
+  a.a_stages = sa;
+  a.b_stages = sb;
+  a.raw_slots = rs;
   static PerDeviceOnce configured;
   int dev = 0;
   cudaGetDevice(&dev);
   if (!configured.done(dev)) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<DT, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<DT, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, device_smem_optin());
     if (e != cudaSuccess) return e;
     configured.set(dev);
   }
-  dim3 grid((unsigned)((a.n_rows + BM - 1) / BM), (unsigned)((a.m + BN - 1) / BN), (unsigned)a.splits);
-  return launch_pdl(gemm_tc_kernel<DT, BN>, grid, dim3(TC_THREADS), (size_t)SMEM, s, map, a);
+  const size_t smem = (size_t)(sa * a_stage + sb * b_stage + rs * SLOT_BYTES) + BAR_BYTES + 1024;
+  return launch_pdl(gemm_tc_kernel<DT, SPLIT>, dim3((unsigned)(2 * pairs)), dim3(TC_THREADS), smem, s, map, a);
 }
 
 template <int DT>
-cudaError_t launch_tc_dt(const CUtensorMap& map, const GemmArgs& a, int bn, cudaStream_t s) {
-  return bn == 64 ? launch_tc_bn<DT, 64>(map, a, s) : bn == 128 ? launch_tc_bn<DT, 128>(map, a, s) : launch_tc_bn<DT, 256>(map, a, s);
+cudaError_t launch_tc_dt(const CUtensorMap& map, const GemmArgs& a, int pairs, cudaStream_t s) {
+  return a.split_k ? launch_tc_split<DT, true>(map, a, pairs, s) : launch_tc_split<DT, false>(map, a, pairs, s);
 }
 
 }  // namespace
 
-static int pick_bn(int64_t n_rows, int64_t m, int sm_count) {
-  static const int bn_env = tuning_env("TURQ_GEMM_BN", 0);
-  return plan_gemm_bn(n_rows, m, sm_count, bn_env);
+// Activation rows per pair tile for the height class of plan_gemm_bn: the rows dealt out evenly.
+static int tile_rows(int64_t m, int cls) {
+  const int64_t mt = (m + cls - 1) / cls;
+  return (int)(((m + mt - 1) / mt + 15) / 16 * 16);
 }
 
-static int pick_splits(int64_t n_rows, int64_t m, int64_t k, int sm_count) {
-  static const int env = tuning_env("TURQ_GEMM_SPLITK", -1);
-  return plan_gemm_splits(n_rows, m, k, sm_count, env);
+size_t gemm_tc_scratch_bytes(int64_t m, int64_t k) {
+  return (((size_t)m * (size_t)k * 2 + 255) & ~(size_t)255) + (((size_t)m * 4 + 255) & ~(size_t)255) + 256;
 }
 
-size_t gemm_tc_scratch_bytes(int64_t m, int64_t k, int64_t n_rows, int sm_count) {
-  const int splits = pick_splits(n_rows, m, k, sm_count);
-  const size_t part = splits > 1 ? (((size_t)splits * (size_t)m * (size_t)n_rows * 4 + 255) & ~(size_t)255) : 0;
-  return (((size_t)m * (size_t)k * 2 + 255) & ~(size_t)255) + (((size_t)m * 4 + 255) & ~(size_t)255) + 256 + part;
-}
+// Per sibling: partial sums of a 64-row decode batch [CTA][64][128] and the ready flags [CTA][4][8].
+static size_t ws_partial_bytes(int sms) { return (size_t)sms * 64 * BM * 4; }
+static size_t ws_flag_words(int sms) { return (size_t)sms * 4 * 8; }
+size_t gemm_tc_workspace_bytes(int sms) { return GEMM_SIBLINGS * (ws_partial_bytes(sms) + ws_flag_words(sms) * 4); }
 
 cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int64_t k, const void* x, int x_dtype,
-                           int64_t m, float* y, const float* bias, uint8_t* scratch, int sm_count, cudaStream_t s,
-                           int* launches, int* dev_status_word, bool x_prepared, const unsigned* y_toggle, float* y_alt) {
-  if (k % BK != 0 || m <= 0 || m > INT32_MAX || k > INT32_MAX) return cudaErrorInvalidValue;
+                           int64_t m, float* y, const float* bias, uint8_t* scratch, uint8_t* workspace, int sm_count, cudaStream_t s,
+                           int* launches, int* dev_status_word, int sibling, const unsigned* y_toggle, float* y_alt) {
+  if (k % BK != 0 || m <= 0 || m > INT32_MAX || k > INT32_MAX || sibling < 0 || sibling >= GEMM_SIBLINGS) return cudaErrorInvalidValue;
   EncodeTiledFn enc = encode_fn();
   if (!enc) return cudaErrorNotSupported;
   __half* xh = reinterpret_cast<__half*>(scratch);
   float* rscale = reinterpret_cast<float*>(scratch + (((size_t)m * (size_t)k * 2 + 255) & ~(size_t)255));
   cudaError_t e = cudaSuccess;
-  if (!x_prepared) {  // several weights that read the same x share one conversion
+  if (sibling == 0) {  // several weights that read the same x share one conversion
     e = launch_pdl(prep_act_kernel, dim3((unsigned)m), dim3(256), 0, s, x, (int)(x_dtype == TQ_BF16), k, xh, rscale);
     if (launches) (*launches)++;
     if (e != cudaSuccess) return e;
   }
 
+  const int bn = tile_rows(m, plan_gemm_bn(n_rows, m, sm_count));
   CUtensorMap map;
   const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
   const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-  const int bn = pick_bn(n_rows, m, sm_count);
-  const int splits = pick_splits(n_rows, m, k, sm_count);
-  float* partial = reinterpret_cast<float*>(scratch + (((size_t)m * (size_t)k * 2 + 255) & ~(size_t)255) +
-                                            (((size_t)m * 4 + 255) & ~(size_t)255) + 256);
-  const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)bn};
+  const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)bn / 2};
   const cuuint32_t estr[2] = {1, 1};
   CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, xh, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -639,34 +935,37 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
   GemmArgs a{};
   a.tiles = tiles;
   a.n_rows = n_rows;
+  a.row_tiles = (int)((n_rows + TQ_TILE_ROWS - 1) / TQ_TILE_ROWS);
   a.ktiles = (int)(k / tq_block_elems(dtype));
-  a.k = (int)k;
+  a.kblocks = (int)(k / BK);
+  a.KU = (int)((k + UNIT_K - 1) / UNIT_K);
   a.m = (int)m;
+  a.bn = bn;
+  a.mt = (int)((m + bn - 1) / bn);
+  const int64_t n_tiles = (n_rows + 2 * BM - 1) / (2 * BM);
+  const GemmWork work = plan_gemm_work(n_rows, m, k, a.mt, sm_count);
+  const int64_t total = n_tiles * (work.split_k ? a.KU : a.mt);
+  if (total > (int64_t)1 << 30) return cudaErrorInvalidValue;
+  a.total = (int)total;
+  a.split_k = work.split_k;
+  a.sibling = sibling > 0;
   a.rscale = rscale;
-  a.y = splits > 1 ? partial : y;
+  a.y = y;
   a.bias = bias;
+  a.partial = reinterpret_cast<float*>(workspace + sibling * ws_partial_bytes(sm_count));
+  a.flags = reinterpret_cast<int*>(workspace + GEMM_SIBLINGS * ws_partial_bytes(sm_count)) + sibling * ws_flag_words(sm_count);
   a.status = dev_status_word;
-  a.splits = splits;
-  a.y_toggle = splits > 1 ? nullptr : y_toggle;  // with split-K the reduction launch picks the buffer
+  a.y_toggle = y_toggle;
   a.y_alt = y_alt;
   switch (dtype) {
-    case TQ_Q8_0: e = launch_tc_dt<TQ_Q8_0>(map, a, bn, s); break;
-    case TQ_Q4_K: e = launch_tc_dt<TQ_Q4_K>(map, a, bn, s); break;
-    case TQ_Q5_K: e = launch_tc_dt<TQ_Q5_K>(map, a, bn, s); break;
-    case TQ_Q6_K: e = launch_tc_dt<TQ_Q6_K>(map, a, bn, s); break;
+    case TQ_Q8_0: e = launch_tc_dt<TQ_Q8_0>(map, a, work.pairs, s); break;
+    case TQ_Q4_K: e = launch_tc_dt<TQ_Q4_K>(map, a, work.pairs, s); break;
+    case TQ_Q5_K: e = launch_tc_dt<TQ_Q5_K>(map, a, work.pairs, s); break;
+    case TQ_Q6_K: e = launch_tc_dt<TQ_Q6_K>(map, a, work.pairs, s); break;
     default: return cudaErrorInvalidValue;
   }
-  if (launches) (*launches)++;
-  if (e != cudaSuccess || splits == 1) return e;
-  const int64_t total = m * n_rows;
-  e = launch_pdl(splitk_reduce_kernel, dim3((unsigned)((total + 1023) / 1024)), dim3(256), 0, s, (const float*)partial, splits,
-                 total, n_rows, bias, y, y_toggle, y_alt);
   if (launches) (*launches)++;
   return e;
 }
 
 }  // namespace turq
-
-#ifdef TURQ_TRACE
-extern "C" int turq_debug_read_gemm_trace(unsigned long long* host, int n) { return turq::read_gemm_trace(host, n); }
-#endif

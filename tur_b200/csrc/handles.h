@@ -25,6 +25,7 @@ struct turq_ctx {
   unsigned* done_count = nullptr;     // device memory: calls signalled so far
   unsigned done_expected = 0;         // host: calls launched so far
   uint8_t* gemv_ws = nullptr;  // split row-tile workspace of the streaming GEMV (zeroed once)
+  uint8_t* gemm_ws = nullptr;  // partial sums and ready flags of the tensor-core GEMM's split K loops (zeroed once)
   cudaStream_t own_stream = nullptr;
   int auto_policy = 0;  // what TURQ_MODE_AUTO resolves to: 0 = by row count, else a fixed turq_mode
   int64_t launches = 0;

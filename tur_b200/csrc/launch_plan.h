@@ -44,10 +44,10 @@ inline int64_t gemv_split_start(const GemvSplit& p, int64_t total_units, int b) 
   return u < total_units ? u : total_units;
 }
 
-// ---- tcgen05 GEMM (128 weight rows per CTA)
+// ---- tcgen05 GEMM (pairs of CTAs, 256 weight rows per pair)
 
-// Activation rows per CTA: 64 for decode batches; 256 for prefill, unless twice as many CTAs
-// still fit the SMs in one wave - then 128, which doubles the CTA count for the same work.
+// Class of the activation rows per pair tile: 64 for decode batches; 256 for prefill, unless twice
+// as many tiles still fit the SMs in one wave - then 128, which doubles the pairs at work.
 inline int plan_gemm_bn(int64_t n_rows, int64_t m, int sm_count, int force = 0) {
   if (force == 64 || force == 128 || force == 256) return force;
   int bn = m <= 64 ? 64 : 256;
@@ -55,20 +55,45 @@ inline int plan_gemm_bn(int64_t n_rows, int64_t m, int sm_count, int force = 0) 
   return bn;
 }
 
-// Split-K for decode batches (one 64-row activation tile): when the 128-row weight tiles alone
-// leave SMs without a CTA, the K loop of every tile is shared out over several CTAs (at least 8
-// blocks of 64 each, at most 16 CTAs). The split depends on the weight's shape only, so a row's
+// Split-K for decode batches (one activation tile of at most 64 rows): when the weight's row tiles
+// alone leave SMs without work, the K loop of every tile is shared out over several pairs (at least
+// 8 blocks of 64 each, at most 16 pairs). The split depends on the weight's shape only, so a row's
 // result does not depend on the batch it is in; prefill (more than 64 rows) never splits.
 // force: -1 = choose, 0 = never, > 0 = that many (still at least 8 blocks each).
 inline int plan_gemm_splits(int64_t n_rows, int64_t m, int64_t k, int sm_count, int force = -1) {
   if (m > 64 || force == 0) return 1;
-  const int64_t tiles = (n_rows + 127) / 128;
-  int64_t s = tiles > 0 ? sm_count / tiles : 1;
+  const int64_t tiles = (n_rows + 255) / 256;
+  int64_t s = tiles > 0 ? sm_count / 2 / tiles : 1;
   const int64_t by_k = (k / 64) / 8;
   if (force > 0) s = force;
   if (s > by_k) s = by_k;
   if (s > 16) s = 16;
   return s < 2 ? 1 : (int)s;
+}
+
+// Pairs of CTAs and what is dealt out to them: whole tiles (round robin), or - decode batches - the
+// units of 256 k of all tiles in one even split. With plan_gemm_splits() > 1 the pairs are a multiple
+// of the tiles, so every cut is the same in every tile; a weight with more tiles than half the pairs
+// is cut wherever the even split falls (at least two units per pair).
+struct GemmWork {
+  int pairs;
+  int split_k;
+};
+inline GemmWork plan_gemm_work(int64_t n_rows, int64_t m, int64_t k, int mt, int sm_count) {
+  const int64_t tiles = (n_rows + 255) / 256, slots = sm_count / 2 > 0 ? sm_count / 2 : 1;
+  GemmWork w{};
+  if (m > 64) {
+    w.pairs = (int)(tiles * mt < slots ? tiles * mt : slots);
+    return w;
+  }
+  const int splits = plan_gemm_splits(n_rows, m, k, sm_count);
+  const int64_t units = tiles * ((k + 255) / 256);
+  int64_t pairs = splits > 1 ? tiles * splits : slots;
+  if (splits == 1 && pairs > units / 2) pairs = units / 2;
+  if (splits == 1 && pairs < tiles && pairs < slots) pairs = tiles < slots ? tiles : slots;
+  w.pairs = pairs > 0 ? (int)pairs : 1;
+  w.split_k = 1;
+  return w;
 }
 
 }  // namespace turq
