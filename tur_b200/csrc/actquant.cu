@@ -147,11 +147,15 @@ static cudaError_t launch_act(int fmt, const void* x, int x_dtype, int64_t m, in
     int64_t warps = m * (k >> 8);
     int64_t blocks = (warps + 3) / 4;
     if (blocks > (int64_t)device_sm_count() * 16) blocks = (int64_t)device_sm_count() * 16;
+    cudaError_t e = prefer_matmul_carveout<quant_q8k_kernel>();
+    if (e != cudaSuccess) return e;
     return launch_pdl(quant_q8k_kernel, (unsigned)blocks, threads, s, x, is_bf16, m, k, out);
   } else if (fmt == TQ_Q8_0) {
     int64_t warps = m * (((k >> 5) + 7) >> 3);
     int64_t blocks = (warps + 3) / 4;
     if (blocks > (int64_t)device_sm_count() * 16) blocks = (int64_t)device_sm_count() * 16;
+    cudaError_t e = prefer_matmul_carveout<quant_q8_0_kernel>();
+    if (e != cudaSuccess) return e;
     return launch_pdl(quant_q8_0_kernel, (unsigned)blocks, threads, s, x, is_bf16, m, k, out);
   } else {
     return cudaErrorInvalidValue;

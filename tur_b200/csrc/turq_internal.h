@@ -36,6 +36,20 @@ struct PerDeviceOnce {
   void set(int dev) { if (dev >= 0 && dev < 64) mask.fetch_or(1ull << dev, std::memory_order_release); }
 };
 
+// Small kernels that run between the matmuls ask for the same shared-memory carve-out as those (the
+// largest): an SM changes its split only when it is empty, so a launch that wants another one cannot
+// become resident beside the tail of its predecessor.
+template <auto Kernel>
+inline cudaError_t prefer_matmul_carveout() {
+  static PerDeviceOnce configured;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (configured.done(dev)) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  if (e == cudaSuccess) configured.set(dev);
+  return e;
+}
+
 struct ActPackPlan {
   size_t off_qs, off_dsc, off_bs16, off_bs32, total;
 };
