@@ -523,7 +523,7 @@ def run_gpu(args):
                     "us_per_launch": dom_us, "launches": dom_launches, "algorithmic_flops": dom_flops, "traffic": None}
     else:
         roofline = {"bound": "hbm",
-                    "kernel": ("gemm_tc (+ activation prep, split-K reduction) " if tensor_path else "gemv_stream ") + members
+                    "kernel": ("gemm_tc (+ activation prep) " if tensor_path else "gemv_stream ") + members
                               + " as issued in the pass (one multi-weight launch where the path has one; activation "
                               "quantization included)",
                     "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,

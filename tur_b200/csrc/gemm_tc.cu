@@ -19,25 +19,29 @@
 //   * warps 3..6    epilogue: tcgen05.ld the accumulator, undo the row scale, add bias, store. The
 //                   accumulator is double buffered (2 x 256 TMEM columns), so the next tile's MMAs
 //                   run meanwhile;
-//   * warps 7..22   dequantize (two groups of eight on alternate 64-k blocks) from the raw ring to
-//                   f16 with packed half arithmetic, store in the K-major 128B-swizzled layout,
-//                   fence to the async proxy and arrive on the leader's barrier.
+//   * warps 7..22   dequantize (two groups of eight, each two 64-k blocks of a unit) from the raw ring
+//                   to f16 with packed half arithmetic and arrive on the leader's barrier. Prefill:
+//                   into shared memory, K-major 128B-swizzled. Decode batches: into TMEM (tcgen05.st),
+//                   where their few accumulator columns leave room for three units.
 // MMA roles: A = weights (rows = TMEM lanes), B = activations (columns).
 // Work: more than 64 rows: whole tiles, dealt out to persistent pairs. Decode batches (<= 64 rows,
 // one activation tile): the K loop of a tile is shared between pairs; the pair that holds a tile's
 // first unit adds the others' partial sums in pair order (fixed order, no float atomics).
 //
 // What bounds it. Prefill: the tensor pipe (81 % of active cycles at 12288 x 4096 Q4_K, 2048 rows), the
-// power limit and the last wave of tiles. Decode batches: issue slots - the dequantization costs about
-// 75 warp instructions per 1024 weights - and some 8 us of hand-overs (conversion, first activation
-// tile, partial sums). Why it is split this way, measured with graph replay, conversion included, against
-// one CTA per 128 rows with weights prefetched into registers and one ring for both operands:
-//   Q4_K 12288 x 4096, 2048 rows  231 -> 163 us (1267 TFLOP/s)   Q6_K 4096 x 12288, 512 rows  105 -> 75 us
-//   Q4_K 12288 x 4096, 64 rows   31.5 -> 24 us                   Q6_K 5120 x 25600, 64 rows   85 -> 57 us
-// Steps on the way: an MMA loop whose control flow is warp-uniform (210 -> 173 us at 2048 rows: with
-// one divergent thread the descriptors of every MMA went through moves to uniform registers), remote
-// arrivals without a cluster-scope release (270 -> 210 us; the proxy fence already orders the operand
-// tile), two 64-k blocks per weight stage (fewer fences and barrier rounds per dequantize warp).
+// power limit and the last wave of tiles. Decode batches: the rounds of barriers between the warps
+// (without any dequantization and a quarter of the MMAs the 25600 x 5120 launch below still takes 26 us)
+// and some 7 us of hand-overs (conversion, first activation tile, partial sums).
+// Measured with graph replay, conversion included, against one CTA per 128 rows with weights prefetched
+// into registers, one ring for both operands and split-K sums added by a second launch:
+//   Q4_K 12288 x 4096, 2048 rows  231 -> 157 us (1310 TFLOP/s)   Q6_K 5120 x 25600, 64 rows  85 -> 48 us
+//   Q5_K 2560 x 2560, 32 rows    10.1 -> 9.0 us
+// Steps on the way: an MMA loop whose control flow is warp-uniform (2048 rows: 210 -> 173 us; with one
+// divergent thread the descriptors of every MMA went through moves to uniform registers); remote arrivals
+// without a cluster-scope release (270 -> 210 us; the proxy fence already orders the operand tile); no
+// way out of that loop on an expired wait (Q4_K 25600 x 5120, 32 rows: 42 -> 37 us); the decode weight
+// operand in TMEM (37 -> 34 us: its stores and the MMA's reads were two thirds of the shared-memory
+// traffic); whole units per decode stage (34 -> 33 us, Q6_K 5120 x 25600 51 -> 48 us).
 // Every wait is bounded; on expiry the CTA records TURQ_E_TIMEOUT, releases its TMEM and returns.
 #include <cstdlib>
 #include <cuda.h>
@@ -60,7 +64,6 @@ constexpr int BK = 64;       // k per operand block (one 128-byte swizzle row of
 constexpr int UNIT_K = 256;  // k per unit of raw weight bytes (four blocks)
 constexpr int MAX_ST = 8;    // operand stages
 constexpr int MAX_RAW = 8;   // raw ring slots
-constexpr int KA = 2;                 // blocks per weight stage: what one dequantize warp makes of a unit
 constexpr int A_BYTES = BM * BK * 2;  // 16 KB per block
 constexpr int DQ_WARP0 = 7;        // first dequantize warp; warps 3..6 are the epilogue, one per TMEM lane quarter (warp & 3)
 constexpr int DQ_WARPS = 8;        // warps that together produce one stage of the weight operand
@@ -104,6 +107,15 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatil
   *abort_flag = 1;
   return false;
 }
+// The same for loops that do not look at the result: after an expiry the abort flag makes every further
+// wait return soon, and what such a loop then does stays within its buffers. Without the way out of
+// the loop its control flow is the same for the whole warp and its addresses stay in uniform registers.
+__device__ __noinline__ void bar_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  bar_wait(bar, parity, abort_flag);
+}
+__device__ __forceinline__ void bar_pass(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  if (!bar_try(bar, parity)) bar_wait_slow(bar, parity, abort_flag);
+}
 // The barriers of a pair's leader collect arrivals of both CTAs.
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank) {
   uint32_t r;
@@ -135,13 +147,14 @@ __device__ __forceinline__ void commit_to_pair(uint64_t* bar) {
 // of the tensor-core mode (the bit-exact f32 decode lives in decode.cuh).
 __device__ __forceinline__ __half2 u2h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 __device__ __forceinline__ uint32_t h22u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
-// The f16 operands keep the elements of every aligned group of four in the order 0, 2, 1, 3 (weights
-// here, activations in the conversion kernel): those are the pairs a word gives without a shuffle.
+// k order of both f16 operands: a 16-k chunk (one MMA) of an aligned 32 holds, for c = 0..3, elements
+// 8c + {0, 2, 1, 3} (first chunk) or 8c + 4 + {0, 2, 1, 3} (second) - what lane column c of a fragment
+// tile finds in one word, in the pairs the word gives without a shuffle. The same for prefill and decode
+// batches, so that a row's bits do not depend on which of the two it is in.
 // bytes (b0, b2) / (b1, b3) of a word of small integers -> half2 (1024 + b0, 1024 + b2) / ...
 __device__ __forceinline__ __half2 pair02(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5240)); }
 __device__ __forceinline__ __half2 pair13(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5341)); }
 __device__ __forceinline__ __half2 pair01(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5140)); }
-__device__ __forceinline__ __half2 pair23(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5342)); }
 
 // Raw bytes of one unit (16 weight rows x 256 k) as they lie in a ring slot.
 template <int DT> struct UnitGeom {
@@ -180,9 +193,13 @@ template <int DT>
 __device__ __forceinline__ void dequant_block(const uint8_t* t, const UnitScales& us, int i, int e, int lane, uint8_t* a_rows) {
   const int g = lane >> 2, c = lane & 3, odd = g & 1;
   uint8_t* const row = a_rows + g * 128;
+  const uint32_t o0 = (uint32_t)((((4 * odd) ^ (c >> 1) ^ g) << 4) + 8 * (c & 1));
+  auto store = [&](int hr, int h, const uint4& o) {  // the eight elements of sub-block h ^ odd
+    *reinterpret_cast<uint2*>(row + hr * 1024 + (o0 ^ (h << 6))) = make_uint2(o.x, o.y);
+    *reinterpret_cast<uint2*>(row + hr * 1024 + (o0 ^ (h << 6) ^ 32u)) = make_uint2(o.z, o.w);
+  };
   if constexpr (DT == TQ_Q8_0) {
     const __half2 off = __float2half2_rn(1152.f);  // 1024 + 128: bytes are biased by xor 0x80
-    const uint32_t o0 = (uint32_t)(((4 * odd + c) ^ g) << 4);
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       const uint8_t* tt = t + (2 * i + (h ^ odd)) * 544;
@@ -197,14 +214,13 @@ __device__ __forceinline__ void dequant_block(const uint8_t* t, const UnitScales
         o.y = h22u(__hmul2(__hsub2(pair13(w[hr][0]), off), d2));
         o.z = h22u(__hmul2(__hsub2(pair02(w[hr][1]), off), d2));
         o.w = h22u(__hmul2(__hsub2(pair13(w[hr][1]), off), d2));
-        *reinterpret_cast<uint4*>(row + hr * 1024 + (o0 ^ (h << 6))) = o;
+        store(hr, h, o);
       }
     }
   } else if constexpr (DT == TQ_Q4_K || DT == TQ_Q5_K) {
     constexpr int QS = DT == TQ_Q4_K ? TQ_Q4K_QS : TQ_Q5K_QS;
     const uint4 q = lds_v4(t + QS + 512 * i + 16 * lane);
     const uint32_t w[2][2] = {{q.x, q.y}, {q.z, q.w}};
-    const uint32_t o0 = (uint32_t)(((4 * odd + c) ^ g) << 4);
     uint32_t dl2[2], ml2[2];
 #pragma unroll
     for (int hr = 0; hr < 2; hr++) {
@@ -229,7 +245,7 @@ __device__ __forceinline__ void dequant_block(const uint8_t* t, const UnitScales
           o.y = h22u(__hfma2(__hsub2(u2h2(((w[hr][0] >> 8) & mask) | magic), off), dl, ml));
           o.z = h22u(__hfma2(__hsub2(u2h2((w[hr][1] & mask) | magic), off), dl, ml));
           o.w = h22u(__hfma2(__hsub2(u2h2(((w[hr][1] >> 8) & mask) | magic), off), dl, ml));
-          *reinterpret_cast<uint4*>(row + hr * 1024 + (o0 ^ (h << 6))) = o;
+          store(hr, h, o);
         }
       } else {
         const __half2 off = __float2half2_rn(1024.f);
@@ -246,43 +262,138 @@ __device__ __forceinline__ void dequant_block(const uint8_t* t, const UnitScales
           o.y = h22u(__hfma2(__hsub2(pair13(m0), off), dl, ml));
           o.z = h22u(__hfma2(__hsub2(pair02(m1), off), dl, ml));
           o.w = h22u(__hfma2(__hsub2(pair13(m1), off), dl, ml));
-          *reinterpret_cast<uint4*>(row + hr * 1024 + (o0 ^ (h << 6))) = o;
+          store(hr, h, o);
         }
       }
     }
-  } else {  // Q6_K: the block is sub-blocks 4i .. 4i+3 (16 elements each)
-    const uint4 ql = lds_v4(t + TQ_Q6K_QL + 512 * i + 16 * lane);
-    const uint4 q2 = lds_v4(t + TQ_Q6K_QH + 512 * (i >> 1) + 16 * lane);
-    const uint32_t db = lds_u16(t + TQ_Q6K_D + 2 * g) | (lds_u16(t + TQ_Q6K_D + 2 * (g + 8)) << 16);
-    const __half2 off = __float2half2_rn(1056.f);  // 1024 + 32
+  } else {  // Q6_K: a lane takes its eight elements of every 32 from the two lanes that hold them in the tile
+    const int nib = c >> 1, la = 4 * g + 2 * (c & 1);
+    const uint8_t* const qhp = t + TQ_Q6K_QH + 512 * (i >> 1) + 4 * (i & 1) + 16 * la;
+    const uint4 qa = lds_v4(t + TQ_Q6K_QL + 512 * i + 16 * la), qb = lds_v4(t + TQ_Q6K_QL + 512 * i + 16 * la + 16);
+    const __half2 off = __float2half2_rn(1056.f);     // 1024 + 32
     const __half2 off_sc = __float2half2_rn(1152.f);  // 1024 + 128: the int8 scales are biased by xor 0x80
-    const uint32_t o0 = (uint32_t)((((4 * odd) ^ (c >> 1) ^ g) << 4) + 8 * (c & 1));
 #pragma unroll
     for (int hr = 0; hr < 2; hr++) {
-      const uint32_t wa = hr ? ql.z : ql.x, wb = hr ? ql.w : ql.y;
-      const uint32_t qhw = (i & 1) ? (hr ? q2.w : q2.y) : (hr ? q2.z : q2.x);
-      // d * scale in half arithmetic (exact product, one rounding - as the f32 route gives)
-      const __half2 dd = u2h2(__byte_perm(db, 0u, hr ? 0x3232 : 0x1010));
+      const uint32_t qh[2] = {ld_u32(qhp + 8 * hr), ld_u32(qhp + 16 + 8 * hr)};
+      // d * scale of sub-blocks 4i + nib and 4i + 2 + nib in half arithmetic (exact product, one rounding)
+      const __half2 dd = __half2half2(__ushort_as_half((unsigned short)lds_u16(t + TQ_Q6K_D + 2 * (g + 8 * hr))));
       const uint32_t scb = ld_u32(t + 16 * (g + 8 * hr) + 4 * i) ^ 0x80808080u;
-      const __half2 dl01 = __hmul2(dd, __hsub2(pair01(scb), off_sc)), dl23 = __hmul2(dd, __hsub2(pair23(scb), off_sc));
-      // odd rows take sub-blocks 2, 3, 0, 1
-      const uint32_t w2[2] = {odd ? wb : wa, odd ? wa : wb};
-      const uint32_t dl2[2] = {h22u(odd ? dl23 : dl01), h22u(odd ? dl01 : dl23)};
-      const uint32_t qv = odd ? __funnelshift_l(qhw, qhw, 28) : qhw;  // fields 2, 3 down to 0, 1 (and 0, 1 up, bytes rotated)
-      const uint32_t qu = odd ? __funnelshift_l(qhw, qhw, 4) : qhw;   // fields 0, 1 up to 2, 3
+      const uint32_t dl2 = h22u(__hmul2(dd, __hsub2(pair02(scb >> (8 * nib)), off_sc)));
 #pragma unroll
-      for (int jj = 0; jj < 4; jj++) {
-        const int nib = jj & 1, sh = 2 * jj;
-        const __half2 dl = u2h2(__byte_perm(dl2[jj >> 1], 0u, nib ? 0x3232 : 0x1010));
-        uint32_t m = (nib ? (w2[jj >> 1] >> 4) : w2[jj >> 1]) & 0x0F0F0F0Fu;
-        m |= (sh <= 4 ? ((jj < 2 ? qv : qu) << (4 - sh)) : (qu >> (sh - 4))) & 0x30303030u;
-        uint2 o;
-        o.x = h22u(__hmul2(__hsub2(pair02(m), off), dl));
-        o.y = h22u(__hmul2(__hsub2(pair13(m), off), dl));
-        *reinterpret_cast<uint2*>(row + hr * 1024 + (o0 ^ (jj << 5))) = o;
+      for (int h = 0; h < 2; h++) {
+        const int s = h ^ odd;
+        const __half2 dl = u2h2(__byte_perm(dl2, 0u, s ? 0x3232u : 0x1010u));
+        const uint32_t qlw[2] = {s ? (hr ? qa.w : qa.y) : (hr ? qa.z : qa.x), s ? (hr ? qb.w : qb.y) : (hr ? qb.z : qb.x)};
+        const int rot = 4 - 4 * s - 2 * nib;  // brings 2-bit field 2s + nib of the qh word to bits 4..5 of every byte
+        const uint32_t m0 = ((qlw[0] >> (4 * nib)) & 0x0F0F0F0Fu) | (__funnelshift_l(qh[0], qh[0], rot) & 0x30303030u);
+        const uint32_t m1 = ((qlw[1] >> (4 * nib)) & 0x0F0F0F0Fu) | (__funnelshift_l(qh[1], qh[1], rot) & 0x30303030u);
+        uint4 o;
+        o.x = h22u(__hmul2(__hsub2(pair02(m0), off), dl));
+        o.y = h22u(__hmul2(__hsub2(pair13(m0), off), dl));
+        o.z = h22u(__hmul2(__hsub2(pair02(m1), off), dl));
+        o.w = h22u(__hmul2(__hsub2(pair13(m1), off), dl));
+        store(hr, h, o);
       }
     }
   }
+}
+
+// The same 64-k block as registers of a tcgen05.st 16x256b.x4 (decode batches keep the weight operand in
+// TMEM): register 4j + 2h + e of lane 4g + c holds columns 8j + 2c + e of row g + 8h, two f16 each, so
+// chunk j (16 k, one MMA) has from this lane the elements 32 (j / 2) + 8c + 4 (j % 2) + {0, 2, 1, 3}.
+template <int DT>
+__device__ __forceinline__ void dequant_frag(const uint8_t* t, const UnitScales& us, int i, int e, int lane, uint32_t (&o)[16]) {
+  const int g = lane >> 2, c = lane & 3;
+  if constexpr (DT == TQ_Q8_0) {
+    const __half2 off = __float2half2_rn(1152.f);  // 1024 + 128: bytes are biased by xor 0x80
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+      const uint8_t* tt = t + (2 * i + s) * 544;
+      const uint4 q = lds_v4(tt + TQ_Q8_0_QS + 16 * lane);
+      const uint32_t w[2][2] = {{q.x ^ 0x80808080u, q.y ^ 0x80808080u}, {q.z ^ 0x80808080u, q.w ^ 0x80808080u}};
+#pragma unroll
+      for (int hr = 0; hr < 2; hr++) {
+        const __half2 d2 = __half2half2(__ushort_as_half((unsigned short)lds_u16(tt + 2 * (g + 8 * hr))));
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+          o[4 * (2 * s + b) + 2 * hr] = h22u(__hmul2(__hsub2(pair02(w[hr][b]), off), d2));
+          o[4 * (2 * s + b) + 2 * hr + 1] = h22u(__hmul2(__hsub2(pair13(w[hr][b]), off), d2));
+        }
+      }
+    }
+  } else if constexpr (DT == TQ_Q4_K || DT == TQ_Q5_K) {
+    constexpr int QS = DT == TQ_Q4_K ? TQ_Q4K_QS : TQ_Q5K_QS;
+    const uint4 q = lds_v4(t + QS + 512 * i + 16 * lane);
+    const uint32_t w[2][2] = {{q.x, q.y}, {q.z, q.w}};
+    uint32_t qh[2][2] = {{0, 0}, {0, 0}};
+    if constexpr (DT == TQ_Q5_K) {
+      const uint4 h4 = lds_v4(t + TQ_Q5K_QH + 16 * lane);
+      qh[0][0] = h4.x; qh[0][1] = h4.y; qh[1][0] = h4.z; qh[1][1] = h4.w;
+    }
+#pragma unroll
+    for (int hr = 0; hr < 2; hr++) {
+      const int src = 2 * (g + 8 * hr) + e;
+      const __half2 dl2 = u2h2(__shfl_sync(0xFFFFFFFFu, us.dl, src)), ml2 = u2h2(__shfl_sync(0xFFFFFFFFu, us.ml, src));
+#pragma unroll
+      for (int s = 0; s < 2; s++) {  // sub-blocks 2i (low nibbles) and 2i + 1 (high nibbles)
+        const __half2 dl = s ? __high2half2(dl2) : __low2half2(dl2), ml = s ? __high2half2(ml2) : __low2half2(ml2);
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+          __half2 v02, v13;
+          if constexpr (DT == TQ_Q4_K) {
+            // A nibble becomes a half without being moved: under the exponent of 1024 the low nibble counts
+            // ones, under that of 64 the high nibble (16 units of 1/16) does; the offset subtracts exactly.
+            const uint32_t mask = s ? 0x00F000F0u : 0x000F000Fu, magic = s ? 0x54005400u : 0x64006400u;
+            v02 = __hsub2(u2h2((w[hr][b] & mask) | magic), u2h2(magic));
+            v13 = __hsub2(u2h2(((w[hr][b] >> 8) & mask) | magic), u2h2(magic));
+          } else {
+            const __half2 off = __float2half2_rn(1024.f);
+            // the sub-block's bit, brought to bit 4 of every byte
+            const uint32_t m = ((w[hr][b] >> (4 * s)) & 0x0F0F0F0Fu) |
+                               (__funnelshift_l(qh[hr][b], qh[hr][b], 4 - (2 * i + s)) & 0x10101010u);
+            v02 = __hsub2(pair02(m), off);
+            v13 = __hsub2(pair13(m), off);
+          }
+          o[4 * (2 * s + b) + 2 * hr] = h22u(__hfma2(v02, dl, ml));
+          o[4 * (2 * s + b) + 2 * hr + 1] = h22u(__hfma2(v13, dl, ml));
+        }
+      }
+    }
+  } else {  // Q6_K: a lane takes its eight elements of every 32 from the two lanes that hold them in the tile
+    const int nib = c >> 1, la = 4 * g + 2 * (c & 1);
+    const uint8_t* const qhp = t + TQ_Q6K_QH + 512 * (i >> 1) + 4 * (i & 1) + 16 * la;
+    const uint4 qa = lds_v4(t + TQ_Q6K_QL + 512 * i + 16 * la), qb = lds_v4(t + TQ_Q6K_QL + 512 * i + 16 * la + 16);
+    const __half2 off = __float2half2_rn(1056.f);     // 1024 + 32
+    const __half2 off_sc = __float2half2_rn(1152.f);  // 1024 + 128: the int8 scales are biased by xor 0x80
+#pragma unroll
+    for (int hr = 0; hr < 2; hr++) {
+      const uint32_t ql[2][2] = {{hr ? qa.z : qa.x, hr ? qb.z : qb.x}, {hr ? qa.w : qa.y, hr ? qb.w : qb.y}};
+      const uint32_t qh[2] = {ld_u32(qhp + 8 * hr), ld_u32(qhp + 16 + 8 * hr)};
+      // d * scale of sub-blocks 4i + nib and 4i + 2 + nib in half arithmetic (exact product, one rounding)
+      const __half2 dd = __half2half2(__ushort_as_half((unsigned short)lds_u16(t + TQ_Q6K_D + 2 * (g + 8 * hr))));
+      const uint32_t scb = ld_u32(t + 16 * (g + 8 * hr) + 4 * i) ^ 0x80808080u;
+      const __half2 dl2 = __hmul2(dd, __hsub2(pair02(scb >> (8 * nib)), off_sc));
+#pragma unroll
+      for (int s = 0; s < 2; s++) {
+        const __half2 dl = s ? __high2half2(dl2) : __low2half2(dl2);
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+          // 2-bit field 2s + nib of the qh word, brought to bits 4..5 of every byte
+          const uint32_t m = ((ql[s][b] >> (4 * nib)) & 0x0F0F0F0Fu) |
+                             (__funnelshift_l(qh[b], qh[b], 4 - 4 * s - 2 * nib) & 0x30303030u);
+          o[4 * (2 * s + b) + 2 * hr] = h22u(__hmul2(__hsub2(pair02(m), off), dl));
+          o[4 * (2 * s + b) + 2 * hr + 1] = h22u(__hmul2(__hsub2(pair13(m), off), dl));
+        }
+      }
+    }
+  }
+}
+__device__ __forceinline__ void tmem_store_block(uint32_t taddr, const uint32_t (&o)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+      "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(o[8]), "r"(o[9]), "r"(o[10]),
+      "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]), "r"(o[15])
+      : "memory");
 }
 
 struct GemmArgs {
@@ -455,7 +566,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
   constexpr int TB = TileGeom<DT>::BYTES;
   constexpr int UB = UnitGeom<DT>::BYTES;
   constexpr int SLOT_BYTES = 8 * UB;
-  constexpr int KB = SPLIT ? 2 : 1;  // 64-k blocks per activation stage
+  // 64-k blocks per stage of the weight and of the activation operand. Decode batches: a whole unit, since
+  // with few activation rows it is the barrier rounds of the MMA loop that separate the MMAs.
+  constexpr int KA = SPLIT ? 4 : 2, KB = SPLIT ? 4 : 1;
+  // Decode batches (SPLIT) need few accumulator columns: their weight operand lies in the rest of TMEM,
+  // 32 columns per 64-k block, instead of in shared memory.
+  constexpr int ACC_COLS = SPLIT ? 64 : 256;
+  constexpr int A_COL0 = 2 * ACC_COLS;
+  constexpr int A_COLS = 32;  // per block
   constexpr int CH = SPLIT ? 8 : 16;  // columns per epilogue step
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // 1024-byte alignment for the swizzled tiles; the same offsets in both CTAs of the pair
@@ -463,7 +581,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
   const int SA = a.a_stages, SB = a.b_stages, RS = a.raw_slots;
   const int b_bytes = a.bn * (BK * 2 / 2);  // this CTA's half of the activation tile, per block
   uint8_t* sA = smem;
-  uint8_t* sB = sA + SA * KA * A_BYTES;
+  uint8_t* sB = sA + (SPLIT ? 0 : SA * KA * A_BYTES);
   uint8_t* sRaw = sB + SB * KB * b_bytes;
   // The two operands have rings of their own: an activation tile is a trip to L2 away and needs many
   // stages in flight, a weight tile comes from this SM's raw ring and needs few.
@@ -487,7 +605,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < SA; s++) {
-      bar_init(&a_full[s], 2 * DQ_WARPS);
+      bar_init(&a_full[s], (SPLIT ? 2 : 1) * 2 * DQ_WARPS);
       bar_init(&a_empty[s], 1);
     }
     for (int s = 0; s < SB; s++) {
@@ -522,32 +640,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
   int t, ka, kb;
   if (warp == 0) {
     // ------------------------------------------------------------ raw weight bytes -> ring
-    if (lane == 0) {
-      int slot = 0;
-      uint32_t ph = 0;
-      bool ok = true;
-      while (ok && seg.next(t, ka, kb)) {
-        const int rt0 = (t / a.mt) * 16 + (int)rank * 8;
-        int nlive = a.row_tiles - rt0;
-        nlive = nlive < 0 ? 0 : nlive > 8 ? 8 : nlive;
-        for (int ku = ka; ku < kb; ku++) {
-          ok = bar_wait(&raw_empty[slot], ph ^ 1u, abort_flag);
-          if (!ok) break;
-          int nt = a.ktiles - ku * UnitGeom<DT>::TILES;
-          if (nt > UnitGeom<DT>::TILES) nt = UnitGeom<DT>::TILES;
-          const uint32_t bytes = (uint32_t)(nt * TB);
-          bar_expect_tx(&raw_full[slot], bytes * (uint32_t)nlive);
-          const uint8_t* src = a.tiles + ((int64_t)rt0 * a.ktiles + (int64_t)ku * UnitGeom<DT>::TILES) * TB;
-          uint8_t* dst = sRaw + slot * SLOT_BYTES;
-          for (int r = 0; r < nlive; r++) {
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(s_u32(dst)),
-                         "l"(src), "r"(bytes), "r"(s_u32(&raw_full[slot]))
-                         : "memory");
-            src += (int64_t)a.ktiles * TB;
-            dst += UB;
-          }
-          if (++slot == RS) { slot = 0; ph ^= 1u; }
-        }
+    // Lane r < 8 copies row-tile r's share of the unit: issued by one lane, the eight copies of a unit
+    // took 600 ns one after the other, half of what the unit lasts.
+    int slot = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    while (ok && seg.next(t, ka, kb)) {
+      const int rt0 = (t / a.mt) * 16 + (int)rank * 8;
+      int nlive = a.row_tiles - rt0;
+      nlive = nlive < 0 ? 0 : nlive > 8 ? 8 : nlive;
+      const uint8_t* const row = a.tiles + (int64_t)(rt0 + lane) * a.ktiles * TB;
+      for (int ku = ka; ku < kb; ku++) {
+        ok = __all_sync(0xFFFFFFFFu, bar_wait(&raw_empty[slot], ph ^ 1u, abort_flag));
+        if (!ok) break;
+        int nt = a.ktiles - ku * UnitGeom<DT>::TILES;
+        if (nt > UnitGeom<DT>::TILES) nt = UnitGeom<DT>::TILES;
+        const uint32_t bytes = (uint32_t)(nt * TB);
+        if (lane == 0) bar_expect_tx(&raw_full[slot], bytes * (uint32_t)nlive);
+        __syncwarp();
+        if (lane < nlive)
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                           s_u32(sRaw + slot * SLOT_BYTES + lane * UB)),
+                       "l"(row + (int64_t)ku * UB), "r"(bytes), "r"(s_u32(&raw_full[slot]))
+                       : "memory");
+        if (++slot == RS) { slot = 0; ph ^= 1u; }
       }
     }
   } else if (warp == 1) {
@@ -586,7 +702,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
   } else if (warp == 2) {
     // ------------------------------------------------------------ MMA issuer
     // The whole warp walks the loop and one elected lane issues: control flow and descriptors stay
-    // warp-uniform.
+    // warp-uniform. This loop's own instructions are what separates the MMAs of consecutive stages when
+    // there are few activation rows.
     if (rank == 0) {
       // instruction descriptor: f32 accumulate, f16 x f16, both K-major, N = bn, M = 256
       const uint32_t idesc = (1u << 4) | ((uint32_t)(a.bn >> 3) << 17) | ((uint32_t)(2 * BM >> 4) << 24);
@@ -595,50 +712,56 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
       constexpr uint64_t desc_hi = (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
       const uint32_t a_lo0 = (s_u32(sA) & 0x3FFFFu) >> 4, b_lo0 = (s_u32(sB) & 0x3FFFFu) >> 4;
       const uint32_t b_step = (uint32_t)b_bytes >> 4;
-      bool ok = true;
+      const bool issuer = elect_one();
       int s = 0, sb = 0, nseg = 0;
       uint32_t ph = 0, bph = 0;
-      while (ok && seg.next(t, ka, kb)) {
+      while (seg.next(t, ka, kb)) {
         const int acc = nseg & 1;
         const uint32_t aph = (uint32_t)(nseg >> 1) & 1u;
         nseg++;
-        ok = bar_wait(&acc_empty[acc], aph ^ 1u, abort_flag);
-        ok = __all_sync(0xFFFFFFFFu, ok);
-        if (!ok) break;
+        bar_pass(&acc_empty[acc], aph ^ 1u, abort_flag);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t d = tmem_base + (uint32_t)(acc * 256);
+        const uint32_t d = tmem_base + (uint32_t)(acc * ACC_COLS);
         uint32_t accumulate = 0;  // the first MMA of the tile overwrites the accumulator
         const int k1 = kb * 4 < a.kblocks ? kb * 4 : a.kblocks;
-        for (int k = ka * 4; k < k1 && ok; k += KA) {
-          const int nk = k1 - k < KA ? k1 - k : KA;
+        for (int k = ka * 4; k < k1; k += KA) {
           const uint64_t da0 = desc_hi | (uint64_t)(a_lo0 + (uint32_t)(s * KA) * (A_BYTES >> 4));
+          bar_pass(&a_full[s], ph, abort_flag);
 #pragma unroll
           for (int b = 0; b < KA; b++) {
-            if (b < nk) {
+            if (b == 0 || k + b < k1) {
+              const bool last = b == KA - 1 || k + b + 1 >= k1;
               if (b % KB == 0) {
-                ok = (b > 0 || bar_wait(&a_full[s], ph, abort_flag)) && bar_wait(&b_full[sb], bph, abort_flag);
-                ok = __all_sync(0xFFFFFFFFu, ok);
-                if (!ok) break;
+                bar_pass(&b_full[sb], bph, abort_flag);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
               }
               const uint64_t db0 = desc_hi | (uint64_t)(b_lo0 + (uint32_t)(sb * KB + b % KB) * b_step);
-              if (elect_one()) {
+              if (issuer) {
 #pragma unroll
                 for (int kk = 0; kk < BK / 16; kk++) {
-                  asm volatile(
-                      "{\n\t.reg .pred p;\n\t"
-                      "setp.ne.b32 p, %4, 0;\n\t"
-                      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-                      "l"(da0 + (uint64_t)(b * (A_BYTES >> 4) + 2 * kk)), "l"(db0 + (uint64_t)(2 * kk)), "r"(idesc),
-                      "r"(b + kk > 0 ? 1u : accumulate)
-                      : "memory");
+                  if constexpr (SPLIT) {  // weight operand in TMEM
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\t"
+                        "setp.ne.b32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+                        "r"(tmem_base + (uint32_t)(A_COL0 + (s * KA + b) * A_COLS + 8 * kk)), "l"(db0 + (uint64_t)(2 * kk)), "r"(idesc),
+                        "r"(b + kk > 0 ? 1u : accumulate)
+                        : "memory");
+                  } else {
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\t"
+                        "setp.ne.b32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+                        "l"(da0 + (uint64_t)(b * (A_BYTES >> 4) + 2 * kk)), "l"(db0 + (uint64_t)(2 * kk)), "r"(idesc),
+                        "r"(b + kk > 0 ? 1u : accumulate)
+                        : "memory");
+                  }
                 }
                 // release the stages to both CTAs' producers once these MMAs have read them
-                if (b % KB == KB - 1 || b == nk - 1) commit_to_pair(&b_empty[sb]);
-                if (b == nk - 1) commit_to_pair(&a_empty[s]);
+                if (KB == 1 || last) commit_to_pair(&b_empty[sb]);
+                if (last) commit_to_pair(&a_empty[s]);
               }
-              __syncwarp();
-              if (b % KB == KB - 1 || b == nk - 1) {
+              if (KB == 1 || last) {
                 if (++sb == SB) { sb = 0; bph ^= 1u; }
               }
             }
@@ -646,9 +769,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
           accumulate = 1u;
           if (++s == SA) { s = 0; ph ^= 1u; }
         }
-        if (ok && elect_one()) commit_to_pair(seg.last() ? last_full : &acc_full[acc]);
-        __syncwarp();
+        if (issuer) commit_to_pair(seg.last() ? last_full : &acc_full[acc]);
       }
+      __syncwarp();
     }
   } else if (warp < DQ_WARP0) {
     // ------------------------------------------------------------ epilogue
@@ -665,7 +788,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
       if (!(seg.last() ? bar_wait(last_full, 0, abort_flag) : bar_wait(&acc_full[acc], aph, abort_flag))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // the last epilogue is shared with the dequantize warps, which have nothing left to do
-      epilogue<CH, SPLIT>(a, ybase, t, ka, kb, pair, pairs, (int)rank, quarter, lane, tmem_base + (uint32_t)(acc * 256), 0,
+      epilogue<CH, SPLIT>(a, ybase, t, ka, kb, pair, pairs, (int)rank, quarter, lane, tmem_base + (uint32_t)(acc * ACC_COLS), 0,
                           seg.last() ? HELPERS : 1, abort_flag);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -673,40 +796,52 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
     }
   } else {
     // ------------------------------------------------------------ dequantize
-    const int dqw = warp - DQ_WARP0;    // 0..15
-    const int grp = dqw / DQ_WARPS;     // this warp's group takes the blocks i = grp, grp + 2 of a unit
-    const int dq = dqw % DQ_WARPS;      // row-tile of 16 rows inside the CTA's 128 rows
+    // A warp reaches one quarter of TMEM's lanes (warp & 3), 32 rows: two of the four warps of a quarter
+    // take one 16-row tile each for one group, two for the other. A group makes blocks 2 grp, 2 grp + 1.
+    const int dqw = (warp - DQ_WARP0) >> 2;  // 0..3 within the quarter
+    const int grp = dqw >> 1;
+    const int dq = 2 * (warp & 3) + (dqw & 1);  // row-tile of 16 rows inside the CTA's 128 rows
     const uint32_t a_full0 = map_to_rank(s_u32(&a_full[0]), 0);
     int slot = 0, s = 0, nseg = 0;
     uint32_t rph = 0, ph = 0;
-    bool ok = true;
     int lt = 0, lka = 0, lkb = 0;  // the last segment
-    while (ok && seg.next(t, ka, kb)) {
+    while (seg.next(t, ka, kb)) {
       lt = t; lka = ka; lkb = kb;
       nseg++;
       const bool live = (t / a.mt) * 16 + (int)rank * 8 + dq < a.row_tiles;  // rows beyond the weight are never stored
-      for (int ku = ka; ku < kb && ok; ku++) {
-        ok = bar_wait(&raw_full[slot], rph, abort_flag);
-        if (!ok) break;
+      for (int ku = ka; ku < kb; ku++) {
+        bar_pass(&raw_full[slot], rph, abort_flag);
         const uint8_t* raw = sRaw + slot * SLOT_BYTES + dq * UB;
         int nb = a.kblocks - 4 * ku;
         if (nb > 4) nb = 4;
-        nb -= KA * grp;  // this group makes the unit's blocks KA * grp, KA * grp + 1: one stage
-        if (nb > 0) {
-          const UnitScales us = unit_scales<DT>(raw, KA * grp + (lane & 1), lane);
-          int si = s + grp;
+        nb -= 2 * grp;  // this group makes the unit's blocks 2 grp, 2 grp + 1
+        if (SPLIT || nb > 0) {
+          const UnitScales us = unit_scales<DT>(raw, 2 * grp + (lane & 1), lane);
+          int si = SPLIT ? s : s + grp;
           uint32_t phi = ph;
           if (si >= SA) { si -= SA; phi ^= 1u; }
-          ok = bar_wait(&a_empty[si], phi ^ 1u, abort_flag);
-          if (!ok) break;
+          bar_pass(&a_empty[si], phi ^ 1u, abort_flag);
+          if constexpr (SPLIT) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-          for (int b = 0; b < KA; b++)
-            if (live && b < nb) dequant_block<DT>(raw, us, KA * grp + b, b, lane, sA + (si * KA + b) * A_BYTES + dq * 16 * 128);
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> visible to the MMA
+            for (int b = 0; b < 2; b++)
+              if (live && b < nb) {
+                uint32_t o[16];
+                dequant_frag<DT>(raw, us, 2 * grp + b, b, lane, o);
+                tmem_store_block(tmem_base + ((uint32_t)(16 * dq) << 16) + (uint32_t)(A_COL0 + (si * KA + 2 * grp + b) * A_COLS), o);
+              }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          } else {
+#pragma unroll
+            for (int b = 0; b < 2; b++)
+              if (live && b < nb) dequant_block<DT>(raw, us, 2 * grp + b, b, lane, sA + (si * KA + b) * A_BYTES + dq * 16 * 128);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> visible to the MMA
+          }
           __syncwarp();
           if (lane == 0) bar_arrive_cluster(a_full0 + 8u * (uint32_t)si);
         }
-        s += a.kblocks - 4 * ku > KA ? 2 : 1;
+        s += !SPLIT && a.kblocks - 4 * ku > KA ? 2 : 1;
         if (s >= SA) { s -= SA; ph ^= 1u; }
         __syncwarp();
         if (lane == 0) bar_arrive(&raw_empty[slot]);
@@ -714,14 +849,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
       }
     }
     // nothing left to dequantize: help with the epilogue of the last segment
-    if (ok && nseg > 0) {
+    if (nseg > 0) {
       if (!a.sibling) asm volatile("griddepcontrol.wait;" ::: "memory");
       float* ybase = a.y;
       if (a.y_toggle && ((*reinterpret_cast<const volatile unsigned*>(a.y_toggle) + 1u) & 1u)) ybase = a.y_alt;
       const int acc = (nseg - 1) & 1;
       if (bar_wait(last_full, 0, abort_flag)) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        epilogue<CH, SPLIT>(a, ybase, lt, lka, lkb, pair, pairs, (int)rank, warp & 3, lane, tmem_base + (uint32_t)(acc * 256),
+        epilogue<CH, SPLIT>(a, ybase, lt, lka, lkb, pair, pairs, (int)rank, warp & 3, lane, tmem_base + (uint32_t)(acc * ACC_COLS),
                             (warp - DQ_WARP0) / 4 + 1, HELPERS, abort_flag);
       }
     }
@@ -752,7 +887,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
 // largest magnitude into [8192, 16384): rows of large values do not overflow f16 and rows of
 // tiny values do not sink into its subnormals. rscale[m] undoes the scale exactly in the
 // epilogue. Rows that are all zero, or hold an infinity or NaN, are converted as they are.
-// Every aligned group of four k keeps the order 0, 2, 1, 3 (pair02 / pair13 above). One CTA per row;
+// The row is written in the operands' k order (above). One CTA per row;
 // up to 4096 values stay in registers between the two passes. At 48 registers a thread a CTA fits
 // beside a CTA of the GEMM, so the conversion of the next call is resident before this call ends.
 __global__ void __launch_bounds__(256, 5) prep_act_kernel(const void* __restrict__ x, int is_bf16, int64_t k,
@@ -802,7 +937,10 @@ __global__ void __launch_bounds__(256, 5) prep_act_kernel(const void* __restrict
     for (int h = 0; h < 2; h++)
 #pragma unroll
       for (int e = 0; e < 2; e++) o[2 * h + e] = h22u(__floats2half2_rn(u[4 * h + e] * s, u[4 * h + e + 2] * s));
-    *reinterpret_cast<uint4*>(xh + row0 + i) = make_uint4(o[0], o[1], o[2], o[3]);
+    // the two fours of an eight belong to two 16-k chunks
+    __half* const p = xh + row0 + (i & ~(int64_t)31) + (i & 31) / 2;
+    *reinterpret_cast<uint2*>(p) = make_uint2(o[0], o[1]);
+    *reinterpret_cast<uint2*>(p + 16) = make_uint2(o[2], o[3]);
   };
 #pragma unroll
   for (int j = 0; j < KEEP; j++) {
@@ -854,17 +992,18 @@ template <int DT, bool SPLIT>
 cudaError_t launch_tc_split(const CUtensorMap& map, GemmArgs a, int pairs, cudaStream_t s) {
   constexpr int SLOT_BYTES = 8 * UnitGeom<DT>::BYTES;
   constexpr int BAR_BYTES = (4 * MAX_ST + 2 * MAX_RAW + 5) * 8 + 8;
-  // Shared memory: three raw slots and weight stages (two where that leaves no room for four
-  // activation blocks in flight), the rest for activation stages and raw slots.
-  // (A dequantize warp only waits on the stages it fills itself. Behind a unit of one stage - an
+  // Shared memory: three raw slots and (prefill) three weight stages, two where that leaves no room for
+  // four activation blocks in flight, the rest for activation stages and raw slots. Decode batches have
+  // their three weight stages in TMEM.
+  // (A prefill dequantize warp only waits on the stages it fills itself. Behind a unit of one stage - an
   // in-feature count that is no multiple of 256 - it is three stages on from its last wait; with two
   // stages it could then wait two phases ahead of the barrier, which the parity does not tell apart.)
   // 4 KB stay free for a CTA of the next call's conversion kernel.
   const int budget = device_smem_optin() - 1024 - BAR_BYTES - 4096;
-  const int a_stage = KA * A_BYTES, b_stage = (SPLIT ? 2 : 1) * a.bn * BK;
+  const int a_stage = SPLIT ? 0 : 2 * A_BYTES, b_stage = (SPLIT ? 4 : 1) * a.bn * BK;
   int sa = 3, sb = SPLIT ? 3 : 4, rs = 3;
   auto left = [&]() { return budget - sa * a_stage - sb * b_stage - rs * SLOT_BYTES; };
-  if (left() < 0 && a.kblocks % 4 == 0) sa = 2;
+  if (!SPLIT && left() < 0 && a.kblocks % 4 == 0) sa = 2;
   if (left() < 0) rs = 2;
   if (left() < 0) sb = 3;
   if (left() < 0) return cudaErrorInvalidConfiguration;
@@ -917,6 +1056,8 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
   float* rscale = reinterpret_cast<float*>(scratch + (((size_t)m * (size_t)k * 2 + 255) & ~(size_t)255));
   cudaError_t e = cudaSuccess;
   if (sibling == 0) {  // several weights that read the same x share one conversion
+    e = prefer_matmul_carveout<prep_act_kernel>();
+    if (e != cudaSuccess) return e;
     e = launch_pdl(prep_act_kernel, dim3((unsigned)m), dim3(256), 0, s, x, (int)(x_dtype == TQ_BF16), k, xh, rscale);
     if (launches) (*launches)++;
     if (e != cudaSuccess) return e;
