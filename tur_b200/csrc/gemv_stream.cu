@@ -35,8 +35,9 @@
 namespace turq {
 
 constexpr int NW = 8;                  // consumer warps
-constexpr int THREADS = (NW + 2) * 32; // + producer warp + epilogue warp
+constexpr int THREADS = (NW + 2) * 32; // + producer warp + epilogue warp; a wide CTA has two such sets
 constexpr int RED_SLOTS = 2;           // partial-sum hand-over buffers between consumers and epilogue
+constexpr int red_slots_of(int halves, int mg) { return halves == 2 && mg == 1 ? 1 : RED_SLOTS; }  // wide: room for 8 x 12288 planes
 constexpr int MAX_STAGES = 6;
 constexpr uint32_t SPIN_LIMIT = 1u << 23;
 constexpr long long WAIT_CYCLES = 2000000000ll;  // about one second of SM clock
@@ -99,7 +100,9 @@ extern "C" int turq_debug_read_trace(unsigned long long* host, int n) {
 
 struct SmemPlan {
   int ring, act_qs, act_dsc, act_bs16, act_bs32, red, bars, total, qs_stride;
+  int ring_step, red_step, bars_step;  // wide CTAs: from one half's to the other's
 };
+constexpr int bar_bytes(int red_slots) { return (MAX_STAGES * NW + MAX_STAGES + 2 * red_slots) * 8; }
 
 constexpr int MAX_PARTS = 4;  // weights that share one activation and one launch (q|k|v, gate|up)
 
@@ -131,6 +134,7 @@ struct StreamArgs {
   int stages;
   int stage_bytes;
   SmemPlan sp;
+  int vgrid;            // CTAs of the work split; a wide CTA stands for two of them
   // Row-parallel linear of a tensor-parallel group, small outputs: the CTAs that finish last
   // perform the exchange themselves (signal the peers, wait, add all ranks' partial results in rank
   // order into xchg.out) - compute and collective in one kernel. y / y_alt are then the two
@@ -140,11 +144,12 @@ struct StreamArgs {
 };
 
 inline SmemPlan plan_smem(int dtype, int mg, bool fused /* planes in shared memory */, int rows_cap, int k, int stages, int stage_bytes,
-                          int dtype2 = -1) {
+                          int dtype2 = -1, int halves = 1, int red_slots = RED_SLOTS) {
   auto up = [](int v) { return (v + 127) & ~127; };
   SmemPlan p{};
   p.ring = 0;
-  int off = up(stages * stage_bytes);
+  p.ring_step = up(stages * stage_bytes);
+  int off = halves * p.ring_step;
   p.qs_stride = k + 32;
   p.act_qs = off;
   if (fused) {
@@ -157,9 +162,11 @@ inline SmemPlan plan_smem(int dtype, int mg, bool fused /* planes in shared memo
     if (dtype == TQ_Q4_K || dtype == TQ_Q5_K) off = up(off + rows_cap * (k / 32) * 2);
   }
   p.red = off;
-  off = up(off + RED_SLOTS * NW * mg * 128 * 4);
+  p.red_step = up(red_slots * NW * mg * 128 * 4);
+  off += halves * p.red_step;
   p.bars = off;
-  off += (MAX_STAGES * NW + MAX_STAGES + 2 * RED_SLOTS) * 8 + 8 /* abort flag */ + 8 /* act_full */ + 16;
+  p.bars_step = bar_bytes(red_slots);
+  off += halves * p.bars_step + 8 /* abort flag */ + 8 /* act_full */ + 16;
   p.total = off;
   return p;
 }
@@ -201,8 +208,14 @@ constexpr int ACT_STAGED = 2;  // bulk-copied from global scratch into shared me
 // DT2 != DT: a mixed launch (attn_q|k in Q4_K or Q5_K beside attn_v in Q6_K, as the K-quant
 // mixes store them); parts flagged in part_alt hold DT2 tiles. Both types have one tile per
 // 256 elements, so the walk over tiles is the same; ring slots are sized for the larger tile.
-template <int DT, int MG, int ACT, int DT2 = DT>
-__global__ void __launch_bounds__(THREADS, 2) gemv_stream_kernel(const __grid_constant__ StreamArgs a) {
+//
+// HALVES == 2 (wide): one CTA per SM with two sets of warps. Each set does exactly what a CTA of the
+// split does (same share, same sums, same bits), but both read one copy of the activation planes,
+// which leaves the rings what a second copy would take: 16 rows of 4096 values, or 8 of 12288, fit.
+template <int DT, int MG, int ACT, int DT2 = DT, int HALVES = 1>
+__global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kernel(const __grid_constant__ StreamArgs a) {
+  static_assert(HALVES == 1 || ACT == ACT_STAGED, "wide CTAs share staged planes");
+  constexpr int RSLOTS = red_slots_of(HALVES, MG);
   constexpr bool MIXED = DT2 != DT;
   constexpr int TB = TileGeom<DT>::BYTES;
   constexpr int TB2 = TileGeom<DT2>::BYTES;
@@ -214,18 +227,22 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_stream_kernel(const __grid_co
   constexpr bool NEED32 = DT == TQ_Q4_K || DT == TQ_Q5_K || DT2 == TQ_Q4_K || DT2 == TQ_Q5_K;
   extern __shared__ __align__(128) uint8_t smem[];
   const SmemPlan& sp = a.sp;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + sp.bars);  // [stage][consumer warp]: one tile each
+  const int half = HALVES == 2 ? (int)threadIdx.x / THREADS : 0;
+  const int htid = (int)threadIdx.x - half * THREADS;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + sp.bars + half * sp.bars_step);  // [stage][consumer warp]: one tile each
   uint64_t* empty = full + MAX_STAGES * NW;
   uint64_t* red_full = empty + MAX_STAGES;
-  uint64_t* red_empty = red_full + RED_SLOTS;
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(red_empty + RED_SLOTS);
-  uint64_t* act_full = red_empty + RED_SLOTS + 1;  // ACT_STAGED: the planes have landed
-  float* red = reinterpret_cast<float*>(smem + sp.red);
+  uint64_t* red_empty = red_full + RSLOTS;
+  uint64_t* const common = reinterpret_cast<uint64_t*>(smem + sp.bars + HALVES * sp.bars_step);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(common);
+  uint64_t* act_full = common + 1;  // ACT_STAGED: the planes have landed
+  float* red = reinterpret_cast<float*>(smem + sp.red + half * sp.red_step);
+  uint8_t* const ring = smem + sp.ring + half * sp.ring_step;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = htid >> 5, lane = threadIdx.x & 31;
   if (warp == 0) TRACE(0);
   const int KU = a.KU;
-  const int G = gridDim.x, b = blockIdx.x;
+  const int G = a.vgrid, b = HALVES * (int)blockIdx.x + half;
   auto start_of = [&](int bb) {
     const int u = bb * a.split_q + (bb < a.split_r ? bb : a.split_r);
     return u < a.total_units ? u : a.total_units;
@@ -235,7 +252,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_stream_kernel(const __grid_co
   {
     // one barrier per thread: ~60 mbarrier.init in sequence on one thread cost most of a
     // microsecond before the first copy could be issued
-    const int tid = (int)threadIdx.x;
+    const int tid = htid;
     const int nfull = a.stages * NW;
     int i = tid;
     bool did = true;
@@ -243,13 +260,15 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_stream_kernel(const __grid_co
       mbar_init(&full[i], 1);
     } else if ((i -= nfull) < a.stages) {
       mbar_init(&empty[i], NW);
-    } else if ((i -= a.stages) < RED_SLOTS) {
+    } else if ((i -= a.stages) < RSLOTS) {
       mbar_init(&red_full[i], NW);
-    } else if ((i -= RED_SLOTS) < RED_SLOTS) {
+    } else if ((i -= RSLOTS) < RSLOTS) {
       mbar_init(&red_empty[i], 1);
-    } else if (i == RED_SLOTS) {
-      mbar_init(act_full, 1);
-      *abort_flag = 0;
+    } else if (i == RSLOTS) {
+      if (half == 0) {
+        mbar_init(act_full, 1);
+        *abort_flag = 0;
+      }
     } else {
       did = false;
     }
@@ -288,7 +307,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_stream_kernel(const __grid_co
       // The first ring fill goes out before the planes: weights never depend on the preceding
       // kernels, the planes have to wait for them. The consumers cannot free a stage before they
       // have the planes, so the planes are requested before the first wait that needs a free stage.
-      bool planes_pending = ACT == ACT_STAGED;
+      bool planes_pending = ACT == ACT_STAGED && half == 0;
       StageWalk w;
       w.init(u0, u1, KU);
       int slot = 0, issued = 0;
@@ -313,7 +332,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_stream_kernel(const __grid_co
         }
         const int tb = (MIXED && a.part_alt[part]) ? TB2 : TB;
         const uint8_t* src = a.tiles[part] + ((int64_t)rt_in_part * a.ktiles + (int64_t)w.ku * GROUP) * tb;
-        uint8_t* dst = smem + sp.ring + slot * a.stage_bytes;
+        uint8_t* dst = ring + slot * a.stage_bytes;
         for (int i = 0; i < n; i++) {
           int nt = a.ktiles - (w.ku + i) * GROUP;
           if (nt > GROUP) nt = GROUP;
@@ -441,7 +460,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_stream_kernel(const __grid_co
         const int kt = (w.ku + warp) * GROUP;
         int left = a.ktiles - kt;
         if (left > GROUP) left = GROUP;
-        const uint8_t* tile = smem + sp.ring + slot * a.stage_bytes + warp * UNIT_BYTES;
+        const uint8_t* tile = ring + slot * a.stage_bytes + warp * UNIT_BYTES;
         bool alt = false;
         if constexpr (MIXED) {
           int part = 0;
@@ -487,7 +506,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_stream_kernel(const __grid_co
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&red_full[rs]);
-        if (++rs == RED_SLOTS) { rs = 0; rph ^= 1u; }
+        if (++rs == RSLOTS) { rs = 0; rph ^= 1u; }
       }
     }
     if (warp == 0) TRACE(5);
@@ -600,7 +619,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_stream_kernel(const __grid_co
       } else if (!whole) {
         for (int cb = lane; cb < ncontrib; cb += 32) a.flags[b + 1 + cb] = 0;  // consumed: zero again for the next launch
       }
-      if (++rs == RED_SLOTS) { rs = 0; rph ^= 1u; }
+      if (++rs == RSLOTS) { rs = 0; rph ^= 1u; }
       seg_ka = kb == KU ? 0 : kb;
     }
     TRACE(6);
@@ -614,7 +633,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_stream_kernel(const __grid_co
       __threadfence_system();
     }
   }
-  if (a.xchg_on) {
+  if constexpr (HALVES == 1) if (a.xchg_on) {
     // The CTAs that finish last exchange: the last `nb` tickets (nb = enough CTAs for one float4
     // group per thread, at most 16) wait the short while until every CTA of the launch has
     // written its part of the slot, then ticket order gives each its share of the result and the
@@ -691,20 +710,21 @@ size_t gemv_workspace_flags_bytes(int sms) { return (size_t)sms * 4 * 4; }
 
 // Launches with the programmatic-stream-serialization attribute (the kernel orders itself
 // against its predecessor with griddepcontrol.wait).
-template <int DT, int MG, int ACT, int DT2 = DT>
+template <int DT, int MG, int ACT, int DT2 = DT, int HALVES = 1>
 static cudaError_t launch_one(StreamArgs a, int grid, int smem_bytes, cudaStream_t s, bool after_quant = false) {
   static PerDeviceOnce configured;  // per instantiation; the attribute is per device function
   int dev = 0;
   cudaGetDevice(&dev);
   if (!configured.done(dev)) {
-    cudaError_t e = cudaFuncSetAttribute(gemv_stream_kernel<DT, MG, ACT, DT2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemv_stream_kernel<DT, MG, ACT, DT2, HALVES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          smem_budget());
     if (e != cudaSuccess) return e;
     configured.set(dev);
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(THREADS);
+  a.vgrid = grid;
+  cfg.gridDim = dim3((unsigned)((grid + HALVES - 1) / HALVES));
+  cfg.blockDim = dim3(HALVES * THREADS);
   cfg.dynamicSmemBytes = (size_t)smem_bytes;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -720,12 +740,12 @@ static cudaError_t launch_one(StreamArgs a, int grid, int smem_bytes, cudaStream
   static const int pdl = tuning_env("TURQ_GEMV_PDL", 1);
   static const int pdl_pair = tuning_env("TURQ_GEMV_PDL_PAIR", 1);
   cfg.numAttrs = (pdl || (after_quant && pdl_pair)) ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, gemv_stream_kernel<DT, MG, ACT, DT2>, a);
+  return cudaLaunchKernelEx(&cfg, gemv_stream_kernel<DT, MG, ACT, DT2, HALVES>, a);
 }
 
 // DT2 != DT: parts whose dtype field is DT2 hold tiles of that type (one launch for the K-quant
 // mixes' attn_q|k|v). Returns cudaErrorNotSupported, before anything is launched, when a mixed
-// call would need a variant that is not instantiated (more than 8 rows, planes in global memory).
+// call would need a variant that is not instantiated (planes in global memory, more than 8 rows per launch in narrow CTAs).
 template <int DT, int DT2 = DT>
 static cudaError_t launch_dt(const GemvPart* parts, int nparts, int64_t k, const void* x, int x_dtype,
                              uint8_t* act_scratch, int64_t m, uint8_t* workspace, int* status, int sm_count,
@@ -769,15 +789,34 @@ static cudaError_t launch_dt(const GemvPart* parts, int nparts, int64_t k, const
   // more than the one pass of the quantization launch, so the planes are always staged.
   // planes_ready: a preceding launch of the caller (RMSNorm prologue) already left the planes of
   // these rows in act_scratch.
+  // Wide CTAs (planes shared by two sets of warps) where a CTA's half of the shared memory is too small for
+  // the planes but an SM's is not; with more than 8 rows that do not fit either way, 8 rows at a time (the
+  // second pass finds the weights in L2). Reading the planes from global memory in the MMA loop instead
+  // waits for an L2 trip per fragment: 16 rows, Q4_K gate|up 2 x 12288 x 4096 40.7 us against 33.2 us wide,
+  // attn_q|k|v (one mixed launch instead of two) 26.8 against 17.5 us, Q6_K 4096 x 12288 31.2 against
+  // 30.6 us in two passes. The shares and sums are those of the narrow CTAs, bit for bit.
+  auto wide_stages = [&](int rows, int mg) {
+    int st = MAX_STAGES;
+    for (; st >= 2; st--)
+      if (plan_smem(DT, mg, true, rows, (int)k, st, stage_bytes, DT2, 2, red_slots_of(2, mg)).total <= smem_budget()) break;
+    return st;
+  };
+  bool wide = false;
+  int step = 32;  // rows per launch
   int act_mode = (gemv_int8_fuses_act(DT, m, k) && !x_remote && !planes_ready) ? ACT_FUSED : ACT_GLOBAL;
   {
     const int rows0 = (int)(m < 32 ? m : 32), mg0 = rows0 <= 8 ? 1 : rows0 <= 16 ? 2 : 4;
     if (act_mode == ACT_FUSED && stages_for(true, ctas_per_sm, rows0, mg0) < 2) act_mode = ACT_GLOBAL;
     static const int stage_env = tuning_env("TURQ_GEMV_STAGED", 1);
     if (act_mode == ACT_GLOBAL && m <= 16 && stage_env && stages_for(true, ctas_per_sm, rows0, mg0) >= 2) act_mode = ACT_STAGED;
+    if (act_mode == ACT_GLOBAL && m <= 16 && !xchg && ctas_per_sm == 2) {
+      if (wide_stages(rows0, mg0) >= 2) wide = true;
+      else if (m > 8 && wide_stages(8, 1) >= 2) { wide = true; step = 8; }
+      if (wide) act_mode = ACT_STAGED;
+    }
   }
   const bool fused = act_mode == ACT_FUSED, planes_in_smem = act_mode != ACT_GLOBAL;
-  if (MIXED && (m > 8 || act_mode == ACT_GLOBAL)) return cudaErrorNotSupported;
+  if (MIXED && ((m > 8 && !wide) || act_mode == ACT_GLOBAL)) return cudaErrorNotSupported;
   // Work split. Whole row-tiles per CTA when that keeps most CTA slots busy (or the problem
   // is small): no row-tile is shared, so no partial sums cross CTAs. Otherwise an even split
   // in tiles, with the hand-over of split row-tiles. Depends on the shape only, never on M.
@@ -796,8 +835,8 @@ static cudaError_t launch_dt(const GemvPart* parts, int nparts, int64_t k, const
     if (launches) (*launches)++;
     if (e != cudaSuccess) return e;
   }
-  for (int64_t m0 = 0; m0 < m; m0 += 32) {
-    const int rows = (int)(m - m0 < 32 ? m - m0 : 32);
+  for (int64_t m0 = 0; m0 < m; m0 += step) {
+    const int rows = (int)(m - m0 < step ? m - m0 : step);
     const int mg = rows <= 8 ? 1 : rows <= 16 ? 2 : 4;
     StreamArgs a{};
     for (int p = 0; p < nparts; p++) {
@@ -836,14 +875,17 @@ static cudaError_t launch_dt(const GemvPart* parts, int nparts, int64_t k, const
     a.partial = reinterpret_cast<float*>(workspace);
     a.flags = reinterpret_cast<int*>(workspace + gemv_workspace_flags_offset(sm_count));
     a.status = status;
-    const int stages = stages_for(planes_in_smem, ctas_per_sm, rows, mg);
+    const int stages = wide ? wide_stages(rows, mg) : stages_for(planes_in_smem, ctas_per_sm, rows, mg);
     if (stages < 2) return cudaErrorInvalidConfiguration;
-    const SmemPlan sp = plan_smem(DT, mg, planes_in_smem, rows, (int)k, stages, stage_bytes, DT2);
+    const SmemPlan sp = wide ? plan_smem(DT, mg, true, rows, (int)k, stages, stage_bytes, DT2, 2, red_slots_of(2, mg))
+                             : plan_smem(DT, mg, planes_in_smem, rows, (int)k, stages, stage_bytes, DT2);
     a.stages = stages;
     a.stage_bytes = stage_bytes;
     a.sp = sp;
     cudaError_t e;
-    if constexpr (MIXED) {
+    if (wide) {
+      e = mg == 1 ? launch_one<DT, 1, ACT_STAGED, DT2, 2>(a, grid, sp.total, s, true) : launch_one<DT, 2, ACT_STAGED, DT2, 2>(a, grid, sp.total, s, true);
+    } else if constexpr (MIXED) {
       e = act_mode == ACT_FUSED ? launch_one<DT, 1, ACT_FUSED, DT2>(a, grid, sp.total, s)
                                 : launch_one<DT, 1, ACT_STAGED, DT2>(a, grid, sp.total, s, true);
     } else if (act_mode == ACT_FUSED) {

@@ -92,7 +92,7 @@ cudaError_t launch_gemv_int8(int dtype, const uint8_t* tiles, int64_t n_rows, in
                              uint8_t* workspace, int* status, int sm_count, cudaStream_t s, int* launches);
 // The same for several weights of one in-feature count that share x: one launch over the
 // concatenated rows (q|k|v, gate|up) per weight type - and a single one for Q4_K or Q5_K parts
-// beside Q6_K parts at up to 8 rows - each part with its own output and bias. x_remote: x is
+// beside Q6_K parts while the planes fit shared memory - each part with its own output and bias. x_remote: x is
 // mapped host memory; it is then read exactly once, by the quantization launch. planes_ready: the
 // caller's own prologue launch already wrote the quantized planes of these rows to act_scratch.
 struct TpArgs;  // tp_exchange.cuh: xchg != nullptr (one part, m <= 32) makes the launch's last CTA run
