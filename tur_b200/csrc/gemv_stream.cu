@@ -14,8 +14,8 @@
 //   * Quantized activations (template parameter ACT): up to 4096 values the CTA quantizes
 //     them itself into shared memory while the first weight stages are in flight; otherwise a
 //     launch of its own quantizes them once into global scratch and the CTAs either bulk-copy
-//     the planes into shared memory (up to 16 rows, when they fit) or read them from global
-//     memory in the MMA loop. The GEMV that follows its quantization launch is started with
+//     the planes into shared memory (up to 16 rows, when they fit; one copy for two sets of
+//     warps where a copy per CTA would not) or read them from global memory in the MMA loop. The GEMV that follows its quantization launch is started with
 //     programmatic stream serialization: its CTAs set up while that launch still runs and
 //     order themselves behind it with griddepcontrol.wait.
 //   * Several weights that share x run as one launch over their concatenated row-tiles, also
@@ -100,7 +100,6 @@ extern "C" int turq_debug_read_trace(unsigned long long* host, int n) {
 
 struct SmemPlan {
   int ring, act_qs, act_dsc, act_bs16, act_bs32, red, bars, total, qs_stride;
-  int ring_step, red_step, bars_step;  // wide CTAs: from one half's to the other's
 };
 constexpr int bar_bytes(int red_slots) { return (MAX_STAGES * NW + MAX_STAGES + 2 * red_slots) * 8; }
 
@@ -133,8 +132,8 @@ struct StreamArgs {
   int* status;
   int stages;
   int stage_bytes;
+  int vgrid;            // wide CTAs: CTAs of the work split (a wide CTA stands for two of them)
   SmemPlan sp;
-  int vgrid;            // CTAs of the work split; a wide CTA stands for two of them
   // Row-parallel linear of a tensor-parallel group, small outputs: the CTAs that finish last
   // perform the exchange themselves (signal the peers, wait, add all ranks' partial results in rank
   // order into xchg.out) - compute and collective in one kernel. y / y_alt are then the two
@@ -148,8 +147,7 @@ inline SmemPlan plan_smem(int dtype, int mg, bool fused /* planes in shared memo
   auto up = [](int v) { return (v + 127) & ~127; };
   SmemPlan p{};
   p.ring = 0;
-  p.ring_step = up(stages * stage_bytes);
-  int off = halves * p.ring_step;
+  int off = halves * stages * stage_bytes;  // stage_bytes is a multiple of 128 for every type
   p.qs_stride = k + 32;
   p.act_qs = off;
   if (fused) {
@@ -162,11 +160,9 @@ inline SmemPlan plan_smem(int dtype, int mg, bool fused /* planes in shared memo
     if (dtype == TQ_Q4_K || dtype == TQ_Q5_K) off = up(off + rows_cap * (k / 32) * 2);
   }
   p.red = off;
-  p.red_step = up(red_slots * NW * mg * 128 * 4);
-  off += halves * p.red_step;
+  off += halves * red_slots * NW * mg * 128 * 4;
   p.bars = off;
-  p.bars_step = bar_bytes(red_slots);
-  off += halves * p.bars_step + 8 /* abort flag */ + 8 /* act_full */ + 16;
+  off += halves * bar_bytes(red_slots) + 8 /* abort flag */ + 8 /* act_full */ + 16;
   p.total = off;
   return p;
 }
@@ -229,20 +225,20 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
   const SmemPlan& sp = a.sp;
   const int half = HALVES == 2 ? (int)threadIdx.x / THREADS : 0;
   const int htid = (int)threadIdx.x - half * THREADS;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + sp.bars + half * sp.bars_step);  // [stage][consumer warp]: one tile each
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + sp.bars + half * bar_bytes(RSLOTS));  // [stage][consumer warp]: one tile each
   uint64_t* empty = full + MAX_STAGES * NW;
   uint64_t* red_full = empty + MAX_STAGES;
   uint64_t* red_empty = red_full + RSLOTS;
-  uint64_t* const common = reinterpret_cast<uint64_t*>(smem + sp.bars + HALVES * sp.bars_step);
+  uint64_t* const common = reinterpret_cast<uint64_t*>(smem + sp.bars + HALVES * bar_bytes(RSLOTS));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(common);
   uint64_t* act_full = common + 1;  // ACT_STAGED: the planes have landed
-  float* red = reinterpret_cast<float*>(smem + sp.red + half * sp.red_step);
-  uint8_t* const ring = smem + sp.ring + half * sp.ring_step;
+  float* red = reinterpret_cast<float*>(smem + sp.red + half * (RSLOTS * NW * MG * 128 * 4));
+  uint8_t* const ring = smem + sp.ring + half * (a.stages * a.stage_bytes);
 
   const int warp = htid >> 5, lane = threadIdx.x & 31;
   if (warp == 0) TRACE(0);
   const int KU = a.KU;
-  const int G = a.vgrid, b = HALVES * (int)blockIdx.x + half;
+  const int G = HALVES == 1 ? (int)gridDim.x : a.vgrid, b = HALVES * (int)blockIdx.x + half;
   auto start_of = [&](int bb) {
     const int u = bb * a.split_q + (bb < a.split_r ? bb : a.split_r);
     return u < a.total_units ? u : a.total_units;
