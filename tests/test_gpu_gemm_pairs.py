@@ -62,25 +62,64 @@ def test_decode_batches_share_the_k_loop(tq, dt, n, k):
     tq.context().poll_status()
 
 
-@pytest.mark.parametrize("m", [33, 300])
-def test_weights_of_one_call_run_side_by_side(tq, m):
-    """Four weights of different types and sizes that share x: the later ones start beside the first
-    one and whatever follows the call has to wait for all of them."""
+@pytest.fixture(scope="module")
+def four_weights(tq):
+    """Weights of different types and sizes that share x, in an order in which the number of CTAs falls and rises."""
     k = 1024
     shapes = [(oracle.Q4_K, 4096), (oracle.Q6_K, 272), (oracle.Q5_K, 16), (oracle.Q4_K, 1000)]
     ws = [make_weight(t, n, k, SEED + 7200 + n) for t, n in shapes]
-    mms = [tq.QMatMul.from_arc(tq.QTensor.new(w, tq.GgmlDType(t), (n, k))) for w, (t, n) in zip(ws, shapes)]
-    x = np.random.default_rng(SEED + 7201).standard_normal((m, k)).astype(np.float32)
-    xd = torch.from_numpy(x).cuda()
-    want = [mm.forward(xd, mode=tq.Mode.TENSOR_CORE) for mm in mms]
-    outs = [torch.empty(m, n, device="cuda") for _, n in shapes]
-    for _ in range(20):
-        for o in outs:
-            o.fill_(float("nan"))
-        tq.QMatMul.forward_multi(mms, xd, outs=outs, mode=tq.Mode.TENSOR_CORE)
-        got = torch.cat([o.flatten() for o in outs])       # a launch of another kind right behind the call
-        xd.mul_(1.0)
-        assert torch.equal(got, torch.cat([w_.flatten() for w_ in want]))
-    for o, w, (t, n) in zip(want, ws, shapes):
-        assert oracle.rel_fro(o.cpu().numpy(), oracle.matmul_f64(t, w, n, k, x)) < TOL
+    return k, shapes, ws, [tq.QMatMul.from_arc(tq.QTensor.new(w, tq.GgmlDType(t), (n, k))) for w, (t, n) in zip(ws, shapes)]
+
+
+def rows_of_all_magnitudes(m, k, seed):
+    """Every row by its own power of two, so that the row scales of one x are not those of another."""
+    rng = np.random.default_rng(seed)
+    return (rng.standard_normal((m, k)) * 2.0 ** rng.integers(-8, 9, (m, 1))).astype(np.float32)
+
+
+@pytest.mark.parametrize("m", [33, 300])
+def test_weights_of_one_call_run_side_by_side(tq, four_weights, m):
+    """The later weights of a call start beside the first one, whatever follows the call waits for all
+    of them, and none of them reads the operand, the row scales or the partial sums of another call:
+    calls on different x are issued back to back, with no other kernel between them."""
+    k, shapes, ws, mms = four_weights
+    xs = [rows_of_all_magnitudes(m, k, SEED + 7201 + i) for i in range(4)]
+    xd = [torch.from_numpy(x).cuda() for x in xs]
+    want = [[mm.forward(x, mode=tq.Mode.TENSOR_CORE) for mm in mms] for x in xd]
+    for x, ys in zip(xs, want):
+        for y, w, (t, n) in zip(ys, ws, shapes):
+            ref = oracle.matmul_f64(t, w, n, k, x)
+            scale = np.linalg.norm(ref, axis=1, keepdims=True)         # row by row: the magnitudes differ
+            assert oracle.rel_fro(y.cpu().numpy() / scale, ref / scale) < TOL
+    for order in (slice(None), slice(None, None, -1)):
+        outs = [[torch.full((m, n), float("nan"), device="cuda") for _, n in shapes[order]] for _ in range(20)]
+        for i, o in enumerate(outs):
+            tq.QMatMul.forward_multi(mms[order], xd[i % 4], outs=o, mode=tq.Mode.TENSOR_CORE)
+        got = [torch.cat([y.flatten() for y in o]) for o in outs]      # launches of another kind behind the last call
+        for i, g in enumerate(got):
+            assert torch.equal(g, torch.cat([y.flatten() for y in want[i % 4][order]])), i
+    tq.context().poll_status()
+
+
+@pytest.mark.parametrize("m", [33, 300])
+def test_captured_call_of_several_weights_on_changing_rows(tq, four_weights, m):
+    k, shapes, _, mms = four_weights
+    xs = [torch.from_numpy(rows_of_all_magnitudes(m, k, SEED + 7301 + i)).cuda() for i in range(3)]
+    want = [[mm.forward(x, mode=tq.Mode.TENSOR_CORE) for mm in mms] for x in xs]
+    x = xs[0].clone()
+    tq.context().reserve(m, k, 4096)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        with torch.cuda.graph(graph, stream=stream):
+            outs = [torch.empty((m, n), device="cuda") for _, n in shapes]
+            tq.QMatMul.forward_multi(mms, x, outs=outs, mode=tq.Mode.TENSOR_CORE)
+            tq.QMatMul.forward_multi(mms, x, outs=outs, mode=tq.Mode.TENSOR_CORE)
+        for i in range(9):
+            x.copy_(xs[i % 3])
+            graph.replay()
+            for o, w in zip(outs, want[i % 3]):
+                assert torch.equal(o, w), i
+    torch.cuda.current_stream().wait_stream(stream)
     tq.context().poll_status()

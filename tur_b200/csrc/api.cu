@@ -258,7 +258,8 @@ int32_t turq_ctx_poll_status(turq_ctx* ctx, void* stream) {
     *static_cast<volatile int*>(ctx->host_status) = 0;
     // a kernel that gave up may have left hand-over flags or claim counters set
     cudaMemsetAsync(ctx->gemv_ws, 0, turq::gemv_workspace_bytes(ctx->sm_count), s);
-    cudaMemsetAsync(ctx->gemm_ws, 0, turq::gemm_tc_workspace_bytes(ctx->sm_count), s);
+    cudaMemsetAsync(ctx->gemm_ws + turq::gemm_tc_workspace_flags_offset(ctx->sm_count), 0,
+                    turq::gemm_tc_workspace_flags_bytes(ctx->sm_count), s);
     cudaStreamSynchronize(s);
     if (st == TURQ_E_INVALID_ARG) return fail(ctx, st, "an embedding lookup was given an id outside the table");
     return fail(ctx, st, "a kernel gave up a bounded device-side wait (status %d)", st);
@@ -528,8 +529,12 @@ static int32_t qmatmul_multi_impl(turq_ctx* ctx, int32_t count, const turq_qtens
       int launches = 0;
       cudaError_t e = turq::launch_gemm_tc(qts[i]->dtype, qts[i]->tiles, qts[i]->n_rows, k, dev_x, x_dtype, m, dev_ys[i],
                                            dev_biases ? dev_biases[i] : nullptr, ctx->scratch, ctx->gemm_ws, ctx->sm_count,
-                                           static_cast<cudaStream_t>(stream), &launches, ctx->dev_status, i);
+                                           static_cast<cudaStream_t>(stream), &launches, ctx->dev_status, i,
+                                           i + 1 < count ? qts[i + 1]->n_rows : 0);
       ctx->launches += launches;
+      if (e != cudaSuccess && i > 0)  // the launch before this one has set its go-ahead words
+        cudaMemsetAsync(ctx->gemm_ws + turq::gemm_tc_workspace_flags_offset(ctx->sm_count), 0,
+                        turq::gemm_tc_workspace_flags_bytes(ctx->sm_count), static_cast<cudaStream_t>(stream));
       if (e != cudaSuccess) return cuda_fail(ctx, e, "qmatmul_multi launch");
     }
     return TURQ_OK;
@@ -832,7 +837,7 @@ int32_t qmatmul_for_exchange(turq_ctx* ctx, const turq_qtensor* qt, const void* 
     if (st != TURQ_OK) return st;
     int launches = 0;
     cudaError_t e = launch_gemm_tc(qt->dtype, qt->tiles, qt->n_rows, qt->n_cols, dev_x, x_dtype, m, s0, local_bias, ctx->scratch,
-                                   ctx->gemm_ws, ctx->sm_count, s, &launches, ctx->dev_status, 0, toggle, s1);
+                                   ctx->gemm_ws, ctx->sm_count, s, &launches, ctx->dev_status, 0, 0, toggle, s1);
     ctx->launches += launches;
     if (e != cudaSuccess) return cuda_fail(ctx, e, "row-parallel GEMM launch");
     return TURQ_OK;

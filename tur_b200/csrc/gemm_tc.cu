@@ -409,6 +409,9 @@ struct GemmArgs {
   int total;        // split_k: units of all tiles, shared out evenly; else: tiles
   int split_k;
   int sibling;      // the preceding launch belongs to the same call and reads the same x (see the kernel)
+  int* go;          // [CTA] a sibling's go-ahead words, zero between launches
+  int* next_go;     // those of the launch behind this one, which has next_ctas CTAs (0: no sibling follows)
+  int next_ctas;
   int a_stages, b_stages, raw_slots;
   const float* rscale;  // [m] factor undoing the f16 row scaling
   float* y;             // [m, n_rows]
@@ -460,6 +463,24 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
   return v;
 }
 __device__ __forceinline__ void st_release(int* p, int v) { asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
+
+// Siblings (the later weights of a call) run beside their predecessor, so griddepcontrol.wait, which
+// waits for its end, cannot be what makes the shared operand visible to them. Instead every CTA of a
+// sibling takes one go-ahead word that the launch before it released, once that launch itself could see
+// the operand and the end of everything older than the call. A word is taken by exchanging it for zero:
+// an exchange follows the write that it reads immediately in the word's order of writes, so a word set
+// for an earlier call, which that call's exchange has taken, cannot be read again.
+__device__ __forceinline__ bool take_go(int* p, volatile int* abort_flag) {
+  const long long t0 = clock64();
+  for (;;) {
+    int v;
+    asm volatile("atom.acquire.gpu.global.exch.b32 %0, [%1], 0;" : "=r"(v) : "l"(p) : "memory");
+    if (v != 0) return true;
+    if (*abort_flag || clock64() - t0 > TC_WAIT_CYCLES) break;
+  }
+  *abort_flag = 1;
+  return false;
+}
 
 // Epilogue of one segment for one TMEM lane quarter (32 weight rows): columns in chunks of CH, the
 // chunks h0, h0 + hstep, ... A pair that does not hold the tile's first unit parks its sums in
@@ -596,7 +617,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
   uint64_t* acc_full = raw_empty + MAX_RAW;
   uint64_t* acc_empty = acc_full + 2;  // leader only
   uint64_t* last_full = acc_empty + 2;  // the pair's last accumulator is complete
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(last_full + 1);
+  uint64_t* go_taken = last_full + 1;   // siblings: this CTA's go-ahead word has been taken
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(go_taken + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -621,6 +643,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
       bar_init(&acc_empty[s], 8);
     }
     bar_init(last_full, 1);
+    bar_init(go_taken, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -671,16 +694,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
     if (lane == 0) {
       // Programmatic stream serialization: the f16 operand comes from the conversion launch before
       // this one (the weight side starts without waiting). A sibling launch (the next weight of a
-      // call, same x) starts once every CTA of the GEMM before it has come past this point, so the
-      // operand is complete and everything older than the call has finished: it does not wait here
-      // and runs beside its predecessor; it waits before it ends (below), so that whoever waits for
-      // it has waited for all of the call.
+      // call, same x) has a GEMM before it, beside which it runs: it waits for its go-ahead word
+      // instead, and before it ends (below) for that GEMM's end, so that whoever waits for it has
+      // waited for all of the call. The proxy fence carries what the word's acquire made visible over
+      // to the tensor copies.
       asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
-      if (!a.sibling) asm volatile("griddepcontrol.wait;" ::: "memory");
-      asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+      bool ok = true;
+      if (a.sibling) {
+        ok = take_go(a.go + blockIdx.x, abort_flag);
+        asm volatile("fence.proxy.async.global;" ::: "memory");
+        bar_arrive(go_taken);
+      } else {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+      }
       int s = 0;
       uint32_t ph = 0;
-      bool ok = true;
       while (ok && seg.next(t, ka, kb)) {
         const int row = (t % a.mt) * a.bn + (int)rank * (a.bn >> 1);
         const int k1 = kb * 4 < a.kblocks ? kb * 4 : a.kblocks;
@@ -775,7 +803,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
     }
   } else if (warp < DQ_WARP0) {
     // ------------------------------------------------------------ epilogue
-    if (!a.sibling) asm volatile("griddepcontrol.wait;" ::: "memory");  // y may still be read, the row scales still written
+    // y may still be read, the row scales still written
+    if (a.sibling) bar_wait(go_taken, 0, abort_flag);
+    else asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (warp == 3) {
+      // what this launch has waited for a sibling behind it need not wait for again
+      for (int c = (int)(blockIdx.x + lane * gridDim.x); c < a.next_ctas; c += 32 * (int)gridDim.x) st_release(a.next_go + c, 1);
+      __syncwarp();
+      if (lane == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     float* ybase = a.y;
     if (a.y_toggle && ((*reinterpret_cast<const volatile unsigned*>(a.y_toggle) + 1u) & 1u)) ybase = a.y_alt;
     const int quarter = warp & 3;
@@ -850,7 +886,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
     }
     // nothing left to dequantize: help with the epilogue of the last segment
     if (nseg > 0) {
-      if (!a.sibling) asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (a.sibling) bar_wait(go_taken, 0, abort_flag);
+      else asm volatile("griddepcontrol.wait;" ::: "memory");
       float* ybase = a.y;
       if (a.y_toggle && ((*reinterpret_cast<const volatile unsigned*>(a.y_toggle) + 1u) & 1u)) ybase = a.y_alt;
       const int acc = (nseg - 1) & 1;
@@ -991,7 +1028,7 @@ EncodeTiledFn encode_fn() {
 template <int DT, bool SPLIT>
 cudaError_t launch_tc_split(const CUtensorMap& map, GemmArgs a, int pairs, cudaStream_t s) {
   constexpr int SLOT_BYTES = 8 * UnitGeom<DT>::BYTES;
-  constexpr int BAR_BYTES = (4 * MAX_ST + 2 * MAX_RAW + 5) * 8 + 8;
+  constexpr int BAR_BYTES = (4 * MAX_ST + 2 * MAX_RAW + 6) * 8 + 8;
   // Shared memory: three raw slots and (prefill) three weight stages, two where that leaves no room for
   // four activation blocks in flight, the rest for activation stages and raw slots. Decode batches have
   // their three weight stages in TMEM.
@@ -1041,15 +1078,29 @@ size_t gemm_tc_scratch_bytes(int64_t m, int64_t k) {
   return (((size_t)m * (size_t)k * 2 + 255) & ~(size_t)255) + (((size_t)m * 4 + 255) & ~(size_t)255) + 256;
 }
 
-// Per sibling: partial sums of a 64-row decode batch [CTA][64][128] and the ready flags [CTA][4][8].
+// Per weight of a call: partial sums of a 64-row decode batch [CTA][64][128]; behind them, again per
+// weight, the ready flags [CTA][4][8] and the go-ahead words [CTA].
 static size_t ws_partial_bytes(int sms) { return (size_t)sms * 64 * BM * 4; }
-static size_t ws_flag_words(int sms) { return (size_t)sms * 4 * 8; }
-size_t gemm_tc_workspace_bytes(int sms) { return GEMM_SIBLINGS * (ws_partial_bytes(sms) + ws_flag_words(sms) * 4); }
+static size_t ws_flag_words(int sms) { return (size_t)sms * (4 * 8 + 1); }
+size_t gemm_tc_workspace_flags_offset(int sms) { return GEMM_SIBLINGS * ws_partial_bytes(sms); }
+size_t gemm_tc_workspace_flags_bytes(int sms) { return GEMM_SIBLINGS * ws_flag_words(sms) * 4; }
+size_t gemm_tc_workspace_bytes(int sms) { return gemm_tc_workspace_flags_offset(sms) + gemm_tc_workspace_flags_bytes(sms); }
+
+// Activation rows per pair tile, activation tiles and pairs of a launch.
+struct TcShape { int bn, mt; GemmWork work; };
+static TcShape tc_shape(int64_t n_rows, int64_t m, int64_t k, int sm_count) {
+  TcShape p;
+  p.bn = tile_rows(m, plan_gemm_bn(n_rows, m, sm_count));
+  p.mt = (int)((m + p.bn - 1) / p.bn);
+  p.work = plan_gemm_work(n_rows, m, k, p.mt, sm_count);
+  return p;
+}
 
 cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int64_t k, const void* x, int x_dtype,
                            int64_t m, float* y, const float* bias, uint8_t* scratch, uint8_t* workspace, int sm_count, cudaStream_t s,
-                           int* launches, int* dev_status_word, int sibling, const unsigned* y_toggle, float* y_alt) {
-  if (k % BK != 0 || m <= 0 || m > INT32_MAX || k > INT32_MAX || sibling < 0 || sibling >= GEMM_SIBLINGS) return cudaErrorInvalidValue;
+                           int* launches, int* dev_status_word, int sibling, int64_t next_rows, const unsigned* y_toggle, float* y_alt) {
+  if (k % BK != 0 || m <= 0 || m > INT32_MAX || k > INT32_MAX || sibling < 0 ||
+      sibling + (next_rows > 0 ? 1 : 0) >= GEMM_SIBLINGS) return cudaErrorInvalidValue;
   EncodeTiledFn enc = encode_fn();
   if (!enc) return cudaErrorNotSupported;
   __half* xh = reinterpret_cast<__half*>(scratch);
@@ -1063,7 +1114,8 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
     if (e != cudaSuccess) return e;
   }
 
-  const int bn = tile_rows(m, plan_gemm_bn(n_rows, m, sm_count));
+  const TcShape shape = tc_shape(n_rows, m, k, sm_count);
+  const int bn = shape.bn;
   CUtensorMap map;
   const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
   const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
@@ -1082,9 +1134,9 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
   a.KU = (int)((k + UNIT_K - 1) / UNIT_K);
   a.m = (int)m;
   a.bn = bn;
-  a.mt = (int)((m + bn - 1) / bn);
+  a.mt = shape.mt;
   const int64_t n_tiles = (n_rows + 2 * BM - 1) / (2 * BM);
-  const GemmWork work = plan_gemm_work(n_rows, m, k, a.mt, sm_count);
+  const GemmWork& work = shape.work;
   const int64_t total = n_tiles * (work.split_k ? a.KU : a.mt);
   if (total > (int64_t)1 << 30) return cudaErrorInvalidValue;
   a.total = (int)total;
@@ -1094,7 +1146,10 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
   a.y = y;
   a.bias = bias;
   a.partial = reinterpret_cast<float*>(workspace + sibling * ws_partial_bytes(sm_count));
-  a.flags = reinterpret_cast<int*>(workspace + GEMM_SIBLINGS * ws_partial_bytes(sm_count)) + sibling * ws_flag_words(sm_count);
+  a.flags = reinterpret_cast<int*>(workspace + gemm_tc_workspace_flags_offset(sm_count)) + sibling * ws_flag_words(sm_count);
+  a.go = a.flags + (size_t)sm_count * 4 * 8;
+  a.next_go = a.go + ws_flag_words(sm_count);
+  a.next_ctas = next_rows > 0 ? 2 * tc_shape(next_rows, m, k, sm_count).work.pairs : 0;
   a.status = dev_status_word;
   a.y_toggle = y_toggle;
   a.y_alt = y_alt;
