@@ -123,3 +123,58 @@ def test_captured_call_of_several_weights_on_changing_rows(tq, four_weights, m):
                 assert torch.equal(o, w), i
     torch.cuda.current_stream().wait_stream(stream)
     tq.context().poll_status()
+
+
+def test_contexts_on_streams_of_their_own(tq, four_weights):
+    """Decode batches whose pairs wait for one another's partial sums, and calls of several weights, from
+    two threads with a context and a stream each: neither waits for or disturbs the other."""
+    import threading
+    k, shapes, ws, mms = four_weights
+    xs = {m: torch.from_numpy(rows_of_all_magnitudes(m, k, SEED + 7400 + m)).cuda() for m in (17, 64, 300)}
+    want = {m: [mm.forward(x, mode=tq.Mode.TENSOR_CORE) for mm in mms] for m, x in xs.items()}
+    torch.cuda.synchronize()
+    errors = []
+
+    def worker():
+        try:
+            ctx = tq.new_context()
+            mine = [tq.QMatMul.from_arc(tq.QTensor.new(w, tq.GgmlDType(t), (n, k), ctx=ctx)) for w, (t, n) in zip(ws, shapes)]
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                for it in range(30):
+                    got = {m: tq.QMatMul.forward_multi(mine, x, mode=tq.Mode.TENSOR_CORE) for m, x in xs.items()}
+                    stream.synchronize()
+                    if not all(torch.equal(g, w) for m in xs for g, w in zip(got[m], want[m])):
+                        errors.append(it)
+                ctx.poll_status()
+        except Exception as e:  # reported to the main thread
+            errors.append(repr(e))
+
+    threads = [threading.Thread(target=worker) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+
+
+@pytest.mark.parametrize("k", [320, 384, 576, 1728, 2624])
+@pytest.mark.parametrize("m", [2048, 2999])
+def test_prefill_pairs_with_several_tiles_and_a_short_last_unit(tq, k, m):
+    """Q8_0 in-features that are no multiple of 256 with 256-row tiles, several for every pair: the set-up with
+    three weight stages, two raw slots and three activation stages, a unit of one or two stages followed
+    by the next tile, and the accumulators' hand-over there. Every activation row, weight rows all over the tiles."""
+    n = 5000
+    w = make_weight(oracle.Q8_0, n, k, SEED + 7500 + k)
+    x = rows_of_all_magnitudes(m, k, SEED + 7501 + m)
+    rows = np.unique(np.r_[0:n:41, 255:n:256, 256:n:256, n - 1])
+    mm = tq.QMatMul.from_arc(tq.QTensor.new(w, tq.GgmlDType(oracle.Q8_0), (n, k)))
+    xd = torch.from_numpy(x).cuda()
+    y = mm.forward(xd, mode=tq.Mode.TENSOR_CORE)
+    assert torch.equal(mm.forward(xd, mode=tq.Mode.TENSOR_CORE), y)
+    got = y[:, torch.from_numpy(rows).cuda()].cpu().numpy().astype(np.float64)
+    ref = oracle.matmul_f64(oracle.Q8_0, np.ascontiguousarray(w.reshape(n, -1)[rows]).reshape(-1), len(rows), k, x)
+    err = np.linalg.norm(got - ref, axis=1) / np.linalg.norm(ref, axis=1)      # row by row: the magnitudes differ
+    # 123 or more outputs a row: a row's error stays within a few of the whole matrix' standard deviations
+    assert err.max() < TOL, (int(err.argmax()), err.max())
+    tq.context().poll_status()
