@@ -470,16 +470,18 @@ __device__ __forceinline__ void st_release(int* p, int v) { asm volatile("st.rel
 // the operand and the end of everything older than the call. A word is taken by exchanging it for zero:
 // an exchange follows the write that it reads immediately in the word's order of writes, so a word set
 // for an earlier call, which that call's exchange has taken, cannot be read again.
-__device__ __forceinline__ bool take_go(int* p, volatile int* abort_flag) {
+// The words are there when the sibling starts or soon after: every CTA of the launch before it has then
+// started and waits for nothing more before it releases them. Taken after the CTA's set-up and released
+// before dependents may start, they cost up to 1.2 us a sibling (Q8_0 2560 + 640 + 640 rows x 2560, 32
+// activation rows, us a call: 15.8 without, 18.2 so, 16.1 as it is; Q4_K + Q4_K + Q6_K 4096 + 1024 + 1024 x 4096,
+// 300 rows: 34.1, 36.3, 35.3).
+__device__ __forceinline__ bool take_go(int* p) {
   const long long t0 = clock64();
-  for (;;) {
-    int v;
+  int v;
+  do {
     asm volatile("atom.acquire.gpu.global.exch.b32 %0, [%1], 0;" : "=r"(v) : "l"(p) : "memory");
-    if (v != 0) return true;
-    if (*abort_flag || clock64() - t0 > TC_WAIT_CYCLES) break;
-  }
-  *abort_flag = 1;
-  return false;
+  } while (v == 0 && clock64() - t0 <= TC_WAIT_CYCLES);
+  return v != 0;
 }
 
 // Epilogue of one segment for one TMEM lane quarter (32 weight rows): columns in chunks of CH, the
@@ -617,14 +619,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
   uint64_t* acc_full = raw_empty + MAX_RAW;
   uint64_t* acc_empty = acc_full + 2;  // leader only
   uint64_t* last_full = acc_empty + 2;  // the pair's last accumulator is complete
-  uint64_t* go_taken = last_full + 1;   // siblings: this CTA's go-ahead word has been taken
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(go_taken + 1);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(last_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = blockIdx.x & 1u;  // rank in the cluster of two
   const int pair = (int)(blockIdx.x >> 1), pairs = (int)(gridDim.x >> 1);
 
+  // Siblings: beside the set-up, whose barrier then orders every warp of the CTA behind the word's acquire.
+  bool go = true;
+  if (a.sibling && warp == 1 && lane == 0) go = take_go(a.go + blockIdx.x);
   if (threadIdx.x == 0) {
     for (int s = 0; s < SA; s++) {
       bar_init(&a_full[s], (SPLIT ? 2 : 1) * 2 * DQ_WARPS);
@@ -643,7 +647,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
       bar_init(&acc_empty[s], 8);
     }
     bar_init(last_full, 1);
-    bar_init(go_taken, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -694,21 +697,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
     if (lane == 0) {
       // Programmatic stream serialization: the f16 operand comes from the conversion launch before
       // this one (the weight side starts without waiting). A sibling launch (the next weight of a
-      // call, same x) has a GEMM before it, beside which it runs: it waits for its go-ahead word
-      // instead, and before it ends (below) for that GEMM's end, so that whoever waits for it has
+      // call, same x) has a GEMM before it, beside which it runs: its go-ahead word stands for that
+      // wait, and before it ends (below) it waits for that GEMM's end, so that whoever waits for it has
       // waited for all of the call. The proxy fence carries what the word's acquire made visible over
       // to the tensor copies.
       asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
-      bool ok = true;
       if (a.sibling) {
-        ok = take_go(a.go + blockIdx.x, abort_flag);
+        if (!go) *abort_flag = 1;
         asm volatile("fence.proxy.async.global;" ::: "memory");
-        bar_arrive(go_taken);
       } else {
         asm volatile("griddepcontrol.wait;" ::: "memory");
       }
+      asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
       int s = 0;
       uint32_t ph = 0;
+      bool ok = true;
       while (ok && seg.next(t, ka, kb)) {
         const int row = (t % a.mt) * a.bn + (int)rank * (a.bn >> 1);
         const int k1 = kb * 4 < a.kblocks ? kb * 4 : a.kblocks;
@@ -803,15 +806,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
     }
   } else if (warp < DQ_WARP0) {
     // ------------------------------------------------------------ epilogue
-    // y may still be read, the row scales still written
-    if (a.sibling) bar_wait(go_taken, 0, abort_flag);
-    else asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (warp == 3) {
-      // what this launch has waited for a sibling behind it need not wait for again
+    if (!a.sibling) asm volatile("griddepcontrol.wait;" ::: "memory");  // y may still be read, the row scales still written
+    if (warp == 3)  // what this launch has waited for, a sibling behind it need not wait for again
       for (int c = (int)(blockIdx.x + lane * gridDim.x); c < a.next_ctas; c += 32 * (int)gridDim.x) st_release(a.next_go + c, 1);
-      __syncwarp();
-      if (lane == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    }
     float* ybase = a.y;
     if (a.y_toggle && ((*reinterpret_cast<const volatile unsigned*>(a.y_toggle) + 1u) & 1u)) ybase = a.y_alt;
     const int quarter = warp & 3;
@@ -886,8 +883,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
     }
     // nothing left to dequantize: help with the epilogue of the last segment
     if (nseg > 0) {
-      if (a.sibling) bar_wait(go_taken, 0, abort_flag);
-      else asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (!a.sibling) asm volatile("griddepcontrol.wait;" ::: "memory");
       float* ybase = a.y;
       if (a.y_toggle && ((*reinterpret_cast<const volatile unsigned*>(a.y_toggle) + 1u) & 1u)) ybase = a.y_alt;
       const int acc = (nseg - 1) & 1;
@@ -1028,7 +1024,7 @@ EncodeTiledFn encode_fn() {
 template <int DT, bool SPLIT>
 cudaError_t launch_tc_split(const CUtensorMap& map, GemmArgs a, int pairs, cudaStream_t s) {
   constexpr int SLOT_BYTES = 8 * UnitGeom<DT>::BYTES;
-  constexpr int BAR_BYTES = (4 * MAX_ST + 2 * MAX_RAW + 6) * 8 + 8;
+  constexpr int BAR_BYTES = (4 * MAX_ST + 2 * MAX_RAW + 5) * 8 + 8;
   // Shared memory: three raw slots and (prefill) three weight stages, two where that leaves no room for
   // four activation blocks in flight, the rest for activation stages and raw slots. Decode batches have
   // their three weight stages in TMEM.
