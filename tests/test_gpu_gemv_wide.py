@@ -1,7 +1,8 @@
 """Integer-scheme launches whose activation planes are shared by two sets of warps of one CTA per SM:
 the row counts and in-feature counts at which a CTA's half of the shared memory is too small for them
-(and, beyond eight rows of 12288 values, an SM's too: two passes), an odd number of shares, row-tiles
-cut between shares, mixed types. A row's bits are those it has alone."""
+and, on either side, those at which they stay in global memory; an odd number of shares, row-tiles
+cut between shares, one hand-over buffer (8 rows of 12288 values), mixed types. A row's bits are those
+it has alone, and a weight is streamed once."""
 import numpy as np
 import pytest
 
@@ -37,6 +38,22 @@ def test_rows_keep_their_bits(tq, dt, n, k):
     few = rows[:2].cpu().numpy()
     # the integers are exact; f32 sums over k / 32 blocks in another order: sqrt(512) * 2^-24 at most
     assert oracle.rel_fro(few, oracle.qmatmul(dt, w, n, k, x[:2])) < 2e-6
+    tq.context().poll_status()
+
+
+@pytest.mark.parametrize("dt", [oracle.Q8_0, oracle.Q4_K, oracle.Q5_K, oracle.Q6_K])
+@pytest.mark.parametrize("n,k,rows", [(9600, 4096, (13, 16)), (4096, 12288, (4, 8, 9, 16)), (5120, 8192, (8, 12, 16))])
+def test_rows_keep_their_bits_in_large_weights(tq, dt, n, k, rows):
+    """9600 rows: every type runs wide with row-tiles cut between shares; 5120: cut, where only Q8_0 and Q6_K run wide."""
+    from tur_b200.workloads import random_blocks
+    mm = tq.QMatMul.from_arc(tq.QTensor.new(random_blocks(dt, n, k, SEED + 8200 + n, torch.device("cuda", 0)), tq.GgmlDType(dt), (n, k)))
+    xd = torch.from_numpy(np.random.default_rng(SEED + 8201 + k).standard_normal((16, k)).astype(np.float32)).cuda()
+    alone = torch.cat([mm.forward(xd[r:r + 1], mode=tq.Mode.INT8_ACT) for r in range(16)])
+    for m in rows:
+        l0 = tq.context().launch_count()
+        y = mm.forward(xd[:m], mode=tq.Mode.INT8_ACT)
+        assert tq.context().launch_count() - l0 == 2, "one quantization of x, one pass over the weight"
+        assert torch.equal(y, alone[:m])
     tq.context().poll_status()
 
 

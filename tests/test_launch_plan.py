@@ -21,6 +21,10 @@ long long split_start(int grid, int q, int r, long long total, int b) {
   turq::GemvSplit p{grid, q, r, false};
   return turq::gemv_split_start(p, total, b);
 }
+int gemv_wide(int reads, int rows, int row_tiles, int KU, int slots) {
+  return turq::plan_gemv_wide(static_cast<turq::GemvPlaneReads>(reads), rows, turq::plan_gemv_split(row_tiles, KU, slots),
+                              (long long)row_tiles * KU, KU, slots);
+}
 int gemm_bn(long long n, long long m, int sms, int force) { return turq::plan_gemm_bn(n, m, sms, force); }
 void gemm_work(long long n, long long m, long long k, int mt, int sms, int* out) {
   turq::GemmWork w = turq::plan_gemm_work(n, m, k, mt, sms);
@@ -86,6 +90,24 @@ def test_split_choice_follows_the_stated_rule(plan):
     assert out[3] == 0 and out[0] == SLOTS
     plan.plan_split(64, 16, SLOTS, -1, out)        # 1024 rows: small -> whole row-tiles on 64 CTAs
     assert (out[0], out[3]) == (64, 1)
+
+
+Q8_0, Q6_K, Q45_K = 0, 1, 2      # how the MMA loop reads the planes
+
+
+@pytest.mark.parametrize("reads,unit,n,k,narrow,wide", [
+    (Q8_0, 128, 512, 8192, (), (8, 12, 16)), (Q8_0, 128, 5120, 25600, (), (3, 4, 5)),
+    (Q6_K, 256, 4096, 12288, (), (4, 8)), (Q6_K, 256, 640, 6144, (), (8, 12)),
+    (Q6_K, 256, 5120, 25600, (2, 3), (4,)),                          # cut shares of about one row-tile
+    (Q45_K, 256, 4096, 12288, (), (6, 8, 9)), (Q45_K, 256, 25600, 5120, (), (12, 16)), (Q45_K, 256, 9600, 8192, (), (8, 14)),
+    (Q45_K, 256, 5120, 8192, (8, 9, 12), ()), (Q45_K, 256, 6144, 6144, (9, 11, 16), ()), (Q45_K, 256, 5120, 25600, (3, 5), ()),
+    (Q45_K, 256, 640, 8192, (8, 14), ()), (Q45_K, 256, 128, 16384, (4, 8), ()),      # no more shares than SMs
+    (Q45_K, 256, 2560, 8192, (7, 8), (9, 12)),                       # a share for a little more than every SM
+])
+def test_wide_launches_where_they_are_faster(plan, reads, unit, n, k, narrow, wide):
+    """The sizes at which both forms were measured: what was slower wide stays narrow."""
+    for rows in narrow + wide:
+        assert bool(plan.gemv_wide(reads, rows, -(-n // 16), k // unit, SLOTS)) == (rows in wide), rows
 
 
 @pytest.mark.parametrize("n,k", [(8192, 5120), (1024, 5120), (5120, 8192), (25600, 5120), (5120, 25600), (2560, 2560),

@@ -15,7 +15,8 @@
 //     them itself into shared memory while the first weight stages are in flight; otherwise a
 //     launch of its own quantizes them once into global scratch and the CTAs either bulk-copy
 //     the planes into shared memory (up to 16 rows, when they fit; one copy for two sets of
-//     warps where a copy per CTA would not) or read them from global memory in the MMA loop. The GEMV that follows its quantization launch is started with
+//     warps where a copy per CTA would not and that is faster) or read them from global memory
+//     in the MMA loop. The GEMV that follows its quantization launch is started with
 //     programmatic stream serialization: its CTAs set up while that launch still runs and
 //     order themselves behind it with griddepcontrol.wait.
 //   * Several weights that share x run as one launch over their concatenated row-tiles, also
@@ -37,7 +38,10 @@ namespace turq {
 constexpr int NW = 8;                  // consumer warps
 constexpr int THREADS = (NW + 2) * 32; // + producer warp + epilogue warp; a wide CTA has two such sets
 constexpr int RED_SLOTS = 2;           // partial-sum hand-over buffers between consumers and epilogue
-constexpr int red_slots_of(int halves, int mg) { return halves == 2 && mg == 1 ? 1 : RED_SLOTS; }  // wide: room for 8 x 12288 planes
+// Wide CTAs of up to 8 rows have one buffer, which leaves room for 8 x 12288 planes. Two where they fit measured the
+// same (one / two, us: Q6_K 4096 x 12288, 6 rows 14.75 / 14.73; Q8_0 5120 x 25600, 4 rows 33.4 / 33.5; Q4_K 9600 x 8192,
+// 8 rows 18.0 / 18.1).
+constexpr int red_slots_of(int halves, int mg) { return halves == 2 && mg == 1 ? 1 : RED_SLOTS; }
 constexpr int MAX_STAGES = 6;
 constexpr uint32_t SPIN_LIMIT = 1u << 23;
 constexpr long long WAIT_CYCLES = 2000000000ll;  // about one second of SM clock
@@ -778,41 +782,6 @@ static cudaError_t launch_dt(const GemvPart* parts, int nparts, int64_t k, const
       if (plan_smem(DT, mg, planes_in_smem, rows, (int)k, st, stage_bytes, DT2).total <= share) break;
     return st;
   };
-  // Activation planes: quantized in the kernel (few rows), else quantized once by a launch of
-  // their own and then either bulk-copied into every CTA's shared memory (up to 16 rows, when
-  // they fit beside a two-stage ring) or read from global memory by the MMA loop.
-  // x_remote: x lives in mapped host memory - every CTA reading it over the bus would cost far
-  // more than the one pass of the quantization launch, so the planes are always staged.
-  // planes_ready: a preceding launch of the caller (RMSNorm prologue) already left the planes of
-  // these rows in act_scratch.
-  // Wide CTAs (planes shared by two sets of warps) where a CTA's half of the shared memory is too small for
-  // the planes but an SM's is not; with more than 8 rows that do not fit either way, 8 rows at a time (the
-  // second pass finds the weights in L2). Reading the planes from global memory in the MMA loop instead
-  // waits for an L2 trip per fragment: 16 rows, Q4_K gate|up 2 x 12288 x 4096 40.7 us against 33.2 us wide,
-  // attn_q|k|v (one mixed launch instead of two) 26.8 against 17.5 us, Q6_K 4096 x 12288 31.2 against
-  // 30.6 us in two passes. The shares and sums are those of the narrow CTAs, bit for bit.
-  auto wide_stages = [&](int rows, int mg) {
-    int st = MAX_STAGES;
-    for (; st >= 2; st--)
-      if (plan_smem(DT, mg, true, rows, (int)k, st, stage_bytes, DT2, 2, red_slots_of(2, mg)).total <= smem_budget()) break;
-    return st;
-  };
-  bool wide = false;
-  int step = 32;  // rows per launch
-  int act_mode = (gemv_int8_fuses_act(DT, m, k) && !x_remote && !planes_ready) ? ACT_FUSED : ACT_GLOBAL;
-  {
-    const int rows0 = (int)(m < 32 ? m : 32), mg0 = rows0 <= 8 ? 1 : rows0 <= 16 ? 2 : 4;
-    if (act_mode == ACT_FUSED && stages_for(true, ctas_per_sm, rows0, mg0) < 2) act_mode = ACT_GLOBAL;
-    static const int stage_env = tuning_env("TURQ_GEMV_STAGED", 1);
-    if (act_mode == ACT_GLOBAL && m <= 16 && stage_env && stages_for(true, ctas_per_sm, rows0, mg0) >= 2) act_mode = ACT_STAGED;
-    if (act_mode == ACT_GLOBAL && m <= 16 && !xchg && ctas_per_sm == 2) {
-      if (wide_stages(rows0, mg0) >= 2) wide = true;
-      else if (m > 8 && wide_stages(8, 1) >= 2) { wide = true; step = 8; }
-      if (wide) act_mode = ACT_STAGED;
-    }
-  }
-  const bool fused = act_mode == ACT_FUSED, planes_in_smem = act_mode != ACT_GLOBAL;
-  if (MIXED && ((m > 8 && !wide) || act_mode == ACT_GLOBAL)) return cudaErrorNotSupported;
   // Work split. Whole row-tiles per CTA when that keeps most CTA slots busy (or the problem
   // is small): no row-tile is shared, so no partial sums cross CTAs. Otherwise an even split
   // in tiles, with the hand-over of split row-tiles. Depends on the shape only, never on M.
@@ -824,6 +793,37 @@ static cudaError_t launch_dt(const GemvPart* parts, int nparts, int64_t k, const
   GemvSplit split = interleave ? plan_gemv_split(row_tiles_all / 2, 2 * KU, slots, -1) : plan_gemv_split(row_tiles_all, KU, slots, split_env);
   if (interleave && !split.aligned) return cudaErrorNotSupported;
   const int grid = split.grid, split_q = split.split_q, split_r = split.split_r;
+  // Activation planes: quantized in the kernel (few rows), else quantized once by a launch of
+  // their own and then either bulk-copied into every CTA's shared memory (up to 16 rows, when
+  // they fit beside a two-stage ring) or read from global memory by the MMA loop.
+  // x_remote: x lives in mapped host memory - every CTA reading it over the bus would cost far
+  // more than the one pass of the quantization launch, so the planes are always staged.
+  // planes_ready: a preceding launch of the caller (RMSNorm prologue) already left the planes of
+  // these rows in act_scratch.
+  // Wide CTAs (planes shared by two sets of warps) where a CTA's half of the shared memory is too small for
+  // the planes but an SM's is not, and plan_gemv_wide says that this beats planes in global memory. The
+  // shares and sums are those of the narrow CTAs, bit for bit.
+  auto wide_stages = [&](int rows, int mg) {
+    int st = MAX_STAGES;
+    for (; st >= 2; st--)
+      if (plan_smem(DT, mg, true, rows, (int)k, st, stage_bytes, DT2, 2, red_slots_of(2, mg)).total <= smem_budget()) break;
+    return st;
+  };
+  bool wide = false;
+  int act_mode = (gemv_int8_fuses_act(DT, m, k) && !x_remote && !planes_ready) ? ACT_FUSED : ACT_GLOBAL;
+  {
+    const int rows0 = (int)(m < 32 ? m : 32), mg0 = rows0 <= 8 ? 1 : rows0 <= 16 ? 2 : 4;
+    if (act_mode == ACT_FUSED && stages_for(true, ctas_per_sm, rows0, mg0) < 2) act_mode = ACT_GLOBAL;
+    static const int stage_env = tuning_env("TURQ_GEMV_STAGED", 1);
+    if (act_mode == ACT_GLOBAL && m <= 16 && stage_env && stages_for(true, ctas_per_sm, rows0, mg0) >= 2) act_mode = ACT_STAGED;
+    if (act_mode == ACT_GLOBAL && m <= 16 && !xchg && ctas_per_sm == 2) {
+      constexpr GemvPlaneReads reads = DT == TQ_Q8_0 ? GemvPlaneReads::q8_0 : DT == TQ_Q6_K || MIXED ? GemvPlaneReads::q6_k : GemvPlaneReads::q45_k;
+      wide = plan_gemv_wide(reads, (int)m, split, T, KU, slots) && wide_stages(rows0, mg0) >= 2;
+      if (wide) act_mode = ACT_STAGED;
+    }
+  }
+  const bool fused = act_mode == ACT_FUSED, planes_in_smem = act_mode != ACT_GLOBAL;
+  if (MIXED && ((m > 8 && !wide) || act_mode == ACT_GLOBAL)) return cudaErrorNotSupported;
   const size_t x_es = x_dtype == TQ_BF16 ? 2 : 4;
   ActPackPlan plan = plan_act_pack(fmt, m, k);
   if (!fused && !planes_ready) {
@@ -831,8 +831,8 @@ static cudaError_t launch_dt(const GemvPart* parts, int nparts, int64_t k, const
     if (launches) (*launches)++;
     if (e != cudaSuccess) return e;
   }
-  for (int64_t m0 = 0; m0 < m; m0 += step) {
-    const int rows = (int)(m - m0 < step ? m - m0 : step);
+  for (int64_t m0 = 0; m0 < m; m0 += 32) {
+    const int rows = (int)(m - m0 < 32 ? m - m0 : 32);
     const int mg = rows <= 8 ? 1 : rows <= 16 ? 2 : 4;
     StreamArgs a{};
     for (int p = 0; p < nparts; p++) {

@@ -1,6 +1,6 @@
 // Host-side launch arithmetic of the GEMV and the GEMM, free of CUDA so that it can be
 // compiled and checked on a machine without a GPU: how the tiles of a weight are dealt out to
-// CTAs, how many CTAs share the K loop of a GEMM tile, which activation-tile height is used.
+// CTAs, which launches share their activation planes, how many CTAs share the K loop of a GEMM tile, which activation-tile height is used.
 #pragma once
 #include <cstdint>
 
@@ -42,6 +42,29 @@ inline GemvSplit plan_gemv_split(int row_tiles, int KU, int slots, int force = -
 inline int64_t gemv_split_start(const GemvSplit& p, int64_t total_units, int b) {
   const int64_t u = (int64_t)b * p.split_q + (b < p.split_r ? b : p.split_r);
   return u < total_units ? u : total_units;
+}
+
+// Whether a launch of up to 16 rows whose activation planes fit an SM's shared memory, but not a CTA's half
+// of it, runs as wide CTAs (one copy of the planes and two sets of warps per SM) or reads the planes from
+// global memory. What the wide form saves is the way to L2 per activation fragment, most for Q8_0 (an
+// f32 scale per 32 values beside the quants) and Q6_K (four-byte fragments), least for Q4_K and Q5_K; a
+// mixed launch also spares a launch per type. What it costs is ring stages (two to four instead of six)
+// and, where there are no more shares than SMs, half of the SMs. Measured on B200, global against wide, us:
+//   Q8_0        512 x 8192, 8 rows 13.7 / 9.7   5120 x 25600, 4 rows 41.4 / 33.4   2560 x 8192, 8 rows 13.5 / 13.7
+//   Q6_K        4096 x 12288, 4 rows 14.8 / 13.8   2048 x 5120, 12 rows 13.0 / 10.6
+//     shares cut, shorter than two row-tiles: 5120 x 25600, 2 rows 27.9 / 28.8   5120 x 13312, 7 rows 21.2 / 20.6
+//   Q4_K, Q5_K  4096 x 12288 Q4_K, 8 rows 14.0 / 12.7   25600 x 5120 Q4_K, 12 rows 41.4 / 33.5
+//     shares cut, shorter than two row-tiles: 5120 x 8192 Q4_K, 8 / 12 rows 14.3 / 15.4, 18.6 / 17.9
+//                                             6144 x 6144 Q4_K, 11 rows 16.6 / 17.3
+//     an SM for every share: 128 x 16384 Q4_K, 8 rows 11.5 / 13.4   640 x 8192 Q4_K, 8 / 12 rows 8.2 / 9.0, 12.7 / 11.4
+//     a third of the slots idle: 2560 x 8192 Q5_K, 8 / 12 rows 10.4 / 10.8, 14.3 / 12.9
+enum class GemvPlaneReads { q8_0, q6_k /* also mixed launches */, q45_k };
+inline bool plan_gemv_wide(GemvPlaneReads reads, int rows, const GemvSplit& split, int64_t total_units, int KU, int slots) {
+  const bool cut_short = !split.aligned && total_units < (int64_t)2 * KU * split.grid;
+  if (reads == GemvPlaneReads::q8_0) return true;
+  if (reads == GemvPlaneReads::q6_k) return rows > 3 || !cut_short;
+  if (cut_short || 2 * split.grid <= slots) return false;
+  return rows > 8 || (int64_t)split.grid * 10 >= (int64_t)slots * 7;
 }
 
 // ---- tcgen05 GEMM (pairs of CTAs, 256 weight rows per pair)
