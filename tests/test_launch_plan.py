@@ -126,6 +126,12 @@ def test_gemm_split_k_invariants(plan, n, k):
     assert plan.gemm_splits(n, 64, k, sms, 0) == 1
 
 
+def test_long_k_loops_are_shared_by_five_pairs_at_most(plan):
+    """More pairs were slower than the GEMM with a summing launch of its own at 48 to 64 rows."""
+    for n, k, cuts in ((1024, 5120, 5), (512, 8192, 5), (2560, 8192, 5), (5120, 25600, 3), (1024, 4096, 8), (640, 2560, 5)):
+        assert plan.gemm_splits(n, 64, k, 148, -1) == cuts
+
+
 def test_gemm_activation_tile_choice(plan):
     sms = 148
     assert plan.gemm_bn(12288, 64, sms, 0) == 64

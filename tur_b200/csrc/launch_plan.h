@@ -80,7 +80,7 @@ inline int plan_gemm_bn(int64_t n_rows, int64_t m, int sm_count, int force = 0) 
 
 // Split-K for decode batches (one activation tile of at most 64 rows): when the weight's row tiles
 // alone leave SMs without work, the K loop of every tile is shared out over several pairs (at least
-// 8 blocks of 64 each, at most 16 pairs). The split depends on the weight's shape only, so a row's
+// 8 blocks of 64 each, at most 5 pairs if it is longer than 4096). The split depends on the weight's shape only, so a row's
 // result does not depend on the batch it is in; prefill (more than 64 rows) never splits.
 // force: -1 = choose, 0 = never, > 0 = that many (still at least 8 blocks each).
 inline int plan_gemm_splits(int64_t n_rows, int64_t m, int64_t k, int sm_count, int force = -1) {
@@ -90,7 +90,11 @@ inline int plan_gemm_splits(int64_t n_rows, int64_t m, int64_t k, int sm_count, 
   const int64_t by_k = (k / 64) / 8;
   if (force > 0) s = force;
   if (s > by_k) s = by_k;
-  if (s > 16) s = 16;
+  // Long K loops: five pairs a tile. The owner adds the others' sums two pairs at a time (twice over beyond
+  // 40 rows), which soon costs more than the units it saves. Up to 16 pairs / 5, us a call: Q8_0 2560 x 8192, 32 / 64
+  // rows 13.9 / 13.2, 18.9 / 15.6; Q4_K 1024 x 5120, 32 / 64 rows 10.0 / 10.3, 12.9 / 11.7; Q8_0 512 x 8192,
+  // 64 rows 15.3 / 14.0. At 16 units a cut still pays: Q4_K 1024 x 4096, 32 / 64 rows 8.9 / 9.5, 11.5 / 11.1.
+  if (k > 16 * 256 && s > 5) s = 5;
   return s < 2 ? 1 : (int)s;
 }
 
