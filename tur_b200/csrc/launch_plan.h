@@ -1,6 +1,7 @@
 // Host-side launch arithmetic of the GEMV and the GEMM, free of CUDA so that it can be
 // compiled and checked on a machine without a GPU: how the tiles of a weight are dealt out to
-// CTAs, which launches share their activation planes, how many CTAs share the K loop of a GEMM tile, which activation-tile height is used.
+// CTAs, which launches share their activation planes, how many CTAs share the K loop of a GEMM tile,
+// which activation-tile height is used.
 #pragma once
 #include <cstdint>
 
@@ -71,8 +72,7 @@ inline bool plan_gemv_wide(GemvPlaneReads reads, int rows, const GemvSplit& spli
 
 // Class of the activation rows per pair tile: 64 for decode batches; 256 for prefill, unless twice
 // as many tiles still fit the SMs in one wave - then 128, which doubles the pairs at work.
-inline int plan_gemm_bn(int64_t n_rows, int64_t m, int sm_count, int force = 0) {
-  if (force == 64 || force == 128 || force == 256) return force;
+inline int plan_gemm_bn(int64_t n_rows, int64_t m, int sm_count) {
   int bn = m <= 64 ? 64 : 256;
   if (bn == 256 && 2 * ((n_rows + 127) / 128) * ((m + 255) / 256) <= sm_count) bn = 128;
   return bn;
@@ -80,15 +80,14 @@ inline int plan_gemm_bn(int64_t n_rows, int64_t m, int sm_count, int force = 0) 
 
 // Split-K for decode batches (one activation tile of at most 64 rows): when the weight's row tiles
 // alone leave SMs without work, the K loop of every tile is shared out over several pairs (at least
-// 8 blocks of 64 each, at most 5 pairs if it is longer than 4096). The split depends on the weight's shape only, so a row's
-// result does not depend on the batch it is in; prefill (more than 64 rows) never splits.
-// force: -1 = choose, 0 = never, > 0 = that many (still at least 8 blocks each).
-inline int plan_gemm_splits(int64_t n_rows, int64_t m, int64_t k, int sm_count, int force = -1) {
-  if (m > 64 || force == 0) return 1;
+// 8 blocks of 64 each, at most 5 pairs if it is longer than 4096). The split depends on the weight's
+// shape only, so a row's result does not depend on which batch of up to 64 rows it is in; prefill (more
+// than 64 rows) never splits, so its f32 sums associate differently.
+inline int plan_gemm_splits(int64_t n_rows, int64_t m, int64_t k, int sm_count) {
+  if (m > 64) return 1;
   const int64_t tiles = (n_rows + 255) / 256;
   int64_t s = tiles > 0 ? sm_count / 2 / tiles : 1;
   const int64_t by_k = (k / 64) / 8;
-  if (force > 0) s = force;
   if (s > by_k) s = by_k;
   // Long K loops: five pairs a tile. The owner adds the others' sums two pairs at a time (twice over beyond
   // 40 rows), which soon costs more than the units it saves. Up to 16 pairs / 5, us a call: Q8_0 2560 x 8192, 32 / 64
@@ -100,8 +99,10 @@ inline int plan_gemm_splits(int64_t n_rows, int64_t m, int64_t k, int sm_count, 
 
 // Pairs of CTAs and what is dealt out to them: whole tiles (round robin), or - decode batches - the
 // units of 256 k of all tiles in one even split. With plan_gemm_splits() > 1 the pairs are a multiple
-// of the tiles, so every cut is the same in every tile; a weight with more tiles than half the pairs
-// is cut wherever the even split falls (at least two units per pair).
+// of the tiles, so every cut is the same in every tile. Otherwise (more tiles than half the pairs, or a
+// K loop too short to be cut in two) the cuts are wherever the even split falls: on all pairs, or on so
+// many that each has two units, but never on fewer pairs than tiles while there are pairs: then a pair
+// may have one unit only.
 struct GemmWork {
   int pairs;
   int split_k;
