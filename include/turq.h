@@ -64,7 +64,10 @@ typedef enum {
  *               grows from 16 to 17 rows. A host that needs a token's result to be independent
  *               of the batch or chunk it arrives in (tur's tests/pipeline_integration.rs:275-369
  *               do) pins one scheme for all row counts with turq_ctx_set_auto_policy or passes
- *               an explicit mode. Within one mode results never depend on the other rows. */
+ *               an explicit mode. Within INT8_ACT and EXACT_F32 a row's bits never depend on the
+ *               other rows. TENSOR_CORE has one order of its f32 sums for up to 64 rows and one
+ *               for more: the values of the other rows and their number within either range
+ *               change nothing, but from 64 to 65 rows the last bits of a row may. */
 typedef enum {
   TURQ_MODE_AUTO = 0,
   TURQ_MODE_INT8_ACT = 1,

@@ -96,17 +96,17 @@ def test_mixed_type_qkv_launch_at_the_8b_shapes(tq, m):
 
 
 @pytest.mark.parametrize("dt,n,k,m,nrows", [
-    (Q4_K, 12288, 4096, 2048, 192),    # cfg3 ffn_gate, grid.y = 8
-    (Q4_K, 12288, 4096, 8192, 96),     # grid.y = 32
+    (Q4_K, 12288, 4096, 2048, 192),    # cfg3 ffn_gate, 8 activation tiles
+    (Q4_K, 12288, 4096, 8192, 96),     # 32 activation tiles
     (Q6_K, 4096, 12288, 2048, 128),    # cfg3 ffn_down
     (Q6_K, 4096, 12288, 8192, 64),
     (Q5_K, 12288, 4096, 512, 192),     # cfg3 Q5_K_M variant
-    (Q6_K, 5120, 25600, 64, 256),      # cfg5 ffn_down, decode batch: split-K over 40 tiles
-    (Q4_K, 1024, 5120, 64, 256),       # cfg5 attn_k: 8 tiles -> 16 K splits of 5 blocks
+    (Q6_K, 5120, 25600, 64, 256),      # cfg5 ffn_down, decode batch: the K loops of 20 tiles cut in 3
+    (Q4_K, 1024, 5120, 64, 256),       # cfg5 attn_k: 4 tiles, K loops cut in 10 of 2 units
     (Q6_K, 5120, 25600, 4096, 48),     # cfg5 prefill
     (Q8_0, 2560, 8192, 1024, 128),     # cfg4 Q8_0 ffn_down, prefill
 ], ids=["gate_q4k_m2048", "gate_q4k_m8192", "down_q6k_m2048", "down_q6k_m8192", "gate_q5k_m512",
-        "down32b_q6k_m64_splitk", "k32b_q4k_m64_splitk", "down32b_q6k_m4096", "down3b_q8_0_m1024"])
+        "down32b_q6k_m64_shared_k", "k32b_q4k_m64_shared_k", "down32b_q6k_m4096", "down3b_q8_0_m1024"])
 def test_tensor_core_scheme_at_config_shapes(tq, dt, n, k, m, nrows):
     rng = np.random.default_rng(SEED + n + k + m)
     qt, blocks2d = make(tq, dt, n, k, SEED + n + 1)

@@ -252,7 +252,7 @@ def test_tensor_core_mode_matches_f64_oracle(tq, dt, n, k, m):
     assert oracle.rel_fro(yb, oracle.matmul_f64(dt, w, n, k, xb.float().cpu().numpy())) < TOL
     # AUTO picks this path for prefill-sized M and results do not depend on the batch
     if 17 < m <= 64:
-        # decode batches: split-K depends on the weight's shape only, not on the batch
+        # decode batches: how the K loops are cut depends on the weight's shape only, not on the batch
         y17 = mm.forward(xd[:17], mode=tq.Mode.TENSOR_CORE)
         assert torch.equal(y17, mm.forward(xd, mode=tq.Mode.TENSOR_CORE)[:17])
     if m > 64:
@@ -477,10 +477,11 @@ def test_weight_quantizer_rejects_what_it_cannot_do(tq):
 
 @pytest.mark.parametrize("dt,n,k,m", [(oracle.Q8_0, 256, 1728, 100), (oracle.Q4_K, 256, 1792, 40), (oracle.Q6_K, 384, 1792, 40),
                                       (oracle.Q5_K, 128, 1792, 17)],
-                         ids=["q8_0_27_blocks_unsplit", "q4k_split_9_9_10", "q6k_split_9_9_10", "q5k_split"])
+                         ids=["q8_0_27_blocks_uncut", "q4k_7_units_cut_2_2_3", "q6k_7_units_cut_2_2_3", "q5k_7_units_cut_2_2_3"])
 def test_tensor_core_k_loop_with_an_odd_number_of_blocks(tq, dt, n, k, m):
-    """The GEMM's MMA thread handles two 64-wide K-blocks per barrier round; a K loop (or a CTA's
-    share of it under split-K) with an odd count ends on a half-filled pair."""
+    """Prefill: a stage of the GEMM's weight operand holds two 64-wide K-blocks, and a K loop with an odd
+    count of them (Q8_0) ends on a half-filled stage. Decode batches: a K loop of an odd number of 256-wide
+    units (K-quants are whole units) is cut unevenly between the pairs of CTAs that share it."""
     w = make_weight(dt, n, k, SEED + 3100 + k)
     rng = np.random.default_rng(SEED + 3101 + m)
     x = rng.standard_normal((m, k)).astype(np.float32)

@@ -174,10 +174,10 @@ def test_prefill_sized_row_parallel_product_is_cut_into_chunks(tq):
     tq.context().poll_status()
 
 
-@pytest.mark.parametrize("m", [40, 300], ids=["split_k_reduction_picks_the_slot", "gemm_epilogue_picks_the_slot"])
+@pytest.mark.parametrize("m", [40, 300], ids=["owner_of_a_shared_k_loop_picks_the_slot", "gemm_epilogue_picks_the_slot"])
 def test_tensor_core_product_lands_in_the_exchange_slot_without_a_copy(tq, m):
-    """In the tensor-core mode the GEMM's epilogue (or, for decode batches, its split-K
-    reduction) reads the call counter on the device and writes the slot of the upcoming call
+    """In the tensor-core mode the GEMM's epilogue (for decode batches that of the pair of CTAs that adds
+    the others' partial sums) reads the call counter on the device and writes the slot of the upcoming call
     itself. Four calls in a row alternate the slots; the stand-in peer contributes fresh data to
     each, so a product written to the wrong slot would show."""
     from tur_b200.tensor_parallel import TPGroup

@@ -444,11 +444,12 @@ int32_t turq_quantize_weights(turq_ctx* ctx, int32_t dtype, const float* dev_x, 
   return TURQ_OK;
 }
 
-// TURQ_MODE_AUTO: the integer GEMV up to 16 rows, the tcgen05 GEMM above (64-row activation
-// tiles with split-K for decode batches, 128/256-row tiles for prefill). Measured on B200 at 32
-// and 64 rows the GEMM is ahead for every weight shape of the benchmark configurations.
+// TURQ_MODE_AUTO: the integer GEMV up to 16 rows, the tcgen05 GEMM above (one activation tile and
+// shared K loops for decode batches of up to 64 rows, tiles of up to 256 rows for prefill). Measured
+// on B200 at 32 and 64 rows the GEMM is ahead for every weight shape of the benchmark configurations.
 // A context whose policy was pinned with turq_ctx_set_auto_policy uses that one scheme for every
-// row count, so a token's result does not depend on the batch or chunk it arrives in.
+// row count, so a token's result does not depend on the batch or chunk it arrives in (in the
+// tensor-core scheme: but for the association of its f32 sums, which differs from 64 to 65 rows).
 static int32_t auto_mode(const turq_ctx* ctx, int64_t n_rows, int64_t n_cols, int64_t m) {
   (void)n_rows;
   if (ctx->auto_policy != TURQ_MODE_AUTO) {

@@ -28,7 +28,7 @@
 // one activation tile): the K loop of a tile is shared between pairs; the pair that holds a tile's
 // first unit adds the others' partial sums in pair order (fixed order, no float atomics).
 //
-// What bounds it. Prefill: the tensor pipe (81 % of active cycles at 12288 x 4096 Q4_K, 2048 rows), the
+// What bounds it. Prefill: the tensor pipe (89 % of active cycles at 12288 x 4096 Q4_K, 2048 rows), the
 // power limit and the last wave of tiles. Decode batches: the rounds of barriers between the warps
 // (without any dequantization and a quarter of the MMAs the 25600 x 5120 launch below still takes 26 us)
 // and some 7 us of hand-overs (conversion, first activation tile, partial sums).
@@ -36,12 +36,12 @@
 // into registers, one ring for both operands and split-K sums added by a second launch:
 //   Q4_K 12288 x 4096, 2048 rows  231 -> 157 us (1310 TFLOP/s)   Q6_K 5120 x 25600, 64 rows  85 -> 48 us
 //   Q5_K 2560 x 2560, 32 rows    10.1 -> 9.0 us
-// Steps on the way: an MMA loop whose control flow is warp-uniform (2048 rows: 210 -> 173 us; with one
-// divergent thread the descriptors of every MMA went through moves to uniform registers); remote arrivals
-// without a cluster-scope release (270 -> 210 us; the proxy fence already orders the operand tile); no
-// way out of that loop on an expired wait (Q4_K 25600 x 5120, 32 rows: 42 -> 37 us); the decode weight
-// operand in TMEM (37 -> 34 us: its stores and the MMA's reads were two thirds of the shared-memory
-// traffic); whole units per decode stage (34 -> 33 us, Q6_K 5120 x 25600 51 -> 48 us).
+// Steps on the way: an MMA loop walked by the whole warp, one lane issuing, instead of by one divergent
+// thread (2048 rows: 210 -> 173 us); remote arrivals without a cluster-scope release (270 -> 210 us; the
+// proxy fence already orders the operand tile); no way out of that loop on an expired wait (Q4_K
+// 25600 x 5120, 32 rows: 42 -> 37 us); the decode weight operand in TMEM (37 -> 34 us: its stores and the
+// MMA's reads were two thirds of the shared-memory traffic); whole units per decode stage (34 -> 33 us,
+// Q6_K 5120 x 25600 51 -> 48 us).
 // Every wait is bounded; on expiry the CTA records TURQ_E_TIMEOUT, releases its TMEM and returns.
 #include <cstdlib>
 #include <cuda.h>
@@ -108,8 +108,8 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatil
   return false;
 }
 // The same for loops that do not look at the result: after an expiry the abort flag makes every further
-// wait return soon, and what such a loop then does stays within its buffers. Without the way out of
-// the loop its control flow is the same for the whole warp and its addresses stay in uniform registers.
+// wait return soon, and what such a loop then does stays within its buffers. Without the way out the
+// loop's control flow is the same for the whole warp.
 __device__ __noinline__ void bar_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   bar_wait(bar, parity, abort_flag);
 }
@@ -150,7 +150,8 @@ __device__ __forceinline__ uint32_t h22u(__half2 h) { return *reinterpret_cast<u
 // k order of both f16 operands: a 16-k chunk (one MMA) of an aligned 32 holds, for c = 0..3, elements
 // 8c + {0, 2, 1, 3} (first chunk) or 8c + 4 + {0, 2, 1, 3} (second) - what lane column c of a fragment
 // tile finds in one word, in the pairs the word gives without a shuffle. The same for prefill and decode
-// batches, so that a row's bits do not depend on which of the two it is in.
+// batches, so that one conversion serves both. (Their f32 sums still associate differently: decode batches
+// cut the K loops, prefill does not.)
 // bytes (b0, b2) / (b1, b3) of a word of small integers -> half2 (1024 + b0, 1024 + b2) / ...
 __device__ __forceinline__ __half2 pair02(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5240)); }
 __device__ __forceinline__ __half2 pair13(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5341)); }
@@ -489,6 +490,10 @@ __device__ __forceinline__ bool take_go(int* p) {
 // the workspace; the one that does adds the others' in pair order. Ready flags are per lane quarter
 // and chunk residue modulo HELPERS, so whoever takes a chunk finds it complete whether the other
 // side's last epilogue was shared between warps or not.
+// The wait for the flags ends: a pair waits for pairs of higher index only, and those that add to a tile
+// do not wait before they do. CTAs start in the order of their index, so of a launch's resident pairs only
+// the one that owns the tile in which the first missing pair begins can wait for a pair that has not
+// started; all others end and make room for it, whatever else runs on the GPU.
 template <int CH, bool SPLIT>
 __device__ __forceinline__ void epilogue(const GemmArgs& a, float* ybase, int t, int ka, int kb, int pair, int pairs, int rank,
                                          int quarter, int lane, uint32_t tmem, int h0, int hstep, volatile int* abort_flag) {
