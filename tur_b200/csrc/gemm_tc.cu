@@ -28,13 +28,13 @@
 // one activation tile): the K loop of a tile is shared between pairs; the pair that holds a tile's
 // first unit adds the others' partial sums in pair order (fixed order, no float atomics).
 //
-// What bounds it. Prefill: the tensor pipe (89 % of active cycles at 12288 x 4096 Q4_K, 2048 rows), the
+// What bounds it. Prefill: the tensor pipe (90 % of active cycles at 12288 x 4096 Q4_K, 2048 rows), the
 // power limit and the last wave of tiles. Decode batches: the rounds of barriers between the warps
 // (without any dequantization and a quarter of the MMAs the 25600 x 5120 launch below still takes 26 us)
 // and some 7 us of hand-overs (conversion, first activation tile, partial sums).
 // Measured with graph replay, conversion included, against one CTA per 128 rows with weights prefetched
 // into registers, one ring for both operands and split-K sums added by a second launch:
-//   Q4_K 12288 x 4096, 2048 rows  231 -> 157 us (1310 TFLOP/s)   Q6_K 5120 x 25600, 64 rows  85 -> 48 us
+//   Q4_K 12288 x 4096, 2048 rows  231 -> 161 us (1280 TFLOP/s)   Q6_K 5120 x 25600, 64 rows  85 -> 48 us
 //   Q5_K 2560 x 2560, 32 rows    10.1 -> 9.0 us
 // Steps on the way: an MMA loop walked by the whole warp, one lane issuing, instead of by one divergent
 // thread (2048 rows: 210 -> 173 us); remote arrivals without a cluster-scope release (270 -> 210 us; the
