@@ -1,0 +1,51 @@
+"""Cluster sizes of the decode-batch GEMM (plan_batch_cluster in tur_b200/csrc/launch_plan.h), compiled with g++ and checked
+on the CPU: every CTA of a cluster has units of its own, the measured choices are the ones taken, and the weights of a
+transformer layer that share an activation agree, so that they go out as one launch."""
+import ctypes
+import os
+import subprocess
+import tempfile
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+SHIM = r"""
+#include "launch_plan.h"
+extern "C" int batch_cluster(int tiles, int KU, const int* resident) { return turq::plan_batch_cluster(tiles, KU, resident); }
+"""
+B200 = [0, 148, 74, 45, 33, 26, 22]     # clusters of 1..6 CTAs that are resident at once
+
+
+@pytest.fixture(scope="module")
+def cluster():
+    with tempfile.TemporaryDirectory() as d:
+        src, so = os.path.join(d, "shim.cpp"), os.path.join(d, "shim.so")
+        open(src, "w").write(SHIM)
+        subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", os.path.join(ROOT, "tur_b200", "csrc"), src, "-o", so], check=True)
+        lib = ctypes.CDLL(so)
+
+        def call(n, k, resident=B200):
+            return lib.batch_cluster(-(-n // 128), -(-k // 256), (ctypes.c_int * 7)(*resident))
+        yield call
+
+
+def test_every_cta_has_units(cluster):
+    for resident in (B200, [0, 16, 8, 5, 4, 3, 2], [0, 1, 1, 1, 1, 1, 1]):
+        for n in (1, 128, 129, 640, 2560, 4096, 5120, 12288, 25600, 151936):
+            for k in (64, 256, 320, 512, 768, 1024, 2560, 4096, 6144, 8192, 25600):
+                c = cluster(n, k, resident)
+                assert 1 <= c <= 6 and c <= -(-k // 256), (n, k, c)
+                ku = -(-k // 256)
+                shares = [ku * (r + 1) // c - ku * r // c for r in range(c)]
+                assert min(shares) >= 1 and sum(shares) == ku
+
+
+@pytest.mark.parametrize("n,k,want", [(8192, 2560, 1), (12288, 4096, 2), (25600, 5120, 1), (3072, 1024, 2), (4096, 4096, 4), (2560, 2560, 4),
+                                      (5120, 25600, 3), (5120, 8192, 3), (2560, 8192, 6), (1024, 2048, 4)])
+def test_measured_choices(cluster, n, k, want):
+    assert cluster(n, k) == want
+
+
+@pytest.mark.parametrize("hidden,q,kv", [(1024, 2048, 1024), (2560, 2560, 640), (4096, 4096, 1024), (5120, 8192, 1024), (4096, 4096, 4096)])
+def test_projections_of_a_layer_share_a_launch(cluster, hidden, q, kv):
+    assert cluster(q, hidden) == cluster(kv, hidden)

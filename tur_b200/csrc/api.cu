@@ -183,7 +183,7 @@ int32_t turq_ctx_create(int32_t device, turq_ctx** out) {
   *ctx->host_done = 0;
   ctx->sm_count = prop.multiProcessorCount;
   const size_t ws_bytes = turq::gemv_workspace_bytes(ctx->sm_count);
-  const size_t gemm_ws_bytes = turq::gemm_tc_workspace_bytes(ctx->sm_count);
+  const size_t gemm_ws_bytes = turq::gemm_workspace_bytes(ctx->sm_count);
   if (cudaMalloc(reinterpret_cast<void**>(&ctx->gemv_ws), ws_bytes) != cudaSuccess ||
       cudaMemset(ctx->gemv_ws, 0, ws_bytes) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void**>(&ctx->gemm_ws), gemm_ws_bytes) != cudaSuccess ||
@@ -258,8 +258,7 @@ int32_t turq_ctx_poll_status(turq_ctx* ctx, void* stream) {
     *static_cast<volatile int*>(ctx->host_status) = 0;
     // a kernel that gave up may have left hand-over flags or claim counters set
     cudaMemsetAsync(ctx->gemv_ws, 0, turq::gemv_workspace_bytes(ctx->sm_count), s);
-    cudaMemsetAsync(ctx->gemm_ws + turq::gemm_tc_workspace_flags_offset(ctx->sm_count), 0,
-                    turq::gemm_tc_workspace_flags_bytes(ctx->sm_count), s);
+    cudaMemsetAsync(ctx->gemm_ws, 0, turq::gemm_workspace_bytes(ctx->sm_count), s);
     cudaStreamSynchronize(s);
     if (st == TURQ_E_INVALID_ARG) return fail(ctx, st, "an embedding lookup was given an id outside the table");
     return fail(ctx, st, "a kernel gave up a bounded device-side wait (status %d)", st);
@@ -444,8 +443,8 @@ int32_t turq_quantize_weights(turq_ctx* ctx, int32_t dtype, const float* dev_x, 
   return TURQ_OK;
 }
 
-// TURQ_MODE_AUTO: the integer GEMV up to 16 rows, the tcgen05 GEMM above (one activation tile and
-// shared K loops for decode batches of up to 64 rows, tiles of up to 256 rows for prefill). Measured
+// TURQ_MODE_AUTO: the integer GEMV up to 16 rows, the tcgen05 GEMMs above (gemm_batch.cu for decode
+// batches of up to 64 rows, gemm_tc.cu for prefill). Measured
 // on B200 at 32 and 64 rows the GEMM is ahead for every weight shape of the benchmark configurations.
 // A context whose policy was pinned with turq_ctx_set_auto_policy uses that one scheme for every
 // row count, so a token's result does not depend on the batch or chunk it arrives in (in the
@@ -487,8 +486,13 @@ int32_t turq_qmatmul(turq_ctx* ctx, const turq_qtensor* qt, const void* dev_x, i
   } else if (mode == TURQ_MODE_TENSOR_CORE) {
     int32_t st = ensure(ctx, &ctx->scratch, &ctx->scratch_bytes, turq::gemm_tc_scratch_bytes(m, k));
     if (st != TURQ_OK) return st;
-    e = turq::launch_gemm_tc(qt->dtype, qt->tiles, qt->n_rows, k, dev_x, x_dtype, m, dev_y, dev_bias, ctx->scratch,
-                             ctx->gemm_ws, ctx->sm_count, s, &launches, ctx->dev_status);
+    if (m <= turq::GEMM_BATCH_ROWS) {
+      const turq::GemvPart part{qt->tiles, qt->n_rows, dev_y, dev_bias, qt->dtype, nullptr};
+      e = turq::launch_gemm_batch(&part, 1, k, dev_x, x_dtype, m, ctx->scratch, s, &launches, ctx->dev_status);
+    } else {
+      e = turq::launch_gemm_tc(qt->dtype, qt->tiles, qt->n_rows, k, dev_x, x_dtype, m, dev_y, dev_bias, ctx->scratch,
+                               ctx->gemm_ws, ctx->sm_count, s, &launches, ctx->dev_status);
+    }
   } else {
     return fail(ctx, TURQ_E_INVALID_ARG, "unknown mode %d", mode);
   }
@@ -526,6 +530,17 @@ static int32_t qmatmul_multi_impl(turq_ctx* ctx, int32_t count, const turq_qtens
     TQ_CUDA(ctx, cudaSetDevice(ctx->device));
     int32_t st = ensure(ctx, &ctx->scratch, &ctx->scratch_bytes, turq::gemm_tc_scratch_bytes(m, k));
     if (st != TURQ_OK) return st;
+    if (m <= turq::GEMM_BATCH_ROWS) {
+      turq::GemvPart parts[4];
+      for (int i = 0; i < count; i++)
+        parts[i] = turq::GemvPart{qts[i]->tiles, qts[i]->n_rows, dev_ys[i], dev_biases ? dev_biases[i] : nullptr, qts[i]->dtype, nullptr};
+      int launches = 0;
+      cudaError_t e = turq::launch_gemm_batch(parts, count, k, dev_x, x_dtype, m, ctx->scratch, static_cast<cudaStream_t>(stream),
+                                              &launches, ctx->dev_status);
+      ctx->launches += launches;
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "qmatmul_multi launch");
+      return TURQ_OK;
+    }
     for (int i = 0; i < count; i++) {
       int launches = 0;
       cudaError_t e = turq::launch_gemm_tc(qts[i]->dtype, qts[i]->tiles, qts[i]->n_rows, k, dev_x, x_dtype, m, dev_ys[i],
@@ -534,8 +549,7 @@ static int32_t qmatmul_multi_impl(turq_ctx* ctx, int32_t count, const turq_qtens
                                            i + 1 < count ? qts[i + 1]->n_rows : 0);
       ctx->launches += launches;
       if (e != cudaSuccess && i > 0)  // the launch before this one has set its go-ahead words
-        cudaMemsetAsync(ctx->gemm_ws + turq::gemm_tc_workspace_flags_offset(ctx->sm_count), 0,
-                        turq::gemm_tc_workspace_flags_bytes(ctx->sm_count), static_cast<cudaStream_t>(stream));
+        cudaMemsetAsync(ctx->gemm_ws, 0, turq::gemm_workspace_bytes(ctx->sm_count), static_cast<cudaStream_t>(stream));
       if (e != cudaSuccess) return cuda_fail(ctx, e, "qmatmul_multi launch");
     }
     return TURQ_OK;
@@ -837,8 +851,11 @@ int32_t qmatmul_for_exchange(turq_ctx* ctx, const turq_qtensor* qt, const void* 
     int32_t st = ensure(ctx, &ctx->scratch, &ctx->scratch_bytes, gemm_tc_scratch_bytes(m, qt->n_cols));
     if (st != TURQ_OK) return st;
     int launches = 0;
-    cudaError_t e = launch_gemm_tc(qt->dtype, qt->tiles, qt->n_rows, qt->n_cols, dev_x, x_dtype, m, s0, local_bias, ctx->scratch,
-                                   ctx->gemm_ws, ctx->sm_count, s, &launches, ctx->dev_status, 0, 0, toggle, s1);
+    const GemvPart part{qt->tiles, qt->n_rows, s0, local_bias, qt->dtype, s1};
+    cudaError_t e = m <= GEMM_BATCH_ROWS
+                        ? launch_gemm_batch(&part, 1, qt->n_cols, dev_x, x_dtype, m, ctx->scratch, s, &launches, ctx->dev_status, toggle)
+                        : launch_gemm_tc(qt->dtype, qt->tiles, qt->n_rows, qt->n_cols, dev_x, x_dtype, m, s0, local_bias, ctx->scratch,
+                                         ctx->gemm_ws, ctx->sm_count, s, &launches, ctx->dev_status, 0, 0, toggle, s1);
     ctx->launches += launches;
     if (e != cudaSuccess) return cuda_fail(ctx, e, "row-parallel GEMM launch");
     return TURQ_OK;

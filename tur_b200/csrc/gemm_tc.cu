@@ -1,5 +1,5 @@
-// QMatMul::forward on the 5th-generation tensor cores (tcgen05 / TMEM): prefill and decode batches
-// of more than 16 rows.
+// QMatMul::forward on the 5th-generation tensor cores (tcgen05 / TMEM) for prefill: more than 64
+// activation rows (up to 64: gemm_batch.cu).
 //
 //   y[m, n] = sum_k x[m, k] * W[n, k]      W quantized (device fragment tiles), x f32 or bf16
 //
@@ -20,28 +20,18 @@
 //                   accumulator is double buffered (2 x 256 TMEM columns), so the next tile's MMAs
 //                   run meanwhile;
 //   * warps 7..22   dequantize (two groups of eight, each two 64-k blocks of a unit) from the raw ring
-//                   to f16 with packed half arithmetic and arrive on the leader's barrier. Prefill:
-//                   into shared memory, K-major 128B-swizzled. Decode batches: into TMEM (tcgen05.st),
-//                   where their few accumulator columns leave room for three units.
+//                   to f16 with packed half arithmetic into shared memory, K-major 128B-swizzled, and
+//                   arrive on the leader's barrier.
 // MMA roles: A = weights (rows = TMEM lanes), B = activations (columns).
-// Work: more than 64 rows: whole tiles, dealt out to persistent pairs. Decode batches (<= 64 rows,
-// one activation tile): the K loop of a tile is shared between pairs; the pair that holds a tile's
-// first unit adds the others' partial sums in pair order (fixed order, no float atomics).
+// Work: whole tiles, dealt out to persistent pairs.
 //
-// What bounds it. Prefill: the tensor pipe (90 % of active cycles at 12288 x 4096 Q4_K, 2048 rows), the
-// power limit and the last wave of tiles. Decode batches: the rounds of barriers between the warps
-// (without any dequantization and a quarter of the MMAs the 25600 x 5120 launch below still takes 26 us)
-// and some 7 us of hand-overs (conversion, first activation tile, partial sums).
+// What bounds it: the tensor pipe (90 % of active cycles at 12288 x 4096 Q4_K, 2048 rows), the
+// power limit and the last wave of tiles.
 // Measured with graph replay, conversion included, against one CTA per 128 rows with weights prefetched
-// into registers, one ring for both operands and split-K sums added by a second launch:
-//   Q4_K 12288 x 4096, 2048 rows  231 -> 161 us (1280 TFLOP/s)   Q6_K 5120 x 25600, 64 rows  85 -> 48 us
-//   Q5_K 2560 x 2560, 32 rows    10.1 -> 9.0 us
+// into registers and one ring for both operands: Q4_K 12288 x 4096, 2048 rows  231 -> 161 us (1280 TFLOP/s).
 // Steps on the way: an MMA loop walked by the whole warp, one lane issuing, instead of by one divergent
 // thread (2048 rows: 210 -> 173 us); remote arrivals without a cluster-scope release (270 -> 210 us; the
-// proxy fence already orders the operand tile); no way out of that loop on an expired wait (Q4_K
-// 25600 x 5120, 32 rows: 42 -> 37 us); the decode weight operand in TMEM (37 -> 34 us: its stores and the
-// MMA's reads were two thirds of the shared-memory traffic); whole units per decode stage (34 -> 33 us,
-// Q6_K 5120 x 25600 51 -> 48 us).
+// proxy fence already orders the operand tile).
 // Every wait is bounded; on expiry the CTA records TURQ_E_TIMEOUT, releases its TMEM and returns.
 #include <cstdlib>
 #include <cuda.h>
@@ -50,18 +40,14 @@
 #include <cstdio>
 
 #include "actquant.cuh"
-#include "device_utils.cuh"
-#include "gemv_tile.cuh"
 #include "launch_plan.h"
+#include "tc_common.cuh"
 #include "turq_internal.h"
 
 namespace turq {
 
 namespace {
 
-constexpr int BM = 128;      // weight rows per CTA; a pair's MMA covers 2 * BM
-constexpr int BK = 64;       // k per operand block (one 128-byte swizzle row of f16)
-constexpr int UNIT_K = 256;  // k per unit of raw weight bytes (four blocks)
 constexpr int MAX_ST = 8;    // operand stages
 constexpr int MAX_RAW = 8;   // raw ring slots
 constexpr int A_BYTES = BM * BK * 2;  // 16 KB per block
@@ -73,62 +59,10 @@ constexpr int TC_THREADS = (DQ_WARP0 + DQ_WARPS * DQ_GROUPS) * 32;
 // Register bound (72) of the kernel: leaves a CTA of the conversion kernel room beside it on an SM.
 constexpr int TC_REG_THREADS = 896;
 constexpr int TMEM_COLS = 512;     // two accumulators of 256 columns
-constexpr long long TC_WAIT_CYCLES = 4000000000ll;
 
-__device__ __forceinline__ uint32_t s_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(s_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void bar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void bar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(s_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool bar_try(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(s_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  if (bar_try(bar, parity)) return true;  // the common case costs one poll, no clock read
-  const long long t0 = clock64();
-  for (uint32_t i = 0;; i++) {
-    if (bar_try(bar, parity)) return true;
-    if ((i & 255u) == 255u && (*abort_flag || clock64() - t0 > TC_WAIT_CYCLES)) break;
-  }
-  *abort_flag = 1;
-  return false;
-}
-// The same for loops that do not look at the result: after an expiry the abort flag makes every further
-// wait return soon, and what such a loop then does stays within its buffers. Without the way out the
-// loop's control flow is the same for the whole warp.
-__device__ __noinline__ void bar_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  bar_wait(bar, parity, abort_flag);
-}
-__device__ __forceinline__ void bar_pass(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  if (!bar_try(bar, parity)) bar_wait_slow(bar, parity, abort_flag);
-}
 // The barriers of a pair's leader collect arrivals of both CTAs.
-__device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
 __device__ __forceinline__ void bar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
 }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -138,52 +72,6 @@ __device__ __forceinline__ void commit_to_pair(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(s_u32(bar)),
                "h"((unsigned short)3)
                : "memory");
-}
-
-// ---- dequantization to f16 with packed half arithmetic (two elements per instruction).
-// An integer q <= 1023 becomes the half 1024 + q by OR-ing it under the exponent 0x6400;
-// subtracting the offset is exact, so the only roundings are the f16 sub-block scale / min
-// and the final multiply-add. The error stays a few 1e-4 of the value, inside the 2e-3 budget
-// of the tensor-core mode (the bit-exact f32 decode lives in decode.cuh).
-__device__ __forceinline__ __half2 u2h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
-__device__ __forceinline__ uint32_t h22u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
-// k order of both f16 operands: a 16-k chunk (one MMA) of an aligned 32 holds, for c = 0..3, elements
-// 8c + {0, 2, 1, 3} (first chunk) or 8c + 4 + {0, 2, 1, 3} (second) - what lane column c of a fragment
-// tile finds in one word, in the pairs the word gives without a shuffle. The same for prefill and decode
-// batches, so that one conversion serves both. (Their f32 sums still associate differently: decode batches
-// cut the K loops, prefill does not.)
-// bytes (b0, b2) / (b1, b3) of a word of small integers -> half2 (1024 + b0, 1024 + b2) / ...
-__device__ __forceinline__ __half2 pair02(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5240)); }
-__device__ __forceinline__ __half2 pair13(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5341)); }
-__device__ __forceinline__ __half2 pair01(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5140)); }
-
-// Raw bytes of one unit (16 weight rows x 256 k) as they lie in a ring slot.
-template <int DT> struct UnitGeom {
-  static constexpr int TILES = UNIT_K / TileGeom<DT>::ELEMS;  // device tiles per unit: 8 (Q8_0) or 1
-  static constexpr int BYTES = TILES * TileGeom<DT>::BYTES;   // per row-tile
-};
-
-// Scales of the two 64-k blocks of a unit that a warp dequantizes (Q4_K / Q5_K): lane 2r + e holds,
-// for row r of the row-tile and block e of the warp's two, the f16 scale and negated min of the
-// block's two sub-blocks. Worked out once per unit and row instead of by every lane that needs them.
-struct UnitScales { uint32_t dl, ml; };
-template <int DT>
-__device__ __forceinline__ UnitScales unit_scales(const uint8_t* t, int i, int lane) {
-  UnitScales u{0u, 0u};
-  if constexpr (DT == TQ_Q4_K || DT == TQ_Q5_K) {
-    const __half2 off = __float2half2_rn(1024.f);
-    const uint4 hd = lds_v4(t + 16 * (lane >> 1));
-    // Half arithmetic only (no int->float / float->half conversions, which share one narrow pipe):
-    // d * sc is exact in f32, so one f16 multiply rounds it the same way.
-    const __half2 dd = u2h2(__byte_perm(hd.x, 0u, 0x1010)), mm = u2h2(__byte_perm(hd.x, 0u, 0x3232));
-    // 6-bit scales / mins of sub-blocks 0..3 or 4..7, one per byte; block i needs bytes 2(i&1), 2(i&1)+1
-    const uint32_t scw = i >= 2 ? ((hd.w & 0x0F0F0F0Fu) | ((hd.y >> 2) & 0x30303030u)) : (hd.y & 0x3F3F3F3Fu);
-    const uint32_t mnw = i >= 2 ? (((hd.w >> 4) & 0x0F0F0F0Fu) | ((hd.z >> 2) & 0x30303030u)) : (hd.z & 0x3F3F3F3Fu);
-    const int sh = 16 * (i & 1);
-    u.dl = h22u(__hmul2(dd, __hsub2(pair01(scw >> sh), off)));
-    u.ml = h22u(__hneg2(__hmul2(mm, __hsub2(pair01(mnw >> sh), off))));
-  }
-  return u;
 }
 
 // Dequantizes 64-k block i of a unit (t: the row-tile's raw bytes in shared memory), block e of the
@@ -299,104 +187,6 @@ __device__ __forceinline__ void dequant_block(const uint8_t* t, const UnitScales
   }
 }
 
-// The same 64-k block as registers of a tcgen05.st 16x256b.x4 (decode batches keep the weight operand in
-// TMEM): register 4j + 2h + e of lane 4g + c holds columns 8j + 2c + e of row g + 8h, two f16 each, so
-// chunk j (16 k, one MMA) has from this lane the elements 32 (j / 2) + 8c + 4 (j % 2) + {0, 2, 1, 3}.
-template <int DT>
-__device__ __forceinline__ void dequant_frag(const uint8_t* t, const UnitScales& us, int i, int e, int lane, uint32_t (&o)[16]) {
-  const int g = lane >> 2, c = lane & 3;
-  if constexpr (DT == TQ_Q8_0) {
-    const __half2 off = __float2half2_rn(1152.f);  // 1024 + 128: bytes are biased by xor 0x80
-#pragma unroll
-    for (int s = 0; s < 2; s++) {
-      const uint8_t* tt = t + (2 * i + s) * 544;
-      const uint4 q = lds_v4(tt + TQ_Q8_0_QS + 16 * lane);
-      const uint32_t w[2][2] = {{q.x ^ 0x80808080u, q.y ^ 0x80808080u}, {q.z ^ 0x80808080u, q.w ^ 0x80808080u}};
-#pragma unroll
-      for (int hr = 0; hr < 2; hr++) {
-        const __half2 d2 = __half2half2(__ushort_as_half((unsigned short)lds_u16(tt + 2 * (g + 8 * hr))));
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-          o[4 * (2 * s + b) + 2 * hr] = h22u(__hmul2(__hsub2(pair02(w[hr][b]), off), d2));
-          o[4 * (2 * s + b) + 2 * hr + 1] = h22u(__hmul2(__hsub2(pair13(w[hr][b]), off), d2));
-        }
-      }
-    }
-  } else if constexpr (DT == TQ_Q4_K || DT == TQ_Q5_K) {
-    constexpr int QS = DT == TQ_Q4_K ? TQ_Q4K_QS : TQ_Q5K_QS;
-    const uint4 q = lds_v4(t + QS + 512 * i + 16 * lane);
-    const uint32_t w[2][2] = {{q.x, q.y}, {q.z, q.w}};
-    uint32_t qh[2][2] = {{0, 0}, {0, 0}};
-    if constexpr (DT == TQ_Q5_K) {
-      const uint4 h4 = lds_v4(t + TQ_Q5K_QH + 16 * lane);
-      qh[0][0] = h4.x; qh[0][1] = h4.y; qh[1][0] = h4.z; qh[1][1] = h4.w;
-    }
-#pragma unroll
-    for (int hr = 0; hr < 2; hr++) {
-      const int src = 2 * (g + 8 * hr) + e;
-      const __half2 dl2 = u2h2(__shfl_sync(0xFFFFFFFFu, us.dl, src)), ml2 = u2h2(__shfl_sync(0xFFFFFFFFu, us.ml, src));
-#pragma unroll
-      for (int s = 0; s < 2; s++) {  // sub-blocks 2i (low nibbles) and 2i + 1 (high nibbles)
-        const __half2 dl = s ? __high2half2(dl2) : __low2half2(dl2), ml = s ? __high2half2(ml2) : __low2half2(ml2);
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-          __half2 v02, v13;
-          if constexpr (DT == TQ_Q4_K) {
-            // A nibble becomes a half without being moved: under the exponent of 1024 the low nibble counts
-            // ones, under that of 64 the high nibble (16 units of 1/16) does; the offset subtracts exactly.
-            const uint32_t mask = s ? 0x00F000F0u : 0x000F000Fu, magic = s ? 0x54005400u : 0x64006400u;
-            v02 = __hsub2(u2h2((w[hr][b] & mask) | magic), u2h2(magic));
-            v13 = __hsub2(u2h2(((w[hr][b] >> 8) & mask) | magic), u2h2(magic));
-          } else {
-            const __half2 off = __float2half2_rn(1024.f);
-            // the sub-block's bit, brought to bit 4 of every byte
-            const uint32_t m = ((w[hr][b] >> (4 * s)) & 0x0F0F0F0Fu) |
-                               (__funnelshift_l(qh[hr][b], qh[hr][b], 4 - (2 * i + s)) & 0x10101010u);
-            v02 = __hsub2(pair02(m), off);
-            v13 = __hsub2(pair13(m), off);
-          }
-          o[4 * (2 * s + b) + 2 * hr] = h22u(__hfma2(v02, dl, ml));
-          o[4 * (2 * s + b) + 2 * hr + 1] = h22u(__hfma2(v13, dl, ml));
-        }
-      }
-    }
-  } else {  // Q6_K: a lane takes its eight elements of every 32 from the two lanes that hold them in the tile
-    const int nib = c >> 1, la = 4 * g + 2 * (c & 1);
-    const uint8_t* const qhp = t + TQ_Q6K_QH + 512 * (i >> 1) + 4 * (i & 1) + 16 * la;
-    const uint4 qa = lds_v4(t + TQ_Q6K_QL + 512 * i + 16 * la), qb = lds_v4(t + TQ_Q6K_QL + 512 * i + 16 * la + 16);
-    const __half2 off = __float2half2_rn(1056.f);     // 1024 + 32
-    const __half2 off_sc = __float2half2_rn(1152.f);  // 1024 + 128: the int8 scales are biased by xor 0x80
-#pragma unroll
-    for (int hr = 0; hr < 2; hr++) {
-      const uint32_t ql[2][2] = {{hr ? qa.z : qa.x, hr ? qb.z : qb.x}, {hr ? qa.w : qa.y, hr ? qb.w : qb.y}};
-      const uint32_t qh[2] = {ld_u32(qhp + 8 * hr), ld_u32(qhp + 16 + 8 * hr)};
-      // d * scale of sub-blocks 4i + nib and 4i + 2 + nib in half arithmetic (exact product, one rounding)
-      const __half2 dd = __half2half2(__ushort_as_half((unsigned short)lds_u16(t + TQ_Q6K_D + 2 * (g + 8 * hr))));
-      const uint32_t scb = ld_u32(t + 16 * (g + 8 * hr) + 4 * i) ^ 0x80808080u;
-      const __half2 dl2 = __hmul2(dd, __hsub2(pair02(scb >> (8 * nib)), off_sc));
-#pragma unroll
-      for (int s = 0; s < 2; s++) {
-        const __half2 dl = s ? __high2half2(dl2) : __low2half2(dl2);
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-          // 2-bit field 2s + nib of the qh word, brought to bits 4..5 of every byte
-          const uint32_t m = ((ql[s][b] >> (4 * nib)) & 0x0F0F0F0Fu) |
-                             (__funnelshift_l(qh[b], qh[b], 4 - 4 * s - 2 * nib) & 0x30303030u);
-          o[4 * (2 * s + b) + 2 * hr] = h22u(__hmul2(__hsub2(pair02(m), off), dl));
-          o[4 * (2 * s + b) + 2 * hr + 1] = h22u(__hmul2(__hsub2(pair13(m), off), dl));
-        }
-      }
-    }
-  }
-}
-__device__ __forceinline__ void tmem_store_block(uint32_t taddr, const uint32_t (&o)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-      "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(o[8]), "r"(o[9]), "r"(o[10]),
-      "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]), "r"(o[15])
-      : "memory");
-}
-
 struct GemmArgs {
   const uint8_t* tiles;
   int64_t n_rows;   // weight rows (output features)
@@ -407,8 +197,7 @@ struct GemmArgs {
   int m;            // activation rows
   int bn;           // activation rows per pair tile: a multiple of 16, at most 256
   int mt;           // activation tiles
-  int total;        // split_k: units of all tiles, shared out evenly; else: tiles
-  int split_k;
+  int total;        // tiles
   int sibling;      // the preceding launch belongs to the same call and reads the same x (see the kernel)
   int* go;          // [CTA] a sibling's go-ahead words, zero between launches
   int* next_go;     // those of the launch behind this one, which has next_ctas CTAs (0: no sibling follows)
@@ -417,8 +206,6 @@ struct GemmArgs {
   const float* rscale;  // [m] factor undoing the f16 row scaling
   float* y;             // [m, n_rows]
   const float* bias;
-  float* partial;       // [CTA][bn / 4][128][4]: partial sums of a CTA that does not own its first tile
-  int* flags;           // [CTA][4 lane quarters][8, HELPERS used], all zero between launches
   int* status;
   // exchange slots (tp.cu): with y_toggle set, the result goes to y_alt instead of y when the
   // word it points to, plus one, is odd - read after the preceding kernels have completed
@@ -426,44 +213,22 @@ struct GemmArgs {
   float* y_alt;
 };
 
-// The tiles (or shares of tiles) a pair works on, in order; every role of both CTAs walks the same list.
-struct Segments {
-  int u, u1, step, KU;
-  bool split;
-  __device__ __forceinline__ static int start(const GemmArgs& a, int pair, int pairs) {
-    return (int)((int64_t)a.total * pair / pairs);
-  }
+// The tiles a pair works on, in order; every role of both CTAs walks the same list.
+struct Tiles {
+  int u, total, step;
   __device__ __forceinline__ void init(const GemmArgs& a, int pair, int pairs) {
-    split = a.split_k != 0;
-    KU = a.KU;
-    u = split ? start(a, pair, pairs) : pair;
-    u1 = split ? start(a, pair + 1, pairs) : a.total;
+    u = pair;
+    total = a.total;
     step = pairs;
   }
-  __device__ __forceinline__ bool last() const { return u >= u1; }  // after next(): nothing follows
-  // units [ka, kb) of tile `t`
-  __device__ __forceinline__ bool next(int& t, int& ka, int& kb) {
-    if (u >= u1) return false;
-    if (!split) {
-      t = u; ka = 0; kb = KU;
-      u += step;
-      return true;
-    }
-    t = u / KU;
-    ka = u - t * KU;
-    kb = ka + (u1 - u);
-    if (kb > KU) kb = KU;
-    u += kb - ka;
+  __device__ __forceinline__ bool last() const { return u >= total; }  // after next(): nothing follows
+  __device__ __forceinline__ bool next(int& t) {
+    if (u >= total) return false;
+    t = u;
+    u += step;
     return true;
   }
 };
-
-__device__ __forceinline__ int ld_acquire(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release(int* p, int v) { asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
 
 // Siblings (the later weights of a call) run beside their predecessor, so griddepcontrol.wait, which
 // waits for its end, cannot be what makes the shared operand visible to them. Instead every CTA of a
@@ -485,132 +250,52 @@ __device__ __forceinline__ bool take_go(int* p) {
   return v != 0;
 }
 
-// Epilogue of one segment for one TMEM lane quarter (32 weight rows): columns in chunks of CH, the
-// chunks h0, h0 + hstep, ... A pair that does not hold the tile's first unit parks its sums in
-// the workspace; the one that does adds the others' in pair order. Ready flags are per lane quarter
-// and chunk residue modulo HELPERS, so whoever takes a chunk finds it complete whether the other
-// side's last epilogue was shared between warps or not.
-// The wait for the flags ends: a pair waits for pairs of higher index only, and those that add to a tile
-// do not wait before they do. CTAs start in the order of their index, so of a launch's resident pairs only
-// the one that owns the tile in which the first missing pair begins can wait for a pair that has not
-// started; all others end and make room for it, whatever else runs on the GPU.
-template <int CH, bool SPLIT>
-__device__ __forceinline__ void epilogue(const GemmArgs& a, float* ybase, int t, int ka, int kb, int pair, int pairs, int rank,
-                                         int quarter, int lane, uint32_t tmem, int h0, int hstep, volatile int* abort_flag) {
+// Epilogue of one tile for one TMEM lane quarter (32 weight rows): columns in chunks of 16, the
+// chunks h0, h0 + hstep, ...
+__device__ __forceinline__ void epilogue(const GemmArgs& a, float* ybase, int t, int rank, int quarter, int lane, uint32_t tmem, int h0, int hstep) {
+  constexpr int CH = 16;
   const int m0 = (t % a.mt) * a.bn;
   const int cols = a.m - m0 < a.bn ? a.m - m0 : a.bn;
   const int nchunks = (cols + CH - 1) / CH;
   const int64_t n = (int64_t)(t / a.mt) * (2 * BM) + rank * BM + 32 * quarter + lane;
-  const bool owner = !SPLIT || ka == 0;
-  const int cta = 2 * pair + rank;
-  const int nflags = nchunks < HELPERS ? nchunks : HELPERS;
-  int nother = 0;  // pairs that hold the rest of this tile
-  if (SPLIT && owner && kb < a.KU) {
-    while (pair + 1 + nother < pairs && Segments::start(a, pair + 1 + nother, pairs) < (t + 1) * a.KU) nother++;
-    const long long t0 = clock64();
-    for (int f0 = h0; f0 < nflags; f0 += hstep)
-      for (int o = lane; o < nother; o += 32) {
-        const int* f = a.flags + ((cta + 2 * (o + 1)) * 4 + quarter) * 8 + f0;
-        while (ld_acquire(f) == 0) {
-          if (*abort_flag || clock64() - t0 > TC_WAIT_CYCLES) { *abort_flag = 1; break; }
-        }
-      }
-    __syncwarp();
-  }
-  const float bv = (owner && a.bias && n < a.n_rows) ? a.bias[n] : 0.f;
+  const float bv = (a.bias && n < a.n_rows) ? a.bias[n] : 0.f;
   float* const yp = ybase + (int64_t)m0 * a.n_rows + n;
-  float* const part = a.partial + ((size_t)cta * (a.bn >> 2) * BM + (32 * quarter + lane)) * 4;
-  const size_t part_pair = (size_t)2 * (a.bn >> 2) * BM * 4;  // the same CTA of the next pair
   for (int ch = h0; ch < nchunks; ch += hstep) {
     const int col0 = ch * CH;
     uint32_t v[CH];
     const uint32_t taddr = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)col0;
-    if constexpr (CH == 16) {
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-          "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-            "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-          : "r"(taddr)
-          : "memory");
-    } else {
-      asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                   : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                   : "r"(taddr)
-                   : "memory");
-    }
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-    if (!owner) {
+    if (n < a.n_rows) {
 #pragma unroll
-      for (int j = 0; j < CH; j += 4)
-        __stcg(reinterpret_cast<uint4*>(part + (size_t)((col0 + j) >> 2) * BM * 4), make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]));
-    } else {
-      if constexpr (SPLIT) {
-        constexpr int B = 2;  // other pairs whose sums are in flight at once
-        for (int o = 1; o <= nother; o += B) {
-          float4 p[B][CH / 4];
-#pragma unroll
-          for (int b = 0; b < B; b++)
-#pragma unroll
-            for (int j = 0; j < CH / 4; j++)
-              if (o + b <= nother) p[b][j] = __ldcg(reinterpret_cast<const float4*>(part + (o + b) * part_pair + (size_t)((col0 >> 2) + j) * BM * 4));
-#pragma unroll
-          for (int b = 0; b < B; b++)
-            if (o + b <= nother) {
-#pragma unroll
-              for (int j = 0; j < CH / 4; j++) {
-                v[4 * j] = __float_as_uint(__uint_as_float(v[4 * j]) + p[b][j].x);
-                v[4 * j + 1] = __float_as_uint(__uint_as_float(v[4 * j + 1]) + p[b][j].y);
-                v[4 * j + 2] = __float_as_uint(__uint_as_float(v[4 * j + 2]) + p[b][j].z);
-                v[4 * j + 3] = __float_as_uint(__uint_as_float(v[4 * j + 3]) + p[b][j].w);
-              }
-            }
-        }
-      }
-      if (n < a.n_rows) {
-#pragma unroll
-        for (int j = 0; j < CH; j++)
-          if (col0 + j < cols) yp[(int64_t)(col0 + j) * a.n_rows] = __uint_as_float(v[j]) * a.rscale[m0 + col0 + j] + bv;
-      }
-    }
-  }
-  if constexpr (SPLIT) {
-    if (!owner) {
-      __syncwarp();
-      if (lane == 0)
-        for (int f0 = h0; f0 < nflags; f0 += hstep) st_release(a.flags + (cta * 4 + quarter) * 8 + f0, 1);
-    } else {
-      __syncwarp();
-      for (int f0 = h0; f0 < nflags; f0 += hstep)  // consumed: zero again for the next launch
-        for (int o = lane; o < nother; o += 32) a.flags[((cta + 2 * (o + 1)) * 4 + quarter) * 8 + f0] = 0;
+      for (int j = 0; j < CH; j++)
+        if (col0 + j < cols) yp[(int64_t)(col0 + j) * a.n_rows] = __uint_as_float(v[j]) * a.rscale[m0 + col0 + j] + bv;
     }
   }
 }
 
-// SPLIT: decode batches of at most 64 rows (K loops shared between pairs).
-template <int DT, bool SPLIT>
+template <int DT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_REG_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ GemmArgs a) {
   constexpr int TB = TileGeom<DT>::BYTES;
   constexpr int UB = UnitGeom<DT>::BYTES;
   constexpr int SLOT_BYTES = 8 * UB;
-  // 64-k blocks per stage of the weight and of the activation operand. Decode batches: a whole unit, since
-  // with few activation rows it is the barrier rounds of the MMA loop that separate the MMAs.
-  constexpr int KA = SPLIT ? 4 : 2, KB = SPLIT ? 4 : 1;
-  // Decode batches (SPLIT) need few accumulator columns: their weight operand lies in the rest of TMEM,
-  // 32 columns per 64-k block, instead of in shared memory.
-  constexpr int ACC_COLS = SPLIT ? 64 : 256;
-  constexpr int A_COL0 = 2 * ACC_COLS;
-  constexpr int A_COLS = 32;  // per block
-  constexpr int CH = SPLIT ? 8 : 16;  // columns per epilogue step
+  constexpr int KA = 2;          // 64-k blocks per stage of the weight operand (one per stage of the activation operand)
+  constexpr int ACC_COLS = 256;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // 1024-byte alignment for the swizzled tiles; the same offsets in both CTAs of the pair
   uint8_t* smem = smem_raw + ((1024u - (s_u32(smem_raw) & 1023u)) & 1023u);
   const int SA = a.a_stages, SB = a.b_stages, RS = a.raw_slots;
   const int b_bytes = a.bn * (BK * 2 / 2);  // this CTA's half of the activation tile, per block
   uint8_t* sA = smem;
-  uint8_t* sB = sA + (SPLIT ? 0 : SA * KA * A_BYTES);
-  uint8_t* sRaw = sB + SB * KB * b_bytes;
+  uint8_t* sB = sA + SA * KA * A_BYTES;
+  uint8_t* sRaw = sB + SB * b_bytes;
   // The two operands have rings of their own: an activation tile is a trip to L2 away and needs many
   // stages in flight, a weight tile comes from this SM's raw ring and needs few.
   // a_full[s] (leader only): both CTAs' weight tiles, one arrival per dequantize warp
@@ -636,7 +321,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
   if (a.sibling && warp == 1 && lane == 0) go = take_go(a.go + blockIdx.x);
   if (threadIdx.x == 0) {
     for (int s = 0; s < SA; s++) {
-      bar_init(&a_full[s], (SPLIT ? 2 : 1) * 2 * DQ_WARPS);
+      bar_init(&a_full[s], 2 * DQ_WARPS);
       bar_init(&a_empty[s], 1);
     }
     for (int s = 0; s < SB; s++) {
@@ -666,9 +351,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
 
-  Segments seg;
+  Tiles seg;
   seg.init(a, pair, pairs);
-  int t, ka, kb;
+  int t;
   if (warp == 0) {
     // ------------------------------------------------------------ raw weight bytes -> ring
     // Lane r < 8 copies row-tile r's share of the unit: issued by one lane, the eight copies of a unit
@@ -676,12 +361,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
     int slot = 0;
     uint32_t ph = 0;
     bool ok = true;
-    while (ok && seg.next(t, ka, kb)) {
+    while (ok && seg.next(t)) {
       const int rt0 = (t / a.mt) * 16 + (int)rank * 8;
       int nlive = a.row_tiles - rt0;
       nlive = nlive < 0 ? 0 : nlive > 8 ? 8 : nlive;
       const uint8_t* const row = a.tiles + (int64_t)(rt0 + lane) * a.ktiles * TB;
-      for (int ku = ka; ku < kb; ku++) {
+      for (int ku = 0; ku < a.KU; ku++) {
         ok = __all_sync(0xFFFFFFFFu, bar_wait(&raw_empty[slot], ph ^ 1u, abort_flag));
         if (!ok) break;
         int nt = a.ktiles - ku * UnitGeom<DT>::TILES;
@@ -717,20 +402,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      while (ok && seg.next(t, ka, kb)) {
+      while (ok && seg.next(t)) {
         const int row = (t % a.mt) * a.bn + (int)rank * (a.bn >> 1);
-        const int k1 = kb * 4 < a.kblocks ? kb * 4 : a.kblocks;
-        for (int k = ka * 4; k < k1; k += KB) {
+        for (int k = 0; k < a.kblocks; k++) {
           ok = bar_wait(&b_empty[s], ph ^ 1u, abort_flag);
           if (!ok) break;
-          const int nk = k1 - k < KB ? k1 - k : KB;
-          if (rank == 0) bar_expect_tx(&b_full[s], 2u * (uint32_t)(nk * b_bytes));
-          for (int b = 0; b < nk; b++)
-            asm volatile(
-                "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                    s_u32(sB + (s * KB + b) * b_bytes)),
-                "l"(&xmap), "r"((k + b) * BK), "r"(row), "r"(map_to_rank(s_u32(&b_full[s]), 0))
-                : "memory");
+          if (rank == 0) bar_expect_tx(&b_full[s], 2u * (uint32_t)b_bytes);
+          asm volatile(
+              "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                  s_u32(sB + s * b_bytes)),
+              "l"(&xmap), "r"(k * BK), "r"(row), "r"(map_to_rank(s_u32(&b_full[s]), 0))
+              : "memory");
           if (++s == SB) { s = 0; ph ^= 1u; }
         }
       }
@@ -751,7 +433,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
       const bool issuer = elect_one();
       int s = 0, sb = 0, nseg = 0;
       uint32_t ph = 0, bph = 0;
-      while (seg.next(t, ka, kb)) {
+      while (seg.next(t)) {
         const int acc = nseg & 1;
         const uint32_t aph = (uint32_t)(nseg >> 1) & 1u;
         nseg++;
@@ -759,47 +441,32 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d = tmem_base + (uint32_t)(acc * ACC_COLS);
         uint32_t accumulate = 0;  // the first MMA of the tile overwrites the accumulator
-        const int k1 = kb * 4 < a.kblocks ? kb * 4 : a.kblocks;
-        for (int k = ka * 4; k < k1; k += KA) {
+        for (int k = 0; k < a.kblocks; k += KA) {
           const uint64_t da0 = desc_hi | (uint64_t)(a_lo0 + (uint32_t)(s * KA) * (A_BYTES >> 4));
           bar_pass(&a_full[s], ph, abort_flag);
 #pragma unroll
           for (int b = 0; b < KA; b++) {
-            if (b == 0 || k + b < k1) {
-              const bool last = b == KA - 1 || k + b + 1 >= k1;
-              if (b % KB == 0) {
-                bar_pass(&b_full[sb], bph, abort_flag);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              }
-              const uint64_t db0 = desc_hi | (uint64_t)(b_lo0 + (uint32_t)(sb * KB + b % KB) * b_step);
+            if (b == 0 || k + b < a.kblocks) {
+              const bool last = b == KA - 1 || k + b + 1 >= a.kblocks;
+              bar_pass(&b_full[sb], bph, abort_flag);
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              const uint64_t db0 = desc_hi | (uint64_t)(b_lo0 + (uint32_t)sb * b_step);
               if (issuer) {
 #pragma unroll
                 for (int kk = 0; kk < BK / 16; kk++) {
-                  if constexpr (SPLIT) {  // weight operand in TMEM
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\t"
-                        "setp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
-                        "r"(tmem_base + (uint32_t)(A_COL0 + (s * KA + b) * A_COLS + 8 * kk)), "l"(db0 + (uint64_t)(2 * kk)), "r"(idesc),
-                        "r"(b + kk > 0 ? 1u : accumulate)
-                        : "memory");
-                  } else {
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\t"
-                        "setp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-                        "l"(da0 + (uint64_t)(b * (A_BYTES >> 4) + 2 * kk)), "l"(db0 + (uint64_t)(2 * kk)), "r"(idesc),
-                        "r"(b + kk > 0 ? 1u : accumulate)
-                        : "memory");
-                  }
+                  asm volatile(
+                      "{\n\t.reg .pred p;\n\t"
+                      "setp.ne.b32 p, %4, 0;\n\t"
+                      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+                      "l"(da0 + (uint64_t)(b * (A_BYTES >> 4) + 2 * kk)), "l"(db0 + (uint64_t)(2 * kk)), "r"(idesc),
+                      "r"(b + kk > 0 ? 1u : accumulate)
+                      : "memory");
                 }
                 // release the stages to both CTAs' producers once these MMAs have read them
-                if (KB == 1 || last) commit_to_pair(&b_empty[sb]);
+                commit_to_pair(&b_empty[sb]);
                 if (last) commit_to_pair(&a_empty[s]);
               }
-              if (KB == 1 || last) {
-                if (++sb == SB) { sb = 0; bph ^= 1u; }
-              }
+              if (++sb == SB) { sb = 0; bph ^= 1u; }
             }
           }
           accumulate = 1u;
@@ -819,15 +486,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
     const int quarter = warp & 3;
     const uint32_t empty0 = map_to_rank(s_u32(&acc_empty[0]), 0);
     int nseg = 0;
-    while (seg.next(t, ka, kb)) {
+    while (seg.next(t)) {
       const int acc = nseg & 1;
       const uint32_t aph = (uint32_t)(nseg >> 1) & 1u;
       nseg++;
       if (!(seg.last() ? bar_wait(last_full, 0, abort_flag) : bar_wait(&acc_full[acc], aph, abort_flag))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // the last epilogue is shared with the dequantize warps, which have nothing left to do
-      epilogue<CH, SPLIT>(a, ybase, t, ka, kb, pair, pairs, (int)rank, quarter, lane, tmem_base + (uint32_t)(acc * ACC_COLS), 0,
-                          seg.last() ? HELPERS : 1, abort_flag);
+      epilogue(a, ybase, t, (int)rank, quarter, lane, tmem_base + (uint32_t)(acc * ACC_COLS), 0, seg.last() ? HELPERS : 1);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) bar_arrive_cluster(empty0 + 8u * (uint32_t)acc);
@@ -842,51 +508,38 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
     const uint32_t a_full0 = map_to_rank(s_u32(&a_full[0]), 0);
     int slot = 0, s = 0, nseg = 0;
     uint32_t rph = 0, ph = 0;
-    int lt = 0, lka = 0, lkb = 0;  // the last segment
-    while (seg.next(t, ka, kb)) {
-      lt = t; lka = ka; lkb = kb;
+    int lt = 0;  // the last tile
+    while (seg.next(t)) {
+      lt = t;
       nseg++;
       const bool live = (t / a.mt) * 16 + (int)rank * 8 + dq < a.row_tiles;  // rows beyond the weight are never stored
-      for (int ku = ka; ku < kb; ku++) {
+      for (int ku = 0; ku < a.KU; ku++) {
         bar_pass(&raw_full[slot], rph, abort_flag);
         const uint8_t* raw = sRaw + slot * SLOT_BYTES + dq * UB;
         int nb = a.kblocks - 4 * ku;
         if (nb > 4) nb = 4;
         nb -= 2 * grp;  // this group makes the unit's blocks 2 grp, 2 grp + 1
-        if (SPLIT || nb > 0) {
+        if (nb > 0) {
           const UnitScales us = unit_scales<DT>(raw, 2 * grp + (lane & 1), lane);
-          int si = SPLIT ? s : s + grp;
+          int si = s + grp;
           uint32_t phi = ph;
           if (si >= SA) { si -= SA; phi ^= 1u; }
           bar_pass(&a_empty[si], phi ^ 1u, abort_flag);
-          if constexpr (SPLIT) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-            for (int b = 0; b < 2; b++)
-              if (live && b < nb) {
-                uint32_t o[16];
-                dequant_frag<DT>(raw, us, 2 * grp + b, b, lane, o);
-                tmem_store_block(tmem_base + ((uint32_t)(16 * dq) << 16) + (uint32_t)(A_COL0 + (si * KA + 2 * grp + b) * A_COLS), o);
-              }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          } else {
-#pragma unroll
-            for (int b = 0; b < 2; b++)
-              if (live && b < nb) dequant_block<DT>(raw, us, 2 * grp + b, b, lane, sA + (si * KA + b) * A_BYTES + dq * 16 * 128);
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> visible to the MMA
-          }
+          for (int b = 0; b < 2; b++)
+            if (live && b < nb) dequant_block<DT>(raw, us, 2 * grp + b, b, lane, sA + (si * KA + b) * A_BYTES + dq * 16 * 128);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> visible to the MMA
           __syncwarp();
           if (lane == 0) bar_arrive_cluster(a_full0 + 8u * (uint32_t)si);
         }
-        s += !SPLIT && a.kblocks - 4 * ku > KA ? 2 : 1;
+        s += a.kblocks - 4 * ku > KA ? 2 : 1;
         if (s >= SA) { s -= SA; ph ^= 1u; }
         __syncwarp();
         if (lane == 0) bar_arrive(&raw_empty[slot]);
         if (++slot == RS) { slot = 0; rph ^= 1u; }
       }
     }
-    // nothing left to dequantize: help with the epilogue of the last segment
+    // nothing left to dequantize: help with the epilogue of the last tile
     if (nseg > 0) {
       if (!a.sibling) asm volatile("griddepcontrol.wait;" ::: "memory");
       float* ybase = a.y;
@@ -894,8 +547,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
       const int acc = (nseg - 1) & 1;
       if (bar_wait(last_full, 0, abort_flag)) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        epilogue<CH, SPLIT>(a, ybase, lt, lka, lkb, pair, pairs, (int)rank, warp & 3, lane, tmem_base + (uint32_t)(acc * ACC_COLS),
-                            (warp - DQ_WARP0) / 4 + 1, HELPERS, abort_flag);
+        epilogue(a, ybase, lt, (int)rank, warp & 3, lane, tmem_base + (uint32_t)(acc * ACC_COLS), (warp - DQ_WARP0) / 4 + 1, HELPERS);
       }
     }
   }
@@ -921,15 +573,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
   if (a.sibling && threadIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// x [m, k] (f32 / bf16) -> f16 [m, k] with a per-row power-of-two scale that brings the row's
+// x [m, k] (f32 / bf16) -> f16 with a per-row power-of-two scale that brings the row's
 // largest magnitude into [8192, 16384): rows of large values do not overflow f16 and rows of
 // tiny values do not sink into its subnormals. rscale[m] undoes the scale exactly in the
 // epilogue. Rows that are all zero, or hold an infinity or NaN, are converted as they are.
-// The row is written in the operands' k order (above). One CTA per row;
+// The row is written in the operands' k order (tc_common.cuh): as a row of [m, k] (image_rows = 0, prefill),
+// or as a row of the operand's shared-memory image [k / 64][image_rows][128 bytes], 128B-swizzled, which
+// decode batches copy in whole. One CTA per row;
 // up to 4096 values stay in registers between the two passes. At 48 registers a thread a CTA fits
 // beside a CTA of the GEMM, so the conversion of the next call is resident before this call ends.
-__global__ void __launch_bounds__(256, 5) prep_act_kernel(const void* __restrict__ x, int is_bf16, int64_t k,
-                                                        __half* __restrict__ xh, float* __restrict__ rscale) {
+__global__ void __launch_bounds__(256, 6) prep_act_kernel(const void* __restrict__ x, int is_bf16, int64_t k, int image_rows,
+                                                          __half* __restrict__ xh, float* __restrict__ rscale) {
   __shared__ float wmax[8];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMM behind may start on its weights
   asm volatile("griddepcontrol.wait;" ::: "memory");               // x may still be written, the operand buffer still read
@@ -976,9 +630,17 @@ __global__ void __launch_bounds__(256, 5) prep_act_kernel(const void* __restrict
 #pragma unroll
       for (int e = 0; e < 2; e++) o[2 * h + e] = h22u(__floats2half2_rn(u[4 * h + e] * s, u[4 * h + e + 2] * s));
     // the two fours of an eight belong to two 16-k chunks
-    __half* const p = xh + row0 + (i & ~(int64_t)31) + (i & 31) / 2;
-    *reinterpret_cast<uint2*>(p) = make_uint2(o[0], o[1]);
-    *reinterpret_cast<uint2*>(p + 16) = make_uint2(o[2], o[3]);
+    const int in_block = (int)(i & 32) + (int)(i & 31) / 2;  // inside the 64-k block
+    if (image_rows) {
+      uint8_t* const p = reinterpret_cast<uint8_t*>(xh) + ((i >> 6) * image_rows + blockIdx.x) * 128;
+      const int off = (2 * in_block) ^ ((int)(blockIdx.x & 7) << 4);  // 16-byte chunks exchanged by the row's low bits
+      *reinterpret_cast<uint2*>(p + off) = make_uint2(o[0], o[1]);
+      *reinterpret_cast<uint2*>(p + (off ^ 32)) = make_uint2(o[2], o[3]);
+    } else {
+      __half* const p = xh + row0 + (i & ~(int64_t)63) + in_block;
+      *reinterpret_cast<uint2*>(p) = make_uint2(o[0], o[1]);
+      *reinterpret_cast<uint2*>(p + 16) = make_uint2(o[2], o[3]);
+    }
   };
 #pragma unroll
   for (int j = 0; j < KEEP; j++) {
@@ -991,23 +653,6 @@ __global__ void __launch_bounds__(256, 5) prep_act_kernel(const void* __restrict
     load8(x, is_bf16, row0 + i, u);
     store8(i, u);
   }
-}
-
-// Launch with programmatic stream serialization: the kernel may be scheduled while its
-// predecessor in the stream still runs and orders itself with griddepcontrol.wait.
-template <class... Params, class... Args>
-cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -1026,22 +671,21 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-template <int DT, bool SPLIT>
-cudaError_t launch_tc_split(const CUtensorMap& map, GemmArgs a, int pairs, cudaStream_t s) {
+template <int DT>
+cudaError_t launch_tc_dt(const CUtensorMap& map, GemmArgs a, int pairs, cudaStream_t s) {
   constexpr int SLOT_BYTES = 8 * UnitGeom<DT>::BYTES;
   constexpr int BAR_BYTES = (4 * MAX_ST + 2 * MAX_RAW + 5) * 8 + 8;
-  // Shared memory: three raw slots and (prefill) three weight stages, two where that leaves no room for
-  // four activation blocks in flight, the rest for activation stages and raw slots. Decode batches have
-  // their three weight stages in TMEM.
-  // (A prefill dequantize warp only waits on the stages it fills itself. Behind a unit of one stage - an
+  // Shared memory: three raw slots and three weight stages, two where that leaves no room for
+  // four activation blocks in flight, the rest for activation stages and raw slots.
+  // (A dequantize warp only waits on the stages it fills itself. Behind a unit of one stage - an
   // in-feature count that is no multiple of 256 - it is three stages on from its last wait; with two
   // stages it could then wait two phases ahead of the barrier, which the parity does not tell apart.)
   // 4 KB stay free for a CTA of the next call's conversion kernel.
   const int budget = device_smem_optin() - 1024 - BAR_BYTES - 4096;
-  const int a_stage = SPLIT ? 0 : 2 * A_BYTES, b_stage = (SPLIT ? 4 : 1) * a.bn * BK;
-  int sa = 3, sb = SPLIT ? 3 : 4, rs = 3;
+  const int a_stage = 2 * A_BYTES, b_stage = a.bn * BK;
+  int sa = 3, sb = 4, rs = 3;
   auto left = [&]() { return budget - sa * a_stage - sb * b_stage - rs * SLOT_BYTES; };
-  if (!SPLIT && left() < 0 && a.kblocks % 4 == 0) sa = 2;
+  if (left() < 0 && a.kblocks % 4 == 0) sa = 2;
   if (left() < 0) rs = 2;
   if (left() < 0) sb = 3;
   if (left() < 0) return cudaErrorInvalidConfiguration;
@@ -1054,17 +698,12 @@ cudaError_t launch_tc_split(const CUtensorMap& map, GemmArgs a, int pairs, cudaS
   int dev = 0;
   cudaGetDevice(&dev);
   if (!configured.done(dev)) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<DT, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, device_smem_optin());
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, device_smem_optin());
     if (e != cudaSuccess) return e;
     configured.set(dev);
   }
   const size_t smem = (size_t)(sa * a_stage + sb * b_stage + rs * SLOT_BYTES) + BAR_BYTES + 1024;
-  return launch_pdl(gemm_tc_kernel<DT, SPLIT>, dim3((unsigned)(2 * pairs)), dim3(TC_THREADS), smem, s, map, a);
-}
-
-template <int DT>
-cudaError_t launch_tc_dt(const CUtensorMap& map, const GemmArgs& a, int pairs, cudaStream_t s) {
-  return a.split_k ? launch_tc_split<DT, true>(map, a, pairs, s) : launch_tc_split<DT, false>(map, a, pairs, s);
+  return launch_pdl(gemm_tc_kernel<DT>, dim3((unsigned)(2 * pairs)), dim3(TC_THREADS), smem, s, map, a);
 }
 
 }  // namespace
@@ -1075,17 +714,19 @@ static int tile_rows(int64_t m, int cls) {
   return (int)(((m + mt - 1) / mt + 15) / 16 * 16);
 }
 
-size_t gemm_tc_scratch_bytes(int64_t m, int64_t k) {
-  return (((size_t)m * (size_t)k * 2 + 255) & ~(size_t)255) + (((size_t)m * 4 + 255) & ~(size_t)255) + 256;
-}
+// The f16 operand: rows up to a multiple of 16 for the image of a decode batch.
+size_t gemm_operand_bytes(int64_t m, int64_t k) { return ((size_t)((m + 15) / 16 * 16) * (size_t)k * 2 + 255) & ~(size_t)255; }
+size_t gemm_tc_scratch_bytes(int64_t m, int64_t k) { return gemm_operand_bytes(m, k) + (((size_t)m * 4 + 255) & ~(size_t)255) + 256; }
 
-// Per weight of a call: partial sums of a 64-row decode batch [CTA][64][128]; behind them, again per
-// weight, the ready flags [CTA][4][8] and the go-ahead words [CTA].
-static size_t ws_partial_bytes(int sms) { return (size_t)sms * 64 * BM * 4; }
-static size_t ws_flag_words(int sms) { return (size_t)sms * (4 * 8 + 1); }
-size_t gemm_tc_workspace_flags_offset(int sms) { return GEMM_SIBLINGS * ws_partial_bytes(sms); }
-size_t gemm_tc_workspace_flags_bytes(int sms) { return GEMM_SIBLINGS * ws_flag_words(sms) * 4; }
-size_t gemm_tc_workspace_bytes(int sms) { return gemm_tc_workspace_flags_offset(sms) + gemm_tc_workspace_flags_bytes(sms); }
+// Go-ahead words [weight of the call][CTA].
+size_t gemm_workspace_bytes(int sms) { return (size_t)GEMM_SIBLINGS * sms * 4; }
+
+cudaError_t launch_prep_act(const void* x, int x_dtype, int64_t m, int64_t k, int image_rows, uint8_t* xh, float* rscale, cudaStream_t s) {
+  cudaError_t e = prefer_matmul_carveout<prep_act_kernel>();
+  if (e != cudaSuccess) return e;
+  return launch_pdl(prep_act_kernel, dim3((unsigned)m), dim3(256), 0, s, x, (int)(x_dtype == TQ_BF16), k, image_rows,
+                    reinterpret_cast<__half*>(xh), rscale);
+}
 
 // Activation rows per pair tile, activation tiles and pairs of a launch.
 struct TcShape { int bn, mt; GemmWork work; };
@@ -1100,17 +741,14 @@ static TcShape tc_shape(int64_t n_rows, int64_t m, int64_t k, int sm_count) {
 cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int64_t k, const void* x, int x_dtype,
                            int64_t m, float* y, const float* bias, uint8_t* scratch, uint8_t* workspace, int sm_count, cudaStream_t s,
                            int* launches, int* dev_status_word, int sibling, int64_t next_rows, const unsigned* y_toggle, float* y_alt) {
-  if (k % BK != 0 || m <= 0 || m > INT32_MAX || k > INT32_MAX || sibling < 0 ||
+  if (k % BK != 0 || m <= GEMM_BATCH_ROWS || m > INT32_MAX || k > INT32_MAX || sibling < 0 ||
       sibling + (next_rows > 0 ? 1 : 0) >= GEMM_SIBLINGS) return cudaErrorInvalidValue;
   EncodeTiledFn enc = encode_fn();
   if (!enc) return cudaErrorNotSupported;
-  __half* xh = reinterpret_cast<__half*>(scratch);
-  float* rscale = reinterpret_cast<float*>(scratch + (((size_t)m * (size_t)k * 2 + 255) & ~(size_t)255));
+  float* rscale = reinterpret_cast<float*>(scratch + gemm_operand_bytes(m, k));
   cudaError_t e = cudaSuccess;
   if (sibling == 0) {  // several weights that read the same x share one conversion
-    e = prefer_matmul_carveout<prep_act_kernel>();
-    if (e != cudaSuccess) return e;
-    e = launch_pdl(prep_act_kernel, dim3((unsigned)m), dim3(256), 0, s, x, (int)(x_dtype == TQ_BF16), k, xh, rscale);
+    e = launch_prep_act(x, x_dtype, m, k, 0, scratch, rscale, s);
     if (launches) (*launches)++;
     if (e != cudaSuccess) return e;
   }
@@ -1122,7 +760,7 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
   const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
   const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)bn / 2};
   const cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, xh, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, scratch, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
 
@@ -1138,18 +776,15 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
   a.mt = shape.mt;
   const int64_t n_tiles = (n_rows + 2 * BM - 1) / (2 * BM);
   const GemmWork& work = shape.work;
-  const int64_t total = n_tiles * (work.split_k ? a.KU : a.mt);
+  const int64_t total = n_tiles * a.mt;
   if (total > (int64_t)1 << 30) return cudaErrorInvalidValue;
   a.total = (int)total;
-  a.split_k = work.split_k;
   a.sibling = sibling > 0;
   a.rscale = rscale;
   a.y = y;
   a.bias = bias;
-  a.partial = reinterpret_cast<float*>(workspace + sibling * ws_partial_bytes(sm_count));
-  a.flags = reinterpret_cast<int*>(workspace + gemm_tc_workspace_flags_offset(sm_count)) + sibling * ws_flag_words(sm_count);
-  a.go = a.flags + (size_t)sm_count * 4 * 8;
-  a.next_go = a.go + ws_flag_words(sm_count);
+  a.go = reinterpret_cast<int*>(workspace) + (size_t)sibling * sm_count;
+  a.next_go = a.go + sm_count;
   a.next_ctas = next_rows > 0 ? 2 * tc_shape(next_rows, m, k, sm_count).work.pairs : 0;
   a.status = dev_status_word;
   a.y_toggle = y_toggle;

@@ -69,6 +69,8 @@ inline bool plan_gemv_wide(GemvPlaneReads reads, int rows, const GemvSplit& spli
 }
 
 // ---- tcgen05 GEMM (pairs of CTAs, 256 weight rows per pair)
+// Its product callers have more than 64 rows; what the functions answer for up to 64 is how that kernel shared K loops
+// between pairs before decode batches got a kernel and a plan of their own (plan_batch_cluster below).
 
 // Class of the activation rows per pair tile: 64 for decode batches; 256 for prefill, unless twice
 // as many tiles still fit the SMs in one wave - then 128, which doubles the pairs at work.
@@ -122,6 +124,46 @@ inline GemmWork plan_gemm_work(int64_t n_rows, int64_t m, int64_t k, int mt, int
   w.pairs = pairs > 0 ? (int)pairs : 1;
   w.split_k = 1;
   return w;
+}
+
+// ---- tcgen05 GEMM of decode batches (gemm_batch.cu): clusters of CTAs that share the K loop of 128 weight rows
+
+constexpr int BATCH_MAX_CLUSTER = 6;
+
+// CTAs per cluster for a weight of `tiles` 128-row tiles and `KU` units of 256 k; resident[c]: clusters of c that fit the GPU
+// (on 148 SMs 148, 74, 45, 33, 26, 22). A function of the weight's shape alone: it fixes how the f32 sums associate, so it may depend
+// neither on the batch nor on the other weights of a call. The weights that share an x should agree all the same, or
+// the call takes a launch for each size, hence a rule that goes by what a weight looks like rather than by the best size for each.
+// Measured on B200 with 1 / 2 / 3 / 4 / 6 CTAs, us a call at 32 rows:
+//   more than twice as many rows as columns (ffn_gate|up, heads: called in pairs or large anyway): fewest units in sequence
+//     at twice the tiles, an exchange counted as one unit more
+//     2 x 8192 x 2560 Q5_K 12.8 / 13.0 / 15.4 / 16.2 / 19.7   2 x 12288 x 4096 Q4_K 25.4 / 21.5 / 26.5 / 23.1 / 29.5
+//     2 x 25600 x 5120 Q4_K 46.2 / 46.9 / 51.2 / 52.3 / 64.5  2 x 3072 x 1024 Q8_0 6.1 / 6.0 / 8.6 / 7.0 / 7.0
+//   else up to 23 units (attn_q|k|v, attn_output): four CTAs, but no more than one per two units
+//     4096 + 1024 + 1024 x 4096 15.9 / 10.8 / 14.3 / 10.8 / 12.5     8192 + 1024 + 1024 x 5120 20.6 / 20.1 / 16.9 / 17.0 / 18.2
+//     4096 x 4096 13.4 / 9.2 / 8.8 / 8.1 / 9.2   2560 x 2560 10.0 / 6.7 / 6.7 / 6.8 / 6.8   2048 + 1024 + 1024 x 1024 5.9 / 5.8 / 6.2 / 6.0 / 6.0
+//   else (ffn_down and wide attn_output, called alone): fewest units in sequence
+//     5120 x 25600 Q6_K 88.8 / 50.8 / 40.3 / 52.3 / 40.8   5120 x 8192 Q4_K 24.6 / 15.9 / 13.8 / 16.4 / 14.4
+//     2560 x 8192 Q6_K 28.3 / 16.6 / 13.3 / 11.8 / 11.2
+inline int plan_batch_cluster(int tiles, int KU, const int* resident) {
+  auto rounds = [&](int t, int c) { return (t + resident[c] - 1) / resident[c]; };
+  int best = 1;
+  if (tiles > 4 * KU) {
+    int64_t cost = (int64_t)rounds(2 * tiles, 1) * KU;
+    for (int c = 2; c <= 4; c *= 2) {
+      const int64_t n = (int64_t)rounds(2 * tiles, c) * ((KU + c - 1) / c + 1);
+      if (n < cost) { best = c; cost = n; }
+    }
+  } else if (KU < 24) {
+    best = KU < 8 ? (KU + 1) / 2 : 4;
+  } else {
+    int64_t cost = 0;
+    for (int c = 3; c <= BATCH_MAX_CLUSTER; c++) {
+      const int64_t n = (int64_t)rounds(tiles, c) * ((KU + c - 1) / c);
+      if (c == 3 || n < cost) { best = c; cost = n; }
+    }
+  }
+  return best < KU ? best : KU;
 }
 
 }  // namespace turq

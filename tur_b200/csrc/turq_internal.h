@@ -120,25 +120,31 @@ cudaError_t launch_gemv_f32(int dtype, const uint8_t* tiles, int64_t n_rows, int
                             const void* x, int x_dtype, int64_t m, float* y, const float* bias,
                             int sm_count, cudaStream_t s, int* launches);
 
-// Tensor-core GEMM (tcgen05): x [m, k] -> f16 operand in scratch, then the fused
-// dequantize + MMA kernel. scratch must hold gemm_tc_scratch_bytes(m, k), workspace
-// gemm_tc_workspace_bytes(sm_count), zero-initialised once.
+// Tensor-core GEMM (tcgen05): x [m, k] -> f16 operand in scratch, then the fused dequantize + MMA
+// kernel. scratch must hold gemm_tc_scratch_bytes(m, k).
+// y_toggle / y_alt: the result goes to y_alt instead of y when *y_toggle + 1 is odd (read on the
+// device after the preceding kernels have completed: the exchange slots of tp.cu).
+constexpr int GEMM_BATCH_ROWS = 64;  // decode batches: up to this many rows
+constexpr int GEMM_SIBLINGS = 4;
+size_t gemm_operand_bytes(int64_t m, int64_t k);  // the operand at the start of scratch, the row scales behind it
+size_t gemm_tc_scratch_bytes(int64_t m, int64_t k);
+// The conversion launch: as [m, k], or (image_rows > 0) as the operand image of a decode batch.
+cudaError_t launch_prep_act(const void* x, int x_dtype, int64_t m, int64_t k, int image_rows, uint8_t* xh, float* rscale, cudaStream_t s);
+// Prefill, m > GEMM_BATCH_ROWS. workspace: gemm_workspace_bytes(sm_count) that read zero at launch.
 // sibling: index of the weight in a call whose weights share x. The first one converts x; the later
 // ones (same m, k, x, scratch, workspace, stream, issued directly behind it) reuse the operand and
 // run beside their predecessor. next_rows: out-features of the weight that will be issued as the next
-// sibling (0: none follows); a call that cannot issue it after all has to clear the workspace's flags.
-// y_toggle / y_alt: the result goes to y_alt instead of y when *y_toggle + 1 is odd (read on the
-// device after the preceding kernels have completed: the exchange slots of tp.cu).
-constexpr int GEMM_SIBLINGS = 4;
-size_t gemm_tc_scratch_bytes(int64_t m, int64_t k);
-size_t gemm_tc_workspace_bytes(int sm_count);
-size_t gemm_tc_workspace_flags_offset(int sm_count);  // the part that must read zero at launch
-size_t gemm_tc_workspace_flags_bytes(int sm_count);
+// sibling (0: none follows); a call that cannot issue it after all has to clear the workspace.
+size_t gemm_workspace_bytes(int sm_count);
 cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int64_t k,
                            const void* x, int x_dtype, int64_t m, float* y, const float* bias,
                            uint8_t* scratch, uint8_t* workspace, int sm_count, cudaStream_t s, int* launches,
                            int* dev_status_word, int sibling = 0, int64_t next_rows = 0, const unsigned* y_toggle = nullptr,
                            float* y_alt = nullptr);
+// Decode batches, m <= GEMM_BATCH_ROWS: the weights of a call (each part with its dtype) as one launch per cluster size
+// that their shapes ask for.
+cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, const void* x, int x_dtype, int64_t m, uint8_t* scratch,
+                              cudaStream_t s, int* launches, int* dev_status_word, const unsigned* y_toggle = nullptr);
 
 // QMatMul (no bias) whose result has to land in one of two buffers picked on the device: s1 when
 // (*toggle + 1) is odd, else s0 (the exchange slots of tp.cu). In the integer scheme the GEMV's
