@@ -37,6 +37,7 @@ struct ActOut {
   float* dsc;
   int16_t* bs16;
   int16_t* bs32;
+  ActOrder order;  // of the planes' quants (Q8_K)
 };
 
 // One warp per 256-element block: lane owns elements 8*lane .. 8*lane+7.
@@ -69,10 +70,7 @@ __global__ void __launch_bounds__(128) quant_q8k_kernel(const void* __restrict__
       qs[1] = w1;
       if ((lane & 1) == 0) *reinterpret_cast<int16_t*>(b + 260 + lane) = (int16_t)s16;
     } else {
-      *reinterpret_cast<uint2*>(out.qs + row * k + blk * 256 + lane * 8) = make_uint2(w0, w1);
-      if (lane == 0) out.dsc[wb] = d;
-      if ((lane & 1) == 0) out.bs16[row * (k >> 4) + blk * 16 + (lane >> 1)] = (int16_t)s16;
-      if ((lane & 3) == 0) out.bs32[row * (k >> 5) + blk * 8 + (lane >> 2)] = (int16_t)s32;
+      store_q8k_planes(out.qs, out.order, out.dsc, out.bs16, out.bs32, m, row, blk, lane, w0, w1, d, s16, s32);
     }
   }
 }
@@ -116,8 +114,8 @@ __global__ void __launch_bounds__(128) quant_q8_0_kernel(const void* __restrict_
       qs[2] = (uint16_t)(w1 & 0xFFFF);
       qs[3] = (uint16_t)(w1 >> 16);
     } else {
-      *reinterpret_cast<uint2*>(out.qs + row * k + blk * 32 + (lane & 3) * 8) = make_uint2(w0, w1);
-      if ((lane & 3) == 0) out.dsc[row * nblk + blk] = __half2float(dh);
+      *reinterpret_cast<uint2*>(out.qs + (blk * m + row) * 32 + (lane & 3) * 8) = make_uint2(w0, w1);
+      if ((lane & 3) == 0) out.dsc[blk * m + row] = __half2float(dh);
     }
   }
 }
@@ -170,11 +168,12 @@ cudaError_t launch_quantize_act_wire(int fmt, const void* x, int x_dtype, int64_
   return launch_act(fmt, x, x_dtype, m, k, out, s);
 }
 
-cudaError_t launch_quantize_act_pack(int fmt, const void* x, int x_dtype, int64_t m, int64_t k,
+cudaError_t launch_quantize_act_pack(int fmt, ActOrder order, const void* x, int x_dtype, int64_t m, int64_t k,
                                      uint8_t* scratch, cudaStream_t s) {
   ActPackPlan p = plan_act_pack(fmt, m, k);
   ActOut out{};
   out.wire = nullptr;
+  out.order = order;
   out.qs = reinterpret_cast<int8_t*>(scratch + p.off_qs);
   out.dsc = reinterpret_cast<float*>(scratch + p.off_dsc);
   out.bs16 = reinterpret_cast<int16_t*>(scratch + p.off_bs16);

@@ -3,6 +3,7 @@
 // blocks of the public entry and the planes the GEMV consumes always agree.
 #pragma once
 #include "device_utils.cuh"
+#include "gemv_tile.cuh"
 
 // The Q8_K activation quantizer has three choices on which GGML revisions and candle differ.
 // They are compile-time switches here and (under the TQO_ prefix) in the CPU oracle, which
@@ -108,6 +109,25 @@ __device__ __forceinline__ void quant_block_q8k(const float (&v)[8], int lane, u
   s32 = s16 + __shfl_xor_sync(0xFFFFFFFFu, s16, 2);
   w0 = pack4(q);
   w1 = pack4(q + 4);
+}
+
+// One Q8_K block, 8 values per lane, into the planes (gemv_tile.cuh) of R rows.
+__device__ __forceinline__ void store_q8k_qs(int8_t* qs, ActOrder order, int64_t R, int64_t row, int64_t blk, int lane, uint32_t w0, uint32_t w1) {
+  int8_t* const q = qs + ((4 * blk + (lane >> 3)) * R + row) * 64;
+  const int e = (lane & 7) * 8, r = (int)(row & 7);
+  if (order == ActOrder::order32) {
+    *reinterpret_cast<uint2*>(q + act_offset(ActOrder::order32, r, e)) = make_uint2(w0, w1);
+  } else {
+    *reinterpret_cast<uint32_t*>(q + act_offset(ActOrder::order16, r, e)) = w0;
+    *reinterpret_cast<uint32_t*>(q + act_offset(ActOrder::order16, r, e + 4)) = w1;
+  }
+}
+__device__ __forceinline__ void store_q8k_planes(int8_t* qs, ActOrder order, float* dsc, int16_t* bs16, int16_t* bs32, int64_t R,
+                                                 int64_t row, int64_t blk, int lane, uint32_t w0, uint32_t w1, float d, int s16, int s32) {
+  store_q8k_qs(qs, order, R, row, blk, lane, w0, w1);
+  if (lane == 0) dsc[blk * R + row] = d;
+  if ((lane & 1) == 0) bs16[((2 * blk + (lane >> 4)) * R + row) * 8 + ((lane >> 1) & 7)] = (int16_t)s16;
+  if ((lane & 3) == 0) bs32[(blk * R + row) * 8 + (lane >> 2)] = (int16_t)s32;
 }
 
 // The same Q8_K block held 16 values per lane by one half of a warp (lane & 15 owns elements

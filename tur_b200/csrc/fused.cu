@@ -39,7 +39,9 @@ struct NormQuantArgs {
   int64_t k;
   float* h_out;  // nullable
   int fmt;       // TQ_Q8_K or TQ_Q8_0
+  int64_t m;
   int8_t* qs;
+  int8_t* qs_order16;  // Q8_K: a second copy of the quants, for launches of Q6_K weights alone
   float* dsc;
   int16_t* bs16;
   int16_t* bs32;
@@ -84,10 +86,8 @@ __global__ void __launch_bounds__(256) rmsnorm_quant_kernel(const NormQuantArgs 
       float d;
       int s16, s32;
       quant_block_q8k(v, lane, q0, q1, d, s16, s32);
-      *reinterpret_cast<uint2*>(a.qs + row * k + blk * 256 + lane * 8) = make_uint2(q0, q1);
-      if (lane == 0) a.dsc[row * nblk + blk] = d;
-      if ((lane & 1) == 0) a.bs16[row * (k >> 4) + blk * 16 + (lane >> 1)] = (int16_t)s16;
-      if ((lane & 3) == 0) a.bs32[row * (k >> 5) + blk * 8 + (lane >> 2)] = (int16_t)s32;
+      store_q8k_planes(a.qs, ActOrder::order32, a.dsc, a.bs16, a.bs32, a.m, row, blk, lane, q0, q1, d, s16, s32);
+      store_q8k_qs(a.qs_order16, ActOrder::order16, a.m, row, blk, lane, q0, q1);
     }
   } else {
     const int64_t nblk = k >> 5, groups = (nblk + 7) >> 3;
@@ -116,8 +116,8 @@ __global__ void __launch_bounds__(256) rmsnorm_quant_kernel(const NormQuantArgs 
       __half dh;
       quant_block_q8_0(v, q0, q1, dh);
       if (live) {
-        *reinterpret_cast<uint2*>(a.qs + row * k + blk * 32 + (lane & 3) * 8) = make_uint2(q0, q1);
-        if ((lane & 3) == 0) a.dsc[row * nblk + blk] = __half2float(dh);
+        *reinterpret_cast<uint2*>(a.qs + (blk * a.m + row) * 32 + (lane & 3) * 8) = make_uint2(q0, q1);
+        if ((lane & 3) == 0) a.dsc[blk * a.m + row] = __half2float(dh);
       }
     }
   }
@@ -293,7 +293,7 @@ int32_t turq_rmsnorm_qmatmul_multi(turq_ctx* ctx, int32_t count, const turq_qten
   const bool direct = eff == TURQ_MODE_INT8_ACT && !(k_quant && q8_0);
   const int fmt = q8_0 && !k_quant ? TQ_Q8_0 : TQ_Q8_K;
   const turq::ActPackPlan plan = turq::plan_act_pack(fmt, m, k);
-  int32_t st = turq::api_ensure_scratch(ctx, plan.total);
+  int32_t st = turq::api_ensure_scratch(ctx, turq::norm_scratch_bytes(fmt, m, k));
   if (st != TURQ_OK) return st;
   float* h = dev_h_out;
   if (!direct && !h) {  // the other schemes read h itself
@@ -309,7 +309,9 @@ int32_t turq_rmsnorm_qmatmul_multi(turq_ctx* ctx, int32_t count, const turq_qten
   a.k = k;
   a.h_out = h;
   a.fmt = fmt;
+  a.m = m;
   a.qs = reinterpret_cast<int8_t*>(ctx->scratch + plan.off_qs);
+  a.qs_order16 = reinterpret_cast<int8_t*>(ctx->scratch + plan.total);
   a.dsc = reinterpret_cast<float*>(ctx->scratch + plan.off_dsc);
   a.bs16 = reinterpret_cast<int16_t*>(ctx->scratch + plan.off_bs16);
   a.bs32 = reinterpret_cast<int16_t*>(ctx->scratch + plan.off_bs32);

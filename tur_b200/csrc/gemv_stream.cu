@@ -103,7 +103,7 @@ extern "C" int turq_debug_read_trace(unsigned long long* host, int n) {
 #endif
 
 struct SmemPlan {
-  int ring, act_qs, act_dsc, act_bs16, act_bs32, red, bars, total, qs_stride;
+  int ring, act_qs, act_dsc, act_bs16, act_bs32, red, bars, total;
 };
 constexpr int bar_bytes(int red_slots) { return (MAX_STAGES * NW + MAX_STAGES + 2 * red_slots) * 8; }
 
@@ -129,7 +129,7 @@ struct StreamArgs {
   int total_units;
   const void* x;        // activations of the pass (first row of the pass), f32 or bf16   [ACT_FUSED]
   int x_is_bf16;
-  ActPack gact;         // planes in global scratch, already offset to the pass's first row [other modes]
+  ActPack gact;         // planes in global scratch, already offset to the pass's first row [other modes]; fused: R only
   int rows;             // valid activation rows in this pass (<= 8 * MG)
   float* partial;       // [grid][MG * 128]: partial sums of a CTA's leading split row-tile
   int* flags;           // [grid], all zero between launches
@@ -152,10 +152,9 @@ inline SmemPlan plan_smem(int dtype, int mg, bool fused /* planes in shared memo
   SmemPlan p{};
   p.ring = 0;
   int off = halves * stages * stage_bytes;  // stage_bytes is a multiple of 128 for every type
-  p.qs_stride = k + 32;
   p.act_qs = off;
   if (fused) {
-    off = up(off + rows_cap * p.qs_stride);
+    off = up(off + rows_cap * k);
     p.act_dsc = off;
     off = up(off + rows_cap * (k / (dtype == TQ_Q8_0 ? 32 : 256)) * 4);
     p.act_bs16 = off;  // Q6_K reads the sums of 16, Q4_K / Q5_K the sums of 32
@@ -205,6 +204,9 @@ constexpr int ACT_GLOBAL = 0;  // in global scratch (written by a preceding quan
 constexpr int ACT_FUSED = 1;   // quantized by this CTA into shared memory
 constexpr int ACT_STAGED = 2;  // bulk-copied from global scratch into shared memory at CTA start
 
+// The order of the planes' quants a launch reads.
+constexpr ActOrder order_of(int dt, int dt2) { return dt == TQ_Q6_K && dt2 == TQ_Q6_K ? ActOrder::order16 : ActOrder::order32; }
+
 // DT2 != DT: a mixed launch (attn_q|k in Q4_K or Q5_K beside attn_v in Q6_K, as the K-quant
 // mixes store them); parts flagged in part_alt hold DT2 tiles. Both types have one tile per
 // 256 elements, so the walk over tiles is the same; ring slots are sized for the larger tile.
@@ -217,6 +219,7 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
   static_assert(HALVES == 1 || ACT == ACT_STAGED, "wide CTAs share staged planes");
   constexpr int RSLOTS = red_slots_of(HALVES, MG);
   constexpr bool MIXED = DT2 != DT;
+  constexpr ActOrder ORDER = order_of(DT, DT2);
   constexpr int TB = TileGeom<DT>::BYTES;
   constexpr int TB2 = TileGeom<DT2>::BYTES;
   constexpr int GROUP = TileGeom<DT>::GROUP;
@@ -289,8 +292,7 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
       // without them. They were written by the quantization launch just before this one; with
       // programmatic stream serialization this grid is already resident (barriers set up) when
       // that launch ends, and griddepcontrol.wait orders the copies after it.
-      // One copy per row of quants (the shared-memory rows are padded), one per plane of
-      // scales / sums (sizes rounded up to 16 bytes; the planes are padded on both sides).
+      // One copy per plane (sizes rounded up to 16 bytes; the planes are padded on both sides).
       auto copy_planes = [&]() {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         const int nb = DT == TQ_Q8_0 ? a.k >> 5 : a.k >> 8;
@@ -298,8 +300,7 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
         const uint32_t s16_bytes = NEED16 ? (((uint32_t)(a.rows * (a.k >> 4) * 2) + 15u) & ~15u) : 0u;
         const uint32_t s32_bytes = NEED32 ? (((uint32_t)(a.rows * (a.k >> 5) * 2) + 15u) & ~15u) : 0u;
         mbar_expect_tx(act_full, (uint32_t)(a.rows * a.k) + dsc_bytes + s16_bytes + s32_bytes);
-        for (int r = 0; r < a.rows; r++)
-          bulk_g2s(smem + sp.act_qs + r * sp.qs_stride, a.gact.qs + (size_t)r * a.k, (uint32_t)a.k, act_full);
+        bulk_g2s(smem + sp.act_qs, a.gact.qs, (uint32_t)(a.rows * a.k), act_full);
         bulk_g2s(smem + sp.act_dsc, a.gact.dsc, dsc_bytes, act_full);
         if constexpr (NEED16) bulk_g2s(smem + sp.act_bs16, a.gact.bs16, s16_bytes, act_full);
         if constexpr (NEED32) bulk_g2s(smem + sp.act_bs32, a.gact.bs32, s32_bytes, act_full);
@@ -360,7 +361,6 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
       act.dsc = reinterpret_cast<const float*>(smem + sp.act_dsc);
       act.bs16 = reinterpret_cast<const int16_t*>(smem + sp.act_bs16);
       act.bs32 = reinterpret_cast<const int16_t*>(smem + sp.act_bs32);
-      act.qs_stride = sp.qs_stride;
     }
     if constexpr (ACT == ACT_FUSED) {
       int8_t* sqs = reinterpret_cast<int8_t*>(smem + sp.act_qs);
@@ -383,8 +383,8 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
           __half dh;
           quant_block_q8_0(v, w0, w1, dh);
           if (live) {
-            *reinterpret_cast<uint2*>(sqs + row * sp.qs_stride + blk * 32 + (lane & 3) * 8) = make_uint2(w0, w1);
-            if ((lane & 3) == 0) sdsc[row * nblk + blk] = __half2float(dh);
+            *reinterpret_cast<uint2*>(sqs + (blk * a.rows + row) * 32 + (lane & 3) * 8) = make_uint2(w0, w1);
+            if ((lane & 3) == 0) sdsc[blk * a.rows + row] = __half2float(dh);
           }
         }
       } else {
@@ -418,11 +418,18 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
           int s16, s32;
           quant_block_q8k_half(v, lane, w4, d, s16, s32);
           if (has) {
-            *reinterpret_cast<uint4*>(sqs + row * sp.qs_stride + blk * 256 + hl * 16) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-            if (hl == 0) sdsc[row * nblk + blk] = d;
-            if constexpr (NEED16) sb16[row * (a.k >> 4) + blk * 16 + hl] = (int16_t)s16;
+            int8_t* const q = sqs + ((4 * blk + (hl >> 2)) * a.rows + row) * 64;
+            if constexpr (ORDER == ActOrder::order32) {
+              *reinterpret_cast<uint2*>(q + act_offset(ORDER, row, (hl & 3) * 16)) = make_uint2(w4[0], w4[1]);
+              *reinterpret_cast<uint2*>(q + act_offset(ORDER, row, (hl & 3) * 16 + 8)) = make_uint2(w4[2], w4[3]);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; e++) *reinterpret_cast<uint32_t*>(q + act_offset(ORDER, row, (hl & 3) * 16 + 4 * e)) = w4[e];
+            }
+            if (hl == 0) sdsc[blk * a.rows + row] = d;
+            if constexpr (NEED16) sb16[((2 * blk + (hl >> 3)) * a.rows + row) * 8 + (hl & 7)] = (int16_t)s16;
             if constexpr (NEED32) {
-              if ((hl & 1) == 0) sb32[row * (a.k >> 5) + blk * 8 + (hl >> 1)] = (int16_t)s32;
+              if ((hl & 1) == 0) sb32[(blk * a.rows + row) * 8 + (hl >> 1)] = (int16_t)s32;
             }
           }
         }
@@ -431,12 +438,14 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
       act.dsc = sdsc;
       act.bs16 = sb16;
       act.bs32 = sb32;
-      act.qs_stride = sp.qs_stride;
       consumer_sync();
     }
     if (warp == 0) TRACE(3);
 
     const int g = lane >> 2, c = lane & 3;
+    if constexpr (ACT != ACT_GLOBAL) act.R = a.rows;
+    LaneAct<MG> la;
+    la.init(lane, a.rows, DT == TQ_Q8_0 ? 32 : 64);
     float acc[MG][4];
 #pragma unroll
     for (int mg = 0; mg < MG; mg++)
@@ -471,19 +480,21 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
         bool done_row1 = false;
         if constexpr (MG == 1 && DT != TQ_Q8_0 && DT2 != TQ_Q8_0) {
           if (a.rows == 1) {
+            ActPack one = act;
+            if constexpr (ACT != ACT_GLOBAL) one.R = 1;  // a constant: no multiplications on the way to the planes
             if (MIXED && alt) {
-              tile_mma_row1<DT2>(tile, lane, act, a.k, kt, acc);
+              tile_mma_row1<DT2, ORDER>(tile, lane, one, kt, acc);
             } else {
-              tile_mma_row1<DT>(tile, lane, act, a.k, kt, acc);
+              tile_mma_row1<DT, ORDER>(tile, lane, one, kt, acc);
             }
             done_row1 = true;
           }
         }
         if (!done_row1) {
           if (MIXED && alt) {
-            tile_mma<DT2, MG>(tile, lane, act, a.k, kt, a.rows, left, acc);
+            tile_mma<DT2, MG, ORDER>(tile, lane, act, la, kt, left, acc);
           } else {
-            tile_mma<DT, MG>(tile, lane, act, a.k, kt, a.rows, left, acc);
+            tile_mma<DT, MG, ORDER>(tile, lane, act, la, kt, left, acc);
           }
         }
       }
@@ -827,7 +838,7 @@ static cudaError_t launch_dt(const GemvPart* parts, int nparts, int64_t k, const
   const size_t x_es = x_dtype == TQ_BF16 ? 2 : 4;
   ActPackPlan plan = plan_act_pack(fmt, m, k);
   if (!fused && !planes_ready) {
-    cudaError_t e = launch_quantize_act_pack(fmt, x, x_dtype, m, k, act_scratch, s);
+    cudaError_t e = launch_quantize_act_pack(fmt, order_of(DT, DT2), x, x_dtype, m, k, act_scratch, s);
     if (launches) (*launches)++;
     if (e != cudaSuccess) return e;
   }
@@ -860,12 +871,13 @@ static cudaError_t launch_dt(const GemvPart* parts, int nparts, int64_t k, const
     a.x = static_cast<const uint8_t*>(x) + (size_t)m0 * k * x_es;
     a.x_is_bf16 = x_dtype == TQ_BF16;
     if (!fused) {
-      const int bs = fmt == TQ_Q8_0 ? 32 : 256;
-      a.gact.qs = reinterpret_cast<const int8_t*>(act_scratch + plan.off_qs) + m0 * k;
-      a.gact.dsc = reinterpret_cast<const float*>(act_scratch + plan.off_dsc) + m0 * (k / bs);
-      a.gact.bs16 = reinterpret_cast<const int16_t*>(act_scratch + plan.off_bs16) + m0 * (k / 16);
-      a.gact.bs32 = reinterpret_cast<const int16_t*>(act_scratch + plan.off_bs32) + m0 * (k / 32);
-      a.gact.qs_stride = (int)k;
+      // a prologue's planes hold the quants in both orders
+      const size_t off_qs = planes_ready && fmt == TQ_Q8_K && order_of(DT, DT2) == ActOrder::order16 ? plan.total : plan.off_qs;
+      a.gact.qs = reinterpret_cast<const int8_t*>(act_scratch + off_qs) + m0 * (fmt == TQ_Q8_0 ? 32 : 64);
+      a.gact.dsc = reinterpret_cast<const float*>(act_scratch + plan.off_dsc) + m0;
+      a.gact.bs16 = reinterpret_cast<const int16_t*>(act_scratch + plan.off_bs16) + m0 * 8;
+      a.gact.bs32 = reinterpret_cast<const int16_t*>(act_scratch + plan.off_bs32) + m0 * 8;
+      a.gact.R = (int)m;
     }
     a.rows = rows;
     a.partial = reinterpret_cast<float*>(workspace);

@@ -21,18 +21,54 @@ template <> struct TileGeom<TQ_Q4_K> { static constexpr int BYTES = 2304, ELEMS 
 template <> struct TileGeom<TQ_Q5_K> { static constexpr int BYTES = 2816, ELEMS = 256, GROUP = 1; };
 template <> struct TileGeom<TQ_Q6_K> { static constexpr int BYTES = 3360, ELEMS = 256, GROUP = 1; };
 
-// Quantized activation planes (global scratch or shared memory), indexed by the row number
-// relative to the first row of the pass.
-//   qs    int8  [rows][qs_stride]  element order = input order
-//   dsc   f32   [rows][k/bs]       bs = 256 (Q8_K) or 32 (Q8_0; the f16-rounded scale)
-//   bs16  int16 [rows][k/16]       Q8_K: sums of 16 consecutive qs
-//   bs32  int16 [rows][k/32]       Q8_K: sums of 32 consecutive qs
+// Quantized activation planes (global scratch or shared memory) of R rows, in the order in which the MMA loop reads them: a
+// lane finds what it needs in as few and as wide words as there are, neighbouring rows lie next to each other (no bank
+// conflicts, whole sectors from global memory), and a run of k-tiles is one contiguous range. With row-major planes more than
+// half of the shared-memory wavefronts of a 16-row tile were conflicts (the block sums of four rows in the same banks) and a
+// Q6_K tile read its quants in sixteen words a row. Row-major against this order, us a call, 8 / 16 rows:
+//   2 x 12288 x 4096 Q4_K 19.8 -> 17.5, 33.4 -> 23.6   4096 x 12288 Q6_K 15.8 -> 13.7, 30.6 -> 18.9
+//   2 x 8192 x 2560 Q5_K 11.7 -> 11.3, 16.6 -> 15.4    5120 x 25600 Q6_K (planes in global memory) 35.8 -> 27.0, 61.9 -> 38.9
+//   2 x 8192 x 2560 Q8_0 13.7 -> 12.2, 17.1 -> 16.3
+//   qs    K-quants: [k/64][R][64 bytes], the 64 bytes in one of two orders (ActOrder)
+//         Q8_0:     [k/32][R][32 bytes], element order
+//   dsc   f32   [k/bs][R]          bs = 256 (Q8_K) or 32 (Q8_0; the f16-rounded scale)
+//   bs16  int16 [k/256][2][R][8]   Q8_K: sums of 16 consecutive qs
+//   bs32  int16 [k/256][R][8]      Q8_K: sums of 32 consecutive qs
 struct ActPack {
   const int8_t* qs;
   const float* dsc;
   const int16_t* bs16;
   const int16_t* bs32;
-  int qs_stride;
+  int R;
+};
+
+// Byte offset of element e (0..63) of row r inside the row's 64 bytes of a chunk.
+//   order32 (Q4_K, Q5_K, mixed launches): lane column c's eight bytes of both 32-element sub-blocks, 16 bytes together. The
+//     columns of rows 2, 3, 6, 7 change places pairwise, so that Q6_K tiles of a mixed launch, which read four-byte words,
+//     meet in a bank twice and not four times.
+//   order16 (Q6_K): lane column c's four bytes of all four 16-element sub-blocks, 16 bytes together.
+enum class ActOrder { order32, order16 };
+__host__ __device__ __forceinline__ int act_offset(ActOrder o, int r, int e) {
+  if (o == ActOrder::order32) return 16 * (((e & 31) >> 3) ^ (r & 2)) + 8 * (e >> 5) + (e & 7);
+  return 16 * ((e & 15) >> 2) + 4 * (e >> 4) + (e & 3);
+}
+
+// What a lane needs to find its rows in the planes; the same for every tile. Rows beyond the valid ones are clamped to the last
+// one: their columns of the MMA are not stored.
+template <int MG>
+struct LaneAct {
+  int q[MG];        // offset of row 8 mg + g inside a chunk of qs
+  int r0[MG], r1[MG];  // rows 8 mg + 2 c, 8 mg + 2 c + 1
+  __device__ __forceinline__ void init(int lane, int rows, int row_bytes) {
+    const int g = lane >> 2, c = lane & 3;
+#pragma unroll
+    for (int mg = 0; mg < MG; mg++) {
+      const int b = 8 * mg + g, m0 = 8 * mg + 2 * c;
+      q[mg] = (b < rows ? b : rows - 1) * row_bytes;
+      r0[mg] = m0 < rows ? m0 : rows - 1;
+      r1[mg] = m0 + 1 < rows ? m0 + 1 : rows - 1;
+    }
+  }
 };
 
 __device__ __forceinline__ int sext_byte(uint32_t w, int b) { return (int)(int8_t)((w >> (8 * b)) & 0xFFu); }
@@ -40,14 +76,13 @@ __device__ __forceinline__ uint4 lds_v4(const uint8_t* p) { return *reinterpret_
 __device__ __forceinline__ uint32_t lds_u16(const uint8_t* p) { return *reinterpret_cast<const uint16_t*>(p); }
 
 // One tile (or GROUP consecutive Q8_0 tiles) at shared-memory address t, tile index kt of its
-// row, against the `rows` valid activation rows of the pass; adds into acc[mg][0..3].
-template <int DT, int MG>
-__device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane, const ActPack& act, int k, int kt,
-                                         int rows, int ntiles_left, float (&acc)[MG][4]) {
+// row, against the activation rows of the pass; adds into acc[mg][0..3]. ORDER: the order of the planes' qs.
+template <int DT, int MG, ActOrder ORDER>
+__device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane, const ActPack& act, const LaneAct<MG>& la, int kt,
+                                         int ntiles_left, float (&acc)[MG][4]) {
+  static_assert(DT == TQ_Q8_0 || DT == TQ_Q6_K || ORDER == ActOrder::order32, "Q4_K and Q5_K tiles read order32");
   const int g = lane >> 2, c = lane & 3;
-  const uint4 z4 = make_uint4(0, 0, 0, 0);
   if constexpr (DT == TQ_Q8_0) {
-    const int nb = k >> 5;
 #pragma unroll
     for (int u = 0; u < 4; u++) {
       if (u < ntiles_left) {
@@ -58,12 +93,11 @@ __device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane
         const int kb = kt + u;
 #pragma unroll
         for (int mg = 0; mg < MG; mg++) {
-          const int mb = 8 * mg + g, m0 = 8 * mg + 2 * c, m1 = m0 + 1;
-          const uint2 b = mb < rows ? ld_v2(act.qs + mb * act.qs_stride + kb * 32 + 8 * c) : make_uint2(0, 0);
+          const uint2 b = ld_v2(act.qs + (int64_t)kb * act.R * 32 + la.q[mg] + 8 * c);
           int cc[4] = {0, 0, 0, 0};
           mma_16832<false>(cc, a, b.x, b.y);
-          const float dx0 = m0 < rows ? act.dsc[m0 * nb + kb] : 0.f;
-          const float dx1 = m1 < rows ? act.dsc[m1 * nb + kb] : 0.f;
+          const float* const dsc = act.dsc + (int64_t)kb * act.R;
+          const float dx0 = dsc[la.r0[mg]], dx1 = dsc[la.r1[mg]];
           acc[mg][0] += (float)cc[0] * (dw0 * dx0);
           acc[mg][1] += (float)cc[1] * (dw0 * dx1);
           acc[mg][2] += (float)cc[2] * (dw1 * dx0);
@@ -90,9 +124,8 @@ __device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane
         const int mnh = (int)(((s2 >> 4) & 0x0F0F0F0Fu) | ((s1 >> 2) & 0x30303030u));
 #pragma unroll
         for (int mg = 0; mg < MG; mg++) {
-          const int m0 = 8 * mg + 2 * c, m1 = m0 + 1;
-          const uint4 bs0 = m0 < rows ? ld_v4(act.bs32 + m0 * (k >> 5) + kt * 8) : z4;
-          const uint4 bs1 = m1 < rows ? ld_v4(act.bs32 + m1 * (k >> 5) + kt * 8) : z4;
+          const int16_t* const bs = act.bs32 + (int64_t)kt * act.R * 8;
+          const uint4 bs0 = ld_v4(bs + la.r0[mg] * 8), bs1 = ld_v4(bs + la.r1[mg] * 8);
           // mins: sum_j mn_j * bsum_j, two 16-bit x 8-bit products per instruction
           aM[mg][2 * hr] = __dp2a_hi((int)bs0.w, mnh, __dp2a_lo((int)bs0.z, mnh, __dp2a_hi((int)bs0.y, mnl, __dp2a_lo((int)bs0.x, mnl, 0))));
           aM[mg][2 * hr + 1] = __dp2a_hi((int)bs1.w, mnh, __dp2a_lo((int)bs1.z, mnh, __dp2a_hi((int)bs1.y, mnl, __dp2a_lo((int)bs1.x, mnl, 0))));
@@ -103,7 +136,7 @@ __device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane
     for (int mg = 0; mg < MG; mg++)
 #pragma unroll
       for (int e = 0; e < 4; e++) aE[mg][e] = aO[mg][e] = 0;
-    uint4 qh = z4;
+    uint4 qh = make_uint4(0, 0, 0, 0);
     if constexpr (DT == TQ_Q5_K) qh = lds_v4(t + TQ_Q5K_QH + 16 * lane);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -129,13 +162,10 @@ __device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane
       }
 #pragma unroll
       for (int mg = 0; mg < MG; mg++) {
-        const int mb = 8 * mg + g;
-        const int8_t* xrow = act.qs + mb * act.qs_stride + kt * 256 + 8 * c + 64 * i;
-        const uint2 blo = mb < rows ? ld_v2(xrow) : make_uint2(0, 0);
-        const uint2 bhi = mb < rows ? ld_v2(xrow + 32) : make_uint2(0, 0);
+        const uint4 bx = ld_v4(act.qs + (int64_t)(4 * kt + i) * act.R * 64 + la.q[mg] + 16 * (c ^ ((la.q[mg] >> 6) & 2)));
         int clo[4] = {0, 0, 0, 0}, chi[4] = {0, 0, 0, 0};
-        mma_16832<true>(clo, alo, blo.x, blo.y);
-        mma_16832<true>(chi, ahi, bhi.x, bhi.y);
+        mma_16832<true>(clo, alo, bx.x, bx.y);
+        mma_16832<true>(chi, ahi, bx.z, bx.w);
 #pragma unroll
         for (int hr = 0; hr < 2; hr++) {
           aE[mg][2 * hr] += se[hr] * clo[2 * hr];
@@ -149,9 +179,8 @@ __device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane
     const float dmin[2] = {f16_bits_to_f32(h0.x >> 16), f16_bits_to_f32(h1.x >> 16)};
 #pragma unroll
     for (int mg = 0; mg < MG; mg++) {
-      const int m0 = 8 * mg + 2 * c, m1 = m0 + 1;
-      const float dx0 = m0 < rows ? act.dsc[m0 * (k >> 8) + kt] : 0.f;
-      const float dx1 = m1 < rows ? act.dsc[m1 * (k >> 8) + kt] : 0.f;
+      const float* const dsc = act.dsc + (int64_t)kt * act.R;
+      const float dx0 = dsc[la.r0[mg]], dx1 = dsc[la.r1[mg]];
 #pragma unroll
       for (int hr = 0; hr < 2; hr++) {
         constexpr int SH = DT == TQ_Q4_K ? 4 : 0;
@@ -167,11 +196,10 @@ __device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane
 #pragma unroll
     for (int mg = 0; mg < MG; mg++) {
       // the -32 offset: sum_j sc_j * bsum16_j, two products per instruction
-      const int m0 = 8 * mg + 2 * c, m1 = m0 + 1;
-      const int16_t* b0p = act.bs16 + m0 * (k >> 4) + kt * 16;
-      const int16_t* b1p = act.bs16 + m1 * (k >> 4) + kt * 16;
-      const uint4 p0 = m0 < rows ? ld_v4(b0p) : z4, p1 = m0 < rows ? ld_v4(b0p + 8) : z4;
-      const uint4 q0 = m1 < rows ? ld_v4(b1p) : z4, q1 = m1 < rows ? ld_v4(b1p + 8) : z4;
+      const int16_t* const bs = act.bs16 + (int64_t)kt * act.R * 16;
+      const int16_t* const bh = bs + act.R * 8;
+      const uint4 p0 = ld_v4(bs + la.r0[mg] * 8), p1 = ld_v4(bh + la.r0[mg] * 8);
+      const uint4 q0 = ld_v4(bs + la.r1[mg] * 8), q1 = ld_v4(bh + la.r1[mg] * 8);
       const uint32_t bw0[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
       const uint32_t bw1[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
 #pragma unroll
@@ -190,11 +218,15 @@ __device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane
     for (int i = 0; i < 4; i++) {
       const uint4 ql = lds_v4(t + TQ_Q6K_QL + 512 * i + 16 * lane);
       const uint4 qh = lds_v4(t + TQ_Q6K_QH + 512 * (i >> 1) + 16 * lane);
+      uint4 bx[MG];  // order16: this lane's words of the chunk's four sub-blocks
+      if constexpr (ORDER == ActOrder::order16) {
+#pragma unroll
+        for (int mg = 0; mg < MG; mg++) bx[mg] = ld_v4(act.qs + (int64_t)(4 * kt + i) * act.R * 64 + la.q[mg] + 16 * c);
+      }
       // qh word of this chunk's four sub-blocks: chunk i of ql pairs with qh word (i & 1) of each row
       const uint32_t qh0 = (i & 1) ? qh.y : qh.x, qh1 = (i & 1) ? qh.w : qh.z;
 #pragma unroll
       for (int jj = 0; jj < 4; jj++) {
-        const int j = 4 * i + jj;
         const int tw = jj >> 1, nib = jj & 1;
         const uint32_t w0 = tw ? ql.y : ql.x, w1 = tw ? ql.w : ql.z;
         uint32_t a0 = (nib ? (w0 >> 4) : w0) & 0x0F0F0F0Fu, a1 = (nib ? (w1 >> 4) : w1) & 0x0F0F0F0Fu;
@@ -205,8 +237,13 @@ __device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane
         const int sc0 = sext_byte(scw[0][i], jj), sc1 = sext_byte(scw[1][i], jj);
 #pragma unroll
         for (int mg = 0; mg < MG; mg++) {
-          const int mb = 8 * mg + g;
-          const uint32_t b = mb < rows ? ld_u32(act.qs + mb * act.qs_stride + kt * 256 + 4 * c + 16 * j) : 0u;
+          uint32_t b;
+          if constexpr (ORDER == ActOrder::order16) {
+            b = jj == 0 ? bx[mg].x : jj == 1 ? bx[mg].y : jj == 2 ? bx[mg].z : bx[mg].w;
+          } else {  // elements 16 jj + 4 c ...: column 2 (jj & 1) + c / 2 of sub-block jj / 2, word c & 1
+            b = ld_u32(act.qs + (int64_t)(4 * kt + i) * act.R * 64 + la.q[mg] +
+                       16 * ((2 * (jj & 1) + (c >> 1)) ^ ((la.q[mg] >> 6) & 2)) + 8 * (jj >> 1) + 4 * (c & 1));
+          }
           int cc[4] = {0, 0, 0, 0};
           mma_16816_u8s8(cc, a0, a1, b);
           aI[mg][0] += sc0 * cc[0];
@@ -219,9 +256,8 @@ __device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane
     const float d0 = f16_bits_to_f32(lds_u16(t + TQ_Q6K_D + 2 * g)), d1 = f16_bits_to_f32(lds_u16(t + TQ_Q6K_D + 2 * (g + 8)));
 #pragma unroll
     for (int mg = 0; mg < MG; mg++) {
-      const int m0 = 8 * mg + 2 * c, m1 = m0 + 1;
-      const float dx0 = m0 < rows ? act.dsc[m0 * (k >> 8) + kt] : 0.f;
-      const float dx1 = m1 < rows ? act.dsc[m1 * (k >> 8) + kt] : 0.f;
+      const float* const dsc = act.dsc + (int64_t)kt * act.R;
+      const float dx0 = dsc[la.r0[mg]], dx1 = dsc[la.r1[mg]];
       acc[mg][0] += (dx0 * d0) * (float)aI[mg][0];
       acc[mg][1] += (dx1 * d0) * (float)aI[mg][1];
       acc[mg][2] += (dx0 * d1) * (float)aI[mg][2];
@@ -240,18 +276,18 @@ __device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane
 // float step is the one of the general function - same integers, same float operations, so
 // the result has the bits of tile_mma<DT, 1> with rows = 1. Each lane loads one 8-byte (two
 // 4-byte) activation fragment per tile instead of eight (sixteen).
-template <int DT>
-__device__ __forceinline__ void tile_mma_row1(const uint8_t* __restrict__ t, int lane, const ActPack& act, int k, int kt,
-                                              float (&acc)[1][4]) {
+template <int DT, ActOrder ORDER>
+__device__ __forceinline__ void tile_mma_row1(const uint8_t* __restrict__ t, int lane, const ActPack& act, int kt, float (&acc)[1][4]) {
+  static_assert(DT == TQ_Q6_K || ORDER == ActOrder::order32, "Q4_K and Q5_K tiles read order32");
   static_assert(DT == TQ_Q4_K || DT == TQ_Q5_K || DT == TQ_Q6_K, "single-row variant exists for the K-quants");
   const int g = lane >> 2, c = lane & 3;
-  const float dx0 = act.dsc[kt];
+  const float dx0 = act.dsc[(int64_t)kt * act.R];
   if constexpr (DT == TQ_Q4_K || DT == TQ_Q5_K) {
     constexpr int QS = DT == TQ_Q4_K ? TQ_Q4K_QS : TQ_Q5K_QS;
     constexpr int SH = DT == TQ_Q4_K ? 4 : 0;
     const uint4 h0 = lds_v4(t + 16 * g), h1 = lds_v4(t + 16 * (g + 8));
     const uint4 hh[2] = {h0, h1};
-    const uint4 bs0 = ld_v4(act.bs32 + kt * 8);
+    const uint4 bs0 = ld_v4(act.bs32 + (int64_t)kt * act.R * 8);
     uint32_t scl[2], sch[2];
     int aM[2];
 #pragma unroll
@@ -264,7 +300,7 @@ __device__ __forceinline__ void tile_mma_row1(const uint8_t* __restrict__ t, int
       aM[hr] = __dp2a_hi((int)bs0.w, mnh, __dp2a_lo((int)bs0.z, mnh, __dp2a_hi((int)bs0.y, mnl, __dp2a_lo((int)bs0.x, mnl, 0))));
     }
     // this lane's activation fragment: elements 8c .. 8c+7 of sub-block g
-    const uint2 frag = ld_v2(act.qs + kt * 256 + 32 * g + 8 * c);
+    const uint2 frag = ld_v2(act.qs + (int64_t)(4 * kt + (g >> 1)) * act.R * 64 + 16 * c + 8 * (g & 1));
     int cc[4] = {0, 0, 0, 0};
     uint4 qh = make_uint4(0, 0, 0, 0);
     if constexpr (DT == TQ_Q5_K) qh = lds_v4(t + TQ_Q5K_QH + 16 * lane);
@@ -303,8 +339,8 @@ __device__ __forceinline__ void tile_mma_row1(const uint8_t* __restrict__ t, int
   } else {  // Q6_K: 16 sub-blocks of 16 elements -> two accumulator sets of 8 columns
     const uint4 s0v = lds_v4(t + 16 * g), s1v = lds_v4(t + 16 * (g + 8));
     const uint32_t scw[2][4] = {{s0v.x, s0v.y, s0v.z, s0v.w}, {s1v.x, s1v.y, s1v.z, s1v.w}};
-    const int16_t* b0p = act.bs16 + kt * 16;
-    const uint4 p0 = ld_v4(b0p), p1 = ld_v4(b0p + 8);
+    const int16_t* b0p = act.bs16 + (int64_t)kt * act.R * 16;
+    const uint4 p0 = ld_v4(b0p), p1 = ld_v4(b0p + act.R * 8);
     const uint32_t bw0[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
     int off32[2];
 #pragma unroll
@@ -315,8 +351,9 @@ __device__ __forceinline__ void tile_mma_row1(const uint8_t* __restrict__ t, int
       off32[hr] = -32 * o0;
     }
     // this lane's activation fragments: elements 4c .. 4c+3 of sub-blocks g and g + 8
-    const uint32_t fa = ld_u32(act.qs + kt * 256 + 16 * g + 4 * c);
-    const uint32_t fb = ld_u32(act.qs + kt * 256 + 16 * (g + 8) + 4 * c);
+    const int8_t* const qp = act.qs + (int64_t)(4 * kt + (g >> 2)) * act.R * 64 +
+                             (ORDER == ActOrder::order16 ? 16 * c + 4 * (g & 3) : 16 * (2 * (g & 1) + (c >> 1)) + 8 * ((g >> 1) & 1) + 4 * (c & 1));
+    const uint32_t fa = ld_u32(qp), fb = ld_u32(qp + act.R * 128);
     int ca[4] = {0, 0, 0, 0}, cb[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int i = 0; i < 4; i++) {
