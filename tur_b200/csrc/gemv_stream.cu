@@ -42,6 +42,14 @@ constexpr int RED_SLOTS = 2;           // partial-sum hand-over buffers between 
 // same (one / two, us: Q6_K 4096 x 12288, 6 rows 14.75 / 14.73; Q8_0 5120 x 25600, 4 rows 33.4 / 33.5; Q4_K 9600 x 8192,
 // 8 rows 18.0 / 18.1).
 constexpr int red_slots_of(int halves, int mg) { return halves == 2 && mg == 1 ? 1 : RED_SLOTS; }
+// Consumer warps whose tiles arrive in one copy, on one barrier. The producer needs some 130 cycles to arm a barrier and issue a
+// copy; at a tile a copy that is what a large launch waits for. Copies of 1 / 2 / 4 / 8 tiles, us: 2 x 25600 x 5120 Q4_K, one row
+// 31.8 / 30.2 / 29.8 / 29.7, 8 rows 35.9 / 33.8 / 32.2 / 32.4, 16 rows 48.3 / 46.1 / 45.0 / 44.7; 2 x 12288 x 4096 Q4_K, one row 14.7 /
+// 13.9 / 14.0 / 13.7 (15.3 before this choice), 16 rows 23.6 / 23.9 / 23.6 / 23.7; 4096 x 12288 Q6_K, 8 rows 13.3 / 13.3 / 13.1 / 13.6:
+// with all eight in one copy every warp waits for the last byte of a stage. Eight lanes that issue a copy each were slower
+// than one lane with two copies (2 x 25600 x 5120, one row: 33.3).
+constexpr int TPC = 4;
+constexpr int GROUPS = NW / TPC;       // copies and full barriers of a stage
 constexpr int MAX_STAGES = 6;
 constexpr uint32_t SPIN_LIMIT = 1u << 23;
 constexpr long long WAIT_CYCLES = 2000000000ll;  // about one second of SM clock
@@ -105,7 +113,7 @@ extern "C" int turq_debug_read_trace(unsigned long long* host, int n) {
 struct SmemPlan {
   int ring, act_qs, act_dsc, act_bs16, act_bs32, red, bars, total;
 };
-constexpr int bar_bytes(int red_slots) { return (MAX_STAGES * NW + MAX_STAGES + 2 * red_slots) * 8; }
+constexpr int bar_bytes(int red_slots) { return (MAX_STAGES * GROUPS + MAX_STAGES + 2 * red_slots) * 8; }
 
 constexpr int MAX_PARTS = 4;  // weights that share one activation and one launch (q|k|v, gate|up)
 
@@ -225,15 +233,14 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
   constexpr int GROUP = TileGeom<DT>::GROUP;
   static_assert(!MIXED || (GROUP == 1 && TileGeom<DT2>::GROUP == 1 && TileGeom<DT>::ELEMS == TileGeom<DT2>::ELEMS),
                 "mixed launches pair K-quant types only");
-  constexpr int UNIT_BYTES = (TB2 > TB ? TB2 : TB) * GROUP;
   constexpr bool NEED16 = DT == TQ_Q6_K || DT2 == TQ_Q6_K;
   constexpr bool NEED32 = DT == TQ_Q4_K || DT == TQ_Q5_K || DT2 == TQ_Q4_K || DT2 == TQ_Q5_K;
   extern __shared__ __align__(128) uint8_t smem[];
   const SmemPlan& sp = a.sp;
   const int half = HALVES == 2 ? (int)threadIdx.x / THREADS : 0;
   const int htid = (int)threadIdx.x - half * THREADS;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + sp.bars + half * bar_bytes(RSLOTS));  // [stage][consumer warp]: one tile each
-  uint64_t* empty = full + MAX_STAGES * NW;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + sp.bars + half * bar_bytes(RSLOTS));  // [stage][group of consumer warps]
+  uint64_t* empty = full + MAX_STAGES * GROUPS;
   uint64_t* red_full = empty + MAX_STAGES;
   uint64_t* red_empty = red_full + RSLOTS;
   uint64_t* const common = reinterpret_cast<uint64_t*>(smem + sp.bars + HALVES * bar_bytes(RSLOTS));
@@ -253,10 +260,9 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
   const int u0 = start_of(b), u1 = start_of(b + 1);
 
   {
-    // one barrier per thread: ~60 mbarrier.init in sequence on one thread cost most of a
-    // microsecond before the first copy could be issued
+    // one barrier per thread: mbarrier.init in sequence on one thread would hold up the first copy
     const int tid = htid;
-    const int nfull = a.stages * NW;
+    const int nfull = a.stages * GROUPS;
     int i = tid;
     bool did = true;
     if (i < nfull) {
@@ -321,8 +327,8 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
         }
         issued++;
         if (!mbar_wait(&empty[slot], ph ^ 1u, abort_flag)) break;
-        // one copy per consumer warp (its tile, or its group of Q8_0 tiles), each completing on
-        // that warp's own barrier: a warp starts as soon as its bytes are there
+        // one copy per group of consumer warps (their tiles are contiguous), each completing on the group's
+        // own barrier: it starts as soon as its bytes are there
         int part = 0, rt_in_part;
         if (a.interleave) {
           part = w.rt & 1;
@@ -332,16 +338,23 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
           rt_in_part = w.rt - a.rt_begin[part];
         }
         const int tb = (MIXED && a.part_alt[part]) ? TB2 : TB;
-        const uint8_t* src = a.tiles[part] + ((int64_t)rt_in_part * a.ktiles + (int64_t)w.ku * GROUP) * tb;
+        const int t0 = w.ku * GROUP;
+        int nt = a.ktiles - t0;  // tiles of the stage
+        if (nt > n * GROUP) nt = n * GROUP;
+        const uint8_t* src = a.tiles[part] + ((int64_t)rt_in_part * a.ktiles + t0) * tb;
         uint8_t* dst = ring + slot * a.stage_bytes;
-        for (int i = 0; i < n; i++) {
-          int nt = a.ktiles - (w.ku + i) * GROUP;
-          if (nt > GROUP) nt = GROUP;
-          const uint32_t bytes = (uint32_t)nt * tb;
-          mbar_expect_tx(&full[slot * NW + i], bytes);
-          bulk_g2s(dst + i * UNIT_BYTES, src + (size_t)i * GROUP * tb, bytes, &full[slot * NW + i]);
+#pragma unroll
+        for (int i = 0; i < GROUPS; i++) {
+          int c = nt - i * TPC * GROUP;
+          if (c > TPC * GROUP) c = TPC * GROUP;
+          if (c > 0) {
+            const uint32_t bytes = (uint32_t)c * tb;
+            mbar_expect_tx(&full[slot * GROUPS + i], bytes);
+            bulk_g2s(dst + i * TPC * GROUP * tb, src + (size_t)i * TPC * GROUP * tb, bytes, &full[slot * GROUPS + i]);
+          } else {
+            mbar_arrive(&full[slot * GROUPS + i]);  // unused this stage: keep phases in step
+          }
         }
-        for (int i = n; i < NW; i++) mbar_arrive(&full[slot * NW + i]);  // unused this stage: keep phases in step
         w.advance(n);
         w.next_row_if_needed();
         if (++slot == a.stages) { slot = 0; ph ^= 1u; }
@@ -462,20 +475,20 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
       // producer completes that phase with a plain arrive): a warp that skipped the wait could
       // run more than one phase ahead of the producer, pass a later parity test too early
       // and release the stage twice.
-      if (!mbar_wait(&full[slot * NW + warp], ph, abort_flag)) break;
+      if (!mbar_wait(&full[slot * GROUPS + warp / TPC], ph, abort_flag)) break;
       if (warp == 0 && first) TRACE(4);
       first = false;
       if (warp < n) {
         const int kt = (w.ku + warp) * GROUP;
         int left = a.ktiles - kt;
         if (left > GROUP) left = GROUP;
-        const uint8_t* tile = ring + slot * a.stage_bytes + warp * UNIT_BYTES;
         bool alt = false;
         if constexpr (MIXED) {
           int part = 0;
           while (part + 1 < a.nparts && w.rt >= a.rt_begin[part + 1]) part++;
           alt = a.part_alt[part] != 0;
         }
+        const uint8_t* tile = ring + slot * a.stage_bytes + warp * ((MIXED && alt ? TB2 : TB) * GROUP);
         // one activation row: the single-row tile function (same bits, about half the instructions)
         bool done_row1 = false;
         if constexpr (MG == 1 && DT != TQ_Q8_0 && DT2 != TQ_Q8_0) {
