@@ -53,6 +53,7 @@ class Mode(enum.IntEnum):
 
 _TORCH_TO_GGML = {torch.float32: GgmlDType.F32, torch.float16: GgmlDType.F16, torch.bfloat16: GgmlDType.BF16}
 _GGML_TO_TORCH = {v: k for k, v in _TORCH_TO_GGML.items()}
+_ACTIVATION_CODE = {torch.float32: int(GgmlDType.F32), torch.bfloat16: int(GgmlDType.BF16)}  # activation types of the kernels
 
 
 class _Context:
@@ -113,14 +114,18 @@ def new_context(device: int | torch.device | None = None) -> _Context:
     return _Context(device)
 
 
-def _stream_ptr(device: int) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def _stream_ptr(device: int) -> int:
+    return torch.cuda.current_stream(device).cuda_stream
+
+
+# The same without a Stream object on the way (1.2 us a call), where this build of torch has it.
+_stream_ptr = getattr(torch._C, "_cuda_getCurrentRawStream", _stream_ptr)
 
 
 def _check_operand(t: torch.Tensor, what: str, device: int, dtypes: Sequence[torch.dtype]) -> None:
     """The kernels dereference raw pointers on the weight's device: refuse, before any launch,
     a tensor that lives elsewhere, has another element type or is not dense."""
-    if not t.is_cuda or t.device.index != device:
+    if not t.is_cuda or t.get_device() != device:
         raise TurqError(1, f"{what} lives on {t.device}, the weight on cuda:{device}")
     if t.dtype not in dtypes:
         raise TurqError(3, f"{what} has dtype {t.dtype}, expected one of {[str(d) for d in dtypes]}")
@@ -271,11 +276,11 @@ class QMatMul:
         """x [..., k] -> [..., n] f32. CUDA tensors run stream-ordered on the current stream;
         CPU tensors go through the host-buffer entry (copies inside the call)."""
         qt = self.qtensor
-        n, k = qt.shape()
+        n, k = qt._shape
+        lead = x.shape[:-1]
         if x.dim() < 1 or x.shape[-1] != k:
             raise TurqError(2, f"last dim of x {tuple(x.shape)} must equal in-features {k}")
         mode = self.mode if mode is None else mode
-        lead = tuple(x.shape[:-1])
         lib = _lib.load()
         ctx = qt._ctx
         if not x.is_cuda:
@@ -290,25 +295,33 @@ class QMatMul:
             ctx.check(lib.turq_qmatmul_host(ctx.handle, qt._h, x2.data_ptr(), x2.shape[0], y.data_ptr(), int(mode),
                                             b.data_ptr() if b is not None else None))
             return y if y.shape == (*lead, n) else y.reshape(*lead, n)
-        if x.dtype not in (torch.float32, torch.bfloat16):
-            x = x.to(torch.float32)
-        x2 = x.reshape(-1, k).contiguous()
-        m = x2.shape[0]
-        _check_operand(x2, "x", ctx.device, (torch.float32, torch.bfloat16))
+        # A program that calls its linears one by one waits for this function, not for the GPU: no views, device objects or
+        # conversions that the call does not need (28 linears of a 0.6B model, one row: 14.5 us a call before, 8.8 now).
+        code = _ACTIVATION_CODE.get(x.dtype)
+        if code is None:
+            x, code = x.to(torch.float32), 0
+        if not x.is_contiguous():
+            x = x.contiguous()
+        if x.get_device() != ctx.device:
+            _check_operand(x, "x", ctx.device, (torch.float32, torch.bfloat16))
+        m = x.numel() // k
+        b = None
         if bias is not None:
             _check_operand(bias, "bias", ctx.device, (torch.float32,))
             if bias.numel() != n:
                 raise TurqError(2, f"bias has {bias.numel()} elements, the weight {n} rows")
-        if out is not None:
+            b = bias.data_ptr()
+        if out is None:
+            y = torch.empty((*lead, n), dtype=torch.float32, device=x.device)
+        else:
             _check_operand(out, "out", ctx.device, (torch.float32,))
             if out.numel() != m * n:
                 raise TurqError(2, f"out has {out.numel()} elements, expected {m} x {n}")
-        y = out if out is not None else torch.empty((m, n), dtype=torch.float32, device=qt.device())
-        ctx.check(lib.turq_qmatmul(ctx.handle, qt._h, ctypes.c_void_p(x2.data_ptr()), int(_TORCH_TO_GGML[x2.dtype]), m,
-                                   ctypes.c_void_p(y.data_ptr()), int(mode),
-                                   ctypes.c_void_p(bias.data_ptr()) if bias is not None else None,
-                                   _stream_ptr(ctx.device)))
-        return y.reshape(*lead, n)
+            y = out
+        st = lib.turq_qmatmul(ctx.handle, qt._h, x.data_ptr(), code, m, y.data_ptr(), int(mode), b, _stream_ptr(ctx.device))
+        if st != 0:
+            ctx.check(st)
+        return y if out is None else y.reshape(*lead, n)
 
     __call__ = forward
 
