@@ -1,6 +1,7 @@
-"""Cluster sizes of the decode-batch GEMM (plan_batch_cluster in tur_b200/csrc/launch_plan.h), compiled with g++ and checked
-on the CPU: every CTA of a cluster has units of its own, the measured choices are the ones taken, and the weights of a
-transformer layer that share an activation agree, so that they go out as one launch."""
+"""Cluster sizes of the decode-batch GEMM and tile heights of the prefill GEMM (plan_batch_cluster and plan_gemm_rows in
+tur_b200/csrc/launch_plan.h), compiled with g++ and checked on the CPU: every CTA of a cluster has units of its own, the measured
+choices are the ones taken, the weights of a transformer layer that share an activation agree on a cluster size, so that
+they go out as one launch, and a tile height is a legal one that needs no more time by the plan's measure than 256 rows."""
 import ctypes
 import os
 import subprocess
@@ -12,21 +13,27 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SHIM = r"""
 #include "launch_plan.h"
 extern "C" int batch_cluster(int tiles, int KU, const int* resident) { return turq::plan_batch_cluster(tiles, KU, resident); }
+extern "C" int gemm_rows(long long call_tiles, long long m, int sms) { return turq::plan_gemm_rows(call_tiles, m, sms); }
 """
 B200 = [0, 148, 74, 45, 33, 26, 22]     # clusters of 1..6 CTAs that are resident at once
 
 
 @pytest.fixture(scope="module")
-def cluster():
+def lib():
     with tempfile.TemporaryDirectory() as d:
         src, so = os.path.join(d, "shim.cpp"), os.path.join(d, "shim.so")
         open(src, "w").write(SHIM)
         subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", os.path.join(ROOT, "tur_b200", "csrc"), src, "-o", so], check=True)
         lib = ctypes.CDLL(so)
+        lib.gemm_rows.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int]
+        yield lib
 
-        def call(n, k, resident=B200):
-            return lib.batch_cluster(-(-n // 128), -(-k // 256), (ctypes.c_int * 7)(*resident))
-        yield call
+
+@pytest.fixture(scope="module")
+def cluster(lib):
+    def call(n, k, resident=B200):
+        return lib.batch_cluster(-(-n // 128), -(-k // 256), (ctypes.c_int * 7)(*resident))
+    return call
 
 
 def test_every_cta_has_units(cluster):
@@ -49,3 +56,23 @@ def test_measured_choices(cluster, n, k, want):
 @pytest.mark.parametrize("hidden,q,kv", [(1024, 2048, 1024), (2560, 2560, 640), (4096, 4096, 1024), (5120, 8192, 1024), (4096, 4096, 4096)])
 def test_projections_of_a_layer_share_a_launch(cluster, hidden, q, kv):
     assert cluster(q, hidden) == cluster(kv, hidden)
+
+
+@pytest.mark.parametrize("rows,m,tiles", [((4096, 1024, 1024), 512, 3), ((4096,), 512, 4), ((12288, 12288), 512, 2), ((2560, 640, 640), 1000, 4),
+                                          ((2560,), 1000, 7), ((8192, 8192), 1000, 4), ((4096,), 2048, 9), ((12288, 12288), 2048, 8),
+                                          ((5120,), 4096, 18), ((25600, 25600), 4096, 16), ((12288, 12288), 128, 1)])
+def test_tile_heights_that_were_measured_best(lib, rows, m, tiles):
+    assert -(-m // lib.gemm_rows(sum(-(-n // 256) for n in rows), m, 148)) == tiles
+
+
+def test_tile_heights_are_legal_and_no_worse_than_the_largest(lib):
+    def cost(call, m, b, slots):
+        return -(-call * -(-m // b) // slots) * max(b + 110, 260)
+    for sms in (148, 132, 16, 2, 1):
+        for call in (1, 3, 10, 24, 74, 200, 1187):
+            for m in (65, 80, 129, 255, 256, 257, 999, 2048, 2999, 65535, 2 ** 30):
+                b = lib.gemm_rows(call, m, sms)
+                assert b % 16 == 0 and 16 <= b <= 256, (call, m, b)
+                whole = -(-(-(-m // -(-m // 256))) // 16) * 16
+                slots = max(1, sms // 2)
+                assert cost(call, m, b, slots) <= cost(call, m, whole, slots)

@@ -541,11 +541,13 @@ static int32_t qmatmul_multi_impl(turq_ctx* ctx, int32_t count, const turq_qtens
       if (e != cudaSuccess) return cuda_fail(ctx, e, "qmatmul_multi launch");
       return TURQ_OK;
     }
+    int64_t call_tiles = 0;
+    for (int i = 0; i < count; i++) call_tiles += (qts[i]->n_rows + 255) / 256;
     for (int i = 0; i < count; i++) {
       int launches = 0;
       cudaError_t e = turq::launch_gemm_tc(qts[i]->dtype, qts[i]->tiles, qts[i]->n_rows, k, dev_x, x_dtype, m, dev_ys[i],
                                            dev_biases ? dev_biases[i] : nullptr, ctx->scratch, ctx->gemm_ws, ctx->sm_count,
-                                           static_cast<cudaStream_t>(stream), &launches, ctx->dev_status, i,
+                                           static_cast<cudaStream_t>(stream), &launches, ctx->dev_status, call_tiles, i,
                                            i + 1 < count ? qts[i + 1]->n_rows : 0);
       ctx->launches += launches;
       if (e != cudaSuccess && i > 0)  // the launch before this one has set its go-ahead words
@@ -855,7 +857,7 @@ int32_t qmatmul_for_exchange(turq_ctx* ctx, const turq_qtensor* qt, const void* 
     cudaError_t e = m <= GEMM_BATCH_ROWS
                         ? launch_gemm_batch(&part, 1, qt->n_cols, dev_x, x_dtype, m, ctx->scratch, s, &launches, ctx->dev_status, toggle)
                         : launch_gemm_tc(qt->dtype, qt->tiles, qt->n_rows, qt->n_cols, dev_x, x_dtype, m, s0, local_bias, ctx->scratch,
-                                         ctx->gemm_ws, ctx->sm_count, s, &launches, ctx->dev_status, 0, 0, toggle, s1);
+                                         ctx->gemm_ws, ctx->sm_count, s, &launches, ctx->dev_status, 0, 0, 0, toggle, s1);
     ctx->launches += launches;
     if (e != cudaSuccess) return cuda_fail(ctx, e, "row-parallel GEMM launch");
     return TURQ_OK;

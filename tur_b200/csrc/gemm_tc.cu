@@ -577,13 +577,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
 // largest magnitude into [8192, 16384): rows of large values do not overflow f16 and rows of
 // tiny values do not sink into its subnormals. rscale[m] undoes the scale exactly in the
 // epilogue. Rows that are all zero, or hold an infinity or NaN, are converted as they are.
-// The row is written in the operands' k order (tc_common.cuh): as a row of [m, k] (image_rows = 0, prefill),
+// The row is written in the operands' k order (tc_common.cuh): as a row of [m, k] (prefill),
 // or as a row of the operand's shared-memory image [k / 64][image_rows][128 bytes], 128B-swizzled, which
 // decode batches copy in whole. One CTA per row;
-// up to 4096 values stay in registers between the two passes. At 48 registers a thread a CTA fits
-// beside a CTA of the GEMM, so the conversion of the next call is resident before this call ends.
-__global__ void __launch_bounds__(256, 6) prep_act_kernel(const void* __restrict__ x, int is_bf16, int64_t k, int image_rows,
-                                                          __half* __restrict__ xh, float* __restrict__ rscale) {
+// up to 4096 values stay in registers between the two passes. At 48 registers a thread (40 where the GEMM behind has a warp
+// more) a CTA fits beside a CTA of the GEMM, so the conversion of the next call is resident before this call ends.
+template <bool IMAGE>
+__global__ void __launch_bounds__(256, IMAGE ? 6 : 5) prep_act_kernel(const void* __restrict__ x, int is_bf16, int64_t k, int image_rows,
+                                                                      __half* __restrict__ xh, float* __restrict__ rscale) {
   __shared__ float wmax[8];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMM behind may start on its weights
   asm volatile("griddepcontrol.wait;" ::: "memory");               // x may still be written, the operand buffer still read
@@ -631,7 +632,7 @@ __global__ void __launch_bounds__(256, 6) prep_act_kernel(const void* __restrict
       for (int e = 0; e < 2; e++) o[2 * h + e] = h22u(__floats2half2_rn(u[4 * h + e] * s, u[4 * h + e + 2] * s));
     // the two fours of an eight belong to two 16-k chunks
     const int in_block = (int)(i & 32) + (int)(i & 31) / 2;  // inside the 64-k block
-    if (image_rows) {
+    if constexpr (IMAGE) {
       uint8_t* const p = reinterpret_cast<uint8_t*>(xh) + ((i >> 6) * image_rows + blockIdx.x) * 128;
       const int off = (2 * in_block) ^ ((int)(blockIdx.x & 7) << 4);  // 16-byte chunks exchanged by the row's low bits
       *reinterpret_cast<uint2*>(p + off) = make_uint2(o[0], o[1]);
@@ -708,12 +709,6 @@ cudaError_t launch_tc_dt(const CUtensorMap& map, GemmArgs a, int pairs, cudaStre
 
 }  // namespace
 
-// Activation rows per pair tile for the height class of plan_gemm_bn: the rows dealt out evenly.
-static int tile_rows(int64_t m, int cls) {
-  const int64_t mt = (m + cls - 1) / cls;
-  return (int)(((m + mt - 1) / mt + 15) / 16 * 16);
-}
-
 // The f16 operand: rows up to a multiple of 16 for the image of a decode batch.
 size_t gemm_operand_bytes(int64_t m, int64_t k) { return ((size_t)((m + 15) / 16 * 16) * (size_t)k * 2 + 255) & ~(size_t)255; }
 size_t gemm_tc_scratch_bytes(int64_t m, int64_t k) { return gemm_operand_bytes(m, k) + (((size_t)m * 4 + 255) & ~(size_t)255) + 256; }
@@ -722,17 +717,17 @@ size_t gemm_tc_scratch_bytes(int64_t m, int64_t k) { return gemm_operand_bytes(m
 size_t gemm_workspace_bytes(int sms) { return (size_t)GEMM_SIBLINGS * sms * 4; }
 
 cudaError_t launch_prep_act(const void* x, int x_dtype, int64_t m, int64_t k, int image_rows, uint8_t* xh, float* rscale, cudaStream_t s) {
-  cudaError_t e = prefer_matmul_carveout<prep_act_kernel>();
+  cudaError_t e = image_rows ? prefer_matmul_carveout<prep_act_kernel<true>>() : prefer_matmul_carveout<prep_act_kernel<false>>();
   if (e != cudaSuccess) return e;
-  return launch_pdl(prep_act_kernel, dim3((unsigned)m), dim3(256), 0, s, x, (int)(x_dtype == TQ_BF16), k, image_rows,
+  return launch_pdl(image_rows ? prep_act_kernel<true> : prep_act_kernel<false>, dim3((unsigned)m), dim3(256), 0, s, x, (int)(x_dtype == TQ_BF16), k, image_rows,
                     reinterpret_cast<__half*>(xh), rscale);
 }
 
-// Activation rows per pair tile, activation tiles and pairs of a launch.
+// Activation rows per pair tile, activation tiles and pairs of a launch; call_tiles: 256-row tiles of all weights of the call.
 struct TcShape { int bn, mt; GemmWork work; };
-static TcShape tc_shape(int64_t n_rows, int64_t m, int64_t k, int sm_count) {
+static TcShape tc_shape(int64_t n_rows, int64_t call_tiles, int64_t m, int64_t k, int sm_count) {
   TcShape p;
-  p.bn = tile_rows(m, plan_gemm_bn(n_rows, m, sm_count));
+  p.bn = plan_gemm_rows(call_tiles, m, sm_count);
   p.mt = (int)((m + p.bn - 1) / p.bn);
   p.work = plan_gemm_work(n_rows, m, k, p.mt, sm_count);
   return p;
@@ -740,7 +735,8 @@ static TcShape tc_shape(int64_t n_rows, int64_t m, int64_t k, int sm_count) {
 
 cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int64_t k, const void* x, int x_dtype,
                            int64_t m, float* y, const float* bias, uint8_t* scratch, uint8_t* workspace, int sm_count, cudaStream_t s,
-                           int* launches, int* dev_status_word, int sibling, int64_t next_rows, const unsigned* y_toggle, float* y_alt) {
+                           int* launches, int* dev_status_word, int64_t call_tiles, int sibling, int64_t next_rows, const unsigned* y_toggle,
+                           float* y_alt) {
   if (k % BK != 0 || m <= GEMM_BATCH_ROWS || m > INT32_MAX || k > INT32_MAX || sibling < 0 ||
       sibling + (next_rows > 0 ? 1 : 0) >= GEMM_SIBLINGS) return cudaErrorInvalidValue;
   EncodeTiledFn enc = encode_fn();
@@ -753,7 +749,8 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
     if (e != cudaSuccess) return e;
   }
 
-  const TcShape shape = tc_shape(n_rows, m, k, sm_count);
+  const int64_t n_tiles = (n_rows + 2 * BM - 1) / (2 * BM);
+  const TcShape shape = tc_shape(n_rows, call_tiles > 0 ? call_tiles : n_tiles, m, k, sm_count);
   const int bn = shape.bn;
   CUtensorMap map;
   const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
@@ -774,7 +771,6 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
   a.m = (int)m;
   a.bn = bn;
   a.mt = shape.mt;
-  const int64_t n_tiles = (n_rows + 2 * BM - 1) / (2 * BM);
   const GemmWork& work = shape.work;
   const int64_t total = n_tiles * a.mt;
   if (total > (int64_t)1 << 30) return cudaErrorInvalidValue;
@@ -785,7 +781,7 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
   a.bias = bias;
   a.go = reinterpret_cast<int*>(workspace) + (size_t)sibling * sm_count;
   a.next_go = a.go + sm_count;
-  a.next_ctas = next_rows > 0 ? 2 * tc_shape(next_rows, m, k, sm_count).work.pairs : 0;
+  a.next_ctas = next_rows > 0 ? 2 * tc_shape(next_rows, call_tiles, m, k, sm_count).work.pairs : 0;
   a.status = dev_status_word;
   a.y_toggle = y_toggle;
   a.y_alt = y_alt;

@@ -136,7 +136,8 @@ size_t gemm_operand_bytes(int64_t m, int64_t k);  // the operand at the start of
 size_t gemm_tc_scratch_bytes(int64_t m, int64_t k);
 // The conversion launch: as [m, k], or (image_rows > 0) as the operand image of a decode batch.
 cudaError_t launch_prep_act(const void* x, int x_dtype, int64_t m, int64_t k, int image_rows, uint8_t* xh, float* rscale, cudaStream_t s);
-// Prefill, m > GEMM_BATCH_ROWS. workspace: gemm_workspace_bytes(sm_count) that read zero at launch.
+// Prefill, m > GEMM_BATCH_ROWS. call_tiles: 256-row tiles of all weights of the call, the same for each (0: this is the
+// only one). workspace: gemm_workspace_bytes(sm_count) that read zero at launch.
 // sibling: index of the weight in a call whose weights share x. The first one converts x; the later
 // ones (same m, k, x, scratch, workspace, stream, issued directly behind it) reuse the operand and
 // run beside their predecessor. next_rows: out-features of the weight that will be issued as the next
@@ -145,8 +146,8 @@ size_t gemm_workspace_bytes(int sm_count);
 cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int64_t k,
                            const void* x, int x_dtype, int64_t m, float* y, const float* bias,
                            uint8_t* scratch, uint8_t* workspace, int sm_count, cudaStream_t s, int* launches,
-                           int* dev_status_word, int sibling = 0, int64_t next_rows = 0, const unsigned* y_toggle = nullptr,
-                           float* y_alt = nullptr);
+                           int* dev_status_word, int64_t call_tiles = 0, int sibling = 0, int64_t next_rows = 0,
+                           const unsigned* y_toggle = nullptr, float* y_alt = nullptr);
 // Decode batches, m <= GEMM_BATCH_ROWS: the weights of a call (each part with its dtype) as one launch per cluster size
 // that their shapes ask for.
 cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, const void* x, int x_dtype, int64_t m, uint8_t* scratch,
