@@ -251,17 +251,6 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                "r"(bytes), "r"(s_u32(bar))
                : "memory");
 }
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_size() {
-  uint32_t r;
-  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(r));
-  return r;
-}
-
 // Walks chunks of columns; which CTA of the cluster adds one up, and which of that CTA's chunks it is. No divisions on the way.
 struct Chunk {
   int ch, owner, index;
@@ -758,20 +747,8 @@ cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, cons
     a.raw_slots = room / a.slot_bytes < MAX_RAW ? room / a.slot_bytes : MAX_RAW;
     if (a.raw_slots < 2) return cudaErrorInvalidConfiguration;
     const int clusters = a.items < resident[c] ? a.items : resident[c];
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(clusters * c));
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = (size_t)(ST * bn * 512 + a.raw_slots * a.slot_bytes + a.red_bytes) + BAR_BYTES + 1024;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = (unsigned)c;
-    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
-    e = cudaLaunchKernelEx(&cfg, gemm_batch_kernel, a);
+    const size_t smem = (size_t)(ST * bn * 512 + a.raw_slots * a.slot_bytes + a.red_bytes) + BAR_BYTES + 1024;
+    e = launch_pdl_cluster(gemm_batch_kernel, (unsigned)c, dim3((unsigned)(clusters * c)), dim3(THREADS), smem, s, a);
     if (launches) (*launches)++;
     if (e != cudaSuccess) return e;
   }

@@ -579,30 +579,38 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
 // epilogue. Rows that are all zero, or hold an infinity or NaN, are converted as they are.
 // The row is written in the operands' k order (tc_common.cuh): as a row of [m, k] (prefill),
 // or as a row of the operand's shared-memory image [k / 64][image_rows][128 bytes], 128B-swizzled, which
-// decode batches copy in whole. One CTA per row;
-// up to 4096 values stay in registers between the two passes. At 48 registers a thread (40 where the GEMM behind has a warp
-// more) a CTA fits beside a CTA of the GEMM, so the conversion of the next call is resident before this call ends.
-template <bool IMAGE>
-__global__ void __launch_bounds__(256, IMAGE ? 6 : 5) prep_act_kernel(const void* __restrict__ x, int is_bf16, int64_t k, int image_rows,
-                                                                      __half* __restrict__ xh, float* __restrict__ rscale) {
+// decode batches copy in whole. One CTA per row; up to 4096 values stay in registers between the search for the largest
+// magnitude and the conversion. Rows of more than 16384 values (CLUSTER): a cluster of CTAs, 4096 values each (beyond 8 x 4096 the
+// rest is read again), whose maxima meet in distributed shared memory: Q6_K 5120 x 25600 with the conversion, 32 / 64 rows 41.0 /
+// 47.6 -> 38.4 / 43.4 us. Below that the cluster's barriers cost what the second pass does: 4096 x 12288 17.2 / 20.0 and 18.7 / 20.0.
+// At 48 registers a thread (40 where the GEMM behind has a warp more) a CTA fits beside a CTA of the GEMM, so the conversion
+// of the next call is resident before this call ends.
+constexpr int PREP_THREADS = 256, PREP_KEEP = 2, PREP_VALUES = PREP_THREADS * 8 * PREP_KEEP, PREP_MAX_CLUSTER = 8;
+template <bool IMAGE, bool CLUSTER>
+__global__ void __launch_bounds__(PREP_THREADS, IMAGE ? 6 : 5) prep_act_kernel(const void* __restrict__ x, int is_bf16, int64_t k, int image_rows,
+                                                                               __half* __restrict__ xh, float* __restrict__ rscale) {
   __shared__ float wmax[8];
+  __shared__ float cta_max;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMM behind may start on its weights
   asm volatile("griddepcontrol.wait;" ::: "memory");               // x may still be written, the operand buffer still read
-  constexpr int KEEP = 2;
-  const int64_t row0 = (int64_t)blockIdx.x * k;
-  float v[KEEP][8];
+  const int csize = CLUSTER ? (int)cluster_size() : 1, rank = CLUSTER ? (int)cluster_rank() : 0;
+  const int64_t row = blockIdx.x / csize;
+  // this CTA's columns, in whole 64-k blocks
+  const int64_t per = CLUSTER ? (k / 64 + csize - 1) / csize * 64 : k, c0 = rank * per, c1 = c0 + per < k ? c0 + per : k;
+  const int64_t row0 = row * k;
+  float v[PREP_KEEP][8];
   float amax = 0.f;
 #pragma unroll
-  for (int j = 0; j < KEEP; j++) {
-    const int64_t i = ((int64_t)j * 256 + threadIdx.x) * 8;
-    if (i < k) {
+  for (int j = 0; j < PREP_KEEP; j++) {
+    const int64_t i = c0 + (j * PREP_THREADS + (int)threadIdx.x) * 8;
+    if (i < c1) {
       load8(x, is_bf16, row0 + i, v[j]);
 #pragma unroll
       for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(v[j][e]));
     }
   }
 #pragma unroll 2
-  for (int64_t i = ((int64_t)KEEP * 256 + threadIdx.x) * 8; i < k; i += 2048) {
+  for (int64_t i = c0 + PREP_VALUES + (int)threadIdx.x * 8; i < c1; i += PREP_THREADS * 8) {
     float u[8];
     load8(x, is_bf16, row0 + i, u);
 #pragma unroll
@@ -615,6 +623,17 @@ __global__ void __launch_bounds__(256, IMAGE ? 6 : 5) prep_act_kernel(const void
   amax = wmax[0];
 #pragma unroll
   for (int w = 1; w < 8; w++) amax = fmaxf(amax, wmax[w]);
+  if constexpr (CLUSTER) {
+    if (threadIdx.x == 0) cta_max = amax;
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int r = 0; r < csize; r++) {
+      float other;
+      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(other) : "r"(map_to_rank(s_u32(&cta_max), (uint32_t)r)));
+      amax = fmaxf(amax, other);
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // read: waited for before the CTA ends
+  }
   float s = 1.f;
   if (amax > 0.f && amax < 3.0e38f) {  // also false for NaN
     int e;
@@ -623,7 +642,7 @@ __global__ void __launch_bounds__(256, IMAGE ? 6 : 5) prep_act_kernel(const void
     if (se > 126) se = 126;     // keep the scale and its reciprocal normal numbers
     s = ldexpf(1.f, se);
   }
-  if (threadIdx.x == 0) rscale[blockIdx.x] = 1.f / s;
+  if (threadIdx.x == 0 && rank == 0) rscale[row] = 1.f / s;
   auto store8 = [&](int64_t i, const float (&u)[8]) {
     uint32_t o[4];
 #pragma unroll
@@ -633,8 +652,8 @@ __global__ void __launch_bounds__(256, IMAGE ? 6 : 5) prep_act_kernel(const void
     // the two fours of an eight belong to two 16-k chunks
     const int in_block = (int)(i & 32) + (int)(i & 31) / 2;  // inside the 64-k block
     if constexpr (IMAGE) {
-      uint8_t* const p = reinterpret_cast<uint8_t*>(xh) + ((i >> 6) * image_rows + blockIdx.x) * 128;
-      const int off = (2 * in_block) ^ ((int)(blockIdx.x & 7) << 4);  // 16-byte chunks exchanged by the row's low bits
+      uint8_t* const p = reinterpret_cast<uint8_t*>(xh) + ((i >> 6) * image_rows + row) * 128;
+      const int off = (2 * in_block) ^ ((int)(row & 7) << 4);  // 16-byte chunks exchanged by the row's low bits
       *reinterpret_cast<uint2*>(p + off) = make_uint2(o[0], o[1]);
       *reinterpret_cast<uint2*>(p + (off ^ 32)) = make_uint2(o[2], o[3]);
     } else {
@@ -644,16 +663,17 @@ __global__ void __launch_bounds__(256, IMAGE ? 6 : 5) prep_act_kernel(const void
     }
   };
 #pragma unroll
-  for (int j = 0; j < KEEP; j++) {
-    const int64_t i = ((int64_t)j * 256 + threadIdx.x) * 8;
-    if (i < k) store8(i, v[j]);
+  for (int j = 0; j < PREP_KEEP; j++) {
+    const int64_t i = c0 + (j * PREP_THREADS + (int)threadIdx.x) * 8;
+    if (i < c1) store8(i, v[j]);
   }
 #pragma unroll 2
-  for (int64_t i = ((int64_t)KEEP * 256 + threadIdx.x) * 8; i < k; i += 2048) {
+  for (int64_t i = c0 + PREP_VALUES + (int)threadIdx.x * 8; i < c1; i += PREP_THREADS * 8) {
     float u[8];
     load8(x, is_bf16, row0 + i, u);
     store8(i, u);
   }
+  if constexpr (CLUSTER) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -716,11 +736,22 @@ size_t gemm_tc_scratch_bytes(int64_t m, int64_t k) { return gemm_operand_bytes(m
 // Go-ahead words [weight of the call][CTA].
 size_t gemm_workspace_bytes(int sms) { return (size_t)GEMM_SIBLINGS * sms * 4; }
 
-cudaError_t launch_prep_act(const void* x, int x_dtype, int64_t m, int64_t k, int image_rows, uint8_t* xh, float* rscale, cudaStream_t s) {
-  cudaError_t e = image_rows ? prefer_matmul_carveout<prep_act_kernel<true>>() : prefer_matmul_carveout<prep_act_kernel<false>>();
+template <bool IMAGE, bool CLUSTER>
+static cudaError_t launch_prep(unsigned c, const void* x, int x_dtype, int64_t m, int64_t k, int image_rows, uint8_t* xh, float* rscale, cudaStream_t s) {
+  cudaError_t e = prefer_matmul_carveout<prep_act_kernel<IMAGE, CLUSTER>>();
   if (e != cudaSuccess) return e;
-  return launch_pdl(image_rows ? prep_act_kernel<true> : prep_act_kernel<false>, dim3((unsigned)m), dim3(256), 0, s, x, (int)(x_dtype == TQ_BF16), k, image_rows,
-                    reinterpret_cast<__half*>(xh), rscale);
+  return launch_pdl_cluster(prep_act_kernel<IMAGE, CLUSTER>, CLUSTER ? c : 0, dim3((unsigned)m * c), dim3(PREP_THREADS), 0, s, x, (int)(x_dtype == TQ_BF16), k,
+                            image_rows, reinterpret_cast<__half*>(xh), rscale);
+}
+cudaError_t launch_prep_act(const void* x, int x_dtype, int64_t m, int64_t k, int image_rows, uint8_t* xh, float* rscale, cudaStream_t s) {
+  int64_t c = k > 4 * PREP_VALUES ? (k + PREP_VALUES - 1) / PREP_VALUES : 1;
+  if (c > PREP_MAX_CLUSTER) c = PREP_MAX_CLUSTER;
+  if (m * c > INT32_MAX) c = 1;
+  if (image_rows)
+    return c > 1 ? launch_prep<true, true>((unsigned)c, x, x_dtype, m, k, image_rows, xh, rscale, s)
+                 : launch_prep<true, false>(1, x, x_dtype, m, k, image_rows, xh, rscale, s);
+  return c > 1 ? launch_prep<false, true>((unsigned)c, x, x_dtype, m, k, image_rows, xh, rscale, s)
+               : launch_prep<false, false>(1, x, x_dtype, m, k, image_rows, xh, rscale, s);
 }
 
 // Activation rows per pair tile, activation tiles and pairs of a launch; call_tiles: 256-row tiles of all weights of the call.

@@ -61,6 +61,16 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank) {
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
   return r;
 }
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(r));
+  return r;
+}
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
@@ -121,20 +131,28 @@ __device__ __forceinline__ UnitScales unit_scales(const uint8_t* t, int i, int l
 }
 
 // Launch with programmatic stream serialization: the kernel may be scheduled while its
-// predecessor in the stream still runs and orders itself with griddepcontrol.wait.
+// predecessor in the stream still runs and orders itself with griddepcontrol.wait. In clusters of `cluster` CTAs, or as
+// the kernel is declared (0).
 template <class... Params, class... Args>
-inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+inline cudaError_t launch_pdl_cluster(void (*kernel)(Params...), unsigned cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <class... Params, class... Args>
+inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+  return launch_pdl_cluster(kernel, 0, grid, block, smem, s, args...);
 }
 
 }  // namespace turq
