@@ -70,3 +70,18 @@ def test_one_call_of_several_types_and_cluster_sizes(tq, m):
     tq.QMatMul.forward_multi(mms[:3], x, mode=tq.Mode.TENSOR_CORE)
     assert tq.context().launch_count() - l0 == 2          # one conversion, one GEMM
     tq.context().poll_status()
+
+
+@pytest.mark.parametrize("k,dtype", [(256, torch.float32), (5120, torch.bfloat16), (16640, torch.float32), (33024, torch.bfloat16)])
+def test_one_call_of_both_k_orders(tq, k, dtype):
+    """Q6_K (in an order of its own where K is cut, which 256 columns are not) beside Q4_K: rows converted by one CTA and by several."""
+    rng = np.random.default_rng(SEED + 8200 + k)
+    ws = [(t, *make_weight(t, n, k, SEED + 8201 + n)) for t, n in ((oracle.Q4_K, 150), (oracle.Q6_K, 130))]
+    mms = [tq.QMatMul.from_arc(tq.QTensor.new(w, tq.GgmlDType(t), (n, k))) for t, w, n in ws]
+    x = torch.from_numpy(rng.standard_normal((33, k)).astype(np.float32)).to(dtype).cuda()
+    got = tq.QMatMul.forward_multi(mms, x, mode=tq.Mode.TENSOR_CORE)
+    for (t, w, n), mm, y in zip(ws, mms, got):
+        ref = oracle.matmul_f64(t, w, n, k, x.float().cpu().numpy())
+        assert np.linalg.norm(y.double().cpu().numpy() - ref) / np.linalg.norm(ref) < TOL
+        assert torch.equal(mm.forward(x, mode=tq.Mode.TENSOR_CORE), y)
+    tq.context().poll_status()

@@ -3,7 +3,8 @@
 //   y[m, n] = sum_k x[m, k] * W[n, k]      W quantized (device fragment tiles), x f32 or bf16
 //
 // Step 1 (prep kernel, gemm_tc.cu): x -> f16 with a power-of-two scale per row, written as the shared-memory
-// image of the B operand: 64-k blocks of bn rows x 128 bytes, 128B-swizzled, the blocks of a 256-k unit one behind the other.
+// image of the B operand: 64-k blocks of bn rows x 128 bytes, 128B-swizzled, the blocks of a 256-k unit one behind the other; in
+// the k order that all types share, in one of Q6_K's own (a lane then finds all that it converts in its own words), or both.
 // Step 2 (this kernel): a cluster of C CTAs computes 128 weight rows at a time, each CTA a share of the K loop. A unit is 256 k:
 //   * warps 0, 23   stream the raw quantized tiles of the unit (contiguous bytes per row-tile) into a ring with cp.async.bulk;
 //   * warp 1        one bulk copy of the unit's activation image (no tensor map, no multicast);
@@ -28,11 +29,13 @@
 // Measured with graph replay, conversion included, against pairs of CTAs (cta_group::2) with one launch per weight and partial
 // sums through global memory, us a call:
 //   attn_q|k|v 2560 + 640 + 640 x 2560 Q5_K, Q6_K, 32 rows 16.7 -> 7.6    ffn_gate|up 2 x 8192 x 2560 Q5_K, 32 rows 23.1 -> 12.8
-//   attn_q|k|v 8192 + 1024 + 1024 x 5120 Q4_K, Q6_K, 64 rows 32.2 -> 20.0   ffn_gate|up 2 x 25600 x 5120 Q4_K, 64 rows 68.4 -> 50.0
-//   attn_output 4096 x 4096 Q4_K, 32 rows 11.1 -> 8.1                      ffn_down 5120 x 25600 Q6_K, 64 rows 52.1 -> 47.3
+//   attn_q|k|v 8192 + 1024 + 1024 x 5120 Q4_K, Q6_K, 64 rows 32.2 -> 20.0   ffn_gate|up 2 x 25600 x 5120 Q4_K, 64 rows 68.4 -> 50.4
+//   attn_output 4096 x 4096 Q4_K, 32 rows 11.1 -> 8.1                      ffn_down 5120 x 25600 Q6_K, 64 rows 52.1 -> 40.6
 // Steps on the way (2 x 25600 x 5120, 64 rows): CTAs of their own instead of pairs 68.4 -> 66.6 us; whole units per warp instead of
 // halves of every unit 62.0; a second warp to issue the copies 59.0; partial sums through distributed shared memory instead of
 // global memory (a fence and a flag per chunk: up to 13 us an epilogue) 57.5; the row scales in shared memory 52.7.
+// Q6_K in a k order of its own (5120 x 25600, 32 / 64 rows): 38.3 / 43.0 -> 34.8 / 40.6 us; 4096 x 12288 17.2 / 20.0 -> 16.2 / 19.4;
+// a call that needs both images (the q|k|v above at 64 rows): 19.5 -> 20.0.
 // Every wait is bounded; on expiry the CTA records TURQ_E_TIMEOUT, releases its TMEM and returns.
 #include <atomic>
 
@@ -89,8 +92,9 @@ __device__ __forceinline__ RowScales row_scales(const uint8_t* t, int lane) {
 
 // 64-k block i of a unit (t: the row-tile's raw bytes in shared memory) as registers of a tcgen05.st 16x256b.x4:
 // register 4j + 2h + e of lane 4g + c holds columns 8j + 2c + e of row g + 8h, two f16 each, so
-// chunk j (16 k, one MMA) has from this lane the elements 32 (j / 2) + 8c + 4 (j % 2) + {0, 2, 1, 3}.
-template <int DT>
+// chunk j (16 k, one MMA) has from this lane the elements 32 (j / 2) + 8c + 4 (j % 2) + {0, 2, 1, 3}; in Q6_K's own order
+// (OWN) 16j + 4c + {0, 2, 1, 3}.
+template <int DT, bool OWN>
 __device__ __forceinline__ void dequant_frag(const uint8_t* t, const RowScales& us, int i, int lane, uint32_t (&o)[16]) {
   const int g = lane >> 2, c = lane & 3;
   if constexpr (DT == TQ_Q8_0) {
@@ -157,6 +161,27 @@ __device__ __forceinline__ void dequant_frag(const uint8_t* t, const RowScales& 
         o[4 * (2 + b) + 2 * hr + 1] = h22u(__hfma2(v[1][1], dhi, mhi));
       }
     }
+  } else if constexpr (OWN) {  // chunk j is the block's 16-element sub-block j
+    const uint4 ql = lds_v4(t + TQ_Q6K_QL + 512 * i + 16 * lane), qv = lds_v4(t + TQ_Q6K_QH + 512 * (i >> 1) + 16 * lane);
+    const __half2 off = __float2half2_rn(1056.f);     // 1024 + 32
+    const __half2 off_sc = __float2half2_rn(1152.f);  // 1024 + 128: the int8 scales are biased by xor 0x80
+#pragma unroll
+    for (int hr = 0; hr < 2; hr++) {
+      const uint32_t qh = (i & 1) ? (hr ? qv.w : qv.y) : (hr ? qv.z : qv.x);
+      // d * scale of the four sub-blocks in half arithmetic (exact product, one rounding)
+      const __half2 dd = __half2half2(__ushort_as_half((unsigned short)lds_u16(t + TQ_Q6K_D + 2 * (g + 8 * hr))));
+      const uint32_t scb = ld_u32(t + 16 * (g + 8 * hr) + 4 * i) ^ 0x80808080u;
+      const __half2 d01 = __hmul2(dd, __hsub2(pair01(scb), off_sc)), d23 = __hmul2(dd, __hsub2(pair23(scb), off_sc));
+#pragma unroll
+      for (int jj = 0; jj < 4; jj++) {
+        const __half2 dl = jj == 0 ? __low2half2(d01) : jj == 1 ? __high2half2(d01) : jj == 2 ? __low2half2(d23) : __high2half2(d23);
+        const uint32_t w = jj < 2 ? (hr ? ql.z : ql.x) : (hr ? ql.w : ql.y);
+        const int sh = 2 * jj;  // 2-bit field jj of the qh word moved to bits 4..5 of every byte
+        const uint32_t m = (((jj & 1) ? w >> 4 : w) & 0x0F0F0F0Fu) | ((sh <= 4 ? qh << (4 - sh) : qh >> (sh - 4)) & 0x30303030u);
+        o[4 * jj + 2 * hr] = h22u(__hmul2(__hsub2(pair02(m), off), dl));
+        o[4 * jj + 2 * hr + 1] = h22u(__hmul2(__hsub2(pair13(m), off), dl));
+      }
+    }
   } else {  // Q6_K: a lane takes its eight elements of every 32 from the two lanes that hold them in the tile
     const int nib = c >> 1, la = 4 * g + 2 * (c & 1);
     const uint8_t* const qhp = t + TQ_Q6K_QH + 512 * (i >> 1) + 4 * (i & 1) + 16 * la;
@@ -195,8 +220,13 @@ __device__ __forceinline__ void tmem_store_block(uint32_t taddr, const uint32_t 
 }
 
 
+// Whether a weight is multiplied in the k order of its own tiles. Only where the K loop is cut: a sum that one CTA adds up
+// keeps the MMAs of the prefill kernel, and with them its bits.
+__host__ __device__ __forceinline__ bool own_order(int dtype, int csize) { return dtype == TQ_Q6_K && csize > 1; }
+
 struct BatchPart {
   const uint8_t* tiles;
+  const uint8_t* xh;   // B operand image in the weight's k order: [kblocks][bn][128 bytes]
   float* y;            // [m, n_rows]
   float* y_alt;
   const float* bias;
@@ -217,7 +247,6 @@ struct BatchArgs {
   int bn;               // the same, up to a multiple of 16
   int raw_slots, slot_bytes;
   int red_bytes;        // exchange buffer of a CTA
-  const uint8_t* xh;    // B operand image: [kblocks][bn][128 bytes]
   const float* rscale;  // [m] factor undoing the f16 row scaling
   int* status;
   // exchange slots (tp.cu): with y_toggle set, the result goes to y_alt instead of y when the
@@ -362,7 +391,7 @@ struct DequantPos {
 
 // A warp's share of an item: one 16-row tile (`dq` of the CTA's eight) of every other unit. Whole units, so that what a
 // unit costs beside the conversion itself (barriers, scales, addresses) is spread over four blocks.
-template <int DT>
+template <int DT, bool OWN = false>
 __device__ __forceinline__ void dequant_units(const BatchArgs& a, int ka, int kb, bool live, int dq, int grp, int lane, uint8_t* raw0,
                                               uint64_t* raw_full, uint64_t* raw_empty, uint64_t* full, uint64_t* empty, uint32_t tmem,
                                               DequantPos& pos, volatile int* abort_flag) {
@@ -381,7 +410,7 @@ __device__ __forceinline__ void dequant_units(const BatchArgs& a, int ka, int kb
         for (int b = 0; b < 4; b++)
           if (b == 0 || DT != TQ_Q8_0 || b < nb) {
             uint32_t o[16];
-            dequant_frag<DT>(raw, us, b, lane, o);
+            dequant_frag<DT, OWN>(raw, us, b, lane, o);
             tmem_store_block(dst + (uint32_t)(b * A_COLS), o);
           }
       }
@@ -505,13 +534,14 @@ __global__ void __launch_bounds__(REG_THREADS, 1) gemm_batch_kernel(const __grid
       uint32_t ph = 0;
       bool ok = true;
       while (ok && walk.next(a)) {
+        const uint8_t* const xh = a.part[walk.part].xh;
         for (int ku = ka; ku < kb; ku++) {
           ok = bar_wait(&empty[s], ph ^ 1u, abort_flag);
           if (!ok) break;
           const int nb = a.kblocks - 4 * ku < 4 ? a.kblocks - 4 * ku : 4;
           const uint32_t bytes = (uint32_t)(nb * a.bn * 128);
           bar_expect_tx(&full[s], bytes);
-          bulk_load(sB + s * b_stage, a.xh + (int64_t)ku * b_stage, bytes, &full[s]);
+          bulk_load(sB + s * b_stage, xh + (int64_t)ku * b_stage, bytes, &full[s]);
           if (++s == ST) { s = 0; ph ^= 1u; }
         }
       }
@@ -616,7 +646,12 @@ __global__ void __launch_bounds__(REG_THREADS, 1) gemm_batch_kernel(const __grid
         case TQ_Q8_0: dequant_units<TQ_Q8_0>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag); break;
         case TQ_Q4_K: dequant_units<TQ_Q4_K>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag); break;
         case TQ_Q5_K: dequant_units<TQ_Q5_K>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag); break;
-        default: dequant_units<TQ_Q6_K>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag); break;
+        default:
+          if (own_order(p.dtype, csize))
+            dequant_units<TQ_Q6_K, true>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag);
+          else
+            dequant_units<TQ_Q6_K>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag);
+          break;
       }
     }
     // nothing left to dequantize: help with the epilogue of the last item
@@ -705,9 +740,13 @@ cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, cons
     if ((parts[i].n_rows + BM - 1) / BM > (1 << 24)) return cudaErrorInvalidValue;
     cluster[i] = plan_batch_cluster((int)((parts[i].n_rows + BM - 1) / BM), KU, resident);
   }
-  float* rscale = reinterpret_cast<float*>(scratch + gemm_operand_bytes(m, k));
+  // images of both k orders where a call needs both, the row scales behind them
+  bool own = false, common = false;
+  for (int i = 0; i < nparts; i++) (own_order(parts[i].dtype, cluster[i]) ? own : common) = true;
+  uint8_t* const xh16 = scratch + (common ? gemm_operand_bytes(m, k) : 0);
+  float* rscale = reinterpret_cast<float*>(scratch + ((int)own + (int)common) * gemm_operand_bytes(m, k));
   const int bn = (int)(m + 15) / 16 * 16;
-  e = launch_prep_act(x, x_dtype, m, k, bn, scratch, rscale, s);
+  e = launch_prep_image(x, x_dtype, m, k, bn, common ? scratch : nullptr, own ? xh16 : nullptr, rscale, s);
   if (launches) (*launches)++;
   if (e != cudaSuccess) return e;
 
@@ -720,7 +759,6 @@ cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, cons
     a.KU = KU;
     a.m = (int)m;
     a.bn = bn;
-    a.xh = scratch;
     a.rscale = rscale;
     a.status = dev_status_word;
     a.y_toggle = y_toggle;
@@ -729,6 +767,7 @@ cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, cons
       done[i] = true;
       BatchPart& p = a.part[a.nparts++];
       p.tiles = parts[i].tiles;
+      p.xh = own_order(parts[i].dtype, c) ? xh16 : scratch;
       p.y = parts[i].y;
       p.y_alt = parts[i].y_alt;
       p.bias = parts[i].bias;

@@ -578,7 +578,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
 // tiny values do not sink into its subnormals. rscale[m] undoes the scale exactly in the
 // epilogue. Rows that are all zero, or hold an infinity or NaN, are converted as they are.
 // The row is written in the operands' k order (tc_common.cuh): as a row of [m, k] (prefill),
-// or as a row of the operand's shared-memory image [k / 64][image_rows][128 bytes], 128B-swizzled, which
+// or as a row of the operand's shared-memory images [k / 64][image_rows][128 bytes], 128B-swizzled, which
 // decode batches copy in whole. One CTA per row; up to 4096 values stay in registers between the search for the largest
 // magnitude and the conversion. Rows of more than 16384 values (CLUSTER): a cluster of CTAs, 4096 values each (beyond 8 x 4096 the
 // rest is read again), whose maxima meet in distributed shared memory: Q6_K 5120 x 25600 with the conversion, 32 / 64 rows 41.0 /
@@ -587,22 +587,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
 // of the next call is resident before this call ends.
 constexpr int PREP_THREADS = 256, PREP_KEEP = 2, PREP_VALUES = PREP_THREADS * 8 * PREP_KEEP, PREP_MAX_CLUSTER = 8;
 template <bool IMAGE, bool CLUSTER>
-__global__ void __launch_bounds__(PREP_THREADS, IMAGE ? 6 : 5) prep_act_kernel(const void* __restrict__ x, int is_bf16, int64_t k, int image_rows,
-                                                                               __half* __restrict__ xh, float* __restrict__ rscale) {
+__global__ void __launch_bounds__(PREP_THREADS, IMAGE ? 6 : 5) prep_act_kernel(const void* __restrict__ x, int is_bf16, uint32_t k, int image_rows,
+                                                                               __half* __restrict__ xh, __half* __restrict__ xh16,
+                                                                               float* __restrict__ rscale) {
   __shared__ float wmax[8];
   __shared__ float cta_max;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMM behind may start on its weights
   asm volatile("griddepcontrol.wait;" ::: "memory");               // x may still be written, the operand buffer still read
   const int csize = CLUSTER ? (int)cluster_size() : 1, rank = CLUSTER ? (int)cluster_rank() : 0;
-  const int64_t row = blockIdx.x / csize;
-  // this CTA's columns, in whole 64-k blocks
-  const int64_t per = CLUSTER ? (k / 64 + csize - 1) / csize * 64 : k, c0 = rank * per, c1 = c0 + per < k ? c0 + per : k;
-  const int64_t row0 = row * k;
+  const uint32_t row = blockIdx.x / csize;
+  // this CTA's columns, in whole 64-k blocks (k < 2^31: no sum below leaves 32 bits)
+  const uint32_t per = CLUSTER ? (k / 64 + csize - 1) / csize * 64 : k, c0 = rank * per, c1 = c0 + per < k ? c0 + per : k;
+  const int64_t row0 = (int64_t)row * k;
   float v[PREP_KEEP][8];
   float amax = 0.f;
 #pragma unroll
   for (int j = 0; j < PREP_KEEP; j++) {
-    const int64_t i = c0 + (j * PREP_THREADS + (int)threadIdx.x) * 8;
+    const uint32_t i = c0 + (j * PREP_THREADS + threadIdx.x) * 8;
     if (i < c1) {
       load8(x, is_bf16, row0 + i, v[j]);
 #pragma unroll
@@ -610,7 +611,7 @@ __global__ void __launch_bounds__(PREP_THREADS, IMAGE ? 6 : 5) prep_act_kernel(c
     }
   }
 #pragma unroll 2
-  for (int64_t i = c0 + PREP_VALUES + (int)threadIdx.x * 8; i < c1; i += PREP_THREADS * 8) {
+  for (uint32_t i = c0 + PREP_VALUES + threadIdx.x * 8; i < c1; i += PREP_THREADS * 8) {
     float u[8];
     load8(x, is_bf16, row0 + i, u);
 #pragma unroll
@@ -643,7 +644,7 @@ __global__ void __launch_bounds__(PREP_THREADS, IMAGE ? 6 : 5) prep_act_kernel(c
     s = ldexpf(1.f, se);
   }
   if (threadIdx.x == 0 && rank == 0) rscale[row] = 1.f / s;
-  auto store8 = [&](int64_t i, const float (&u)[8]) {
+  auto store8 = [&](uint32_t i, const float (&u)[8]) {
     uint32_t o[4];
 #pragma unroll
     for (int h = 0; h < 2; h++)
@@ -651,24 +652,30 @@ __global__ void __launch_bounds__(PREP_THREADS, IMAGE ? 6 : 5) prep_act_kernel(c
       for (int e = 0; e < 2; e++) o[2 * h + e] = h22u(__floats2half2_rn(u[4 * h + e] * s, u[4 * h + e + 2] * s));
     // the two fours of an eight belong to two 16-k chunks
     const int in_block = (int)(i & 32) + (int)(i & 31) / 2;  // inside the 64-k block
-    if constexpr (IMAGE) {
-      uint8_t* const p = reinterpret_cast<uint8_t*>(xh) + ((i >> 6) * image_rows + row) * 128;
-      const int off = (2 * in_block) ^ ((int)(row & 7) << 4);  // 16-byte chunks exchanged by the row's low bits
-      *reinterpret_cast<uint2*>(p + off) = make_uint2(o[0], o[1]);
-      *reinterpret_cast<uint2*>(p + (off ^ 32)) = make_uint2(o[2], o[3]);
+    if constexpr (IMAGE) {  // in the common order, in Q6_K's own, or in both
+      const size_t block = (size_t)((i >> 6) * (uint32_t)image_rows + row) * 128;
+      const int swz = (int)(row & 7) << 4;  // 16-byte chunks exchanged by the row's low bits
+      if (xh) {
+        uint8_t* const p = reinterpret_cast<uint8_t*>(xh) + block;
+        const int off = (2 * in_block) ^ swz;
+        *reinterpret_cast<uint2*>(p + off) = make_uint2(o[0], o[1]);
+        *reinterpret_cast<uint2*>(p + (off ^ 32)) = make_uint2(o[2], o[3]);
+      }
+      if (xh16)
+        *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(xh16) + block + ((2 * (int)(i & 63)) ^ swz)) = make_uint4(o[0], o[1], o[2], o[3]);
     } else {
-      __half* const p = xh + row0 + (i & ~(int64_t)63) + in_block;
+      __half* const p = xh + row0 + (i & ~63u) + in_block;
       *reinterpret_cast<uint2*>(p) = make_uint2(o[0], o[1]);
       *reinterpret_cast<uint2*>(p + 16) = make_uint2(o[2], o[3]);
     }
   };
 #pragma unroll
   for (int j = 0; j < PREP_KEEP; j++) {
-    const int64_t i = c0 + (j * PREP_THREADS + (int)threadIdx.x) * 8;
+    const uint32_t i = c0 + (j * PREP_THREADS + threadIdx.x) * 8;
     if (i < c1) store8(i, v[j]);
   }
 #pragma unroll 2
-  for (int64_t i = c0 + PREP_VALUES + (int)threadIdx.x * 8; i < c1; i += PREP_THREADS * 8) {
+  for (uint32_t i = c0 + PREP_VALUES + threadIdx.x * 8; i < c1; i += PREP_THREADS * 8) {
     float u[8];
     load8(x, is_bf16, row0 + i, u);
     store8(i, u);
@@ -731,27 +738,35 @@ cudaError_t launch_tc_dt(const CUtensorMap& map, GemmArgs a, int pairs, cudaStre
 
 // The f16 operand: rows up to a multiple of 16 for the image of a decode batch.
 size_t gemm_operand_bytes(int64_t m, int64_t k) { return ((size_t)((m + 15) / 16 * 16) * (size_t)k * 2 + 255) & ~(size_t)255; }
-size_t gemm_tc_scratch_bytes(int64_t m, int64_t k) { return gemm_operand_bytes(m, k) + (((size_t)m * 4 + 255) & ~(size_t)255) + 256; }
+// One operand, or two images of a decode batch; never less for more rows (a reservation stands for all smaller calls).
+size_t gemm_tc_scratch_bytes(int64_t m, int64_t k) {
+  const size_t rows = gemm_operand_bytes(m, k), images = 2 * gemm_operand_bytes(m < GEMM_BATCH_ROWS ? m : GEMM_BATCH_ROWS, k);
+  return (rows > images ? rows : images) + (((size_t)m * 4 + 255) & ~(size_t)255) + 256;
+}
 
 // Go-ahead words [weight of the call][CTA].
 size_t gemm_workspace_bytes(int sms) { return (size_t)GEMM_SIBLINGS * sms * 4; }
 
 template <bool IMAGE, bool CLUSTER>
-static cudaError_t launch_prep(unsigned c, const void* x, int x_dtype, int64_t m, int64_t k, int image_rows, uint8_t* xh, float* rscale, cudaStream_t s) {
+static cudaError_t launch_prep(unsigned c, const void* x, int x_dtype, int64_t m, int64_t k, int image_rows, uint8_t* xh, uint8_t* xh16, float* rscale,
+                               cudaStream_t s) {
   cudaError_t e = prefer_matmul_carveout<prep_act_kernel<IMAGE, CLUSTER>>();
   if (e != cudaSuccess) return e;
-  return launch_pdl_cluster(prep_act_kernel<IMAGE, CLUSTER>, CLUSTER ? c : 0, dim3((unsigned)m * c), dim3(PREP_THREADS), 0, s, x, (int)(x_dtype == TQ_BF16), k,
-                            image_rows, reinterpret_cast<__half*>(xh), rscale);
+  return launch_pdl_cluster(prep_act_kernel<IMAGE, CLUSTER>, CLUSTER ? c : 0, dim3((unsigned)m * c), dim3(PREP_THREADS), 0, s, x, (int)(x_dtype == TQ_BF16), (uint32_t)k,
+                            image_rows, reinterpret_cast<__half*>(xh), reinterpret_cast<__half*>(xh16), rscale);
 }
-cudaError_t launch_prep_act(const void* x, int x_dtype, int64_t m, int64_t k, int image_rows, uint8_t* xh, float* rscale, cudaStream_t s) {
-  int64_t c = k > 4 * PREP_VALUES ? (k + PREP_VALUES - 1) / PREP_VALUES : 1;
-  if (c > PREP_MAX_CLUSTER) c = PREP_MAX_CLUSTER;
-  if (m * c > INT32_MAX) c = 1;
-  if (image_rows)
-    return c > 1 ? launch_prep<true, true>((unsigned)c, x, x_dtype, m, k, image_rows, xh, rscale, s)
-                 : launch_prep<true, false>(1, x, x_dtype, m, k, image_rows, xh, rscale, s);
-  return c > 1 ? launch_prep<false, true>((unsigned)c, x, x_dtype, m, k, image_rows, xh, rscale, s)
-               : launch_prep<false, false>(1, x, x_dtype, m, k, image_rows, xh, rscale, s);
+static unsigned prep_cluster(int64_t m, int64_t k) {
+  const int64_t c = k > 4 * PREP_VALUES ? (k + PREP_VALUES - 1) / PREP_VALUES : 1;
+  return m * PREP_MAX_CLUSTER > INT32_MAX ? 1u : (unsigned)(c < PREP_MAX_CLUSTER ? c : PREP_MAX_CLUSTER);
+}
+cudaError_t launch_prep_image(const void* x, int x_dtype, int64_t m, int64_t k, int image_rows, uint8_t* xh, uint8_t* xh16, float* rscale, cudaStream_t s) {
+  const unsigned c = prep_cluster(m, k);
+  return c > 1 ? launch_prep<true, true>(c, x, x_dtype, m, k, image_rows, xh, xh16, rscale, s)
+               : launch_prep<true, false>(c, x, x_dtype, m, k, image_rows, xh, xh16, rscale, s);
+}
+static cudaError_t launch_prep_rows(const void* x, int x_dtype, int64_t m, int64_t k, uint8_t* xh, float* rscale, cudaStream_t s) {
+  const unsigned c = prep_cluster(m, k);
+  return c > 1 ? launch_prep<false, true>(c, x, x_dtype, m, k, 0, xh, nullptr, rscale, s) : launch_prep<false, false>(c, x, x_dtype, m, k, 0, xh, nullptr, rscale, s);
 }
 
 // Activation rows per pair tile, activation tiles and pairs of a launch; call_tiles: 256-row tiles of all weights of the call.
@@ -775,7 +790,7 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
   float* rscale = reinterpret_cast<float*>(scratch + gemm_operand_bytes(m, k));
   cudaError_t e = cudaSuccess;
   if (sibling == 0) {  // several weights that read the same x share one conversion
-    e = launch_prep_act(x, x_dtype, m, k, 0, scratch, rscale, s);
+    e = launch_prep_rows(x, x_dtype, m, k, scratch, rscale, s);
     if (launches) (*launches)++;
     if (e != cudaSuccess) return e;
   }

@@ -134,8 +134,8 @@ constexpr int GEMM_BATCH_ROWS = 64;  // decode batches: up to this many rows
 constexpr int GEMM_SIBLINGS = 4;
 size_t gemm_operand_bytes(int64_t m, int64_t k);  // the operand at the start of scratch, the row scales behind it
 size_t gemm_tc_scratch_bytes(int64_t m, int64_t k);
-// The conversion launch: as [m, k], or (image_rows > 0) as the operand image of a decode batch.
-cudaError_t launch_prep_act(const void* x, int x_dtype, int64_t m, int64_t k, int image_rows, uint8_t* xh, float* rscale, cudaStream_t s);
+// The conversion launch of a decode batch: operand images in the common k order (xh) and in Q6_K's own (xh16), either may be null.
+cudaError_t launch_prep_image(const void* x, int x_dtype, int64_t m, int64_t k, int image_rows, uint8_t* xh, uint8_t* xh16, float* rscale, cudaStream_t s);
 // Prefill, m > GEMM_BATCH_ROWS. call_tiles: 256-row tiles of all weights of the call, the same for each (0: this is the
 // only one). workspace: gemm_workspace_bytes(sm_count) that read zero at launch.
 // sibling: index of the weight in a call whose weights share x. The first one converts x; the later
