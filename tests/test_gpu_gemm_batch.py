@@ -85,3 +85,29 @@ def test_one_call_of_both_k_orders(tq, k, dtype):
         assert np.linalg.norm(y.double().cpu().numpy() - ref) / np.linalg.norm(ref) < TOL
         assert torch.equal(mm.forward(x, mode=tq.Mode.TENSOR_CORE), y)
     tq.context().poll_status()
+
+
+# (type, rows, columns, activation rows): tiles of 16 to 128 rows, whole and ragged, narrow and wide accumulators, one item per
+# CTA and several, a last unit of one, two and three 64-k blocks
+TILED = [(oracle.Q4_K, 700, 256, 1024), (oracle.Q8_0, 300, 320, 67), (oracle.Q8_0, 5000, 448, 500), (oracle.Q4_K, 4000, 4096, 65),
+         (oracle.Q5_K, 3000, 5120, 129), (oracle.Q6_K, 5000, 6144, 300), (oracle.Q8_0, 130, 2624, 96), (oracle.Q6_K, 2560, 1024, 1000),
+         (oracle.Q8_0, 8200, 704, 255), (oracle.Q4_K, 12288, 512, 128)]
+
+
+@pytest.mark.parametrize("dt,n,k,m", TILED)
+def test_short_prompts_in_tiles(tq, dt, n, k, m):
+    """65 to 1024 rows in tiles: against the f64 product, and with the bits of a call that is too large for tiles."""
+    w, base = make_weight(dt, n, k, SEED + 8300 + n + k)
+    rng = np.random.default_rng(SEED + 8301 + n)
+    x = (rng.standard_normal((m, k)) * 2.0 ** rng.integers(-8, 9, (m, 1))).astype(np.float32)
+    mm = tq.QMatMul.from_arc(tq.QTensor.new(w, tq.GgmlDType(dt), (n, k)))
+    xd = torch.from_numpy(x).cuda()
+    bias = torch.from_numpy(rng.standard_normal(n).astype(np.float32)).cuda()
+    y = mm.forward(xd, mode=tq.Mode.TENSOR_CORE)
+    ref = oracle.matmul_f64(dt, w[: w.size // n * base], base, k, x)[:, np.arange(n) % base]
+    err = np.linalg.norm(y.double().cpu().numpy() - ref, axis=1) / np.linalg.norm(ref, axis=1)
+    assert err.max() < TOL, (int(err.argmax()), err.max())
+    assert torch.equal(mm.forward(torch.cat([xd] * (1024 // m + 1)), mode=tq.Mode.TENSOR_CORE)[:m], y)
+    a, b = tq.QMatMul.forward_multi([mm, mm], xd, biases=[None, bias], mode=tq.Mode.TENSOR_CORE)
+    assert torch.equal(a, y) and torch.equal(b, y + bias)
+    tq.context().poll_status()

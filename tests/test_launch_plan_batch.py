@@ -14,6 +14,9 @@ SHIM = r"""
 #include "launch_plan.h"
 extern "C" int batch_cluster(int tiles, int KU, const int* resident) { return turq::plan_batch_cluster(tiles, KU, resident); }
 extern "C" int gemm_rows(long long call_tiles, long long m, int sms) { return turq::plan_gemm_rows(call_tiles, m, sms); }
+extern "C" int batch_tile(long long tiles, long long call_tiles, long long m, long long resident, int sms) {
+  return turq::plan_batch_tile(tiles, call_tiles, m, resident, sms);
+}
 """
 B200 = [0, 148, 74, 45, 33, 26, 22]     # clusters of 1..6 CTAs that are resident at once
 
@@ -26,6 +29,7 @@ def lib():
         subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", os.path.join(ROOT, "tur_b200", "csrc"), src, "-o", so], check=True)
         lib = ctypes.CDLL(so)
         lib.gemm_rows.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int]
+        lib.batch_tile.argtypes = [ctypes.c_longlong] * 4 + [ctypes.c_int]
         yield lib
 
 
@@ -76,3 +80,19 @@ def test_tile_heights_are_legal_and_no_worse_than_the_largest(lib):
                 whole = -(-(-(-m // -(-m // 256))) // 16) * 16
                 slots = max(1, sms // 2)
                 assert cost(call, m, b, slots) <= cost(call, m, whole, slots)
+
+
+def test_tiles_of_short_prompts(lib):
+    """A tile is a legal one, no call outside 65..1024 rows is taken, and the measured choices are the ones taken."""
+    def tile(n, m, resident=148, sms=148):
+        return lib.batch_tile(-(-n // 128), -(-n // 256), m, resident, sms)
+    for n in (0, 1, 128, 1000, 4096, 25600, 151936, 2 ** 31):
+        for m in (1, 64, 65, 66, 127, 128, 129, 511, 1000, 1024, 1025, 8192):
+            for resident, sms in ((148, 148), (16, 16), (1, 1)):
+                bn = tile(n, m, resident, sms)
+                assert bn == 0 or (bn % 16 == 0 and 16 <= bn <= 128 and 64 < m <= 1024), (n, m, bn)
+    assert tile(0, 128) == 0
+    for n, m in ((4096, 65), (4096, 128), (4096, 512), (2560, 768), (12288, 128), (12288, 384), (1024, 1000), (25600, 65)):
+        assert tile(n, m) > 0, (n, m)
+    for n, m in ((4096, 1000), (12288, 768), (25600, 256), (25600, 512), (151936, 512)):
+        assert tile(n, m) == 0, (n, m)

@@ -486,9 +486,10 @@ int32_t turq_qmatmul(turq_ctx* ctx, const turq_qtensor* qt, const void* dev_x, i
   } else if (mode == TURQ_MODE_TENSOR_CORE) {
     int32_t st = ensure(ctx, &ctx->scratch, &ctx->scratch_bytes, turq::gemm_tc_scratch_bytes(m, k));
     if (st != TURQ_OK) return st;
-    if (m <= turq::GEMM_BATCH_ROWS) {
-      const turq::GemvPart part{qt->tiles, qt->n_rows, dev_y, dev_bias, qt->dtype, nullptr};
-      e = turq::launch_gemm_batch(&part, 1, k, dev_x, x_dtype, m, ctx->scratch, s, &launches, ctx->dev_status);
+    const turq::GemvPart part{qt->tiles, qt->n_rows, dev_y, dev_bias, qt->dtype, nullptr};
+    if (turq::gemm_batch_takes(&part, 1, m, ctx->sm_count)) {
+      e = turq::launch_gemm_batch(&part, 1, k, dev_x, x_dtype, m, ctx->scratch, s, ctx->gemm_ws, ctx->sm_count, &launches,
+                                  ctx->dev_status);
     } else {
       e = turq::launch_gemm_tc(qt->dtype, qt->tiles, qt->n_rows, k, dev_x, x_dtype, m, dev_y, dev_bias, ctx->scratch,
                                ctx->gemm_ws, ctx->sm_count, s, &launches, ctx->dev_status);
@@ -530,13 +531,13 @@ static int32_t qmatmul_multi_impl(turq_ctx* ctx, int32_t count, const turq_qtens
     TQ_CUDA(ctx, cudaSetDevice(ctx->device));
     int32_t st = ensure(ctx, &ctx->scratch, &ctx->scratch_bytes, turq::gemm_tc_scratch_bytes(m, k));
     if (st != TURQ_OK) return st;
-    if (m <= turq::GEMM_BATCH_ROWS) {
-      turq::GemvPart parts[4];
-      for (int i = 0; i < count; i++)
-        parts[i] = turq::GemvPart{qts[i]->tiles, qts[i]->n_rows, dev_ys[i], dev_biases ? dev_biases[i] : nullptr, qts[i]->dtype, nullptr};
+    turq::GemvPart parts[4];
+    for (int i = 0; i < count; i++)
+      parts[i] = turq::GemvPart{qts[i]->tiles, qts[i]->n_rows, dev_ys[i], dev_biases ? dev_biases[i] : nullptr, qts[i]->dtype, nullptr};
+    if (turq::gemm_batch_takes(parts, count, m, ctx->sm_count)) {
       int launches = 0;
       cudaError_t e = turq::launch_gemm_batch(parts, count, k, dev_x, x_dtype, m, ctx->scratch, static_cast<cudaStream_t>(stream),
-                                              &launches, ctx->dev_status);
+                                              ctx->gemm_ws, ctx->sm_count, &launches, ctx->dev_status);
       ctx->launches += launches;
       if (e != cudaSuccess) return cuda_fail(ctx, e, "qmatmul_multi launch");
       return TURQ_OK;
@@ -854,8 +855,9 @@ int32_t qmatmul_for_exchange(turq_ctx* ctx, const turq_qtensor* qt, const void* 
     if (st != TURQ_OK) return st;
     int launches = 0;
     const GemvPart part{qt->tiles, qt->n_rows, s0, local_bias, qt->dtype, s1};
-    cudaError_t e = m <= GEMM_BATCH_ROWS
-                        ? launch_gemm_batch(&part, 1, qt->n_cols, dev_x, x_dtype, m, ctx->scratch, s, &launches, ctx->dev_status, toggle)
+    cudaError_t e = gemm_batch_takes(&part, 1, m, ctx->sm_count)
+                        ? launch_gemm_batch(&part, 1, qt->n_cols, dev_x, x_dtype, m, ctx->scratch, s, ctx->gemm_ws, ctx->sm_count, &launches,
+                                            ctx->dev_status, toggle)
                         : launch_gemm_tc(qt->dtype, qt->tiles, qt->n_rows, qt->n_cols, dev_x, x_dtype, m, s0, local_bias, ctx->scratch,
                                          ctx->gemm_ws, ctx->sm_count, s, &launches, ctx->dev_status, 0, 0, 0, toggle, s1);
     ctx->launches += launches;

@@ -1,4 +1,5 @@
-// QMatMul::forward on the 5th-generation tensor cores (tcgen05 / TMEM) for decode batches: up to 64 activation rows.
+// QMatMul::forward on the 5th-generation tensor cores (tcgen05 / TMEM) for decode batches, up to 64 activation rows, and for those
+// short prompts (up to 1024 rows) that leave most of the prefill kernel's pairs without work (plan_batch_tile, launch_plan.h).
 //
 //   y[m, n] = sum_k x[m, k] * W[n, k]      W quantized (device fragment tiles), x f32 or bf16
 //
@@ -20,6 +21,12 @@
 // All weights of a call (q|k|v, gate|up; any mix of types) go out as one launch over their 128-row tiles, dealt out round robin
 // to the clusters that fit the GPU. C is a function of the weight's shape alone (launch_plan.h), so a row's bits depend neither on
 // the batch nor on the other weights of the call; weights that want another C go out as a launch of their own.
+//
+// More than 64 rows go in tiles of up to 128 (a tile and 128 weight rows are an item; accumulators of 64 or 128 columns), a launch per
+// weight, side by side. K is not cut then: the sums, and their bits, are those of the prefill kernel. A layer of 4096-wide
+// Q4_K / Q6_K linears at 96 / 128 / 256 / 512 rows: 147 / 150 / 167 / 223 -> 115 / 123 / 149 / 207 us; 2560-wide Q8_0 at 96 / 256: 113 / 125 ->
+// 71 / 84; 1024-wide Q8_0 at 96 / 256 / 512: 64 / 70 / 75 -> 40 / 49 / 58. A unit takes 0.67 us with 16 rows, 0.72 with 64 (dequantize), 0.9 with 96
+// and 1.05 with 128: 82 KB of operands a unit, 8 to 9 TB/s from L2 over all CTAs, where a pair of the prefill kernel shares its rows.
 //
 // What bounds it. Small weights: the chain conversion (1.0 us) - its completion (0.7) - first activation image (0.6) - MMAs of
 // the share - exchange (0.6) - stores and exit, some 5 us. Large ones: the issue slots and the ALU pipe of the dequantize warps
@@ -47,11 +54,8 @@ namespace turq {
 
 namespace {
 
-constexpr int ST = 3;              // operand stages (units): 128 TMEM columns and bn * 512 bytes each
 constexpr int MAX_RAW = 10;        // raw ring slots
-constexpr int ACC_COLS = 64;
-constexpr int A_COL0 = 2 * ACC_COLS;
-constexpr int A_COLS = 32;         // per 64-k block
+constexpr int A_COLS = 32;         // TMEM columns of a 64-k block of the weight operand
 constexpr int CH = 8;              // columns of a chunk: what a CTA of the cluster adds up as a whole
 constexpr int CH_BYTES = BM * CH * 4;
 constexpr int EP_WARPS = 4;
@@ -62,8 +66,19 @@ constexpr int RAW_WARP2 = DQ_WARP0 + DQ_WARPS;  // the second raw producer
 constexpr int THREADS = (RAW_WARP2 + 1) * 32;
 // Register bound (72) of the kernel: leaves a CTA of the conversion kernel room beside it on an SM.
 constexpr int REG_THREADS = 896;
-constexpr int TMEM_COLS = 512;     // two accumulators, three stages of the weight operand
+constexpr int TMEM_COLS = 512;     // two accumulators, the stages of the weight operand
 constexpr int MAX_PARTS = 4;
+// The forms of the kernel. COLS: columns of an accumulator. 64 leaves TMEM for three operand stages of a unit each; 128 for eight
+// blocks, as four stages of half a unit, so that a group of dequantize warps makes one half while the MMAs read the other; the
+// activations then have stages of their own, three. TILED: more than 64 rows, in tiles of up to COLS rows; K is not cut.
+template <int COLS, bool TILED> struct Form {
+  static constexpr bool WIDE = COLS > 64;
+  static constexpr int HALVES = WIDE ? 2 : 1;       // stages of a unit
+  static constexpr int BPS = 4 / HALVES;            // 64-k blocks of a stage
+  static constexpr int ST = WIDE ? 4 : 3;           // stages: of the weight operand, or of both
+  static constexpr int BST = 3;                     // stages of the activations, bn * BPS * 128 bytes each
+  static constexpr int A_COL0 = 2 * COLS;
+};
 
 // Sub-block scales of a unit (Q4_K / Q5_K): lane 2r + h holds, for row r of the row-tile, the f16 scales and negated mins of
 // sub-blocks 4h, 4h + 1 (dl[0], ml[0]) and 4h + 2, 4h + 3 (dl[1], ml[1]). Worked out once per unit and row instead of by
@@ -226,7 +241,7 @@ __host__ __device__ __forceinline__ bool own_order(int dtype, int csize) { retur
 
 struct BatchPart {
   const uint8_t* tiles;
-  const uint8_t* xh;   // B operand image in the weight's k order: [kblocks][bn][128 bytes]
+  const uint8_t* xh;   // B operand image in the weight's k order: [mt][kblocks][bn][128 bytes]
   float* y;            // [m, n_rows]
   float* y_alt;
   const float* bias;
@@ -234,7 +249,7 @@ struct BatchPart {
   int row_tiles;       // 16-row tiles of the weight
   int ktiles;          // device tiles per row-tile
   int dtype;
-  int item0;           // the first of the weight's items (128-row tiles)
+  int item0;           // the first of the weight's items (128 weight rows by a tile of activation rows)
 };
 
 struct BatchArgs {
@@ -244,18 +259,24 @@ struct BatchArgs {
   int kblocks;          // k / 64
   int KU;               // units of 256 k per row (the last one of a Q8_0 weight may hold fewer blocks)
   int m;                // activation rows
-  int bn;               // the same, up to a multiple of 16
+  int bn;               // rows of a tile, a multiple of 16
+  int mt;               // tiles of bn rows (1 up to 64 rows)
   int raw_slots, slot_bytes;
   int red_bytes;        // exchange buffer of a CTA
   const float* rscale;  // [m] factor undoing the f16 row scaling
   int* status;
+  // tiled form (tc_common.cuh): the preceding launch belongs to the same call and reads the same x; go-ahead words [CTA] of this
+  // launch and of the one behind it, which has next_ctas CTAs (0: none follows)
+  int sibling;
+  int *go, *next_go;
+  int next_ctas;
   // exchange slots (tp.cu): with y_toggle set, the result goes to y_alt instead of y when the
   // word it points to, plus one, is odd - read after the preceding kernels have completed
   const unsigned* y_toggle;
 };
 
-// The 128-row tiles a cluster works on, in order; every role of all its CTAs walks the same list.
-struct Walk {
+// The items a cluster works on, in order; every role of all its CTAs walks the same list.
+template <bool TILED> struct Walk {
   int item, part, step;
   __device__ __forceinline__ void init(int first, int clusters) {
     item = first - clusters;
@@ -269,7 +290,18 @@ struct Walk {
     return true;
   }
   __device__ __forceinline__ bool last(const BatchArgs& a) const { return item + step >= a.items; }
-  __device__ __forceinline__ int row_tile(const BatchArgs& a) const { return (item - a.part[part].item0) * (BM / TQ_TILE_ROWS); }
+  __device__ __forceinline__ int row_tile(const BatchArgs& a) const {
+    const int i = item - a.part[part].item0;
+    return (TILED ? i / a.mt : i) * (BM / TQ_TILE_ROWS);
+  }
+  __device__ __forceinline__ int m0(const BatchArgs& a) const {  // the first activation row
+    const int i = item - a.part[part].item0;
+    return TILED ? i % a.mt * a.bn : 0;
+  }
+  __device__ __forceinline__ int rows(const BatchArgs& a) const {
+    const int left = a.m - m0(a);
+    return TILED && left > a.bn ? a.bn : left;
+  }
 };
 
 __device__ __forceinline__ void commit_to(uint64_t* bar) {
@@ -294,9 +326,10 @@ struct Chunk {
 // Epilogue of one item for one TMEM lane quarter (32 weight rows): of the chunks h0, h0 + hstep, ... those that other CTAs
 // add up are sent to them, then those of this CTA (chunk % cluster size == rank) are added and stored.
 // Exchange buffer of a CTA: [its chunks][other ranks][CH / 4][BM] of four columns.
-__device__ __forceinline__ void epilogue(const BatchArgs& a, const Walk& w, int rank, int csize, int quarter, int lane, uint32_t tmem,
+template <bool TILED>
+__device__ __forceinline__ void epilogue(const BatchArgs& a, const Walk<TILED>& w, int rank, int csize, int quarter, int lane, uint32_t tmem,
                                          int h0, int hstep, const float* scale, uint8_t* red, uint64_t* red_full, uint32_t parity, volatile int* abort_flag) {
-  const int nchunks = (a.m + CH - 1) / CH;
+  const int m0 = w.m0(a), rows = w.rows(a), nchunks = (rows + CH - 1) / CH;
   const uint32_t taddr = tmem + ((uint32_t)(32 * quarter) << 16);
   const int row = 32 * quarter + lane;
   float v[CH];
@@ -333,7 +366,8 @@ __device__ __forceinline__ void epilogue(const BatchArgs& a, const Walk& w, int 
   const float bv = (p.bias && live) ? p.bias[n] : 0.f;
   float* ybase = p.y;
   if (a.y_toggle && ((*reinterpret_cast<const volatile unsigned*>(a.y_toggle) + 1u) & 1u)) ybase = p.y_alt;
-  float* const yp = ybase + n;
+  float* const yp = ybase + (TILED ? (int64_t)m0 * p.n_rows : 0) + n;
+  scale += m0;
   bool waited = csize == 1;
   for (Chunk c(h0, csize); c.ch < nchunks; c.advance(hstep, csize)) {
     if (c.owner != rank) continue;
@@ -373,7 +407,7 @@ __device__ __forceinline__ void epilogue(const BatchArgs& a, const Walk& w, int 
       const float4 r0 = *reinterpret_cast<const float4*>(scale + ch * CH), r1 = *reinterpret_cast<const float4*>(scale + ch * CH + 4);
       const float r[CH] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
       float* yc = yp + (int64_t)(ch * CH) * p.n_rows;
-      const int cols = a.m - ch * CH;
+      const int cols = rows - ch * CH;
 #pragma unroll
       for (int j = 0; j < CH; j++) {
         if (j < cols) *yc = v[j] * r[j] + bv;
@@ -391,7 +425,7 @@ struct DequantPos {
 
 // A warp's share of an item: one 16-row tile (`dq` of the CTA's eight) of every other unit. Whole units, so that what a
 // unit costs beside the conversion itself (barriers, scales, addresses) is spread over four blocks.
-template <int DT, bool OWN = false>
+template <class F, int DT, bool OWN = false>
 __device__ __forceinline__ void dequant_units(const BatchArgs& a, int ka, int kb, bool live, int dq, int grp, int lane, uint8_t* raw0,
                                               uint64_t* raw_full, uint64_t* raw_empty, uint64_t* full, uint64_t* empty, uint32_t tmem,
                                               DequantPos& pos, volatile int* abort_flag) {
@@ -402,44 +436,53 @@ __device__ __forceinline__ void dequant_units(const BatchArgs& a, int ka, int kb
       const uint8_t* raw = raw0 + slot * a.slot_bytes + dq * UnitGeom<DT>::BYTES;
       const int nb = a.kblocks - 4 * ku;
       const RowScales us = row_scales<DT>(raw, lane);
-      bar_pass(&empty[pos.s], pos.ph ^ 1u, abort_flag);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t dst = tmem + ((uint32_t)(16 * dq) << 16) + (uint32_t)(A_COL0 + pos.s * 4 * A_COLS);
-      if (live) {
 #pragma unroll
-        for (int b = 0; b < 4; b++)
-          if (b == 0 || DT != TQ_Q8_0 || b < nb) {
-            uint32_t o[16];
-            dequant_frag<DT, OWN>(raw, us, b, lane, o);
-            tmem_store_block(dst + (uint32_t)(b * A_COLS), o);
+      for (int h = 0; h < F::HALVES; h++) {
+        bar_pass(&empty[pos.s + h], pos.ph ^ 1u, abort_flag);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t dst = tmem + ((uint32_t)(16 * dq) << 16) + (uint32_t)(F::A_COL0 + (pos.s + h) * F::BPS * A_COLS);
+        if (live) {
+#pragma unroll
+          for (int e = 0; e < F::BPS; e++) {
+            const int b = h * F::BPS + e;
+            if (b == 0 || DT != TQ_Q8_0 || b < nb) {
+              uint32_t o[16];
+              dequant_frag<DT, OWN>(raw, us, b, lane, o);
+              tmem_store_block(dst + (uint32_t)(e * A_COLS), o);
+            }
           }
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) bar_arrive(&full[pos.s + h]);
       }
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) {
-        bar_arrive(&full[pos.s]);
-        bar_arrive(&raw_empty[pos.use]);
-      }
+      if (lane == 0) bar_arrive(&raw_empty[pos.use]);
     }
     pos.turn ^= 1;
-    if (++pos.s == ST) { pos.s = 0; pos.ph ^= 1u; }
+    pos.s += F::HALVES;
+    if (pos.s == F::ST) { pos.s = 0; pos.ph ^= 1u; }
     if (++pos.use == 2 * a.raw_slots) { pos.use = 0; pos.rph ^= 1u; }
   }
 }
 
+template <int COLS, bool TILED>
 __global__ void __launch_bounds__(REG_THREADS, 1) gemm_batch_kernel(const __grid_constant__ BatchArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // 1024-byte alignment for the swizzled operand; the same offsets in all CTAs of the cluster
   uint8_t* const smem = smem_raw + ((1024u - (s_u32(smem_raw) & 1023u)) & 1023u);
-  const int b_stage = a.bn * 512;
+  using F = Form<COLS, TILED>;
+  constexpr int ST = F::ST, BST = F::BST;
+  const int b_stage = a.bn * F::BPS * 128;
   uint8_t* const sB = smem;
-  uint8_t* const sRaw = sB + ST * b_stage;
+  uint8_t* const sRaw = sB + BST * b_stage;
   uint8_t* const sRed = sRaw + a.raw_slots * a.slot_bytes;
   float* const sScale = reinterpret_cast<float*>(sRed + a.red_bytes);  // row scales
-  uint64_t* const full = reinterpret_cast<uint64_t*>(sScale + GEMM_BATCH_ROWS);  // both operands of a stage
+  uint64_t* const full = reinterpret_cast<uint64_t*>(sScale + (TILED ? a.mt * a.bn : GEMM_BATCH_ROWS));  // both operands of a stage (wide: the weights)
   uint64_t* const empty = full + ST;
-  uint64_t* const raw_full = empty + ST;
+  uint64_t* const b_full = F::WIDE ? empty + ST : full;      // the activations' stages
+  uint64_t* const b_empty = F::WIDE ? b_full + BST : empty;
+  uint64_t* const raw_full = F::WIDE ? b_empty + BST : empty + ST;
   uint64_t* const raw_empty = raw_full + 2 * MAX_RAW;
   uint64_t* const acc_full = raw_empty + 2 * MAX_RAW;
   uint64_t* const acc_empty = acc_full + 2;
@@ -450,13 +493,20 @@ __global__ void __launch_bounds__(REG_THREADS, 1) gemm_batch_kernel(const __grid
   uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(red_free + 1);
   volatile int* const abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = (int)cluster_rank(), csize = (int)cluster_size();
+  const int rank = TILED ? 0 : (int)cluster_rank(), csize = TILED ? 1 : (int)cluster_size();
 
+  // Siblings: beside the set-up, whose barrier then orders every warp of the CTA behind the word's acquire.
+  bool go = true;
+  if (TILED && a.sibling && warp == 1 && lane == 0) go = take_go(a.go + blockIdx.x);
   if (warp == 0) {
     // one barrier per lane
     if (lane < ST) {
-      bar_init(&full[lane], DQ_WARPS / 2 + 1);
+      bar_init(&full[lane], DQ_WARPS / 2 + (F::WIDE ? 0 : 1));
       bar_init(&empty[lane], 1);
+    }
+    if (F::WIDE && lane < BST) {
+      bar_init(&b_full[lane], 1);
+      bar_init(&b_empty[lane], 1);
     }
     if (lane < 2 * a.raw_slots) {
       bar_init(&raw_full[lane], 1);
@@ -487,7 +537,7 @@ __global__ void __launch_bounds__(REG_THREADS, 1) gemm_batch_kernel(const __grid
   // this CTA's share of the K loop, the same for every item
   const int ka = a.KU * rank / csize, kb = a.KU * (rank + 1) / csize;
 
-  Walk walk;
+  Walk<TILED> walk;
   walk.init((int)blockIdx.x / csize, (int)gridDim.x / csize);
   if (warp == 0 || warp == RAW_WARP2) {
     // ------------------------------------------------------------ raw weight bytes -> ring (lane r: row-tile r)
@@ -527,22 +577,29 @@ __global__ void __launch_bounds__(REG_THREADS, 1) gemm_batch_kernel(const __grid
     // ------------------------------------------------------------ activation image -> stages
     if (lane == 0) {
       // Programmatic stream serialization: the image comes from the conversion launch before this one (the
-      // weight side starts without waiting).
-      asm volatile("griddepcontrol.wait;" ::: "memory");
+      // weight side starts without waiting). A sibling's go-ahead word stands for that wait; the proxy fence carries what
+      // its acquire made visible over to the bulk copies.
+      if (TILED && a.sibling) {
+        if (!go) *abort_flag = 1;
+        asm volatile("fence.proxy.async.global;" ::: "memory");
+      } else {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+      }
       asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
       while (ok && walk.next(a)) {
-        const uint8_t* const xh = a.part[walk.part].xh;
-        for (int ku = ka; ku < kb; ku++) {
-          ok = bar_wait(&empty[s], ph ^ 1u, abort_flag);
+        const uint8_t* xh = a.part[walk.part].xh;
+        if (TILED) xh += (int64_t)walk.m0(a) * a.kblocks * 128;
+        for (int ku = F::HALVES * ka; ok && ku < F::HALVES * kb; ku++) {
+          ok = bar_wait(&b_empty[s], ph ^ 1u, abort_flag);
           if (!ok) break;
-          const int nb = a.kblocks - 4 * ku < 4 ? a.kblocks - 4 * ku : 4;
+          const int left = a.kblocks - F::BPS * ku, nb = left < 0 ? 0 : left < F::BPS ? left : F::BPS;
           const uint32_t bytes = (uint32_t)(nb * a.bn * 128);
-          bar_expect_tx(&full[s], bytes);
-          bulk_load(sB + s * b_stage, xh + (int64_t)ku * b_stage, bytes, &full[s]);
-          if (++s == ST) { s = 0; ph ^= 1u; }
+          bar_expect_tx(&b_full[s], bytes);
+          if (!F::WIDE || nb > 0) bulk_load(sB + s * b_stage, xh + (int64_t)ku * b_stage, bytes, &b_full[s]);
+          if (++s == BST) { s = 0; ph ^= 1u; }
         }
       }
     }
@@ -556,55 +613,61 @@ __global__ void __launch_bounds__(REG_THREADS, 1) gemm_batch_kernel(const __grid
     constexpr uint64_t desc_hi = (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
     const uint32_t b_lo0 = (s_u32(sB) & 0x3FFFFu) >> 4, b_step = (uint32_t)(a.bn * 128) >> 4;
     const bool issuer = elect_one();
-    int s = 0, nitem = 0;
-    uint32_t ph = 0;
+    int s = 0, sb = 0, nitem = 0;
+    uint32_t ph = 0, bph = 0;
     while (walk.next(a)) {
       const int acc = nitem & 1;
       const uint32_t aph = (uint32_t)(nitem >> 1) & 1u;
       nitem++;
       bar_pass(&acc_empty[acc], aph ^ 1u, abort_flag);
-      const uint32_t d = tmem_base + (uint32_t)(acc * ACC_COLS);
+      const uint32_t d = tmem_base + (uint32_t)(acc * COLS);
       uint32_t accumulate = 0;  // the first MMA of the item overwrites the accumulator
-      for (int ku = ka; ku < kb; ku++) {
-        const int nb = a.kblocks - 4 * ku;
+      for (int ku = F::HALVES * ka; ku < F::HALVES * kb; ku++) {
+        const int nb = a.kblocks - F::BPS * ku;
+        if (!F::WIDE) sb = s;
         bar_pass(&full[s], ph, abort_flag);
+        if (F::WIDE) bar_pass(&b_full[sb], bph, abort_flag);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (issuer) {
 #pragma unroll
-          for (int b = 0; b < 4; b++) {
-            if (b == 0 || b < nb) {
-              const uint64_t db = desc_hi | (uint64_t)(b_lo0 + (uint32_t)(s * 4 + b) * b_step);
+          for (int b = 0; b < F::BPS; b++) {
+            if ((!F::WIDE && b == 0) || b < nb) {
+              const uint64_t db = desc_hi | (uint64_t)(b_lo0 + (uint32_t)(sb * F::BPS + b) * b_step);
 #pragma unroll
               for (int kk = 0; kk < BK / 16; kk++)
                 asm volatile(
                     "{\n\t.reg .pred p;\n\t"
                     "setp.ne.b32 p, %4, 0;\n\t"
                     "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
-                    "r"(tmem_base + (uint32_t)(A_COL0 + (s * 4 + b) * A_COLS + 8 * kk)), "l"(db + (uint64_t)(2 * kk)), "r"(idesc),
+                    "r"(tmem_base + (uint32_t)(F::A_COL0 + (s * F::BPS + b) * A_COLS + 8 * kk)), "l"(db + (uint64_t)(2 * kk)), "r"(idesc),
                     "r"(b + kk > 0 ? 1u : accumulate)
                     : "memory");
             }
           }
-          commit_to(&empty[s]);  // frees both operands once these MMAs have read them
+          commit_to(&empty[s]);  // frees the operands once these MMAs have read them
+          if (F::WIDE) commit_to(&b_empty[sb]);
         }
         __syncwarp();
         accumulate = 1u;
         if (++s == ST) { s = 0; ph ^= 1u; }
+        if (F::WIDE && ++sb == BST) { sb = 0; bph ^= 1u; }
       }
       if (issuer) commit_to(walk.last(a) ? last_full : &acc_full[acc]);
       __syncwarp();
     }
   } else if (warp < DQ_WARP0) {
     // ------------------------------------------------------------ epilogue
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // y may still be read, the row scales still written
+    if (!TILED || !a.sibling) asm volatile("griddepcontrol.wait;" ::: "memory");  // y may still be read, the row scales still written
+    if (TILED && warp == 3)  // what this launch has waited for, a sibling behind it need not wait for again
+      for (int i = (int)(blockIdx.x + lane * gridDim.x); i < a.next_ctas; i += 32 * (int)gridDim.x) st_release(a.next_go + i, 1);
     if (csize > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");  // before anything is sent
     const int quarter = warp & 3;
     // In shared memory, where no store to y keeps a load of the next scale behind it (every load on its own: 2800 cycles a chunk)
-    if (warp < 5) sScale[(warp - 3) * 32 + lane] = (warp - 3) * 32 + lane < a.m ? a.rscale[(warp - 3) * 32 + lane] : 0.f;
+    for (int i = (warp - 3) * 32 + lane; i < (TILED ? a.mt * a.bn : GEMM_BATCH_ROWS); i += EP_WARPS * 32) sScale[i] = i < a.m ? a.rscale[i] : 0.f;
     asm volatile("bar.sync 2, %0;" ::"n"(EP_WARPS * 32) : "memory");
     // bytes an item's exchange brings this CTA
     const int nchunks = (a.m + CH - 1) / CH, mine = (nchunks - rank + csize - 1) / csize;
-    const uint32_t incoming = (uint32_t)(mine * (csize - 1) * CH_BYTES);
+    const uint32_t incoming = TILED ? 0u : (uint32_t)(mine * (csize - 1) * CH_BYTES);
     int nitem = 0;
     while (walk.next(a)) {
       const int acc = nitem & 1;
@@ -616,7 +679,7 @@ __global__ void __launch_bounds__(REG_THREADS, 1) gemm_batch_kernel(const __grid
       if (nitem > 0 && csize > 1) bar_pass(red_free, (uint32_t)(nitem - 1) & 1u, abort_flag);
       // the last epilogue is shared with the dequantize warps, which have nothing left to do
       if (last) asm volatile("bar.sync 1, %0;" ::"n"((EP_WARPS + DQ_WARPS) * 32) : "memory");
-      epilogue(a, walk, rank, csize, quarter, lane, tmem_base + (uint32_t)(acc * ACC_COLS), 0, last ? HELPERS : 1, sScale, sRed,
+      epilogue(a, walk, rank, csize, quarter, lane, tmem_base + (uint32_t)(acc * COLS), 0, last ? HELPERS : 1, sScale, sRed,
                last ? red_last : red_full, last ? 0u : (uint32_t)nitem & 1u, abort_flag);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -636,32 +699,32 @@ __global__ void __launch_bounds__(REG_THREADS, 1) gemm_batch_kernel(const __grid
     const int dq = 2 * (warp & 3) + (dqw & 1);  // row-tile of 16 rows inside the CTA's 128 rows
     DequantPos pos{0, 0, 0, 0u, 0u};
     int nitem = 0;
-    Walk lw = walk;
+    Walk<TILED> lw = walk;
     while (walk.next(a)) {
       lw = walk;
       nitem++;
       const BatchPart& p = a.part[walk.part];
       const bool live = walk.row_tile(a) + dq < p.row_tiles;  // rows beyond the weight are never stored
       switch (p.dtype) {
-        case TQ_Q8_0: dequant_units<TQ_Q8_0>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag); break;
-        case TQ_Q4_K: dequant_units<TQ_Q4_K>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag); break;
-        case TQ_Q5_K: dequant_units<TQ_Q5_K>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag); break;
+        case TQ_Q8_0: dequant_units<F, TQ_Q8_0>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag); break;
+        case TQ_Q4_K: dequant_units<F, TQ_Q4_K>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag); break;
+        case TQ_Q5_K: dequant_units<F, TQ_Q5_K>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag); break;
         default:
           if (own_order(p.dtype, csize))
-            dequant_units<TQ_Q6_K, true>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag);
+            dequant_units<F, TQ_Q6_K, true>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag);
           else
-            dequant_units<TQ_Q6_K>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag);
+            dequant_units<F, TQ_Q6_K>(a, ka, kb, live, dq, grp, lane, sRaw, raw_full, raw_empty, full, empty, tmem_base, pos, abort_flag);
           break;
       }
     }
     // nothing left to dequantize: help with the epilogue of the last item
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!TILED || !a.sibling) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (csize > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     const int acc = (nitem - 1) & 1;
     bar_pass(last_full, 0, abort_flag);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("bar.sync 1, %0;" ::"n"((EP_WARPS + DQ_WARPS) * 32) : "memory");
-    epilogue(a, lw, rank, csize, warp & 3, lane, tmem_base + (uint32_t)(acc * ACC_COLS), dqw + 1, HELPERS, sScale, sRed, red_last, 0u, abort_flag);
+    epilogue(a, lw, rank, csize, warp & 3, lane, tmem_base + (uint32_t)(acc * COLS), dqw + 1, HELPERS, sScale, sRed, red_last, 0u, abort_flag);
   }
   // (every thread waits for the cluster's set-up before it arrives for its end)
   if (csize > 1 && (warp < 3 || warp == RAW_WARP2)) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
@@ -684,9 +747,15 @@ __global__ void __launch_bounds__(REG_THREADS, 1) gemm_batch_kernel(const __grid
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(TMEM_COLS) : "memory");
   }
+  // whoever waits for this launch has then waited for all of the call
+  if (TILED && a.sibling && threadIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-constexpr int BAR_BYTES = GEMM_BATCH_ROWS * 4 + (2 * ST + 4 * MAX_RAW + 8) * 8 + 8;  // and the row scales
+// Barriers and row scales.
+template <int COLS, bool TILED> constexpr int bar_bytes(int scales) {
+  using F = Form<COLS, TILED>;
+  return scales * 4 + (2 * F::ST + (F::WIDE ? 2 * F::BST : 0) + 4 * MAX_RAW + 8) * 8 + 8;
+}
 
 int part_slot_bytes(int dtype) { return 8 * (dtype == TQ_Q8_0 ? UnitGeom<TQ_Q8_0>::TILES : 1) * tq_tile_bytes(dtype); }
 
@@ -708,7 +777,7 @@ int resident_clusters(int c) {
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaOccupancyMaxActiveClusters(&n, gemm_batch_kernel, &cfg) != cudaSuccess || n <= 0) {
+  if (cudaOccupancyMaxActiveClusters(&n, gemm_batch_kernel<64, false>, &cfg) != cudaSuccess || n <= 0) {
     cudaGetLastError();
     n = device_sm_count() / c;
   }
@@ -717,53 +786,90 @@ int resident_clusters(int c) {
   return n;
 }
 
-}  // namespace
+// Exchange buffer of a CTA: the sums of its share of the columns from the others of the cluster.
+int exchange_bytes(int bn, int c) { return (bn / CH + c - 1) / c * (c - 1) * CH_BYTES; }
 
-cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, const void* x, int x_dtype, int64_t m, uint8_t* scratch,
-                              cudaStream_t s, int* launches, int* dev_status_word, const unsigned* y_toggle) {
-  if (k % BK != 0 || k > INT32_MAX || m <= 0 || m > GEMM_BATCH_ROWS || nparts < 1 || nparts > MAX_PARTS) return cudaErrorInvalidValue;
+template <int COLS, bool TILED>
+cudaError_t launch_form(BatchArgs& a, int c, int clusters, cudaStream_t s) {
+  using F = Form<COLS, TILED>;
+  a.red_bytes = exchange_bytes(a.bn, c);
+  // 4 KB stay free for a CTA of the next call's conversion kernel.
+  const int fixed = F::BST * F::BPS * a.bn * 128 + a.red_bytes + bar_bytes<COLS, TILED>(TILED ? a.mt * a.bn : GEMM_BATCH_ROWS) + 1024;
+  const int room = device_smem_optin() - 4096 - fixed;
+  a.raw_slots = room / a.slot_bytes < MAX_RAW ? room / a.slot_bytes : MAX_RAW;
+  if (room < 0 || a.raw_slots < 2) return cudaErrorInvalidConfiguration;
   static PerDeviceOnce configured;
   int dev = 0;
   cudaGetDevice(&dev);
-  cudaError_t e;
   if (!configured.done(dev)) {
-    e = cudaFuncSetAttribute(gemm_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, device_smem_optin());
+    cudaError_t e = cudaFuncSetAttribute(gemm_batch_kernel<COLS, TILED>, cudaFuncAttributeMaxDynamicSharedMemorySize, device_smem_optin());
     if (e != cudaSuccess) return e;
     configured.set(dev);
   }
+  return launch_pdl_cluster(gemm_batch_kernel<COLS, TILED>, (unsigned)c, dim3((unsigned)(clusters * c)), dim3(THREADS),
+                            (size_t)(fixed + a.raw_slots * a.slot_bytes), s, a);
+}
+
+}  // namespace
+
+bool gemm_batch_takes(const GemvPart* parts, int nparts, int64_t m, int sm_count) {
+  if (m <= GEMM_BATCH_ROWS) return true;
+  int64_t tiles = 0, call_tiles = 0;  // of 128 and of 256 rows
+  for (int i = 0; i < nparts; i++) {
+    tiles += (parts[i].n_rows + BM - 1) / BM;
+    call_tiles += (parts[i].n_rows + 2 * BM - 1) / (2 * BM);
+  }
+  return plan_batch_tile(tiles, call_tiles, m, resident_clusters(1), sm_count) > 0;
+}
+
+cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, const void* x, int x_dtype, int64_t m, uint8_t* scratch,
+                              cudaStream_t s, uint8_t* workspace, int sm_count, int* launches, int* dev_status_word,
+                              const unsigned* y_toggle) {
+  if (k % BK != 0 || k > INT32_MAX || m <= 0 || m > GEMM_TILED_ROWS || nparts < 1 || nparts > MAX_PARTS) return cudaErrorInvalidValue;
   const int KU = (int)((k + UNIT_K - 1) / UNIT_K);
-  int resident[BATCH_MAX_CLUSTER + 1] = {};
+  const bool tiled = m > GEMM_BATCH_ROWS;
+  int resident[BATCH_MAX_CLUSTER + 1] = {}, cluster[MAX_PARTS];
   for (int c = 1; c <= BATCH_MAX_CLUSTER; c++) resident[c] = resident_clusters(c);
-  int cluster[MAX_PARTS];
+  int64_t tiles = 0, call_tiles = 0;
   for (int i = 0; i < nparts; i++) {
     if (!tq_is_weight_type(parts[i].dtype) || k % tq_block_elems(parts[i].dtype) != 0) return cudaErrorInvalidValue;
-    if ((parts[i].n_rows + BM - 1) / BM > (1 << 24)) return cudaErrorInvalidValue;
-    cluster[i] = plan_batch_cluster((int)((parts[i].n_rows + BM - 1) / BM), KU, resident);
+    const int64_t t = (parts[i].n_rows + BM - 1) / BM;
+    if (t > (1 << 24)) return cudaErrorInvalidValue;
+    tiles += t;
+    call_tiles += (parts[i].n_rows + 2 * BM - 1) / (2 * BM);
+    // beyond 64 rows no sum is cut: all larger calls, this kernel's and the prefill kernel's, have the same bits
+    cluster[i] = tiled ? 1 : plan_batch_cluster((int)t, KU, resident);
   }
+  const int bn = tiled ? plan_batch_tile(tiles, call_tiles, m, resident[1], sm_count) : (int)(m + 15) / 16 * 16;
+  if (bn <= 0) return cudaErrorInvalidValue;
+  const int mt = (int)((m + bn - 1) / bn);
   // images of both k orders where a call needs both, the row scales behind them
   bool own = false, common = false;
   for (int i = 0; i < nparts; i++) (own_order(parts[i].dtype, cluster[i]) ? own : common) = true;
-  uint8_t* const xh16 = scratch + (common ? gemm_operand_bytes(m, k) : 0);
-  float* rscale = reinterpret_cast<float*>(scratch + ((int)own + (int)common) * gemm_operand_bytes(m, k));
-  const int bn = (int)(m + 15) / 16 * 16;
-  e = launch_prep_image(x, x_dtype, m, k, bn, common ? scratch : nullptr, own ? xh16 : nullptr, rscale, s);
+  const size_t image = gemm_operand_bytes((int64_t)mt * bn, k);
+  uint8_t* const xh16 = scratch + (common ? image : 0);
+  float* rscale = reinterpret_cast<float*>(scratch + ((int)own + (int)common) * image);
+  cudaError_t e = launch_prep_image(x, x_dtype, m, k, bn, common ? scratch : nullptr, own ? xh16 : nullptr, rscale, s);
   if (launches) (*launches)++;
   if (e != cudaSuccess) return e;
 
+  const int clusters_max = resident[1] < sm_count ? resident[1] : sm_count;
   bool done[MAX_PARTS] = {};
   for (int i0 = 0; i0 < nparts; i0++) {
     if (done[i0]) continue;
     const int c = cluster[i0];
+    auto items = [&](int i) { return (int)((parts[i].n_rows + BM - 1) / BM) * mt; };
     BatchArgs a{};
     a.kblocks = (int)(k / BK);
     a.KU = KU;
     a.m = (int)m;
     a.bn = bn;
+    a.mt = mt;
     a.rscale = rscale;
     a.status = dev_status_word;
     a.y_toggle = y_toggle;
     for (int i = i0; i < nparts; i++) {
-      if (cluster[i] != c) continue;
+      if (tiled ? i != i0 : cluster[i] != c) continue;
       done[i] = true;
       BatchPart& p = a.part[a.nparts++];
       p.tiles = parts[i].tiles;
@@ -776,20 +882,23 @@ cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, cons
       p.row_tiles = (int)((p.n_rows + TQ_TILE_ROWS - 1) / TQ_TILE_ROWS);
       p.ktiles = (int)(k / tq_block_elems(p.dtype));
       p.item0 = a.items;
-      a.items += (int)((p.n_rows + BM - 1) / BM);
+      a.items += items(i);
       if (part_slot_bytes(p.dtype) > a.slot_bytes) a.slot_bytes = part_slot_bytes(p.dtype);
     }
-    const int nchunks = (int)(m + CH - 1) / CH;
-    a.red_bytes = (nchunks + c - 1) / c * (c - 1) * CH_BYTES;
-    // 4 KB stay free for a CTA of the next call's conversion kernel.
-    const int room = device_smem_optin() - 1024 - BAR_BYTES - 4096 - ST * bn * 512 - a.red_bytes;
-    a.raw_slots = room / a.slot_bytes < MAX_RAW ? room / a.slot_bytes : MAX_RAW;
-    if (a.raw_slots < 2) return cudaErrorInvalidConfiguration;
-    const int clusters = a.items < resident[c] ? a.items : resident[c];
-    const size_t smem = (size_t)(ST * bn * 512 + a.raw_slots * a.slot_bytes + a.red_bytes) + BAR_BYTES + 1024;
-    e = launch_pdl_cluster(gemm_batch_kernel, (unsigned)c, dim3((unsigned)(clusters * c)), dim3(THREADS), smem, s, a);
+    int clusters = c == 1 ? clusters_max : resident[c];
+    if (clusters > a.items) clusters = a.items;
+    if (tiled) {  // the weights of the call one launch each, side by side
+      a.sibling = i0 > 0;
+      a.go = reinterpret_cast<int*>(workspace) + (size_t)i0 * sm_count;
+      a.next_go = a.go + sm_count;
+      a.next_ctas = i0 + 1 == nparts ? 0 : items(i0 + 1) < clusters_max ? items(i0 + 1) : clusters_max;
+    }
+    e = !tiled ? launch_form<64, false>(a, c, clusters, s) : bn <= 64 ? launch_form<64, true>(a, c, clusters, s) : launch_form<128, true>(a, c, clusters, s);
     if (launches) (*launches)++;
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess) {
+      if (a.sibling) cudaMemsetAsync(workspace, 0, gemm_workspace_bytes(sm_count), s);  // go-ahead words that nobody takes
+      return e;
+    }
   }
   return cudaSuccess;
 }

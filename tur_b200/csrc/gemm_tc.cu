@@ -246,26 +246,6 @@ struct Tiles {
   }
 };
 
-// Siblings (the later weights of a call) run beside their predecessor, so griddepcontrol.wait, which
-// waits for its end, cannot be what makes the shared operand visible to them. Instead every CTA of a
-// sibling takes one go-ahead word that the launch before it released, once that launch itself could see
-// the operand and the end of everything older than the call. A word is taken by exchanging it for zero:
-// an exchange follows the write that it reads immediately in the word's order of writes, so a word set
-// for an earlier call, which that call's exchange has taken, cannot be read again.
-// The words are there when the sibling starts or soon after: every CTA of the launch before it has then
-// started and waits for nothing more before it releases them. Taken after the CTA's set-up and released
-// before dependents may start, they cost up to 1.2 us a sibling (Q8_0 2560 + 640 + 640 rows x 2560, 32
-// activation rows, us a call: 15.8 without, 18.2 so, 16.1 as it is; Q4_K + Q4_K + Q6_K 4096 + 1024 + 1024 x 4096,
-// 300 rows: 34.1, 36.3, 35.3).
-__device__ __forceinline__ bool take_go(int* p) {
-  const long long t0 = clock64();
-  int v;
-  do {
-    asm volatile("atom.acquire.gpu.global.exch.b32 %0, [%1], 0;" : "=r"(v) : "l"(p) : "memory");
-  } while (v == 0 && clock64() - t0 <= TC_WAIT_CYCLES);
-  return v != 0;
-}
-
 // Epilogue of one tile for one TMEM lane quarter (32 weight rows): columns in chunks of 16, the
 // chunks h0, h0 + hstep, ...
 __device__ __forceinline__ void epilogue(const GemmArgs& a, float* ybase, int t, int rank, int quarter, int lane, uint32_t tmem, int h0, int hstep) {
@@ -599,8 +579,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
 // tiny values do not sink into its subnormals. rscale[m] undoes the scale exactly in the
 // epilogue. Rows that are all zero, or hold an infinity or NaN, are converted as they are.
 // The row is written in the operands' k order (tc_common.cuh): as a row of [m, k] (prefill),
-// or as a row of the operand's shared-memory images [k / 64][image_rows][128 bytes], 128B-swizzled, which
-// decode batches copy in whole. One CTA per row; up to 4096 values stay in registers between the search for the largest
+// or as a row of the operand's shared-memory images [tile of image_rows rows][k / 64][image_rows][128 bytes], 128B-swizzled,
+// which gemm_batch.cu copies in whole. One CTA per row; up to 4096 values stay in registers between the search for the largest
 // magnitude and the conversion. Rows of more than 16384 values (CLUSTER): a cluster of CTAs, 4096 values each (beyond 8 x 4096 the
 // rest is read again), whose maxima meet in distributed shared memory: Q6_K 5120 x 25600 with the conversion, 32 / 64 rows 41.0 /
 // 47.6 -> 38.4 / 43.4 us. Below that the cluster's barriers cost what the second pass does: 4096 x 12288 17.2 / 20.0 and 18.7 / 20.0.
@@ -665,6 +645,9 @@ __global__ void __launch_bounds__(PREP_THREADS, IMAGE ? 6 : 5) prep_act_kernel(c
     s = ldexpf(1.f, se);
   }
   if (threadIdx.x == 0 && rank == 0) rscale[row] = 1.f / s;
+  // the row in the image of its tile of image_rows rows (a multiple of 16)
+  const uint32_t tile = IMAGE ? row / (uint32_t)image_rows : 0;
+  const uint32_t image_row = IMAGE ? (tile * (k / 64) - tile) * (uint32_t)image_rows + row : 0;  // in rows of 128 bytes
   auto store8 = [&](uint32_t i, const float (&u)[8]) {
     uint32_t o[4];
 #pragma unroll
@@ -674,7 +657,7 @@ __global__ void __launch_bounds__(PREP_THREADS, IMAGE ? 6 : 5) prep_act_kernel(c
     // the two fours of an eight belong to two 16-k chunks
     const int in_block = (int)(i & 32) + (int)(i & 31) / 2;  // inside the 64-k block
     if constexpr (IMAGE) {  // in the common order, in Q6_K's own, or in both
-      const size_t block = (size_t)((i >> 6) * (uint32_t)image_rows + row) * 128;
+      const size_t block = (size_t)((i >> 6) * (uint32_t)image_rows + image_row) * 128;
       const int swz = (int)(row & 7) << 4;  // 16-byte chunks exchanged by the row's low bits
       if (xh) {
         uint8_t* const p = reinterpret_cast<uint8_t*>(xh) + block;
@@ -759,9 +742,11 @@ cudaError_t launch_tc_dt(const CUtensorMap& map, GemmArgs a, int pairs, cudaStre
 
 // The f16 operand: rows up to a multiple of 16 for the image of a decode batch.
 size_t gemm_operand_bytes(int64_t m, int64_t k) { return ((size_t)((m + 15) / 16 * 16) * (size_t)k * 2 + 255) & ~(size_t)255; }
-// One operand, or two images of a decode batch; never less for more rows (a reservation stands for all smaller calls).
+// One operand, two images of a decode batch, or the image of a short prompt, whose last tile of up to GEMM_TILE_ROWS rows is
+// held whole; never less for more rows (a reservation stands for all smaller calls).
 size_t gemm_tc_scratch_bytes(int64_t m, int64_t k) {
-  const size_t rows = gemm_operand_bytes(m, k), images = 2 * gemm_operand_bytes(m < GEMM_BATCH_ROWS ? m : GEMM_BATCH_ROWS, k);
+  const size_t rows = gemm_operand_bytes(m <= GEMM_BATCH_ROWS ? m : m + GEMM_TILE_ROWS, k);
+  const size_t images = 2 * gemm_operand_bytes(m < GEMM_BATCH_ROWS ? m : GEMM_BATCH_ROWS, k);
   return (rows > images ? rows : images) + (((size_t)m * 4 + 255) & ~(size_t)255) + 256;
 }
 

@@ -191,4 +191,32 @@ inline int plan_batch_cluster(int tiles, int KU, const int* resident) {
   return best < KU ? best : KU;
 }
 
+// Activation rows per tile (a multiple of 16, at most 128) with which gemm_batch.cu takes a call of more than 64 rows, without
+// cutting K, or 0: the prefill kernel takes it. tiles, call_tiles: 128-row and 256-row tiles of all weights of the call.
+// What is left idle decides: pairs of CTAs on 256 weight rows leave most of the GPU without work for a short prompt, CTAs of
+// their own on 128 rows and as few activation rows as it takes fill it. Both sides by their waves times the time of a unit of
+// 256 k: here (0.66 + bn / 1000) us up to 64 rows and (0.41 + bn / 200) us beyond, there (plan_gemm_rows) its cost / 218 us; a
+// twelfth has to be gained. Measured on B200, prefill kernel / this one, us a call:
+//   rows                  65            128           256           384           512
+//   4096 x 4096 Q4_K      21.2 / 15.6   22.3 / 15.7   22.7 / 17.8   24.7 / 20.8   25.2 / 22.3   (768: 28.0 / 34.1)
+//   4096 x 12288 Q4_K     50.9 / 38.5   52.7 / 39.7   56.3 / 41.8   60.8 / 50.8   61.1 / 56.0   (768: 73.3 / 92.8)
+//   2560 x 8192 Q8_0      48.2 / 29.5   66.9 / 22.7   63.1 / 27.0   58.7 / 31.3   53.8 / 34.8   (768: 54.8 / 39.5)
+//   12288 x 4096 Q8_0     23.1 / 19.1   29.4 / 21.2   34.2 / 35.7   56.7 / 41.3   57.8 / 55.5
+//   25600 x 5120 Q4_K     46.2 / 39.2   48.8 / 43.6   62.6 / 66.9   86.6 / 101    103 / 127
+//   1024 x 3072 Q8_0      17.1 / 10.6   21.9 / 11.0   22.2 / 13.2   22.3 / 12.3   22.6 / 14.0   (1000: 26.0 / 16.3)
+// and calls of several weights: 4096 + 1024 + 1024 x 4096 Q4_K, Q6_K, 128 / 256 rows 27.7 / 23.6, 29.4 / 26.1; 2 x 12288 x 4096 Q4_K,
+// 128 rows 44.1 / 38.0; 2560 + 640 + 640 x 2560 Q8_0, 256 rows 24.6 / 17.1.
+inline int plan_batch_tile(int64_t tiles, int64_t call_tiles, int64_t m, int64_t resident, int sm_count) {
+  if (m <= 64 || m > 1024) return 0;
+  const int64_t slots = sm_count / 2 > 0 ? sm_count / 2 : 1;
+  const int64_t b = plan_gemm_rows(call_tiles, m, sm_count), mt = (m + b - 1) / b;
+  int64_t best_cost = (call_tiles * mt + slots - 1) / slots * (b + 110 > 260 ? b + 110 : 260) * 9200 / 218;
+  int best = 0;
+  for (int bn = 128; bn >= 16; bn -= 16) {
+    const int64_t cost = (tiles * ((m + bn - 1) / bn) + resident - 1) / resident * (bn <= 64 ? 6600 + 10 * bn : 4100 + 50 * bn);
+    if (cost < best_cost) { best = bn; best_cost = cost; }
+  }
+  return best;
+}
+
 }  // namespace turq

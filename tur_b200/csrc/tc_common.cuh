@@ -101,6 +101,26 @@ __device__ __forceinline__ __half2 pair13(uint32_t w) { return u2h2(__byte_perm(
 __device__ __forceinline__ __half2 pair01(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5140)); }
 __device__ __forceinline__ __half2 pair23(uint32_t w) { return u2h2(__byte_perm(w, 0x64646464u, 0x5342)); }
 
+// Siblings (the later weights of a call) run beside their predecessor, so griddepcontrol.wait, which
+// waits for its end, cannot be what makes the shared operand visible to them. Instead every CTA of a
+// sibling takes one go-ahead word that the launch before it released, once that launch itself could see
+// the operand and the end of everything older than the call. A word is taken by exchanging it for zero:
+// an exchange follows the write that it reads immediately in the word's order of writes, so a word set
+// for an earlier call, which that call's exchange has taken, cannot be read again.
+// The words are there when the sibling starts or soon after: every CTA of the launch before it has then
+// started and waits for nothing more before it releases them. Taken after the CTA's set-up and released
+// before dependents may start, they cost up to 1.2 us a sibling (Q8_0 2560 + 640 + 640 rows x 2560, 32
+// activation rows, us a call: 15.8 without, 18.2 so, 16.1 as it is; Q4_K + Q4_K + Q6_K 4096 + 1024 + 1024 x 4096,
+// 300 rows: 34.1, 36.3, 35.3).
+__device__ __forceinline__ bool take_go(int* p) {
+  const long long t0 = clock64();
+  int v;
+  do {
+    asm volatile("atom.acquire.gpu.global.exch.b32 %0, [%1], 0;" : "=r"(v) : "l"(p) : "memory");
+  } while (v == 0 && clock64() - t0 <= TC_WAIT_CYCLES);
+  return v != 0;
+}
+
 // Raw bytes of one unit (16 weight rows x 256 k) as they lie in a ring slot.
 template <int DT> struct UnitGeom {
   static constexpr int TILES = UNIT_K / TileGeom<DT>::ELEMS;  // device tiles per unit: 8 (Q8_0) or 1

@@ -131,6 +131,8 @@ cudaError_t launch_gemv_f32(int dtype, const uint8_t* tiles, int64_t n_rows, int
 // y_toggle / y_alt: the result goes to y_alt instead of y when *y_toggle + 1 is odd (read on the
 // device after the preceding kernels have completed: the exchange slots of tp.cu).
 constexpr int GEMM_BATCH_ROWS = 64;  // decode batches: up to this many rows
+constexpr int GEMM_TILED_ROWS = 1024;  // the same kernel may take short prompts, up to this many, in tiles of up to GEMM_TILE_ROWS
+constexpr int GEMM_TILE_ROWS = 128;
 constexpr int GEMM_SIBLINGS = 4;
 size_t gemm_operand_bytes(int64_t m, int64_t k);  // the operand at the start of scratch, the row scales behind it
 size_t gemm_tc_scratch_bytes(int64_t m, int64_t k);
@@ -148,10 +150,13 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
                            uint8_t* scratch, uint8_t* workspace, int sm_count, cudaStream_t s, int* launches,
                            int* dev_status_word, int64_t call_tiles = 0, int sibling = 0, int64_t next_rows = 0,
                            const unsigned* y_toggle = nullptr, float* y_alt = nullptr);
-// Decode batches, m <= GEMM_BATCH_ROWS: the weights of a call (each part with its dtype) as one launch per cluster size
-// that their shapes ask for.
+// Whether a call of these weights goes to launch_gemm_batch (to launch_gemm_tc otherwise).
+bool gemm_batch_takes(const GemvPart* parts, int nparts, int64_t m, int sm_count);
+// Decode batches, m <= GEMM_BATCH_ROWS: the weights of a call (each part with its dtype) as one launch per cluster size that
+// their shapes ask for. More rows, where gemm_batch_takes them: a launch per weight, side by side. workspace as above.
 cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, const void* x, int x_dtype, int64_t m, uint8_t* scratch,
-                              cudaStream_t s, int* launches, int* dev_status_word, const unsigned* y_toggle = nullptr);
+                              cudaStream_t s, uint8_t* workspace, int sm_count, int* launches, int* dev_status_word,
+                              const unsigned* y_toggle = nullptr);
 
 // QMatMul (no bias) whose result has to land in one of two buffers picked on the device: s1 when
 // (*toggle + 1) is odd, else s0 (the exchange slots of tp.cu). In the integer scheme the GEMV's
