@@ -50,7 +50,8 @@ inline int64_t gemv_split_start(const GemvSplit& p, int64_t total_units, int b) 
 // global memory. What the wide form saves is the way to L2 per activation fragment, most for Q8_0 (an
 // f32 scale per 32 values beside the quants) and Q6_K (four-byte fragments), least for Q4_K and Q5_K; a
 // mixed launch also spares a launch per type. What it costs is ring stages (two to four instead of six)
-// and, where there are no more shares than SMs, half of the SMs. Measured on B200, global against wide, us:
+// and, where there are no more shares than SMs, half of the SMs. Measured on B200, global against wide, us (with row-major
+// planes; in the order of ActPack both sides are faster):
 //   Q8_0        512 x 8192, 8 rows 13.7 / 9.7   5120 x 25600, 4 rows 41.4 / 33.4   2560 x 8192, 8 rows 13.5 / 13.7
 //   Q6_K        4096 x 12288, 4 rows 14.8 / 13.8   2048 x 5120, 12 rows 13.0 / 10.6
 //     shares cut, shorter than two row-tiles: 5120 x 25600, 2 rows 27.9 / 28.8   5120 x 13312, 7 rows 21.2 / 20.6
@@ -87,7 +88,7 @@ inline int plan_gemm_bn(int64_t n_rows, int64_t m, int sm_count) {
 // 2 / 3 / 4 / 5 / 7 / 8 activation tiles:
 //   512 rows   Q4_K, Q6_K 4096 + 1024 + 1024 x 4096  44.0 / 35.5 / 51.3   Q4_K 4096 x 4096  29.7 / 25.6 / 24.2   2 x 12288 x 4096  85.2 / 93.1 / 110.6
 //   1000 rows  Q8_0 2560 + 640 + 640 x 2560  - / - / 30.2 / 44.7 / 45.1   2560 x 8192  - / - / 62.5 / 58.3 / 56.1 / 98.5
-//   8 / 9 / 10: 2048 rows Q6_K 4096 x 12288 242.7 / 210.6 / 326.3   Q5_K 2 x 12288 x 4096 349 / 371 / 352
+//   8 / 9 / 10: 2048 rows Q6_K 4096 x 12288 242.7 / 210.6 / 326.3 (197 since Q6_K is converted from a lane's own words)   Q5_K 2 x 12288 x 4096 349 / 371 / 352
 // (a choice per weight put the small ones of a call on tiles of 128 rows: a layer at 2048 rows 865 us, at one size 793).
 inline int plan_gemm_rows(int64_t call_tiles, int64_t m, int sm_count) {
   const int64_t slots = sm_count / 2 > 0 ? sm_count / 2 : 1;
