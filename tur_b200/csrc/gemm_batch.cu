@@ -759,6 +759,18 @@ template <int COLS, bool TILED> constexpr int bar_bytes(int scales) {
 
 int part_slot_bytes(int dtype) { return 8 * (dtype == TQ_Q8_0 ? UnitGeom<TQ_Q8_0>::TILES : 1) * tq_tile_bytes(dtype); }
 
+// Allows the kernel all of an SM's shared memory, once per device: before it is launched, and before its occupancy is asked for.
+template <int COLS, bool TILED>
+cudaError_t configure() {
+  static PerDeviceOnce configured;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (configured.done(dev)) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(gemm_batch_kernel<COLS, TILED>, cudaFuncAttributeMaxDynamicSharedMemorySize, device_smem_optin());
+  if (e == cudaSuccess) configured.set(dev);
+  return e;
+}
+
 // Clusters of `c` CTAs that are resident at once (one CTA per SM; SMs at the edge of a GPC stay empty), looked up once per
 // device and size.
 int resident_clusters(int c) {
@@ -777,7 +789,7 @@ int resident_clusters(int c) {
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaOccupancyMaxActiveClusters(&n, gemm_batch_kernel<64, false>, &cfg) != cudaSuccess || n <= 0) {
+  if (configure<64, false>() != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_batch_kernel<64, false>, &cfg) != cudaSuccess || n <= 0) {
     cudaGetLastError();
     n = device_sm_count() / c;
   }
@@ -798,14 +810,8 @@ cudaError_t launch_form(BatchArgs& a, int c, int clusters, cudaStream_t s) {
   const int room = device_smem_optin() - 4096 - fixed;
   a.raw_slots = room / a.slot_bytes < MAX_RAW ? room / a.slot_bytes : MAX_RAW;
   if (room < 0 || a.raw_slots < 2) return cudaErrorInvalidConfiguration;
-  static PerDeviceOnce configured;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!configured.done(dev)) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_batch_kernel<COLS, TILED>, cudaFuncAttributeMaxDynamicSharedMemorySize, device_smem_optin());
-    if (e != cudaSuccess) return e;
-    configured.set(dev);
-  }
+  cudaError_t e = configure<COLS, TILED>();
+  if (e != cudaSuccess) return e;
   return launch_pdl_cluster(gemm_batch_kernel<COLS, TILED>, (unsigned)c, dim3((unsigned)(clusters * c)), dim3(THREADS),
                             (size_t)(fixed + a.raw_slots * a.slot_bytes), s, a);
 }
