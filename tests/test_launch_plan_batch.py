@@ -1,7 +1,8 @@
 """Cluster sizes of the decode-batch GEMM and tile heights of the prefill GEMM (plan_batch_cluster and plan_gemm_rows in
 tur_b200/csrc/launch_plan.h), compiled with g++ and checked on the CPU: every CTA of a cluster has units of its own, the measured
 choices are the ones taken, the weights of a transformer layer that share an activation agree on a cluster size, so that
-they go out as one launch, and a tile height is a legal one that needs no more time by the plan's measure than 256 rows."""
+they go out as one launch, a cluster size goes by the weight's shape and by nothing that a device answers, and a tile height
+is a legal one that needs no more time by the plan's measure than 256 rows."""
 import ctypes
 import os
 import subprocess
@@ -12,13 +13,20 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SHIM = r"""
 #include "launch_plan.h"
-extern "C" int batch_cluster(int tiles, int KU, const int* resident) { return turq::plan_batch_cluster(tiles, KU, resident); }
+extern "C" int batch_cluster(int tiles, int KU) { return turq::plan_batch_cluster(tiles, KU); }
+// asks three times: answers[i] is what the device would say, errors[i] the status that it returns
+extern "C" void ask_three_times(const int* answers, const int* errors, int* asked, int* status, int* out) {
+  std::atomic<int> known{0};
+  for (int i = 0; i < 3; i++) {
+    out[i] = -1;
+    status[i] = turq::ask_once(known, [&](int* n) { ++*asked; *n = answers[i]; return errors[i]; }, &out[i]);
+  }
+}
 extern "C" int gemm_rows(long long call_tiles, long long m, int sms) { return turq::plan_gemm_rows(call_tiles, m, sms); }
-extern "C" int batch_tile(long long tiles, long long call_tiles, long long m, long long resident, int sms) {
-  return turq::plan_batch_tile(tiles, call_tiles, m, resident, sms);
+extern "C" int batch_tile(long long tiles, long long call_tiles, long long m, int sms) {
+  return turq::plan_batch_tile(tiles, call_tiles, m, sms);
 }
 """
-B200 = [0, 148, 74, 45, 33, 26, 22]     # clusters of 1..6 CTAs that are resident at once
 
 
 @pytest.fixture(scope="module")
@@ -29,26 +37,38 @@ def lib():
         subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", os.path.join(ROOT, "tur_b200", "csrc"), src, "-o", so], check=True)
         lib = ctypes.CDLL(so)
         lib.gemm_rows.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int]
-        lib.batch_tile.argtypes = [ctypes.c_longlong] * 4 + [ctypes.c_int]
+        lib.batch_tile.argtypes = [ctypes.c_longlong] * 3 + [ctypes.c_int]
         yield lib
 
 
 @pytest.fixture(scope="module")
 def cluster(lib):
-    def call(n, k, resident=B200):
-        return lib.batch_cluster(-(-n // 128), -(-k // 256), (ctypes.c_int * 7)(*resident))
+    def call(n, k):
+        return lib.batch_cluster(-(-n // 128), -(-k // 256))
     return call
 
 
 def test_every_cta_has_units(cluster):
-    for resident in (B200, [0, 16, 8, 5, 4, 3, 2], [0, 1, 1, 1, 1, 1, 1]):
-        for n in (1, 128, 129, 640, 2560, 4096, 5120, 12288, 25600, 151936):
-            for k in (64, 256, 320, 512, 768, 1024, 2560, 4096, 6144, 8192, 25600):
-                c = cluster(n, k, resident)
-                assert 1 <= c <= 6 and c <= -(-k // 256), (n, k, c)
-                ku = -(-k // 256)
-                shares = [ku * (r + 1) // c - ku * r // c for r in range(c)]
-                assert min(shares) >= 1 and sum(shares) == ku
+    for n in (1, 128, 129, 640, 2560, 4096, 5120, 12288, 25600, 151936):
+        for k in (64, 256, 320, 512, 768, 1024, 2560, 4096, 6144, 8192, 25600):
+            c = cluster(n, k)
+            assert 1 <= c <= 6 and c <= -(-k // 256), (n, k, c)
+            ku = -(-k // 256)
+            shares = [ku * (r + 1) // c - ku * r // c for r in range(c)]
+            assert min(shares) >= 1 and sum(shares) == ku
+
+
+@pytest.mark.parametrize("n,k,want", [(28672, 8192, 2), (3584, 18944, 4), (3072, 8192, 5)])
+def test_cluster_sizes_do_not_follow_the_device(cluster, n, k, want):
+    """Shapes whose size was another one where the device held 48, 36, 28, 24 clusters of 3 to 6 CTAs instead of 45, 33, 26, 22:
+    the size cuts the K loop, so the bits of 17 to 64 rows went with the device. The rule has no such argument now."""
+    assert cluster(n, k) == want
+
+
+def test_a_failed_question_to_the_device_is_returned_and_asked_again(lib):
+    asked, status, out = ctypes.c_int(0), (ctypes.c_int * 3)(), (ctypes.c_int * 3)()
+    lib.ask_three_times((ctypes.c_int * 3)(37, 33, 44), (ctypes.c_int * 3)(1, 0, 0), ctypes.byref(asked), status, out)
+    assert list(status) == [1, 0, 0] and list(out) == [-1, 33, 33] and asked.value == 2
 
 
 @pytest.mark.parametrize("n,k,want", [(8192, 2560, 1), (12288, 4096, 2), (25600, 5120, 1), (3072, 1024, 2), (4096, 4096, 4), (2560, 2560, 4),
@@ -84,12 +104,12 @@ def test_tile_heights_are_legal_and_no_worse_than_the_largest(lib):
 
 def test_tiles_of_short_prompts(lib):
     """A tile is a legal one, no call outside 65..1024 rows is taken, and the measured choices are the ones taken."""
-    def tile(n, m, resident=148, sms=148):
-        return lib.batch_tile(-(-n // 128), -(-n // 256), m, resident, sms)
+    def tile(n, m, sms=148):
+        return lib.batch_tile(-(-n // 128), -(-n // 256), m, sms)
     for n in (0, 1, 128, 1000, 4096, 25600, 151936, 2 ** 31):
         for m in (1, 64, 65, 66, 127, 128, 129, 511, 1000, 1024, 1025, 8192):
-            for resident, sms in ((148, 148), (16, 16), (1, 1)):
-                bn = tile(n, m, resident, sms)
+            for sms in (148, 16, 1):
+                bn = tile(n, m, sms)
                 assert bn == 0 or (bn % 16 == 0 and 16 <= bn <= 128 and 64 < m <= 1024), (n, m, bn)
     assert tile(0, 128) == 0
     for n, m in ((4096, 65), (4096, 128), (4096, 512), (2560, 768), (12288, 128), (12288, 384), (1024, 1000), (25600, 65)):

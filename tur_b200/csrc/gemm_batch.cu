@@ -771,31 +771,30 @@ cudaError_t configure() {
   return e;
 }
 
-// Clusters of `c` CTAs that are resident at once (one CTA per SM; SMs at the edge of a GPC stay empty), looked up once per
-// device and size.
-int resident_clusters(int c) {
+// Clusters of `c` > 1 CTAs that are resident at once (one CTA per SM; SMs at the edge of a GPC stay empty), looked up once per
+// device and size. Sizes the grid; what a cluster computes does not depend on it.
+cudaError_t resident_clusters(int c, int* out) {
   static std::atomic<int> known[64][BATCH_MAX_CLUSTER + 1];
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-  int n = known[dev][c].load(std::memory_order_acquire);
-  if (n > 0) return n;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)c);
-  cfg.blockDim = dim3(THREADS);
-  cfg.dynamicSmemBytes = (size_t)device_smem_optin();
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)c;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (configure<64, false>() != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_batch_kernel<64, false>, &cfg) != cudaSuccess || n <= 0) {
-    cudaGetLastError();
-    n = device_sm_count() / c;
-  }
-  if (n < 1) n = 1;
-  known[dev][c].store(n, std::memory_order_release);
-  return n;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::atomic<int> unkept{0};
+  return static_cast<cudaError_t>(ask_once(dev >= 0 && dev < 64 ? known[dev][c] : unkept, [&](int* n) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)c);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = (size_t)device_smem_optin();
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)c;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t a = configure<64, false>();
+    if (a == cudaSuccess) a = cudaOccupancyMaxActiveClusters(n, gemm_batch_kernel<64, false>, &cfg);
+    if (a != cudaSuccess) cudaGetLastError();  // reported by the call; not left for the next check
+    return (int)a;
+  }, out));
 }
 
 // Exchange buffer of a CTA: the sums of its share of the columns from the others of the cluster.
@@ -825,7 +824,7 @@ bool gemm_batch_takes(const GemvPart* parts, int nparts, int64_t m, int sm_count
     tiles += (parts[i].n_rows + BM - 1) / BM;
     call_tiles += (parts[i].n_rows + 2 * BM - 1) / (2 * BM);
   }
-  return plan_batch_tile(tiles, call_tiles, m, resident_clusters(1), sm_count) > 0;
+  return plan_batch_tile(tiles, call_tiles, m, sm_count) > 0;
 }
 
 cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, const void* x, int x_dtype, int64_t m, uint8_t* scratch,
@@ -834,8 +833,7 @@ cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, cons
   if (k % BK != 0 || k > INT32_MAX || m <= 0 || m > GEMM_TILED_ROWS || nparts < 1 || nparts > MAX_PARTS) return cudaErrorInvalidValue;
   const int KU = (int)((k + UNIT_K - 1) / UNIT_K);
   const bool tiled = m > GEMM_BATCH_ROWS;
-  int resident[BATCH_MAX_CLUSTER + 1] = {}, cluster[MAX_PARTS];
-  for (int c = 1; c <= BATCH_MAX_CLUSTER; c++) resident[c] = resident_clusters(c);
+  int resident[BATCH_MAX_CLUSTER + 1] = {0, sm_count}, cluster[MAX_PARTS];  // a CTA of its own has an SM
   int64_t tiles = 0, call_tiles = 0;
   for (int i = 0; i < nparts; i++) {
     if (!tq_is_weight_type(parts[i].dtype) || k % tq_block_elems(parts[i].dtype) != 0) return cudaErrorInvalidValue;
@@ -844,9 +842,13 @@ cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, cons
     tiles += t;
     call_tiles += (parts[i].n_rows + 2 * BM - 1) / (2 * BM);
     // beyond 64 rows no sum is cut: all larger calls, this kernel's and the prefill kernel's, have the same bits
-    cluster[i] = tiled ? 1 : plan_batch_cluster((int)t, KU, resident);
+    cluster[i] = tiled ? 1 : plan_batch_cluster((int)t, KU);
+    if (!resident[cluster[i]]) {
+      cudaError_t e = resident_clusters(cluster[i], &resident[cluster[i]]);
+      if (e != cudaSuccess) return e;
+    }
   }
-  const int bn = tiled ? plan_batch_tile(tiles, call_tiles, m, resident[1], sm_count) : (int)(m + 15) / 16 * 16;
+  const int bn = tiled ? plan_batch_tile(tiles, call_tiles, m, sm_count) : (int)(m + 15) / 16 * 16;
   if (bn <= 0) return cudaErrorInvalidValue;
   const int mt = (int)((m + bn - 1) / bn);
   // images of both k orders where a call needs both, the row scales behind them
@@ -859,7 +861,6 @@ cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, cons
   if (launches) (*launches)++;
   if (e != cudaSuccess) return e;
 
-  const int clusters_max = resident[1] < sm_count ? resident[1] : sm_count;
   bool done[MAX_PARTS] = {};
   for (int i0 = 0; i0 < nparts; i0++) {
     if (done[i0]) continue;
@@ -891,13 +892,13 @@ cudaError_t launch_gemm_batch(const GemvPart* parts, int nparts, int64_t k, cons
       a.items += items(i);
       if (part_slot_bytes(p.dtype) > a.slot_bytes) a.slot_bytes = part_slot_bytes(p.dtype);
     }
-    int clusters = c == 1 ? clusters_max : resident[c];
+    int clusters = resident[c];
     if (clusters > a.items) clusters = a.items;
     if (tiled) {  // the weights of the call one launch each, side by side
       a.sibling = i0 > 0;
       a.go = reinterpret_cast<int*>(workspace) + (size_t)i0 * sm_count;
       a.next_go = a.go + sm_count;
-      a.next_ctas = i0 + 1 == nparts ? 0 : items(i0 + 1) < clusters_max ? items(i0 + 1) : clusters_max;
+      a.next_ctas = i0 + 1 == nparts ? 0 : items(i0 + 1) < sm_count ? items(i0 + 1) : sm_count;
     }
     e = !tiled ? launch_form<64, false>(a, c, clusters, s) : bn <= 64 ? launch_form<64, true>(a, c, clusters, s) : launch_form<128, true>(a, c, clusters, s);
     if (launches) (*launches)++;

@@ -3,6 +3,7 @@
 // CTAs, which launches share their activation planes, how many CTAs share the K loop of a GEMM tile,
 // which activation-tile height is used.
 #pragma once
+#include <atomic>
 #include <cstdint>
 
 namespace turq {
@@ -155,10 +156,13 @@ inline GemmWork plan_gemm_work(int64_t n_rows, int64_t m, int64_t k, int mt, int
 // ---- tcgen05 GEMM of decode batches (gemm_batch.cu): clusters of CTAs that share the K loop of 128 weight rows
 
 constexpr int BATCH_MAX_CLUSTER = 6;
+// Clusters of 1..6 CTAs, a CTA per SM, that are resident at once on a B200: the model by which the rule below counts rounds. It
+// is not what the device in use answers: how its SMs are spread over GPCs, and a process's share of it, may size a grid, but not cut a K loop.
+constexpr int BATCH_RESIDENT[BATCH_MAX_CLUSTER + 1] = {0, 148, 74, 45, 33, 26, 22};
 
-// CTAs per cluster for a weight of `tiles` 128-row tiles and `KU` units of 256 k; resident[c]: clusters of c that fit the GPU
-// (on 148 SMs 148, 74, 45, 33, 26, 22). A function of the weight's shape alone: it fixes how the f32 sums associate, so it may depend
-// neither on the batch nor on the other weights of a call. The weights that share an x should agree all the same, or
+// CTAs per cluster for a weight of `tiles` 128-row tiles and `KU` units of 256 k. A function of the weight's shape alone: it
+// fixes how the f32 sums associate, so it may depend on neither the batch, the other weights of a call, nor the device or the process.
+// The weights that share an x should agree all the same, or
 // the call takes a launch for each size, hence a rule that goes by what a weight looks like rather than by the best size for each.
 // Measured on B200 with 1 / 2 / 3 / 4 / 6 CTAs, us a call at 32 rows:
 //   more than twice as many rows as columns (ffn_gate|up, heads: called in pairs or large anyway): fewest units in sequence
@@ -171,8 +175,8 @@ constexpr int BATCH_MAX_CLUSTER = 6;
 //   else (ffn_down and wide attn_output, called alone): fewest units in sequence
 //     5120 x 25600 Q6_K 88.8 / 50.8 / 40.3 / 52.3 / 40.8   5120 x 8192 Q4_K 24.6 / 15.9 / 13.8 / 16.4 / 14.4
 //     2560 x 8192 Q6_K 28.3 / 16.6 / 13.3 / 11.8 / 11.2
-inline int plan_batch_cluster(int tiles, int KU, const int* resident) {
-  auto rounds = [&](int t, int c) { return (t + resident[c] - 1) / resident[c]; };
+inline int plan_batch_cluster(int tiles, int KU) {
+  auto rounds = [](int t, int c) { return (t + BATCH_RESIDENT[c] - 1) / BATCH_RESIDENT[c]; };
   int best = 1;
   if (tiles > 4 * KU) {
     int64_t cost = (int64_t)rounds(2 * tiles, 1) * KU;
@@ -192,6 +196,21 @@ inline int plan_batch_cluster(int tiles, int KU, const int* resident) {
   return best < KU ? best : KU;
 }
 
+// A positive number that is asked for once and then known: `ask(&n)` returns an error or 0. Only an answer is kept; an error goes
+// back to the caller, and the next one asks again.
+template <class Ask>
+inline int ask_once(std::atomic<int>& known, Ask ask, int* out) {
+  int n = known.load(std::memory_order_acquire);
+  if (n <= 0) {
+    const int e = ask(&n);
+    if (e != 0) return e;
+    if (n < 1) n = 1;
+    known.store(n, std::memory_order_release);
+  }
+  *out = n;
+  return 0;
+}
+
 // Activation rows per tile (a multiple of 16, at most 128) with which gemm_batch.cu takes a call of more than 64 rows, without
 // cutting K, or 0: the prefill kernel takes it. tiles, call_tiles: 128-row and 256-row tiles of all weights of the call.
 // What is left idle decides: pairs of CTAs on 256 weight rows leave most of the GPU without work for a short prompt, CTAs of
@@ -207,14 +226,14 @@ inline int plan_batch_cluster(int tiles, int KU, const int* resident) {
 //   1024 x 3072 Q8_0      17.1 / 10.6   21.9 / 11.0   22.2 / 13.2   22.3 / 12.3   22.6 / 14.0   (1000: 26.0 / 16.3)
 // and calls of several weights: 4096 + 1024 + 1024 x 4096 Q4_K, Q6_K, 128 / 256 rows 27.7 / 23.6, 29.4 / 26.1; 2 x 12288 x 4096 Q4_K,
 // 128 rows 44.1 / 38.0; 2560 + 640 + 640 x 2560 Q8_0, 256 rows 24.6 / 17.1.
-inline int plan_batch_tile(int64_t tiles, int64_t call_tiles, int64_t m, int64_t resident, int sm_count) {
+inline int plan_batch_tile(int64_t tiles, int64_t call_tiles, int64_t m, int sm_count) {
   if (m <= 64 || m > 1024) return 0;
   const int64_t slots = sm_count / 2 > 0 ? sm_count / 2 : 1;
   const int64_t b = plan_gemm_rows(call_tiles, m, sm_count), mt = (m + b - 1) / b;
   int64_t best_cost = (call_tiles * mt + slots - 1) / slots * (b + 110 > 260 ? b + 110 : 260) * 9200 / 218;
   int best = 0;
   for (int bn = 128; bn >= 16; bn -= 16) {
-    const int64_t cost = (tiles * ((m + bn - 1) / bn) + resident - 1) / resident * (bn <= 64 ? 6600 + 10 * bn : 4100 + 50 * bn);
+    const int64_t cost = (tiles * ((m + bn - 1) / bn) + sm_count - 1) / sm_count * (bn <= 64 ? 6600 + 10 * bn : 4100 + 50 * bn);
     if (cost < best_cost) { best = bn; best_cost = cost; }
   }
   return best;
