@@ -148,3 +148,28 @@ def test_lm_head_topk_and_sharded_merge(tq):
         cand_i.append(i_r)
     mv, mi = tq.topk(torch.cat(cand_v, 1).contiguous(), k, ids=torch.cat(cand_i, 1).contiguous())
     assert torch.equal(mv, vals) and torch.equal(mi, idx)
+
+
+@pytest.mark.parametrize("dt,mode,m", [(oracle.Q4_K, "INT8_ACT", 1600), (oracle.Q5_K, "INT8_ACT", 1600), (oracle.Q4_K, "EXACT_F32", 3000),
+                                       (oracle.Q8_0, "EXACT_F32", 3000)])
+def test_norm_prologue_asks_for_no_memory_that_no_launch_reads(tq, dt, mode, m):
+    """Planes of 1600 x 4096 values (7.9 MB) lie in the 8 MiB that a context starts with; a second copy of the quants, which only
+    Q6_K weights read, does not, nor do the planes of 3000 rows, which the exact scheme does not read. Growing is an
+    allocation inside the call: refused under capture, as such calls were not."""
+    n, k = 32, 4096
+    ctx = tq.new_context()
+    mm = tq.QMatMul.from_arc(tq.QTensor.new(make_weight(dt, n, k, SEED + 91), tq.GgmlDType(dt), (n, k), ctx=ctx))
+    x = torch.from_numpy(np.random.default_rng(SEED + 92).standard_normal((m, k)).astype(np.float32)).cuda()
+    w = torch.ones(k, device="cuda")
+    args = dict(mode=tq.Mode[mode], return_normed=mode != "INT8_ACT")
+    tq.QMatMul.rmsnorm_forward_multi([mm], x[:1], w, 1e-6, **args)      # kernels loaded
+    keep = torch.empty_like(x), torch.empty(m * n, device="cuda")       # what the call returns, in torch's pool beforehand
+    del keep
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    out = tq.QMatMul.rmsnorm_forward_multi([mm], x, w, 1e-6, **args)
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] == free
+    y, h = (out[0][0], out[1]) if mode != "INT8_ACT" else (out[0], torch.nn.functional.rms_norm(x, (k,), w, 1e-6))
+    assert oracle.rel_fro(y.cpu().numpy(), mm.forward(h, mode=tq.Mode[mode]).cpu().numpy()) < (1e-7 if mode != "INT8_ACT" else 2e-3)
+    ctx.poll_status()

@@ -224,7 +224,7 @@ int32_t turq_ctx_reserve(turq_ctx* ctx, int64_t max_m, int64_t max_k, int64_t ma
                 (long long)max_k, (long long)max_n);
   TQ_CUDA(ctx, cudaSetDevice(ctx->device));
   const int64_t k256 = (max_k + 255) / 256 * 256;
-  size_t need = turq::norm_scratch_bytes(TQ_Q8_K, max_m, k256);
+  size_t need = turq::norm_scratch_bytes(TQ_Q8_K, max_m, k256, true);
   const size_t q80 = turq::plan_act_pack(TQ_Q8_0, max_m, k256).total;
   if (q80 > need) need = q80;
   const size_t tc = turq::gemm_tc_scratch_bytes(max_m, k256);  // the tensor-core path's f16 operand

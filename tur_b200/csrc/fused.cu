@@ -40,8 +40,8 @@ struct NormQuantArgs {
   float* h_out;  // nullable
   int fmt;       // TQ_Q8_K or TQ_Q8_0
   int64_t m;
-  int8_t* qs;
-  int8_t* qs_order16;  // Q8_K: a second copy of the quants, for launches of Q6_K weights alone
+  int8_t* qs;          // null: no launch reads planes (the other schemes take h)
+  int8_t* qs_order16;  // Q8_K: a second copy of the quants, for a launch of Q6_K weights alone; null where no weight is Q6_K
   float* dsc;
   int16_t* bs16;
   int16_t* bs32;
@@ -82,12 +82,13 @@ __global__ void __launch_bounds__(256) rmsnorm_quant_kernel(const NormQuantArgs 
         *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
         *reinterpret_cast<float4*>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
       }
+      if (!a.qs) continue;
       uint32_t q0, q1;
       float d;
       int s16, s32;
       quant_block_q8k(v, lane, q0, q1, d, s16, s32);
       store_q8k_planes(a.qs, ActOrder::order32, a.dsc, a.bs16, a.bs32, a.m, row, blk, lane, q0, q1, d, s16, s32);
-      store_q8k_qs(a.qs_order16, ActOrder::order16, a.m, row, blk, lane, q0, q1);
+      if (a.qs_order16) store_q8k_qs(a.qs_order16, ActOrder::order16, a.m, row, blk, lane, q0, q1);
     }
   } else {
     const int64_t nblk = k >> 5, groups = (nblk + 7) >> 3;
@@ -112,6 +113,7 @@ __global__ void __launch_bounds__(256) rmsnorm_quant_kernel(const NormQuantArgs 
 #pragma unroll
         for (int e = 0; e < 8; e++) v[e] = 0.f;
       }
+      if (!a.qs) continue;
       uint32_t q0, q1;
       __half dh;
       quant_block_q8_0(v, q0, q1, dh);
@@ -274,13 +276,14 @@ int32_t turq_rmsnorm_qmatmul_multi(turq_ctx* ctx, int32_t count, const turq_qten
   if (count < 1 || count > 4) return api_fail(ctx, TURQ_E_INVALID_ARG, "count outside 1..4");
   if (x_dtype != TURQ_F32 && x_dtype != TURQ_BF16) return api_fail(ctx, TURQ_E_DTYPE, "activations must be F32 or BF16");
   if (m <= 0 || m > INT32_MAX / 2) return api_fail(ctx, TURQ_E_SHAPE, "m out of range");
-  bool k_quant = false, q8_0 = false;
+  bool k_quant = false, q8_0 = false, q6_k = false;
   int64_t rows_all = 0;
   for (int i = 0; i < count; i++) {
     if (!qts[i] || !dev_ys[i]) return api_fail(ctx, TURQ_E_INVALID_ARG, "null argument");
     if (qts[i]->n_cols != qts[0]->n_cols) return api_fail(ctx, TURQ_E_SHAPE, "weights of one call must share the in-feature count");
     if (qts[i]->device != ctx->device) return api_fail(ctx, TURQ_E_INVALID_ARG, "tensors and context must live on the same device");
     (qts[i]->dtype == TURQ_Q8_0 ? q8_0 : k_quant) = true;
+    q6_k = q6_k || qts[i]->dtype == TURQ_Q6_K;
     rows_all += qts[i]->n_rows;
   }
   const int64_t k = qts[0]->n_cols;
@@ -293,7 +296,8 @@ int32_t turq_rmsnorm_qmatmul_multi(turq_ctx* ctx, int32_t count, const turq_qten
   const bool direct = eff == TURQ_MODE_INT8_ACT && !(k_quant && q8_0);
   const int fmt = q8_0 && !k_quant ? TQ_Q8_0 : TQ_Q8_K;
   const turq::ActPackPlan plan = turq::plan_act_pack(fmt, m, k);
-  int32_t st = turq::api_ensure_scratch(ctx, turq::norm_scratch_bytes(fmt, m, k));
+  int32_t st = TURQ_OK;
+  if (direct) st = turq::api_ensure_scratch(ctx, turq::norm_scratch_bytes(fmt, m, k, q6_k));
   if (st != TURQ_OK) return st;
   float* h = dev_h_out;
   if (!direct && !h) {  // the other schemes read h itself
@@ -310,11 +314,13 @@ int32_t turq_rmsnorm_qmatmul_multi(turq_ctx* ctx, int32_t count, const turq_qten
   a.h_out = h;
   a.fmt = fmt;
   a.m = m;
-  a.qs = reinterpret_cast<int8_t*>(ctx->scratch + plan.off_qs);
-  a.qs_order16 = reinterpret_cast<int8_t*>(ctx->scratch + plan.total);
-  a.dsc = reinterpret_cast<float*>(ctx->scratch + plan.off_dsc);
-  a.bs16 = reinterpret_cast<int16_t*>(ctx->scratch + plan.off_bs16);
-  a.bs32 = reinterpret_cast<int16_t*>(ctx->scratch + plan.off_bs32);
+  if (direct) {
+    a.qs = reinterpret_cast<int8_t*>(ctx->scratch + plan.off_qs);
+    a.qs_order16 = q6_k ? reinterpret_cast<int8_t*>(ctx->scratch + plan.total) : nullptr;
+    a.dsc = reinterpret_cast<float*>(ctx->scratch + plan.off_dsc);
+    a.bs16 = reinterpret_cast<int16_t*>(ctx->scratch + plan.off_bs16);
+    a.bs32 = reinterpret_cast<int16_t*>(ctx->scratch + plan.off_bs32);
+  }
   turq::rmsnorm_quant_kernel<<<(unsigned)m, 256, 0, s>>>(a);
   ctx->launches++;
   e = cudaGetLastError();

@@ -54,9 +54,9 @@ struct ActPackPlan {
   size_t off_qs, off_dsc, off_bs16, off_bs32, total;
 };
 ActPackPlan plan_act_pack(int fmt, int64_t m, int64_t k);
-// The same with the quants of Q8_K in both orders: what the RMSNorm prologue writes.
-inline size_t norm_scratch_bytes(int fmt, int64_t m, int64_t k) {
-  return plan_act_pack(fmt, m, k).total + (fmt == TQ_Q8_K ? (size_t)m * k : 0);
+// What the RMSNorm prologue writes: the same, and where a weight of the call is Q6_K the quants of Q8_K in the other order too.
+inline size_t norm_scratch_bytes(int fmt, int64_t m, int64_t k, bool q6_k) {
+  return plan_act_pack(fmt, m, k).total + (fmt == TQ_Q8_K && q6_k ? (size_t)m * k : 0);
 }
 
 // wire -> device tiles. n_rows may be any positive value; rows are padded to 16.
@@ -99,7 +99,7 @@ cudaError_t launch_gemv_int8(int dtype, const uint8_t* tiles, int64_t n_rows, in
 // concatenated rows (q|k|v, gate|up) per weight type - and a single one for Q4_K or Q5_K parts
 // beside Q6_K parts while the planes fit shared memory - each part with its own output and bias. x_remote: x is
 // mapped host memory; it is then read exactly once, by the quantization launch. planes_ready: the
-// caller's own prologue launch already wrote the quantized planes of these rows to act_scratch, for K-quants with a
+// caller's own prologue launch already wrote the quantized planes of these rows to act_scratch, where a part is Q6_K with a
 // second copy of the quants, in the other order, behind plan.total (norm_scratch_bytes).
 struct TpArgs;  // tp_exchange.cuh: xchg != nullptr (one part, m <= 32) makes the launch's last CTA run
                 // the tensor-parallel all-reduce of the result itself
