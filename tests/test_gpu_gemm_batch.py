@@ -111,3 +111,21 @@ def test_short_prompts_in_tiles(tq, dt, n, k, m):
     a, b = tq.QMatMul.forward_multi([mm, mm], xd, biases=[None, bias], mode=tq.Mode.TENSOR_CORE)
     assert torch.equal(a, y) and torch.equal(b, y + bias)
     tq.context().poll_status()
+
+
+@pytest.mark.parametrize("k,few,many", [(16640, 140, 150), (33024, 70, 1100)])
+def test_long_rows_convert_alike_by_clusters_and_alone(tq, k, few, many):
+    """Few rows are converted by clusters of CTAs, many by a CTA each: the same f16 operand and the same bits, into images of
+    tiles (up to 1024 rows) and into rows."""
+    w, _ = make_weight(oracle.Q4_K, 130, k, SEED + 8400 + k)
+    rng = np.random.default_rng(SEED + 8401 + k)
+    x = (rng.standard_normal((many, k)) * 2.0 ** rng.integers(-8, 9, (many, 1))).astype(np.float32)
+    mm = tq.QMatMul.from_arc(tq.QTensor.new(w, tq.GgmlDType(oracle.Q4_K), (130, k)))
+    xd = torch.from_numpy(x).cuda()
+    y = mm.forward(xd, mode=tq.Mode.TENSOR_CORE)
+    assert torch.equal(mm.forward(xd[:few], mode=tq.Mode.TENSOR_CORE), y[:few])
+    rows = np.r_[0:20, many - 20:many]
+    ref = oracle.matmul_f64(oracle.Q4_K, w, 130, k, x[rows])
+    err = np.linalg.norm(y.cpu().numpy()[rows] - ref, axis=1) / np.linalg.norm(ref, axis=1)
+    assert err.max() < TOL, (int(err.argmax()), err.max())
+    tq.context().poll_status()

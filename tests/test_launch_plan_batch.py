@@ -14,6 +14,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SHIM = r"""
 #include "launch_plan.h"
 extern "C" int batch_cluster(int tiles, int KU) { return turq::plan_batch_cluster(tiles, KU); }
+extern "C" int prep_cluster(long long m, long long k, int sms) { return turq::plan_prep_cluster(m, k, sms); }
 // asks three times: answers[i] is what the device would say, errors[i] the status that it returns
 extern "C" void ask_three_times(const int* answers, const int* errors, int* asked, int* status, int* out) {
   std::atomic<int> known{0};
@@ -38,6 +39,7 @@ def lib():
         lib = ctypes.CDLL(so)
         lib.gemm_rows.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int]
         lib.batch_tile.argtypes = [ctypes.c_longlong] * 3 + [ctypes.c_int]
+        lib.prep_cluster.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int]
         yield lib
 
 
@@ -116,3 +118,15 @@ def test_tiles_of_short_prompts(lib):
         assert tile(n, m) > 0, (n, m)
     for n, m in ((4096, 1000), (12288, 768), (25600, 256), (25600, 512), (151936, 512)):
         assert tile(n, m) == 0, (n, m)
+
+
+def test_rows_are_converted_by_clusters_where_they_are_long_and_few(lib):
+    """Clusters that all fit the GPU at once, none for rows that four CTAs' worth of registers hold or for prompts (25600 values: 177
+    us a call of 4096 rows without, 265 with them)."""
+    for m in (1, 32, 64, 65, 96, 105, 106, 128, 148, 149, 512, 1024, 4096, 2 ** 30):
+        for k in (64, 4096, 16384, 16448, 17408, 25600, 32768, 49152, 2 ** 31 - 64):
+            for sms in (148, 16, 1):
+                c = lib.prep_cluster(m, k, sms)
+                assert 1 <= c <= 8 and (c == 1 or (k > 16384 and c == min(8, -(-k // 4096)) and m * c <= 5 * sms)), (m, k, sms, c)
+    for m, k, c in ((32, 25600, 7), (96, 25600, 7), (128, 25600, 1), (4096, 25600, 1), (64, 17408, 5), (256, 17408, 1), (64, 49152, 8), (64, 16384, 1)):
+        assert lib.prep_cluster(m, k, 148) == c, (m, k)

@@ -581,12 +581,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
 // The row is written in the operands' k order (tc_common.cuh): as a row of [m, k] (prefill),
 // or as a row of the operand's shared-memory images [tile of image_rows rows][k / 64][image_rows][128 bytes], 128B-swizzled,
 // which gemm_batch.cu copies in whole. One CTA per row; up to 4096 values stay in registers between the search for the largest
-// magnitude and the conversion. Rows of more than 16384 values (CLUSTER): a cluster of CTAs, 4096 values each (beyond 8 x 4096 the
-// rest is read again), whose maxima meet in distributed shared memory: Q6_K 5120 x 25600 with the conversion, 32 / 64 rows 41.0 /
-// 47.6 -> 38.4 / 43.4 us. Below that the cluster's barriers cost what the second pass does: 4096 x 12288 17.2 / 20.0 and 18.7 / 20.0.
+// magnitude and the conversion. CLUSTER (few long rows, plan_prep_cluster): a cluster of CTAs a row, 4096 values each (beyond
+// 8 x 4096 the rest is read again), whose maxima meet in distributed shared memory.
 // At 48 registers a thread (40 where the GEMM behind has a warp more) a CTA fits beside a CTA of the GEMM, so the conversion
 // of the next call is resident before this call ends.
-constexpr int PREP_THREADS = 256, PREP_KEEP = 2, PREP_VALUES = PREP_THREADS * 8 * PREP_KEEP, PREP_MAX_CLUSTER = 8;
+constexpr int PREP_THREADS = 256, PREP_KEEP = 2;
+static_assert(PREP_VALUES == PREP_THREADS * 8 * PREP_KEEP, "what the plan counts a CTA to keep");
 template <bool IMAGE, bool CLUSTER>
 __global__ void __launch_bounds__(PREP_THREADS, IMAGE ? 6 : 5) prep_act_kernel(const void* __restrict__ x, int is_bf16, uint32_t k, int image_rows,
                                                                                __half* __restrict__ xh, __half* __restrict__ xh16,
@@ -761,17 +761,13 @@ static cudaError_t launch_prep(unsigned c, const void* x, int x_dtype, int64_t m
   return launch_pdl_cluster(prep_act_kernel<IMAGE, CLUSTER>, CLUSTER ? c : 0, dim3((unsigned)m * c), dim3(PREP_THREADS), 0, s, x, (int)(x_dtype == TQ_BF16), (uint32_t)k,
                             image_rows, reinterpret_cast<__half*>(xh), reinterpret_cast<__half*>(xh16), rscale);
 }
-static unsigned prep_cluster(int64_t m, int64_t k) {
-  const int64_t c = k > 4 * PREP_VALUES ? (k + PREP_VALUES - 1) / PREP_VALUES : 1;
-  return m * PREP_MAX_CLUSTER > INT32_MAX ? 1u : (unsigned)(c < PREP_MAX_CLUSTER ? c : PREP_MAX_CLUSTER);
-}
 cudaError_t launch_prep_image(const void* x, int x_dtype, int64_t m, int64_t k, int image_rows, uint8_t* xh, uint8_t* xh16, float* rscale, cudaStream_t s) {
-  const unsigned c = prep_cluster(m, k);
+  const unsigned c = (unsigned)plan_prep_cluster(m, k, device_sm_count());
   return c > 1 ? launch_prep<true, true>(c, x, x_dtype, m, k, image_rows, xh, xh16, rscale, s)
                : launch_prep<true, false>(c, x, x_dtype, m, k, image_rows, xh, xh16, rscale, s);
 }
 static cudaError_t launch_prep_rows(const void* x, int x_dtype, int64_t m, int64_t k, uint8_t* xh, float* rscale, cudaStream_t s) {
-  const unsigned c = prep_cluster(m, k);
+  const unsigned c = (unsigned)plan_prep_cluster(m, k, device_sm_count());
   return c > 1 ? launch_prep<false, true>(c, x, x_dtype, m, k, 0, xh, nullptr, rscale, s) : launch_prep<false, false>(c, x, x_dtype, m, k, 0, xh, nullptr, rscale, s);
 }
 

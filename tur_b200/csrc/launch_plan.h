@@ -239,4 +239,24 @@ inline int plan_batch_tile(int64_t tiles, int64_t call_tiles, int64_t m, int sm_
   return best;
 }
 
+// ---- conversion of the activations to f16 (prep_act_kernel): a CTA per row, or a cluster of CTAs
+
+constexpr int PREP_VALUES = 4096;      // values of a row that a CTA keeps in registers between its two passes
+constexpr int PREP_MAX_CLUSTER = 8;
+constexpr int PREP_CTAS_PER_SM = 5;    // that are resident at once
+
+// CTAs that share a row of k values: one per 4096 beyond 16384 values, while the clusters of all m rows are resident at once. What
+// they save is a second read of the row, one CTA's chain of it; where there are rows enough to fill the GPU that chain is hidden, and
+// clusters only cost their barriers. Measured on B200 with / without, conversion and a GEMM of 128 weight rows, us a call:
+//   rows        32            64            96            128           256           1200          4096
+//   17408       12.3 / 13.2   13.5 / 14.1   44.3 / 44.3   44.8 / 44.3   49.0 / 45.1   98.6 / 81.7   177 / 124
+//   25600       15.5 / 16.9   17.3 / 17.8   63.7 / 64.2   67.1 / 64.3   71.9 / 65.2   147 / 125     265 / 179
+//   49152       28.6 / 30.0   27.4 / 30.0   119 / 122     123 / 122     128 / 124     255 / 240     423 / 372
+// Up to 16384 values the cluster's barriers cost what the second pass does (12288: 17.2 / 20.0 and 18.7 / 20.0 us at 32 / 64 rows).
+inline int plan_prep_cluster(int64_t m, int64_t k, int sm_count) {
+  if (k <= 4 * PREP_VALUES) return 1;
+  const int64_t want = (k + PREP_VALUES - 1) / PREP_VALUES, c = want < PREP_MAX_CLUSTER ? want : PREP_MAX_CLUSTER;
+  return m <= (int64_t)PREP_CTAS_PER_SM * sm_count / c ? (int)c : 1;
+}
+
 }  // namespace turq
