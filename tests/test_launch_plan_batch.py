@@ -86,7 +86,10 @@ def test_projections_of_a_layer_share_a_launch(cluster, hidden, q, kv):
 
 @pytest.mark.parametrize("rows,m,tiles", [((4096, 1024, 1024), 512, 3), ((4096,), 512, 4), ((12288, 12288), 512, 2), ((2560, 640, 640), 1000, 4),
                                           ((2560,), 1000, 7), ((8192, 8192), 1000, 4), ((4096,), 2048, 9), ((12288, 12288), 2048, 8),
-                                          ((5120,), 4096, 18), ((25600, 25600), 4096, 16), ((12288, 12288), 128, 1)])
+                                          ((5120,), 4096, 18), ((25600, 25600), 4096, 16), ((12288, 12288), 128, 1),
+                                          # a last wave that is nearly empty costs less than a whole one
+                                          ((8192, 8192), 1300, 6), ((8192, 8192), 1500, 6), ((12288, 12288), 1700, 7), ((12288,), 1700, 7),
+                                          ((25600,), 768, 3), ((13824, 13824), 700, 3), ((28672,), 1300, 6), ((1024,), 1300, 17)])
 def test_tile_heights_that_were_measured_best(lib, rows, m, tiles):
     assert -(-m // lib.gemm_rows(sum(-(-n // 256) for n in rows), m, 148)) == tiles
 

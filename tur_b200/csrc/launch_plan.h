@@ -83,22 +83,24 @@ inline int plan_gemm_bn(int64_t n_rows, int64_t m, int sm_count) {
 }
 
 // Activation rows per pair tile (a multiple of 16, at most 256) for a call whose weights have `call_tiles` 256-row tiles in
-// all: the weights of a call run side by side, so what counts is how the tiles of all of them fill the pairs. The fewest
-// waves times the time of a tile; a tile of b rows takes about b + 110 (units of an activation row), and below 150 rows the
-// weights' dequantization holds it at 260. The smaller number of tiles where two are alike. Measured on B200, us a call with
-// 2 / 3 / 4 / 5 / 7 / 8 activation tiles:
-//   512 rows   Q4_K, Q6_K 4096 + 1024 + 1024 x 4096  44.0 / 35.5 / 51.3   Q4_K 4096 x 4096  29.7 / 25.6 / 24.2   2 x 12288 x 4096  85.2 / 93.1 / 110.6
-//   1000 rows  Q8_0 2560 + 640 + 640 x 2560  - / - / 30.2 / 44.7 / 45.1   2560 x 8192  - / - / 62.5 / 58.3 / 56.1 / 98.5
-//   8 / 9 / 10: 2048 rows Q6_K 4096 x 12288 242.7 / 210.6 / 326.3 (197 since Q6_K is converted from a lane's own words)   Q5_K 2 x 12288 x 4096 349 / 371 / 352
-// (a choice per weight put the small ones of a call on tiles of 128 rows: a layer at 2048 rows 865 us, at one size 793).
+// all: the weights of a call run side by side, so what counts is how the tiles of all of them fill the pairs. The least
+// time of a tile times what the tiles take of the pairs: a tile of b rows takes about b + 110 (units of an activation row), and
+// below 90 rows the weights' dequantization holds it at 200; a last wave counts for a third by what is in it and for two thirds
+// whole, since where it is nearly empty the clocks rise with the power that the idle SMs leave. The smaller number of tiles
+// where two are alike. Measured on B200 at every height for 32 calls of 384 to 3000 rows, what the choice loses against the best
+// height of each: 0.13 % in the geometric mean, 6 % at most (a last wave counted whole and tiles held at 260: 0.9 %, 27 %). us a call, tiles of the choice
+// / of the old one: 2 x 8192 x 2560 Q8_0, 1300 rows 109 (6) / 120 (8)   2 x 12288 x 4096 Q4_K, 1700 rows 257 (7) / 269 (9)
+//   25600 x 5120 Q4_K, 768 rows 149 (3) / 157 (4)   1024 x 3072 Q8_0, 1300 rows 21 (17) / 25 (10)
+// A height of its own for every weight put the small ones of a call on tiles of 128 rows (a layer at 2048 rows 865 us, at one height 793).
 inline int plan_gemm_rows(int64_t call_tiles, int64_t m, int sm_count) {
   const int64_t slots = sm_count / 2 > 0 ? sm_count / 2 : 1;
   auto rows_of = [&](int64_t mt) { return ((m + mt - 1) / mt + 15) / 16 * 16; };
   const int64_t cls = plan_gemm_bn(256 * call_tiles, m, sm_count), mt0 = (m + 255) / 256;
   int64_t best = rows_of((m + cls - 1) / cls), best_cost = 0;
   for (int64_t i = -1; i < 3 * mt0 && i < 24; i++) {  // the class above first, then more and more tiles
-    const int64_t b = i < 0 ? best : rows_of(mt0 + i), mt = (m + b - 1) / b;
-    const int64_t cost = (call_tiles * mt + slots - 1) / slots * (b + 110 > 260 ? b + 110 : 260);
+    const int64_t b = i < 0 ? best : rows_of(mt0 + i), tiles = call_tiles * ((m + b - 1) / b);
+    const int64_t whole = (tiles + slots - 1) / slots * slots;  // waves
+    const int64_t cost = (2 * whole + (tiles > slots ? tiles : slots)) * (b + 110 > 200 ? b + 110 : 200);
     if (i < 0 || cost < best_cost || (cost == best_cost && b > best)) {
       best = b;
       best_cost = cost;
