@@ -61,3 +61,18 @@ def test_mixed_launches_and_the_prologue_read_the_same_planes(tq, other, k):
         h = tq.QMatMul.rmsnorm_forward_multi(mms[2:], x[:m], norm, 1e-6, mode=tq.Mode.INT8_ACT)[0]  # Q6_K alone: the other order
         assert torch.equal(y[2], h), m
     tq.context().poll_status()
+
+
+@pytest.mark.parametrize("k", [32, 96, 224, 1056, 4192, 8256])
+def test_q8_0_groups_of_one_to_four_tiles(tq, k):
+    """Whole groups of four tiles take a path of their own, a last group of one to three the other: in-kernel, staged and global
+    planes, one, two and four groups of rows. The bits of a row alone, which are the oracle's up to the order of the sums."""
+    n = 48
+    w, mm = weight(tq, oracle.Q8_0, n, k, SEED + 8400 + k)
+    x = np.random.default_rng(SEED + 8401 + k).standard_normal((32, k)).astype(np.float32)
+    xd = torch.from_numpy(x).cuda()
+    alone = torch.cat([mm.forward(xd[r:r + 1], mode=tq.Mode.INT8_ACT) for r in range(32)])
+    assert oracle.rel_fro(alone.cpu().numpy(), oracle.qmatmul(oracle.Q8_0, w, n, k, x)) < TOL
+    for m in (3, 8, 9, 16, 17, 25, 32):
+        assert torch.equal(mm.forward(xd[:m], mode=tq.Mode.INT8_ACT), alone[:m]), m
+    tq.context().poll_status()

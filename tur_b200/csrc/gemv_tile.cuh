@@ -83,27 +83,36 @@ __device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane
   static_assert(DT == TQ_Q8_0 || DT == TQ_Q6_K || ORDER == ActOrder::order32, "Q4_K and Q5_K tiles read order32");
   const int g = lane >> 2, c = lane & 3;
   if constexpr (DT == TQ_Q8_0) {
+auto one = [&](int u) {
+      const uint8_t* tu = t + 544 * u;
+      const uint4 q = lds_v4(tu + TQ_Q8_0_QS + 16 * lane);
+      const uint32_t a[4] = {q.x, q.z, q.y, q.w};
+      const float dw0 = f16_bits_to_f32(lds_u16(tu + 2 * g)), dw1 = f16_bits_to_f32(lds_u16(tu + 2 * (g + 8)));
+      const int kb = kt + u;
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      if (u < ntiles_left) {
-        const uint8_t* tu = t + 544 * u;
-        const uint4 q = lds_v4(tu + TQ_Q8_0_QS + 16 * lane);
-        const uint32_t a[4] = {q.x, q.z, q.y, q.w};
-        const float dw0 = f16_bits_to_f32(lds_u16(tu + 2 * g)), dw1 = f16_bits_to_f32(lds_u16(tu + 2 * (g + 8)));
-        const int kb = kt + u;
-#pragma unroll
-        for (int mg = 0; mg < MG; mg++) {
-          const uint2 b = ld_v2(act.qs + (int64_t)kb * act.R * 32 + la.q[mg] + 8 * c);
-          int cc[4] = {0, 0, 0, 0};
-          mma_16832<false>(cc, a, b.x, b.y);
-          const float* const dsc = act.dsc + (int64_t)kb * act.R;
-          const float dx0 = dsc[la.r0[mg]], dx1 = dsc[la.r1[mg]];
-          acc[mg][0] += (float)cc[0] * (dw0 * dx0);
-          acc[mg][1] += (float)cc[1] * (dw0 * dx1);
-          acc[mg][2] += (float)cc[2] * (dw1 * dx0);
-          acc[mg][3] += (float)cc[3] * (dw1 * dx1);
-        }
+      for (int mg = 0; mg < MG; mg++) {
+        const uint2 b = ld_v2(act.qs + (int64_t)kb * act.R * 32 + la.q[mg] + 8 * c);
+        int cc[4] = {0, 0, 0, 0};
+        mma_16832<false>(cc, a, b.x, b.y);
+        const float* const dsc = act.dsc + (int64_t)kb * act.R;
+        const float dx0 = dsc[la.r0[mg]], dx1 = dsc[la.r1[mg]];
+        acc[mg][0] += (float)cc[0] * (dw0 * dx0);
+        acc[mg][1] += (float)cc[1] * (dw0 * dx1);
+        acc[mg][2] += (float)cc[2] * (dw1 * dx0);
+        acc[mg][3] += (float)cc[3] * (dw1 * dx1);
       }
+    };
+    // A whole group without a question between its tiles, so that the loads of all four are under way together: asked tile by
+    // tile, every tile waits for its own quants and scales. us a call so / asked, 8 and 16 rows: 128 x 25600 19.2 / 39.1 and
+    // 24.5 / 42.5 (planes in global memory), 4096 x 12288 12.7 / 13.1 and 18.7 / 25.5, 2560 x 8192 12.2 / 12.6 and 13.8 / 15.5.
+    // Four groups of rows have loads enough, and no registers for more (5120 x 25600, 32 rows 80.4 / 73.4).
+    if (MG <= 2 && ntiles_left >= 4) {
+#pragma unroll
+      for (int u = 0; u < 4; u++) one(u);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (u < ntiles_left) one(u);
     }
   } else if constexpr (DT == TQ_Q4_K || DT == TQ_Q5_K) {
     constexpr int QS = DT == TQ_Q4_K ? TQ_Q4K_QS : TQ_Q5K_QS;
