@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(HALVES * THREADS, 3 - HALVES) gemv_stream_kern
 
     const int g = lane >> 2, c = lane & 3;
     if constexpr (ACT != ACT_GLOBAL) act.R = a.rows;
-    LaneAct<MG> la;
+    LaneAct<MG, (MG == 4 && DT == TQ_Q8_0) || (MG == 2 && DT == TQ_Q4_K && !MIXED)> la;
     la.init(lane, a.rows, DT == TQ_Q8_0 ? 32 : 64);
     float acc[MG][4];
 #pragma unroll

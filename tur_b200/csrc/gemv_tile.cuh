@@ -54,17 +54,21 @@ __host__ __device__ __forceinline__ int act_offset(ActOrder o, int r, int e) {
 }
 
 // What a lane needs to find its rows in the planes; the same for every tile. Rows beyond the valid ones are clamped to the last
-// one: their columns of the MMA are not stored.
-template <int MG>
+// one: their columns of the MMA are not stored. GUARD: their quants are not read at all. That pays where reads are what a
+// tile waits for and costs a test per read: Q8_0 with four groups of rows (us a call without / with, 17 / 24 / 32 rows: 128 x 25600 60.9 / 49.5,
+// 67.9 / 54.1, 70.5 / 52.7; 2560 x 2560 12.0 / 10.5, 13.5 / 11.5, 14.0 / 12.4; 5120 x 25600 68.7 / 64.9, 70.0 / 66.6, 73.6 / 68.2) and
+// Q4_K with two (9 rows: 512 x 8192 10.8 / 9.9, 1536 x 8960 11.7 / 10.8; all shapes 2 %). Elsewhere with up to two groups it loses
+// 1 to 6 %, and K-quants with four are even.
+template <int MG, bool GUARD>
 struct LaneAct {
-  int q[MG];        // offset of row 8 mg + g inside a chunk of qs
+  int q[MG];        // offset of row 8 mg + g inside a chunk of qs; GUARD: -1 beyond the valid rows
   int r0[MG], r1[MG];  // rows 8 mg + 2 c, 8 mg + 2 c + 1
   __device__ __forceinline__ void init(int lane, int rows, int row_bytes) {
     const int g = lane >> 2, c = lane & 3;
 #pragma unroll
     for (int mg = 0; mg < MG; mg++) {
       const int b = 8 * mg + g, m0 = 8 * mg + 2 * c;
-      q[mg] = (b < rows ? b : rows - 1) * row_bytes;
+      q[mg] = b < rows ? b * row_bytes : GUARD ? -1 : (rows - 1) * row_bytes;
       r0[mg] = m0 < rows ? m0 : rows - 1;
       r1[mg] = m0 + 1 < rows ? m0 + 1 : rows - 1;
     }
@@ -77,13 +81,14 @@ __device__ __forceinline__ uint32_t lds_u16(const uint8_t* p) { return *reinterp
 
 // One tile (or GROUP consecutive Q8_0 tiles) at shared-memory address t, tile index kt of its
 // row, against the activation rows of the pass; adds into acc[mg][0..3]. ORDER: the order of the planes' qs.
-template <int DT, int MG, ActOrder ORDER>
-__device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane, const ActPack& act, const LaneAct<MG>& la, int kt,
+template <int DT, int MG, ActOrder ORDER, bool GUARD>
+__device__ __forceinline__ void tile_mma(const uint8_t* __restrict__ t, int lane, const ActPack& act, const LaneAct<MG, GUARD>& la, int kt,
                                          int ntiles_left, float (&acc)[MG][4]) {
   static_assert(DT == TQ_Q8_0 || DT == TQ_Q6_K || ORDER == ActOrder::order32, "Q4_K and Q5_K tiles read order32");
+  static_assert(DT != TQ_Q6_K || !GUARD, "Q6_K tiles read clamped rows");
   const int g = lane >> 2, c = lane & 3;
   if constexpr (DT == TQ_Q8_0) {
-auto one = [&](int u) {
+    auto one = [&](int u) {
       const uint8_t* tu = t + 544 * u;
       const uint4 q = lds_v4(tu + TQ_Q8_0_QS + 16 * lane);
       const uint32_t a[4] = {q.x, q.z, q.y, q.w};
@@ -91,7 +96,8 @@ auto one = [&](int u) {
       const int kb = kt + u;
 #pragma unroll
       for (int mg = 0; mg < MG; mg++) {
-        const uint2 b = ld_v2(act.qs + (int64_t)kb * act.R * 32 + la.q[mg] + 8 * c);
+        uint2 b = make_uint2(0, 0);
+        if (!GUARD || la.q[mg] >= 0) b = ld_v2(act.qs + (int64_t)kb * act.R * 32 + la.q[mg] + 8 * c);
         int cc[4] = {0, 0, 0, 0};
         mma_16832<false>(cc, a, b.x, b.y);
         const float* const dsc = act.dsc + (int64_t)kb * act.R;
@@ -171,7 +177,8 @@ auto one = [&](int u) {
       }
 #pragma unroll
       for (int mg = 0; mg < MG; mg++) {
-        const uint4 bx = ld_v4(act.qs + (int64_t)(4 * kt + i) * act.R * 64 + la.q[mg] + 16 * (c ^ ((la.q[mg] >> 6) & 2)));
+        uint4 bx = make_uint4(0, 0, 0, 0);
+        if (!GUARD || la.q[mg] >= 0) bx = ld_v4(act.qs + (int64_t)(4 * kt + i) * act.R * 64 + la.q[mg] + 16 * (c ^ ((la.q[mg] >> 6) & 2)));
         int clo[4] = {0, 0, 0, 0}, chi[4] = {0, 0, 0, 0};
         mma_16832<true>(clo, alo, bx.x, bx.y);
         mma_16832<true>(chi, ahi, bx.z, bx.w);
