@@ -105,7 +105,7 @@ Q8_0, Q6_K, Q45_K = 0, 1, 2      # how the MMA loop reads the planes
     (Q45_K, 256, 2560, 8192, (7, 8), (9, 12)),                       # a share for a little more than every SM
 ])
 def test_wide_launches_where_they_are_faster(plan, reads, unit, n, k, narrow, wide):
-    """The sizes at which both forms were measured: what was slower wide stays narrow."""
+    """The lines of the rule, drawn where both forms were measured with row-major planes; what is measured now stands beside it."""
     for rows in narrow + wide:
         assert bool(plan.gemv_wide(reads, rows, -(-n // 16), k // unit, SLOTS)) == (rows in wide), rows
 

@@ -51,16 +51,19 @@ inline int64_t gemv_split_start(const GemvSplit& p, int64_t total_units, int b) 
 // global memory. What the wide form saves is the way to L2 per activation fragment, most for Q8_0 (an
 // f32 scale per 32 values beside the quants) and Q6_K (four-byte fragments), least for Q4_K and Q5_K; a
 // mixed launch also spares a launch per type. What it costs is ring stages (two to four instead of six)
-// and, where there are no more shares than SMs, half of the SMs. Measured on B200, global against wide, us (with row-major
-// planes; in the order of ActPack both sides are faster):
-//   Q8_0        512 x 8192, 8 rows 13.7 / 9.7   5120 x 25600, 4 rows 41.4 / 33.4   2560 x 8192, 8 rows 13.5 / 13.7
-//   Q6_K        4096 x 12288, 4 rows 14.8 / 13.8   2048 x 5120, 12 rows 13.0 / 10.6
-//     shares cut, shorter than two row-tiles: 5120 x 25600, 2 rows 27.9 / 28.8   5120 x 13312, 7 rows 21.2 / 20.6
-//   Q4_K, Q5_K  4096 x 12288 Q4_K, 8 rows 14.0 / 12.7   25600 x 5120 Q4_K, 12 rows 41.4 / 33.5
-//     shares cut, shorter than two row-tiles: 5120 x 8192 Q4_K, 8 / 12 rows 14.3 / 15.4, 18.6 / 17.9
-//                                             6144 x 6144 Q4_K, 11 rows 16.6 / 17.3
-//     an SM for every share: 128 x 16384 Q4_K, 8 rows 11.5 / 13.4   640 x 8192 Q4_K, 8 / 12 rows 8.2 / 9.0, 12.7 / 11.4
-//     a third of the slots idle: 2560 x 8192 Q5_K, 8 / 12 rows 10.4 / 10.8, 14.3 / 12.9
+// and, where there are no more shares than SMs, half of the SMs. The lines were drawn with row-major planes. Measured on B200
+// with today's, global / wide, us a call ((w) or (g): the other side than the rule's is faster there):
+//   Q8_0        5120 x 25600, 3 / 4 rows 27.9 / 26.7, 28.0 / 27.0   4096 x 12288, 6 / 8 rows 14.2 / 12.2, 14.1 / 12.6
+//               2560 x 8192, 8 / 12 rows 10.7 / 12.1 (g), 13.5 / 13.3   512 x 8192, 12 rows 10.6 / 11.3 (g)
+//   Q6_K        4096 x 12288, 4 / 6 rows 12.4 / 12.3, 12.6 / 12.2   2048 x 5120, 12 rows 10.7 / 9.1   2560 x 8192, 8 rows 9.1 / 8.8
+//               640 x 6144, 8 / 12 rows 6.3 / 7.3 (g), 10.3 / 9.7
+//     shares cut, shorter than two row-tiles: 5120 x 25600, 2 / 3 rows 25.1 / 23.8 (w), 25.5 / 25.1 (w)   5120 x 13312, 5 / 7 rows 17.5 / 17.3, 17.4 / 17.6
+//   Q4_K, Q5_K  4096 x 12288 Q4_K, 6 / 8 rows 10.6 / 9.7, 10.5 / 10.0   25600 x 5120 Q4_K, 12 rows 34.1 / 24.1   9600 x 8192 Q4_K, 8 rows 15.7 / 14.5
+//     shares cut, shorter than two row-tiles: 5120 x 8192 Q4_K, 8 / 9 / 12 rows 12.1 / 12.6, 15.5 / 14.4 (w), 15.8 / 14.9 (w)
+//                                             6144 x 6144 Q4_K, 9 / 16 rows 13.3 / 13.3, 15.4 / 15.0 (w)   5120 x 25600 Q4_K, 3 rows 21.1 / 19.3 (w)
+//     an SM for every share: 128 x 16384 Q4_K, 4 rows 9.5 / 9.9   640 x 8192 Q4_K, 8 / 12 rows 6.6 / 7.1, 10.3 / 9.1 (w)
+//     a third of the slots idle: 2560 x 8192 Q5_K, 8 / 12 rows 8.8 / 8.2 (w), 13.1 / 10.8
+//   mixed (global: a launch per type) 4096 + 1024 + 1024 x 4096, 9 / 12 rows 16.2 / 16.3, 18.7 / 12.9   8192 + 1024 + 1024 x 5120, 9 rows 23.7 / 20.1
 enum class GemvPlaneReads { q8_0, q6_k /* also mixed launches */, q45_k };
 inline bool plan_gemv_wide(GemvPlaneReads reads, int rows, const GemvSplit& split, int64_t total_units, int KU, int slots) {
   const bool cut_short = !split.aligned && total_units < (int64_t)2 * KU * split.grid;
