@@ -1,7 +1,6 @@
 """Host-side launch arithmetic (tur_b200/csrc/launch_plan.h), compiled with g++ and checked on
 the CPU: every tile of a weight is owned by exactly one CTA, whole-row-tile splits are what they
-claim, the workspace is large enough for the grid, and how the GEMM cuts K loops and chooses tiles keeps
-its invariants (at least 8 K blocks per cut, independent of the batch size for decode)."""
+claim, the workspace is large enough for the grid, and the prefill GEMM's tile classes and pairs are what they claim."""
 import ctypes
 import os
 import subprocess
@@ -26,11 +25,7 @@ int gemv_wide(int reads, int rows, int row_tiles, int KU, int slots) {
                               (long long)row_tiles * KU, KU, slots);
 }
 int gemm_bn(long long n, long long m, int sms) { return turq::plan_gemm_bn(n, m, sms); }
-void gemm_work(long long n, long long m, long long k, int mt, int sms, int* out) {
-  turq::GemmWork w = turq::plan_gemm_work(n, m, k, mt, sms);
-  out[0] = w.pairs; out[1] = w.split_k;
-}
-int gemm_splits(long long n, long long m, long long k, int sms) { return turq::plan_gemm_splits(n, m, k, sms); }
+int gemm_pairs(long long tiles, int sms) { return turq::plan_gemm_pairs(tiles, sms); }
 }
 """
 
@@ -46,8 +41,7 @@ def plan():
         lib.split_start.restype = ctypes.c_longlong
         lib.split_start.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_int]
         lib.gemm_bn.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int]
-        lib.gemm_splits.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int]
-        lib.gemm_work.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
+        lib.gemm_pairs.argtypes = [ctypes.c_longlong, ctypes.c_int]
         yield lib
 
 
@@ -110,56 +104,17 @@ def test_wide_launches_where_they_are_faster(plan, reads, unit, n, k, narrow, wi
         assert bool(plan.gemv_wide(reads, rows, -(-n // 16), k // unit, SLOTS)) == (rows in wide), rows
 
 
-@pytest.mark.parametrize("n,k", [(8192, 5120), (1024, 5120), (5120, 8192), (25600, 5120), (5120, 25600), (2560, 2560),
-                                  (640, 2560), (12288, 4096), (4096, 12288), (151936, 4096), (272, 256), (128, 512)])
-def test_gemm_split_k_invariants(plan, n, k):
-    sms = 148
-    decode = {plan.gemm_splits(n, m, k, sms) for m in (17, 32, 48, 64)}
-    assert len(decode) == 1, "the split must not depend on the batch size"
-    s = decode.pop()
-    assert 1 <= s <= 8
-    if s > 1:
-        assert (k // 64) // s >= 8, "at least 8 K blocks per pair"
-        assert s * ((n + 255) // 256) <= sms // 2, "one wave"
-    for m in (65, 512, 4096):
-        assert plan.gemm_splits(n, m, k, sms) == 1
-
-
-def test_long_k_loops_are_shared_by_five_pairs_at_most(plan):
-    """More pairs were slower than the GEMM with a summing launch of its own at 48 to 64 rows."""
-    for n, k, cuts in ((1024, 5120, 5), (512, 8192, 5), (2560, 8192, 5), (5120, 25600, 3), (1024, 4096, 8), (640, 2560, 5)):
-        assert plan.gemm_splits(n, 64, k, 148) == cuts
-
-
 def test_gemm_activation_tile_choice(plan):
     sms = 148
-    assert plan.gemm_bn(12288, 64, sms) == 64
     assert plan.gemm_bn(12288, 2048, sms) == 256
     assert plan.gemm_bn(4096, 512, sms) == 128      # 32 x 2 tiles: doubling still fits one wave
     assert plan.gemm_bn(2560, 1024, sms) == 256     # 20 x 4 tiles: doubling would spill into a second wave
     assert plan.gemm_bn(1024, 2048, sms) == 128
 
 
-@pytest.mark.parametrize("n,k", [(8192, 5120), (1024, 5120), (5120, 25600), (2560, 2560), (640, 2560), (12288, 4096), (4096, 12288),
-                                 (151936, 4096), (272, 256), (1, 64), (9700, 320), (40000, 64), (10000, 768), (300, 8192)])
-def test_gemm_pairs_cover_the_work(plan, n, k):
-    """Decode batches: every pair has work, no more pairs than an SM each for two CTAs, a tile is shared
-    by at most 17 pairs, the same for every batch size. Prefill: never split, no more pairs than tiles."""
-    out = (ctypes.c_int * 2)()
-    tiles, ku = -(-n // 256), -(-k // 256)
-    total = tiles * ku
-    seen = set()
-    for m in (17, 40, 64):
-        plan.gemm_work(n, m, k, 1, 148, out)
-        seen.add((out[0], out[1]))
-    assert len(seen) == 1
-    pairs, split = seen.pop()
-    assert split == 1 and 1 <= pairs <= 74
-    starts = [total * p // pairs for p in range(pairs + 1)]
-    assert starts[0] == 0 and starts[-1] == total and all(b > a for a, b in zip(starts, starts[1:]))
-    splits = plan.gemm_splits(n, 64, k, 148)
-    if splits > 1:
-        assert pairs == tiles * splits and all(t * ku in starts for t in range(tiles)), "no pair holds parts of two tiles"
-    assert max(sum(1 for a, b in zip(starts, starts[1:]) if a < (t + 1) * ku and b > t * ku) for t in range(tiles)) <= 17
-    plan.gemm_work(n, 1000, k, 4, 148, out)
-    assert out[1] == 0 and out[0] == min(74, 4 * tiles)
+@pytest.mark.parametrize("n", [8192, 1024, 5120, 2560, 640, 12288, 4096, 151936, 272, 1, 9700, 40000])
+def test_gemm_pairs_cover_the_work(plan, n):
+    """No more pairs than SMs for two CTAs each, nor than tiles."""
+    tiles = 4 * -(-n // 256)
+    assert plan.gemm_pairs(tiles, 148) == min(74, tiles)
+    assert plan.gemm_pairs(tiles, 1) == 1

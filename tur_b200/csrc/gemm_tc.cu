@@ -772,12 +772,12 @@ static cudaError_t launch_prep_rows(const void* x, int x_dtype, int64_t m, int64
 }
 
 // Activation rows per pair tile, activation tiles and pairs of a launch; call_tiles: 256-row tiles of all weights of the call.
-struct TcShape { int bn, mt; GemmWork work; };
-static TcShape tc_shape(int64_t n_rows, int64_t call_tiles, int64_t m, int64_t k, int sm_count) {
+struct TcShape { int bn, mt, pairs; };
+static TcShape tc_shape(int64_t n_rows, int64_t call_tiles, int64_t m, int sm_count) {
   TcShape p;
   p.bn = plan_gemm_rows(call_tiles, m, sm_count);
   p.mt = (int)((m + p.bn - 1) / p.bn);
-  p.work = plan_gemm_work(n_rows, m, k, p.mt, sm_count);
+  p.pairs = plan_gemm_pairs((n_rows + 2 * BM - 1) / (2 * BM) * p.mt, sm_count);
   return p;
 }
 
@@ -798,7 +798,7 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
   }
 
   const int64_t n_tiles = (n_rows + 2 * BM - 1) / (2 * BM);
-  const TcShape shape = tc_shape(n_rows, call_tiles > 0 ? call_tiles : n_tiles, m, k, sm_count);
+  const TcShape shape = tc_shape(n_rows, call_tiles > 0 ? call_tiles : n_tiles, m, sm_count);
   const int bn = shape.bn;
   CUtensorMap map;
   const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
@@ -819,7 +819,6 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
   a.m = (int)m;
   a.bn = bn;
   a.mt = shape.mt;
-  const GemmWork& work = shape.work;
   const int64_t total = n_tiles * a.mt;
   if (total > (int64_t)1 << 30) return cudaErrorInvalidValue;
   a.total = (int)total;
@@ -829,15 +828,15 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t* tiles, int64_t n_rows, int6
   a.bias = bias;
   a.go = reinterpret_cast<int*>(workspace) + (size_t)sibling * sm_count;
   a.next_go = a.go + sm_count;
-  a.next_ctas = next_rows > 0 ? 2 * tc_shape(next_rows, call_tiles, m, k, sm_count).work.pairs : 0;
+  a.next_ctas = next_rows > 0 ? 2 * tc_shape(next_rows, call_tiles, m, sm_count).pairs : 0;
   a.status = dev_status_word;
   a.y_toggle = y_toggle;
   a.y_alt = y_alt;
   switch (dtype) {
-    case TQ_Q8_0: e = launch_tc_dt<TQ_Q8_0>(map, a, work.pairs, s); break;
-    case TQ_Q4_K: e = launch_tc_dt<TQ_Q4_K>(map, a, work.pairs, s); break;
-    case TQ_Q5_K: e = launch_tc_dt<TQ_Q5_K>(map, a, work.pairs, s); break;
-    case TQ_Q6_K: e = launch_tc_dt<TQ_Q6_K>(map, a, work.pairs, s); break;
+    case TQ_Q8_0: e = launch_tc_dt<TQ_Q8_0>(map, a, shape.pairs, s); break;
+    case TQ_Q4_K: e = launch_tc_dt<TQ_Q4_K>(map, a, shape.pairs, s); break;
+    case TQ_Q5_K: e = launch_tc_dt<TQ_Q5_K>(map, a, shape.pairs, s); break;
+    case TQ_Q6_K: e = launch_tc_dt<TQ_Q6_K>(map, a, shape.pairs, s); break;
     default: return cudaErrorInvalidValue;
   }
   if (launches) (*launches)++;

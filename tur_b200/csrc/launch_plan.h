@@ -1,6 +1,6 @@
 // Host-side launch arithmetic of the GEMV and the GEMM, free of CUDA so that it can be
 // compiled and checked on a machine without a GPU: how the tiles of a weight are dealt out to
-// CTAs, which launches share their activation planes, how many CTAs share the K loop of a GEMM tile,
+// CTAs, which launches share their activation planes, how many CTAs share the K loop of 128 weight rows in decode batches,
 // which activation-tile height is used.
 #pragma once
 #include <atomic>
@@ -73,16 +73,12 @@ inline bool plan_gemv_wide(GemvPlaneReads reads, int rows, const GemvSplit& spli
   return rows > 8 || (int64_t)split.grid * 10 >= (int64_t)slots * 7;
 }
 
-// ---- tcgen05 GEMM (pairs of CTAs, 256 weight rows per pair)
-// Its product callers have more than 64 rows; what the functions answer for up to 64 is how that kernel shared K loops
-// between pairs before decode batches got a kernel and a plan of their own (plan_batch_cluster below).
+// ---- tcgen05 GEMM (pairs of CTAs, 256 weight rows per pair), more than 64 activation rows
 
-// Class of the activation rows per pair tile: 64 for decode batches; 256 for prefill, unless twice
-// as many tiles still fit the SMs in one wave - then 128, which doubles the pairs at work.
+// Class of the activation rows per pair tile: 256, unless twice as many tiles still fit the SMs in one wave - then 128,
+// which doubles the pairs at work.
 inline int plan_gemm_bn(int64_t n_rows, int64_t m, int sm_count) {
-  int bn = m <= 64 ? 64 : 256;
-  if (bn == 256 && 2 * ((n_rows + 127) / 128) * ((m + 255) / 256) <= sm_count) bn = 128;
-  return bn;
+  return 2 * ((n_rows + 127) / 128) * ((m + 255) / 256) <= sm_count ? 128 : 256;
 }
 
 // Activation rows per pair tile (a multiple of 16, at most 256) for a call whose weights have `call_tiles` 256-row tiles in
@@ -112,50 +108,10 @@ inline int plan_gemm_rows(int64_t call_tiles, int64_t m, int sm_count) {
   return (int)best;
 }
 
-// Split-K for decode batches (one activation tile of at most 64 rows): when the weight's row tiles
-// alone leave SMs without work, the K loop of every tile is shared out over several pairs (at least
-// 8 blocks of 64 each, at most 5 pairs if it is longer than 4096). The split depends on the weight's
-// shape only, so a row's result does not depend on which batch of up to 64 rows it is in; prefill (more
-// than 64 rows) never splits, so its f32 sums associate differently.
-inline int plan_gemm_splits(int64_t n_rows, int64_t m, int64_t k, int sm_count) {
-  if (m > 64) return 1;
-  const int64_t tiles = (n_rows + 255) / 256;
-  int64_t s = tiles > 0 ? sm_count / 2 / tiles : 1;
-  const int64_t by_k = (k / 64) / 8;
-  if (s > by_k) s = by_k;
-  // Long K loops: five pairs a tile. The owner adds the others' sums two pairs at a time (twice over beyond
-  // 40 rows), which soon costs more than the units it saves. Up to 16 pairs / 5, us a call: Q8_0 2560 x 8192, 32 / 64
-  // rows 13.9 / 13.2, 18.9 / 15.6; Q4_K 1024 x 5120, 32 / 64 rows 10.0 / 10.3, 12.9 / 11.7; Q8_0 512 x 8192,
-  // 64 rows 15.3 / 14.0. At 16 units a cut still pays: Q4_K 1024 x 4096, 32 / 64 rows 8.9 / 9.5, 11.5 / 11.1.
-  if (k > 16 * 256 && s > 5) s = 5;
-  return s < 2 ? 1 : (int)s;
-}
-
-// Pairs of CTAs and what is dealt out to them: whole tiles (round robin), or - decode batches - the
-// units of 256 k of all tiles in one even split. With plan_gemm_splits() > 1 the pairs are a multiple
-// of the tiles, so every cut is the same in every tile. Otherwise (more tiles than half the pairs, or a
-// K loop too short to be cut in two) the cuts are wherever the even split falls: on all pairs, or on so
-// many that each has two units, but never on fewer pairs than tiles while there are pairs: then a pair
-// may have one unit only.
-struct GemmWork {
-  int pairs;
-  int split_k;
-};
-inline GemmWork plan_gemm_work(int64_t n_rows, int64_t m, int64_t k, int mt, int sm_count) {
-  const int64_t tiles = (n_rows + 255) / 256, slots = sm_count / 2 > 0 ? sm_count / 2 : 1;
-  GemmWork w{};
-  if (m > 64) {
-    w.pairs = (int)(tiles * mt < slots ? tiles * mt : slots);
-    return w;
-  }
-  const int splits = plan_gemm_splits(n_rows, m, k, sm_count);
-  const int64_t units = tiles * ((k + 255) / 256);
-  int64_t pairs = splits > 1 ? tiles * splits : slots;
-  if (splits == 1 && pairs > units / 2) pairs = units / 2;
-  if (splits == 1 && pairs < tiles && pairs < slots) pairs = tiles < slots ? tiles : slots;
-  w.pairs = pairs > 0 ? (int)pairs : 1;
-  w.split_k = 1;
-  return w;
+// Persistent pairs of CTAs for a weight of `tiles` pair tiles, which are dealt out to them whole, round robin.
+inline int plan_gemm_pairs(int64_t tiles, int sm_count) {
+  const int64_t slots = sm_count / 2 > 0 ? sm_count / 2 : 1;
+  return (int)(tiles < slots ? tiles : slots);
 }
 
 // ---- tcgen05 GEMM of decode batches (gemm_batch.cu): clusters of CTAs that share the K loop of 128 weight rows
@@ -220,7 +176,7 @@ inline int ask_once(std::atomic<int>& known, Ask ask, int* out) {
 // cutting K, or 0: the prefill kernel takes it. tiles, call_tiles: 128-row and 256-row tiles of all weights of the call.
 // What is left idle decides: pairs of CTAs on 256 weight rows leave most of the GPU without work for a short prompt, CTAs of
 // their own on 128 rows and as few activation rows as it takes fill it. Both sides by their waves times the time of a unit of
-// 256 k: here (0.66 + bn / 1000) us up to 64 rows and (0.41 + bn / 200) us beyond, there (plan_gemm_rows) its cost / 218 us; a
+// 256 k: here (0.66 + bn / 1000) us up to 64 rows and (0.41 + bn / 200) us beyond, there, with the rows of plan_gemm_rows, (b + 110) / 218 us, at least 260 / 218; a
 // twelfth has to be gained. Measured on B200, prefill kernel / this one, us a call:
 //   rows                  65            128           256           384           512
 //   4096 x 4096 Q4_K      21.2 / 15.6   22.3 / 15.7   22.7 / 17.8   24.7 / 20.8   25.2 / 22.3   (768: 28.0 / 34.1)
