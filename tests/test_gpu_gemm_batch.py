@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import oracle
+import plan_shim
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -31,12 +32,13 @@ def make_weight(dt, n, k, seed):
 # (type, rows, columns, CTAs per cluster on a B200)
 SHAPES = [(oracle.Q4_K, 19000, 256, 1), (oracle.Q8_0, 24300, 320, 1), (oracle.Q4_K, 12200, 4096, 2), (oracle.Q5_K, 700, 1024, 2),
           (oracle.Q6_K, 5000, 6144, 3), (oracle.Q5_K, 8100, 5120, 4), (oracle.Q8_0, 300, 2624, 4), (oracle.Q4_K, 3130, 6400, 5),
-          (oracle.Q6_K, 2560, 8192, 6), (oracle.Q8_0, 130, 6208, 6)]
+          (oracle.Q6_K, 2560, 8192, 6), (oracle.Q8_0, 130, 6208, 5), (oracle.Q8_0, 130, 6464, 6)]
 
 
 @pytest.mark.parametrize("dt,n,k,c", SHAPES)
 def test_clusters_share_the_k_loop(tq, dt, n, k, c):
     """Sums of every cluster size against the f64 product; the bits do not depend on the batch, nor on what ran before."""
+    assert plan_shim.cluster(n, k) == c
     w, base = make_weight(dt, n, k, SEED + 8000 + n + k)
     rng = np.random.default_rng(SEED + 8001 + n)
     x = (rng.standard_normal((64, k)) * 2.0 ** rng.integers(-8, 9, (64, 1))).astype(np.float32)
@@ -87,16 +89,17 @@ def test_one_call_of_both_k_orders(tq, k, dtype):
     tq.context().poll_status()
 
 
-# (type, rows, columns, activation rows): tiles of 16 to 128 rows, whole and ragged, narrow and wide accumulators, one item per
-# CTA and several, a last unit of one, two and three 64-k blocks
-TILED = [(oracle.Q4_K, 700, 256, 1024), (oracle.Q8_0, 300, 320, 67), (oracle.Q8_0, 5000, 448, 500), (oracle.Q4_K, 4000, 4096, 65),
-         (oracle.Q5_K, 3000, 5120, 129), (oracle.Q6_K, 5000, 6144, 300), (oracle.Q8_0, 130, 2624, 96), (oracle.Q6_K, 2560, 1024, 1000),
-         (oracle.Q8_0, 8200, 704, 255), (oracle.Q4_K, 12288, 512, 128)]
+# (type, rows, columns, activation rows, rows of a tile): tiles of 16 to 128 rows, whole and ragged, narrow and wide accumulators,
+# one item per CTA and several, a last unit of one, two and three 64-k blocks
+TILED = [(oracle.Q4_K, 700, 256, 1024, 48), (oracle.Q8_0, 300, 320, 67, 16), (oracle.Q8_0, 5000, 448, 300, 112), (oracle.Q4_K, 4000, 4096, 65, 32),
+         (oracle.Q5_K, 3000, 5120, 129, 32), (oracle.Q6_K, 5000, 6144, 300, 112), (oracle.Q8_0, 130, 2624, 96, 16), (oracle.Q6_K, 2560, 1024, 700, 112),
+         (oracle.Q8_0, 8200, 704, 255, 128), (oracle.Q4_K, 12288, 512, 128, 128)]
 
 
-@pytest.mark.parametrize("dt,n,k,m", TILED)
-def test_short_prompts_in_tiles(tq, dt, n, k, m):
+@pytest.mark.parametrize("dt,n,k,m,rows", TILED)
+def test_short_prompts_in_tiles(tq, dt, n, k, m, rows):
     """65 to 1024 rows in tiles: against the f64 product, and with the bits of a call that is too large for tiles."""
+    assert plan_shim.tile([n], m) == rows and plan_shim.kernel([n], 1024 // m * m + m) == "pairs"
     w, base = make_weight(dt, n, k, SEED + 8300 + n + k)
     rng = np.random.default_rng(SEED + 8301 + n)
     x = (rng.standard_normal((m, k)) * 2.0 ** rng.integers(-8, 9, (m, 1))).astype(np.float32)
