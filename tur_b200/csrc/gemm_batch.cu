@@ -19,14 +19,14 @@
 // a CTA sends its sums of the others' chunks (st.async, completing on the receiver's barrier) and adds those of its own in
 // rank order (fixed order, no float atomics). Clusters have nothing to do with one another.
 // All weights of a call (q|k|v, gate|up; any mix of types) go out as one launch over their 128-row tiles, dealt out round robin
-// to the clusters that fit the GPU. C is a function of the weight's shape alone (launch_plan.h), so a row's bits depend neither on
-// the batch nor on the other weights of the call; weights that want another C go out as a launch of their own.
+// to the clusters that fit the GPU. C is a function of the weight's shape alone (launch_plan.h), so a row's bits depend on
+// neither the batch, the other weights of the call, nor the device; weights that want another C go out as a launch of their own.
 //
 // More than 64 rows go in tiles of up to 128 (a tile and 128 weight rows are an item; accumulators of 64 or 128 columns), a launch per
 // weight, side by side. K is not cut then: the sums, and their bits, are those of the prefill kernel. A layer of 4096-wide
 // Q4_K / Q6_K linears at 96 / 128 / 256 / 512 rows: 147 / 150 / 167 / 223 -> 115 / 123 / 149 / 207 us; 2560-wide Q8_0 at 96 / 256: 113 / 125 ->
 // 71 / 84; 1024-wide Q8_0 at 96 / 256 / 512: 64 / 70 / 75 -> 40 / 49 / 58. A unit takes 0.67 us with 16 rows, 0.72 with 64 (dequantize), 0.9 with 96
-// and 1.05 with 128: 82 KB of operands a unit, 8 to 9 TB/s from L2 over all CTAs, where a pair of the prefill kernel shares its rows.
+// and 1.05 with 128: 64 KB of activations a unit, 9 TB/s from L2 over all CTAs, where a pair of the prefill kernel shares its rows.
 //
 // What bounds it. Small weights: the chain conversion (1.0 us) - its completion (0.7) - first activation image (0.6) - MMAs of
 // the share - exchange (0.6) - stores and exit, some 5 us. Large ones: the issue slots and the ALU pipe of the dequantize warps
@@ -38,11 +38,8 @@
 //   attn_q|k|v 2560 + 640 + 640 x 2560 Q5_K, Q6_K, 32 rows 16.7 -> 7.6    ffn_gate|up 2 x 8192 x 2560 Q5_K, 32 rows 23.1 -> 12.8
 //   attn_q|k|v 8192 + 1024 + 1024 x 5120 Q4_K, Q6_K, 64 rows 32.2 -> 20.0   ffn_gate|up 2 x 25600 x 5120 Q4_K, 64 rows 68.4 -> 50.4
 //   attn_output 4096 x 4096 Q4_K, 32 rows 11.1 -> 8.1                      ffn_down 5120 x 25600 Q6_K, 64 rows 52.1 -> 40.6
-// Steps on the way (2 x 25600 x 5120, 64 rows): CTAs of their own instead of pairs 68.4 -> 66.6 us; whole units per warp instead of
-// halves of every unit 62.0; a second warp to issue the copies 59.0; partial sums through distributed shared memory instead of
-// global memory (a fence and a flag per chunk: up to 13 us an epilogue) 57.5; the row scales in shared memory 52.7.
-// Q6_K in a k order of its own (5120 x 25600, 32 / 64 rows): 38.3 / 43.0 -> 34.8 / 40.6 us; 4096 x 12288 17.2 / 20.0 -> 16.2 / 19.4;
-// a call that needs both images (the q|k|v above at 64 rows): 19.5 -> 20.0.
+// Q6_K in a k order of its own (5120 x 25600, 32 / 64 rows): 38.3 / 43.0 -> 34.8 / 40.6 us; a call that needs both images (the q|k|v
+// above at 64 rows): 19.5 -> 20.0.
 // Every wait is bounded; on expiry the CTA records TURQ_E_TIMEOUT, releases its TMEM and returns.
 #include <atomic>
 

@@ -583,7 +583,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
 // which gemm_batch.cu copies in whole. One CTA per row; up to 4096 values stay in registers between the search for the largest
 // magnitude and the conversion. CLUSTER (few long rows, plan_prep_cluster): a cluster of CTAs a row, 4096 values each (beyond
 // 8 x 4096 the rest is read again), whose maxima meet in distributed shared memory.
-// At 48 registers a thread (40 where the GEMM behind has a warp more) a CTA fits beside a CTA of the GEMM, so the conversion
+// At 48 registers a thread (40 where the GEMM behind has a warp more; the cluster form spills 32 bytes there) a CTA fits beside a CTA of the GEMM, so the conversion
 // of the next call is resident before this call ends.
 constexpr int PREP_THREADS = 256, PREP_KEEP = 2;
 static_assert(PREP_VALUES == PREP_THREADS * 8 * PREP_KEEP, "what the plan counts a CTA to keep");

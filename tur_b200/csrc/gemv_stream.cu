@@ -46,7 +46,9 @@ constexpr int red_slots_of(int halves, int mg) { return halves == 2 && mg == 1 ?
 // copy; at a tile a copy that is what a large launch waits for. Copies of 1 / 2 / 4 / 8 tiles, us: 2 x 25600 x 5120 Q4_K, one row
 // 31.8 / 30.2 / 29.8 / 29.7, 8 rows 35.9 / 33.8 / 32.2 / 32.4, 16 rows 48.3 / 46.1 / 45.0 / 44.7; 2 x 12288 x 4096 Q4_K, one row 14.7 /
 // 13.9 / 14.0 / 13.7 (15.3 before this choice), 16 rows 23.6 / 23.9 / 23.6 / 23.7; 4096 x 12288 Q6_K, 8 rows 13.3 / 13.3 / 13.1 / 13.6:
-// with all eight in one copy every warp waits for the last byte of a stage. Eight lanes that issue a copy each were slower
+// with all eight in one copy every warp waits for the last byte of a stage. Launches of a few stages and one to four rows wait
+// for it with four too (copies of 1 / 4 tiles: 4096 x 4096 Q4_K, 2 / 4 rows 5.47 / 5.60, 5.70 / 5.85; Q8_0 2048 x 1024, one row 2.59 /
+// 2.77), others of that size do not (Q5_K 2560 + 640 + 640 x 2560, 8 rows 6.28 / 5.93): over 407 calls of 1 to 16 rows four are 1.8 % ahead. Eight lanes that issue a copy each were slower
 // than one lane with two copies (2 x 25600 x 5120, one row: 33.3).
 constexpr int TPC = 4;
 constexpr int GROUPS = NW / TPC;       // copies and full barriers of a stage
