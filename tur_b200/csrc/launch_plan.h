@@ -178,7 +178,7 @@ inline int ask_once(std::atomic<int>& known, Ask ask, int* out) {
 // their own on 128 rows and as few activation rows as it takes fill it. Both sides by their waves times the time of a unit of
 // 256 k: here (0.66 + bn / 1000) us up to 64 rows and (0.41 + bn / 200) us beyond, there, with the rows of plan_gemm_rows, (b + 110) / 218 us, at least 260 / 218; a
 // twelfth has to be gained. Measured on B200, prefill kernel / this one, us a call (the prefill side with tiles of 144 rows and
-// more, which its rule took then; where it takes smaller ones now it is up to 20 % faster on the small weights, no less behind):
+// more, which its rule took then; where it takes smaller ones now it is up to 20 % faster on the small weights, and still behind there):
 //   rows                  65            128           256           384           512
 //   4096 x 4096 Q4_K      21.2 / 15.6   22.3 / 15.7   22.7 / 17.8   24.7 / 20.8   25.2 / 22.3   (768: 28.0 / 34.1)
 //   4096 x 12288 Q4_K     50.9 / 38.5   52.7 / 39.7   56.3 / 41.8   60.8 / 50.8   61.1 / 56.0   (768: 73.3 / 92.8)
